@@ -67,6 +67,50 @@ __device__ __forceinline__ bool tri_box_overlap(const double v[3][3], const doub
     return fabs(d) <= r;
 }
 
+// The same axes in FP32, deciding only what is clear of rounding: 0 apart, 1
+// overlap, 2 too close to call (the FP64 axes decide, so the lists are the
+// same).  v: corners relative to the box centre, h: the widened half-extents,
+// W the largest of their sizes, u = 2^-24.  A corner is off by u W, an edge
+// component by 4 u W, so an edge axis' projections and h . |a| are each
+// within 20 u W^2 of the exact ones; a component of the normal is within
+// 48 u W^2, its projections within 240 u W^3.  FP64 runs at 1/64 of the FP32
+// rate here: with the FP64 axes alone a pass over 640,000 triangles took
+// 2.66 ms, with this in front of them 0.47 ms.
+__device__ __forceinline__ int tri_box_overlap32(const float v[3][3], const float h[3]) {
+    const float e0[3] = {v[1][0] - v[0][0], v[1][1] - v[0][1], v[1][2] - v[0][2]};
+    const float e1[3] = {v[2][0] - v[1][0], v[2][1] - v[1][1], v[2][2] - v[1][2]};
+    const float e2[3] = {v[0][0] - v[2][0], v[0][1] - v[2][1], v[0][2] - v[2][2]};
+    const float* E[3] = {e0, e1, e2};
+    float W = fmaxf(h[0], fmaxf(h[1], h[2]));
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) W = fmaxf(W, fabsf(v[c][k]));
+    if (!(W < 4.0f)) return 2;  // also a NaN, or the half-open outermost cells
+    const float err2 = 64.0f * 5.9604645e-08f * W * W, err3 = 512.0f * 5.9604645e-08f * W * W * W;
+    bool sure = true;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
+            const float a1 = -E[j][i2], a2 = E[j][i1];
+            const float p0 = a1 * v[0][i1] + a2 * v[0][i2], p1 = a1 * v[1][i1] + a2 * v[1][i2],
+                        p2 = a1 * v[2][i1] + a2 * v[2][i2];
+            const float r = h[i1] * fabsf(a1) + h[i2] * fabsf(a2);
+            const float gap = fmaxf(fminf(p0, fminf(p1, p2)), -fmaxf(p0, fmaxf(p1, p2))) - r;  // > 0: apart
+            if (gap > err2) return 0;
+            sure &= gap < -err2;
+        }
+    }
+    const float n[3] = {e0[1] * e1[2] - e0[2] * e1[1], e0[2] * e1[0] - e0[0] * e1[2], e0[0] * e1[1] - e0[1] * e1[0]};
+    const float d = n[0] * v[0][0] + n[1] * v[0][1] + n[2] * v[0][2];
+    const float gap = fabsf(d) - (h[0] * fabsf(n[0]) + h[1] * fabsf(n[1]) + h[2] * fabsf(n[2]));
+    if (gap > err3) return 0;
+    sure &= gap < -err3;
+    return sure ? 1 : 2;
+}
+
 // box of fine cell index k on one axis, widened by kAccelEps; the outermost
 // cells reach to infinity because coordinates beyond the box clamp into them
 __device__ __forceinline__ void cell_span(uint32_t k, uint32_t nf, double& lo, double& hi) {
@@ -95,18 +139,30 @@ __global__ void k_accel_cells(uint32_t nT, const TriPlane* __restrict__ plane,
         for (uint32_t y = lo[1]; y <= hi[1]; y++)
             for (uint32_t z = lo[2]; z <= hi[2]; z++) {
                 if (many) {
-                    double bl[3], bh[3], ctr[3], h[3], v[3][3];
+                    double bl[3], bh[3], ctr[3], h[3];
+                    float v32[3][3], h32[3];
                     cell_span(x, nf, bl[0], bh[0]);
                     cell_span(y, nf, bl[1], bh[1]);
                     cell_span(z, nf, bl[2], bh[2]);
                     for (int k = 0; k < 3; k++) {
                         ctr[k] = 0.5 * (bl[k] + bh[k]);
                         h[k] = 0.5 * (bh[k] - bl[k]);
-                        v[0][k] = (double)c0[k] - ctr[k];
-                        v[1][k] = (double)c1[k] - ctr[k];
-                        v[2][k] = (double)c2[k] - ctr[k];
+                        h32[k] = (float)h[k];
+                        v32[0][k] = (float)((double)c0[k] - ctr[k]);
+                        v32[1][k] = (float)((double)c1[k] - ctr[k]);
+                        v32[2][k] = (float)((double)c2[k] - ctr[k]);
                     }
-                    if (!tri_box_overlap(v, h)) continue;
+                    const int clear = tri_box_overlap32(v32, h32);
+                    if (clear == 0) continue;
+                    if (clear == 2) {
+                        double v[3][3];
+                        for (int k = 0; k < 3; k++) {
+                            v[0][k] = (double)c0[k] - ctr[k];
+                            v[1][k] = (double)c1[k] - ctr[k];
+                            v[2][k] = (double)c2[k] - ctr[k];
+                        }
+                        if (!tri_box_overlap(v, h)) continue;
+                    }
                 }
                 uint32_t key = morton3(x, y, z);
                 uint32_t slot = atomicAdd(counter + key, 1u);
