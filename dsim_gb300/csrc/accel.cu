@@ -203,6 +203,79 @@ int launch_accel_cells(bool fill, uint32_t nT, const TriPlane* plane, const TriB
     return kOk;
 }
 
+// ---- cell slabs -----------------------------------------------------------
+// How far a point the float triangle test reports on triangle (u, v) may lie
+// off the triangle, normalised units.  kSlabEps covers the rounding of
+// positions, crossing points and of N . x on both sides (a few 1e-7 each); the
+// rest is the rounding of the Gram system behind the barycentric coordinates,
+// about 40 ulps of the triangle's size over sin^2 of its angle at p1 (64
+// taken).  Infinite, so that its cells cull nothing, for a triangle whose
+// Gram system is nearly singular.
+static constexpr float kSlabEps = 2.5e-5f;
+__device__ __forceinline__ float slab_margin(const TriBary& B, float vv) {
+    const float s2 = 1.0f - (B.uv / B.uu) * (B.uv / vv);
+    if (!(s2 > 1e-5f) || !(B.uu > 0.0f) || !(vv > 0.0f)) return 1e30f;
+    return kSlabEps + 64.0f * 5.9604645e-08f * sqrtf(fmaxf(B.uu, vv)) / s2;
+}
+
+// One thread per cell, in the table's order (x fastest).  N is the sum of the
+// records' normals, each turned to the first one's side, scaled to its largest
+// component 127 and rounded; lo and hi are the range of N . x over the
+// records' corners, widened by each triangle's margin times |N|.
+__global__ void __launch_bounds__(128) k_accel_slabs(uint32_t nf, const TriPlane* __restrict__ plane,
+                                                     const TriBary* __restrict__ bary,
+                                                     const uint32_t* __restrict__ start,
+                                                     const uint32_t* __restrict__ tri,
+                                                     const AccelRecWide* __restrict__ recw,
+                                                     const AccelRecFull* __restrict__ recf, AccelCell* cell) {
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
+    if (x >= nf) return;
+    const uint32_t key = morton3(x, y, z);
+    const uint32_t b0 = start[key], b1 = start[key + 1];
+    AccelCell r;
+    r.first = b0; r.slab = 0u; r.lo = -3.0e38f; r.hi = 3.0e38f;
+    if (b1 > b0) {
+        float sx = 0.0f, sy = 0.0f, sz = 0.0f, rx = 0.0f, ry = 0.0f, rz = 0.0f;
+        for (uint32_t k = b0; k < b1; k++) {
+            const uint32_t t = recf ? __float_as_uint(recf[k].b.w) : (recw ? __float_as_uint(recw[k].pt.w) : tri[k]);
+            const float nx = plane[t].nx, ny = plane[t].ny, nz = plane[t].nz;
+            if (k == b0) { rx = nx; ry = ny; rz = nz; }
+            const float s = nx * rx + ny * ry + nz * rz < 0.0f ? -1.0f : 1.0f;
+            sx += s * nx; sy += s * ny; sz += s * nz;
+        }
+        const float big = fmaxf(fabsf(sx), fmaxf(fabsf(sy), fabsf(sz)));
+        float Nx = 0.0f, Ny = 0.0f, Nz = 0.0f;
+        if (big > 0.0f && big < 1e30f && sx == sx && sy == sy && sz == sz) {
+            Nx = rintf(sx / big * 127.0f); Ny = rintf(sy / big * 127.0f); Nz = rintf(sz / big * 127.0f);
+        }
+        const float len = sqrtf(Nx * Nx + Ny * Ny + Nz * Nz);
+        float lo = 3.0e38f, hi = -3.0e38f;
+        for (uint32_t k = b0; k < b1; k++) {
+            const uint32_t t = recf ? __float_as_uint(recf[k].b.w) : (recw ? __float_as_uint(recw[k].pt.w) : tri[k]);
+            const TriPlane P = plane[t];
+            const TriBary B = bary[t];
+            const float a = Nx * P.p1x + Ny * P.p1y + Nz * P.p1z;
+            const float u = Nx * B.ux + Ny * B.uy + Nz * B.uz, v = Nx * B.vx + Ny * B.vy + Nz * B.vz;
+            const float m = slab_margin(B, P.vv) * len * fmaxf(1.0f, fmaxf(fabsf(P.p1x), fmaxf(fabsf(P.p1y), fabsf(P.p1z))));
+            const float l = a + fminf(0.0f, fminf(u, v)) - m, h = a + fmaxf(0.0f, fmaxf(u, v)) + m;
+            lo = fminf(lo, l); hi = fmaxf(hi, h);
+            if (!(h - l < 1e29f) || !(a + u + v == a + u + v)) { lo = -3.0e38f; hi = 3.0e38f; }
+        }
+        if (len > 0.0f && lo > -1e29f && hi < 1e29f) { r.lo = lo; r.hi = hi; }
+        r.slab = (min(b1 - b0, 255u) << 24) | ((uint32_t)(int)Nx & 0xFFu) | (((uint32_t)(int)Ny & 0xFFu) << 8) |
+                 (((uint32_t)(int)Nz & 0xFFu) << 16);
+    }
+    cell[((size_t)z * nf + y) * nf + x] = r;
+}
+
+int launch_accel_slabs(uint32_t nf, const TriPlane* plane, const TriBary* bary, const uint32_t* start,
+                       const uint32_t* tri, const AccelRecWide* recw, const AccelRecFull* recf, AccelCell* cell,
+                       cudaStream_t st) {
+    k_accel_slabs<<<dim3((nf + 127) / 128, nf, nf), 128, 0, st>>>(nf, plane, bary, start, tri, recw, recf, cell);
+    DSIM_CUDA_TRY(cudaGetLastError());
+    return kOk;
+}
+
 // ---- spin sorting (counting sort on a coarse Morton key) -----------------
 __global__ void k_sort_keys(SpinsSorted S, uint32_t nb, float invLb, uint32_t* keys, uint32_t* hist) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

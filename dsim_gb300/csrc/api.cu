@@ -74,6 +74,7 @@ struct dsim_mesh {
                           // (8, 6, 4), 8 flattened with queued plane survivors, 9 with staged records
     uint64_t accEntries = 0, accBytes = 0;
     uint32_t* acc_start = nullptr;
+    AccelCell* acc_cell = nullptr;
     AccelRec* acc_rec = nullptr;
     uint32_t* acc_tri = nullptr;
     AccelRecWide* acc_recw = nullptr;
@@ -90,7 +91,7 @@ struct dsim_mesh {
     }
     AccelDev acc() const {
         AccelDev a;
-        a.start = acc_start; a.rec = acc_rec; a.tri = acc_tri; a.recw = acc_recw; a.recf = acc_recf; a.nf = nf;
+        a.start = acc_start; a.cell = acc_cell; a.rec = acc_rec; a.tri = acc_tri; a.recw = acc_recw; a.recf = acc_recf; a.nf = nf;
         a.invLf = (float)nf / 2.0f; a.wide = acc_recf ? 2u : (acc_recw ? 1u : 0u);
         return a;
     }
@@ -98,8 +99,8 @@ struct dsim_mesh {
 
 // (Re)build the fine acceleration grid with nf cells per axis (0 removes it).
 static int accel_build(dsim_mesh* m, uint32_t nf) {
-    cudaFree(m->acc_start); cudaFree(m->acc_rec); cudaFree(m->acc_tri); cudaFree(m->acc_recw); cudaFree(m->acc_recf);
-    m->acc_start = nullptr; m->acc_rec = nullptr; m->acc_tri = nullptr; m->acc_recw = nullptr; m->acc_recf = nullptr;
+    cudaFree(m->acc_start); cudaFree(m->acc_cell); cudaFree(m->acc_rec); cudaFree(m->acc_tri); cudaFree(m->acc_recw); cudaFree(m->acc_recf);
+    m->acc_start = nullptr; m->acc_cell = nullptr; m->acc_rec = nullptr; m->acc_tri = nullptr; m->acc_recw = nullptr; m->acc_recf = nullptr;
     m->nf = 0; m->accEntries = 0; m->accBytes = 0;
     if (nf == 0) return kOk;
     if (nf > 1024) { set_last_error(kErrTooLarge, "accel grid: %u cells per axis > 1024", nf); return kErrTooLarge; }
@@ -129,6 +130,8 @@ static int accel_build(dsim_mesh* m, uint32_t nf) {
         }
         if (cudaMemsetAsync(counter, 0, (size_t)nkeys * 4, st) != cudaSuccess) { rc = kErrCuda; break; }
         if ((rc = launch_accel_cells(true, m->nT, m->plane, m->bary, nf, counter, m->acc_start, m->acc_rec, m->acc_tri, m->acc_recw, st, m->acc_recf))) break;
+        if ((rc = dev_alloc(&m->acc_cell, (size_t)nf * nf * nf, &m->accBytes))) break;
+        if ((rc = launch_accel_slabs(nf, m->plane, m->bary, m->acc_start, m->acc_tri, m->acc_recw, m->acc_recf, m->acc_cell, st))) break;
         if (cudaStreamSynchronize(st) != cudaSuccess) { rc = kErrCuda; break; }
         m->nf = nf;
     } while (0);
@@ -136,8 +139,8 @@ static int accel_build(dsim_mesh* m, uint32_t nf) {
     cudaFree(counter);
     cudaFree(scratch);
     if (rc) {
-        cudaFree(m->acc_start); cudaFree(m->acc_rec); cudaFree(m->acc_tri); cudaFree(m->acc_recw); cudaFree(m->acc_recf);
-        m->acc_start = nullptr; m->acc_rec = nullptr; m->acc_tri = nullptr; m->acc_recw = nullptr; m->acc_recf = nullptr; m->nf = 0;
+        cudaFree(m->acc_start); cudaFree(m->acc_cell); cudaFree(m->acc_rec); cudaFree(m->acc_tri); cudaFree(m->acc_recw); cudaFree(m->acc_recf);
+        m->acc_start = nullptr; m->acc_cell = nullptr; m->acc_rec = nullptr; m->acc_tri = nullptr; m->acc_recw = nullptr; m->acc_recf = nullptr; m->nf = 0;
     }
     return rc;
 }
@@ -274,7 +277,7 @@ static void mesh_release(dsim_mesh* m) {
     cudaFree(m->V); cudaFree(m->trgls); cudaFree(m->membrane); cudaFree(m->fiber);
     cudaFree(m->plane); cudaFree(m->bary); cudaFree(m->cell_start); cudaFree(m->cell_tri); cudaFree(m->tri64);
     cudaFree(m->tri_cells);
-    cudaFree(m->acc_start); cudaFree(m->acc_rec); cudaFree(m->acc_tri); cudaFree(m->acc_recw); cudaFree(m->acc_recf);
+    cudaFree(m->acc_start); cudaFree(m->acc_cell); cudaFree(m->acc_rec); cudaFree(m->acc_tri); cudaFree(m->acc_recw); cudaFree(m->acc_recf);
     delete m;
 }
 

@@ -82,6 +82,7 @@ struct State {
     // fine acceleration grid (cells per axis = accelFactor x k_numCubes)
     uint32_t nf = 0;
     uint32_t* acc_start = nullptr;
+    AccelCell* acc_cell = nullptr;
     AccelRecWide* acc_recw = nullptr;
     // spin work buffers for the reordered fast path (grow with N)
     uint32_t cap = 0;
@@ -93,9 +94,9 @@ struct State {
     uint32_t sortEvery = 1000;  // reorder by fine cell once per call of up to 1000 steps
     void release() {
         cudaFree(plane); cudaFree(bary); cudaFree(cell_start); cudaFree(cell_tri);
-        cudaFree(acc_start); cudaFree(acc_recw);
+        cudaFree(acc_start); cudaFree(acc_cell); cudaFree(acc_recw);
         plane = nullptr; bary = nullptr; cell_start = nullptr; cell_tri = nullptr;
-        acc_start = nullptr; acc_recw = nullptr; nf = 0;
+        acc_start = nullptr; acc_cell = nullptr; acc_recw = nullptr; nf = 0;
         have = false;
     }
     SpinsSorted set(int k, uint32_t N) const {
@@ -182,6 +183,8 @@ int derive(State& s, const uint32_t* tic, const uint32_t* cc) {
     if (!rc && cudaMalloc(&s.acc_recw, (size_t)(accTotal ? accTotal : 1) * sizeof(AccelRecWide)) != cudaSuccess) rc = kErrNoMem;
     if (!rc && cudaMemset(counter, 0, (size_t)nkeys * 4) != cudaSuccess) rc = kErrCuda;
     if (!rc) rc = launch_accel_cells(true, nT, s.plane, s.bary, nf, counter, s.acc_start, nullptr, nullptr, s.acc_recw, 0);
+    if (!rc && cudaMalloc(&s.acc_cell, (size_t)nf * nf * nf * sizeof(AccelCell)) != cudaSuccess) rc = kErrNoMem;
+    if (!rc) rc = launch_accel_slabs(nf, s.plane, s.bary, s.acc_start, nullptr, s.acc_recw, nullptr, s.acc_cell, 0);
     cudaFree(counter);
     cudaFree(scr);
     if (rc) { set_last_error(rc, "integrateSystem: building the fine grid failed"); return rc; }
@@ -355,7 +358,7 @@ void integrateSystem(float* pos, unsigned int* randSeed, dsim_spinData* spinInfo
     int cur = 0;
     if ((rc = launch_aos_to_soa(pos, spinInfo, s.set(cur, N), 0))) { fail(rc); return; }
     AccelDev acc;
-    acc.start = s.acc_start; acc.rec = nullptr; acc.tri = nullptr; acc.recw = s.acc_recw; acc.nf = s.nf;
+    acc.start = s.acc_start; acc.cell = s.acc_cell; acc.rec = nullptr; acc.tri = nullptr; acc.recw = s.acc_recw; acc.nf = s.nf;
     acc.invLf = (float)s.nf / 2.0f; acc.wide = 1;
     a.spinKeys = randSeed;
     int rng = s.replay ? kRngReplay : kRngPhiloxPerSpinKey;

@@ -85,8 +85,18 @@ struct __align__(32) AccelRecWide {
 struct __align__(16) AccelRecFull {
     float4 a, b, c, d;
 };
+// One fine cell: its first record, its record count (bits 24-31 of slab; 255:
+// start[] tells) and a slab that holds the cell's triangles: every point x of
+// them has lo <= N . x <= hi for the integer vector N (three signed bytes of
+// slab).  The step kernels skip the records of a cell whose slab both ends of
+// the sub-segment leave on the same side.
+struct __align__(16) AccelCell {
+    uint32_t first, slab;
+    float lo, hi;
+};
 struct AccelDev {
     const uint32_t* start;  // Morton key -> first record (keys + 1 entries)
+    const AccelCell* cell;  // [nf^3] cells, x fastest
     const AccelRec* rec;    // 16-byte records (wide == 0)
     const uint32_t* tri;    // triangle of each record (wide == 0)
     const AccelRecWide* recw;  // 32-byte records (wide == 1)
@@ -109,6 +119,10 @@ __host__ __device__ inline uint32_t accel_keys(uint32_t nf) {
 int launch_accel_cells(bool fill, uint32_t nT, const TriPlane* plane, const TriBary* bary,
                        uint32_t nf, uint32_t* counter, const uint32_t* start, AccelRec* rec,
                        uint32_t* tri, AccelRecWide* recw, cudaStream_t st, AccelRecFull* recf = nullptr);
+// the cells' slabs from their records (any layout) and the triangles' corners
+int launch_accel_slabs(uint32_t nf, const TriPlane* plane, const TriBary* bary, const uint32_t* start,
+                       const uint32_t* tri, const AccelRecWide* recw, const AccelRecFull* recf, AccelCell* cell,
+                       cudaStream_t st);
 int launch_sort_spins(const SpinsSorted& S, const SpinsSorted& D, uint32_t nb, uint32_t* keys,
                       uint32_t* hist, uint32_t* start, uint32_t* scratch, cudaStream_t st);
 int launch_unpermute(const SpinsSorted& S, const SpinsSorted& D, cudaStream_t st);

@@ -225,9 +225,8 @@ __device__ __forceinline__ void flat_round_mode(FlatWarp& H, const MeshDev& g, c
             const uint32_t wd = H.wd[ow], bx = H.box[ow];
             const uint32_t ww1 = (wd >> 8) & 0xFFu, ww2 = wd >> 16;
             const uint32_t iz = q % ww2, r = q / ww2, iy = r % ww1, ix = r / ww1;
-            const uint32_t key = morton3((bx & 1023u) + ix, ((bx >> 10) & 1023u) + iy, (bx >> 20) + iz);
-            b0 = __ldg(acc.start + key);
-            cnt = __ldg(acc.start + key + 1) - b0;
+            cell_records(acc, (bx & 1023u) + ix, ((bx >> 10) & 1023u) + iy, (bx >> 20) + iz, H.ox[ow], H.oy[ow],
+                         H.oz[ow], H.dx[ow], H.dy[ow], H.dz[ow], b0, cnt);
         }
         // pass 2: the items' records, concatenated over the warp
         const uint32_t rincl = warp_incl_scan(cnt, lane);

@@ -431,9 +431,9 @@ __device__ __forceinline__ void local_round(FlatWarp& H, LocalWarp& Lw, const Me
                 const uint32_t wd = H.wd[ow], bx = H.box[ow];
                 const uint32_t ww1 = (wd >> 8) & 0xFFu, ww2 = wd >> 16;
                 const uint32_t iz = q % ww2, r = q / ww2, iy = r % ww1, ix = r / ww1;
-                const uint32_t key = morton3((bx & 1023u) + ix, ((bx >> 10) & 1023u) + iy, (bx >> 20) + iz);
-                b0 = __ldg(acc.start + key);
-                cnt = __ldg(acc.start + key + 1) - b0;
+                cell_records(acc, (bx & 1023u) + ix, ((bx >> 10) & 1023u) + iy, (bx >> 20) + iz,
+                             Lw.gx[ow] + H.ox[ow], Lw.gy[ow] + H.oy[ow], Lw.gz[ow] + H.oz[ow], H.dx[ow], H.dy[ow],
+                             H.dz[ow], b0, cnt);
             }
             rincl = warp_incl_scan(cnt, lane);
             rtotal = __shfl_sync(FULL, rincl, 31);
