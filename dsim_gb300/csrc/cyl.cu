@@ -242,8 +242,9 @@ int build_cyl_grid_gpu(const float4* fibers, uint32_t nF, uint32_t n, uint32_t m
 
 template <int RNG>
 __global__ void __launch_bounds__(256) k_cyl_step(CylDev g, CylStepArgs a, CylSpinsDev S) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S.N) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * a.perWarp + lane;
+    if (lane >= a.perWarp || i >= S.N) return;
     float4 P = S.pos[i];
     uint4 sd4 = reinterpret_cast<const uint4*>(S.seed4)[i];
     float x = P.x, y = P.y, z = P.z, phase = P.w;
@@ -291,10 +292,17 @@ __global__ void __launch_bounds__(256) k_cyl_step(CylDev g, CylStepArgs a, CylSp
     if (status) atomicOr(a.status, status);
 }
 
-int launch_cyl_step(const CylDev& g, const CylStepArgs& a, const CylSpinsDev& S, int rng,
+int launch_cyl_step(const CylDev& g, const CylStepArgs& args, const CylSpinsDev& S, int rng,
                     cudaStream_t st) {
-    if (S.N == 0 || a.iterations == 0) return kOk;
-    dim3 block(128), grid((S.N + 127) / 128);
+    if (S.N == 0 || args.iterations == 0) return kOk;
+    CylStepArgs a = args;
+    // at most 17 warps per SM below 32 spins a warp.  us per step, 64
+    // cylinders, 32 / 16 / 8 / 4 / 2 / 1 spins a warp: 1000 spins 3.9 / 3.5 /
+    // 2.9 / 2.6 / 2.4 / 2.2; 10,000 spins 4.9 / 4.1 / 3.4 / 3.4 / 4.1 / 5.7;
+    // 40,000 spins 5.1 / 4.6 / 6.4; 80,000 spins 5.8 / 7.2
+    a.perWarp = spins_per_warp(S.N, 17);
+    const uint32_t warps = (S.N + a.perWarp - 1) / a.perWarp;
+    dim3 block(128), grid((warps + 3) / 4);
     if (rng == kRngReplay) k_cyl_step<kRngReplay><<<grid, block, 0, st>>>(g, a, S);
     else if (rng == kRngPhilox) k_cyl_step<kRngPhilox><<<grid, block, 0, st>>>(g, a, S);
     else k_cyl_step<kRngPhiloxPerSpinKey><<<grid, block, 0, st>>>(g, a, S);

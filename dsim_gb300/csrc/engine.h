@@ -64,7 +64,20 @@ struct MeshStepArgs {
     uint32_t* tested;     // [N] grid entries scanned (or null)
     const uint32_t* spinKeys;  // per-spin Philox keys [2N] by id (kRngPhiloxPerSpinKey, fast path)
     uint32_t spinBase;    // added to the spin index in the Philox counter (replica shards)
+    uint32_t perWarp;     // spins a warp advances (spins_per_warp; set by the launcher)
 };
+
+// Spins a warp advances: 32 while the spins give every SM `warpsPerSm` warps
+// or more, else the largest power of two below that still does.  With fewer
+// spins than the chip has lanes a step takes as long as one warp's chain, and
+// a warp's chain is the longer the more spins share it (mesh: their records
+// and reflections add up; cylinders: their branches do).
+static constexpr uint32_t kSmCount = 152;
+inline uint32_t spins_per_warp(uint32_t N, uint32_t warpsPerSm) {
+    uint32_t p = 1;
+    while (p < 32 && (N + p - 1) / p > kSmCount * warpsPerSm) p *= 2;
+    return p;
+}
 
 // ---- accel.cu -------------------------------------------------------------
 // Fine acceleration grid: every triangle is listed in each fine cell it
@@ -232,6 +245,7 @@ struct CylStepArgs {
     uint32_t* status;
     uint32_t* counts;
     uint32_t spinBase;    // added to the spin index in the Philox counter (replica shards)
+    uint32_t perWarp;     // spins a warp advances (spins_per_warp; set by the launcher)
 };
 // rng: kRngPhilox (key0/key1), kRngPhiloxPerSpinKey (seed4.x/.y), kRngReplay
 int launch_cyl_step(const CylDev& g, const CylStepArgs& a, const CylSpinsDev& S, int rng,

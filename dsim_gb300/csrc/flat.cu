@@ -50,8 +50,8 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
         if (lane == 0) stage_init(&ws[threadIdx.x >> 5]);
         __syncwarp();
     }
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < S.N;
+    const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * a.perWarp + lane;
+    const bool valid = lane < a.perWarp && i < S.N;
     float x = 0.0f, y = 0.0f, z = 0.0f, mag = 0.0f, phase = 0.0f;
     uint32_t comp = 0, fiber = 0, id = 0;
     if (valid) {
@@ -149,10 +149,17 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
     if (status) atomicOr(a.status, status);
 }
 
-int launch_mesh_step_flat(const MeshDev& g, const AccelDev& acc, const MeshStepArgs& a,
+int launch_mesh_step_flat(const MeshDev& g, const AccelDev& acc, const MeshStepArgs& args,
                           const SpinsSorted& S, int rng, cudaStream_t st, int occupancy, bool queue, bool stage) {
-    if (S.N == 0 || a.iterations == 0) return kOk;
-    dim3 block(kFlatThreads), grid((S.N + kFlatThreads - 1) / kFlatThreads);
+    if (S.N == 0 || args.iterations == 0) return kOk;
+    MeshStepArgs a = args;
+    // at most 14 warps per SM below 32 spins a warp.  us per step, 25 tubes
+    // with myelin, 32 / 16 / 8 / 4 / 2 / 1 spins a warp: 1000 spins 15.8 / 9.5
+    // / 6.6 / 4.9 / 4.1 / 3.9; 8192 spins 17.9 / 11.2 / 7.8 / 6.8 / 8.8 / 10.5;
+    // 32768 spins 19.0 / 13.8 / 14.7; 65536 spins 21.6 / 22.2
+    a.perWarp = spins_per_warp(S.N, 14);
+    const uint32_t warps = (S.N + a.perWarp - 1) / a.perWarp;
+    dim3 block(kFlatThreads), grid((warps + kFlatWarps - 1) / kFlatWarps);
     // one instantiation per record layout keeps each kernel's registers to its own path
     if (a.tested) k_mesh_step_flat<true, 4, 0><<<grid, block, 0, st>>>(g, acc, a, S, rng);
     else if (acc.wide == 2) {
