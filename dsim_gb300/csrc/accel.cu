@@ -218,6 +218,70 @@ __device__ __forceinline__ float slab_margin(const TriBary& B, float vv) {
     return kSlabEps + 64.0f * 5.9604645e-08f * sqrtf(fmaxf(B.uu, vv)) / s2;
 }
 
+// Marks (by the sign of vv) the triangles whose hits need the reference's walk
+// over its cells: those that enter the inside of some reference cell (shrunk
+// by kRegularEps) that does not list them, that lie in more than four cells,
+// or whose float test may report a point farther off (slab_margin).  Any other
+// triangle is listed by the cell of a hit point that keeps 2 kRegularEps from
+// the cell's faces (flat_only_hit).  The reference's overlap test is decided by
+// rounding where a triangle ends on a face, as the rings of a tessellated tube
+// often do, so touching a face alone says nothing.
+__global__ void k_tri_regular(uint32_t nT, uint32_t n, const uint4* __restrict__ cells,
+                              const TriBary* __restrict__ bary, TriPlane* plane) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nT) return;
+    const float eps = kRegularEps;
+    const TriPlane P = plane[t];
+    const TriBary B = bary[t];
+    const uint4 c = cells[t];
+    const float vv = fabsf(P.vv), inv = 0.5f * (float)n, L = 2.0f / (float)n;
+    const float c0[3] = {P.p1x, P.p1y, P.p1z};
+    const float c1[3] = {P.p1x + B.vx, P.p1y + B.vy, P.p1z + B.vz};
+    const float c2[3] = {P.p1x + B.ux, P.p1y + B.uy, P.p1z + B.uz};
+    uint32_t lo[3], hi[3];
+    float mn[3], mx[3];
+    bool regular = c.x != kCellMany && slab_margin(B, vv) <= eps;
+    for (int k = 0; k < 3; k++) {
+        mn[k] = fminf(c0[k], fminf(c1[k], c2[k]));
+        mx[k] = fmaxf(c0[k], fmaxf(c1[k], c2[k]));
+        regular = regular && mn[k] > -2.0f && mx[k] < 2.0f;
+    }
+    for (int k = 0; regular && k < 3; k++) {
+        lo[k] = fine_coord(mn[k], inv, n);
+        hi[k] = fine_coord(mx[k], inv, n);
+        regular = hi[k] - lo[k] < 6u;  // four cells at most are listed
+    }
+    for (uint32_t x = regular ? lo[0] : 1u; regular && x <= hi[0]; x++)
+        for (uint32_t y = lo[1]; regular && y <= hi[1]; y++)
+            for (uint32_t z = lo[2]; regular && z <= hi[2]; z++) {
+                const uint32_t at = x | (y << 10) | (z << 20);
+                if (c.x == at || c.y == at || c.z == at || c.w == at) continue;
+                const uint32_t q[3] = {x, y, z};
+                float v[3][3], h[3];
+                bool apart = false;
+                for (int k = 0; k < 3; k++) {
+                    // the outermost cells are open: to the triangle's own extent
+                    float bl = -1.0f + (float)q[k] * L + eps, bh = -1.0f + (float)(q[k] + 1) * L - eps;
+                    if (q[k] == 0) bl = fminf(bl, mn[k]);
+                    if (q[k] == n - 1) bh = fmaxf(bh, mx[k]);
+                    const float ctr = 0.5f * (bl + bh);
+                    h[k] = 0.5f * (bh - bl);
+                    v[0][k] = c0[k] - ctr; v[1][k] = c1[k] - ctr; v[2][k] = c2[k] - ctr;
+                    apart = apart || mn[k] > bh || mx[k] < bl;
+                }
+                regular = apart || tri_box_overlap32(v, h) == 0;
+            }
+    plane[t].vv = regular ? vv : -vv;
+}
+
+int launch_tri_regular(uint32_t nT, uint32_t n, const uint4* cells, const TriBary* bary, TriPlane* plane,
+                       cudaStream_t st) {
+    if (nT == 0) return kOk;
+    k_tri_regular<<<(nT + 127) / 128, 128, 0, st>>>(nT, n, cells, bary, plane);
+    DSIM_CUDA_TRY(cudaGetLastError());
+    return kOk;
+}
+
 // One thread per cell, in the table's order (x fastest).  N is the sum of the
 // records' normals, each turned to the first one's side, scaled to its largest
 // component 127 and rounded; lo and hi are the range of N . x over the
@@ -256,7 +320,7 @@ __global__ void __launch_bounds__(128) k_accel_slabs(uint32_t nf, const TriPlane
             const TriBary B = bary[t];
             const float a = Nx * P.p1x + Ny * P.p1y + Nz * P.p1z;
             const float u = Nx * B.ux + Ny * B.uy + Nz * B.uz, v = Nx * B.vx + Ny * B.vy + Nz * B.vz;
-            const float m = slab_margin(B, P.vv) * len * fmaxf(1.0f, fmaxf(fabsf(P.p1x), fmaxf(fabsf(P.p1y), fabsf(P.p1z))));
+            const float m = slab_margin(B, fabsf(P.vv)) * len * fmaxf(1.0f, fmaxf(fabsf(P.p1x), fmaxf(fabsf(P.p1y), fabsf(P.p1z))));
             const float l = a + fminf(0.0f, fminf(u, v)) - m, h = a + fmaxf(0.0f, fmaxf(u, v)) + m;
             lo = fminf(lo, l); hi = fmaxf(hi, h);
             if (!(h - l < 1e29f) || !(a + u + v == a + u + v)) { lo = -3.0e38f; hi = 3.0e38f; }

@@ -334,13 +334,14 @@ static int mesh_build(dsim_mesh* m, const std::vector<float>& Vn, const std::vec
         if (m->nT > ncells) {  // the scan scratch is sized for ncells; use a count of its own
             uint32_t* tcount = nullptr;
             if ((rc = dev_alloc(&tcount, m->nT))) break;
-            rc = launch_tri_cell_lists(ncells, m->nT, m->cell_start, m->cell_tri, tcount, m->tri_cells, st);
+            rc = launch_tri_cell_lists(m->n, m->nT, m->cell_start, m->cell_tri, tcount, m->tri_cells, st);
             if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = kErrCuda;
             cudaFree(tcount);
             if (rc) break;
-        } else if ((rc = launch_tri_cell_lists(ncells, m->nT, m->cell_start, m->cell_tri, counter, m->tri_cells, st))) {
+        } else if ((rc = launch_tri_cell_lists(m->n, m->nT, m->cell_start, m->cell_tri, counter, m->tri_cells, st))) {
             break;
         }
+        if ((rc = launch_tri_regular(m->nT, m->n, m->tri_cells, m->bary, m->plane, st))) break;
         std::vector<uint32_t> cs(ncells + 1);
         if (cudaMemcpyAsync(cs.data(), m->cell_start, cs.size() * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) { rc = kErrCuda; break; }

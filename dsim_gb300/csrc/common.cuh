@@ -126,7 +126,7 @@ __device__ __forceinline__ Draw philox_draw(uint32_t spin, uint64_t step, uint32
 // u, v and the three dot products (second 32-B record, read on plane hits only).
 struct __align__(16) TriPlane {
     float nx, ny, nz, p1x;
-    float p1y, p1z, vv;
+    float p1y, p1z, vv;  // the sign of vv is a flag (hit_walk)
     uint32_t info;  // membrane type (bits 0-1) | fiber index << 2
 };
 struct __align__(16) TriBary {

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(128) k_compartments(MeshDev g, AccelDev acc, S
                                 fine_coord(h.z, acc.invLf, acc.nf) != c2)
                                 continue;
                             const uint32_t info = __ldg(&g.plane[t].info);
-                            if (h.type > 1) edgeTypes |= 1u << (info & 3u);
+                            if ((h.type & ~kHitWalk) > 1) edgeTypes |= 1u << (info & 3u);
                             const uint32_t fk = info;  // fiber << 2 | membrane
                             uint32_t s = 0;
                             while (s < nkeys && keys[s] != fk) s++;

@@ -77,6 +77,7 @@ struct State {
     TriBary* bary = nullptr;
     uint32_t* cell_start = nullptr;
     uint32_t* cell_tri = nullptr;
+    uint4* tri_cells = nullptr;
     uint32_t* status = nullptr;
     uint32_t statusHost = 0;
     // fine acceleration grid (cells per axis = accelFactor x k_numCubes)
@@ -93,9 +94,9 @@ struct State {
     uint32_t histNf = 0;
     uint32_t sortEvery = 1000;  // reorder by fine cell once per call of up to 1000 steps
     void release() {
-        cudaFree(plane); cudaFree(bary); cudaFree(cell_start); cudaFree(cell_tri);
+        cudaFree(plane); cudaFree(bary); cudaFree(cell_start); cudaFree(cell_tri); cudaFree(tri_cells);
         cudaFree(acc_start); cudaFree(acc_cell); cudaFree(acc_recw);
-        plane = nullptr; bary = nullptr; cell_start = nullptr; cell_tri = nullptr;
+        plane = nullptr; bary = nullptr; cell_start = nullptr; cell_tri = nullptr; tri_cells = nullptr;
         acc_start = nullptr; acc_cell = nullptr; acc_recw = nullptr; nf = 0;
         have = false;
     }
@@ -157,9 +158,17 @@ int derive(State& s, const uint32_t* tic, const uint32_t* cc) {
     if (!rc && cudaMemcpy(&total, s.cell_start + ncells, 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = kErrCuda;
     if (!rc && cudaMalloc(&s.cell_tri, (size_t)(total ? total : 1) * 4) != cudaSuccess) rc = kErrNoMem;
     if (!rc) rc = launch_dense_to_csr(ncells, s.maxTPC, nT, cc, tic, s.cell_start, s.cell_tri, s.status, 0);
+    // each triangle's reference cells (a hit then needs no list search)
+    uint32_t* perTri = nullptr;
+    if (!rc && (cudaMalloc(&s.tri_cells, (size_t)nT * sizeof(uint4)) != cudaSuccess ||
+                cudaMalloc(&perTri, (size_t)nT * 4) != cudaSuccess))
+        rc = kErrNoMem;
+    if (!rc) rc = launch_tri_cell_lists(s.numCubes, nT, s.cell_start, s.cell_tri, perTri, s.tri_cells, 0);
+    if (!rc) rc = launch_tri_regular(nT, s.numCubes, s.tri_cells, s.bary, s.plane, 0);
     uint32_t st = 0;
     if (!rc && cudaMemcpy(&st, s.status, 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = kErrCuda;
     cudaFree(scratch);
+    cudaFree(perTri);
     if (rc) { set_last_error(rc, "integrateSystem: deriving cell lists failed"); return rc; }
     if (st) {
         set_last_error(kErrFormat, "integrateSystem: trianglesInCubes names a triangle >= %u or a cell above k_maxTrianglesPerCube", nT);
@@ -333,7 +342,7 @@ void integrateSystem(float* pos, unsigned int* randSeed, dsim_spinData* spinInfo
     MeshDev g;
     g.cell_start = s.cell_start; g.cell_tri = s.cell_tri; g.plane = s.plane; g.bary = s.bary;
     g.tri64 = nullptr;
-    g.tri_cells = nullptr;
+    g.tri_cells = s.tri_cells;
     g.n = s.numCubes; g.L = s.cubeLength;
     MeshStepArgs a;
     memset(&a, 0, sizeof(a));

@@ -10,16 +10,15 @@
 // in every fine cell it touches; a collision round works in two flat passes
 // over the whole warp:
 //
-//   1. items: the lanes' fine-cell boxes are concatenated by a warp prefix sum;
-//      32 items at a time, lane m finds its item's owner (binary search over
-//      the prefix by shuffle) and loads that cell's record range, so 32 range
-//      loads are in flight at once;
-//   2. records: a second prefix sum over the 32 ranges concatenates their
-//      records; lane j tests flat record j, j + 32, ... against the owner's
-//      sub-segment, read from a per-warp segment table in shared memory.
+//   1. cells: the lanes' fine-cell boxes are concatenated by a warp prefix sum;
+//      32 cells at a time, lane m looks up its cell's record, so 32 loads are in
+//      flight at once, and keeps it if the owner's sub-segment may meet its slab;
+//   2. records: a second prefix sum concatenates the kept cells' records; lane j
+//      tests flat record j, j + 32, ... against the owner's sub-segment, read
+//      from a per-warp segment table in shared memory.
 //
-// Hits are filed in the owner's slots and resolved by the owner: the first
-// reference cell (in the reference's order) whose list holds one of its hits,
+// Hits are filed in the owner's slots and resolved by the owner: the only hit,
+// or the first reference cell (in the reference's order) whose list holds one,
 // the nearest there, the lowest index on ties; the exact reference-grid scan
 // when the slots overflowed.  Lanes do not advance through the steps in
 // lockstep: a lane whose step ends starts its next step in the next round, so
@@ -52,10 +51,11 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
     }
     const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * a.perWarp + lane;
     const bool valid = lane < a.perWarp && i < S.N;
-    float x = 0.0f, y = 0.0f, z = 0.0f, mag = 0.0f, phase = 0.0f;
+    // the position is o at the top of a step, the start of its current sub-segment within one
+    float ox = 0.0f, oy = 0.0f, oz = 0.0f, mag = 0.0f, phase = 0.0f;
     uint32_t comp = 0, fiber = 0, id = 0;
     if (valid) {
-        x = S.x[i]; y = S.y[i]; z = S.z[i]; mag = S.mag[i]; phase = S.phase[i];
+        ox = S.x[i]; oy = S.y[i]; oz = S.z[i]; mag = S.mag[i]; phase = S.phase[i];
         uint32_t meta = S.meta[i];
         comp = meta & 0xFFu; fiber = meta >> 8;
         id = S.id[i];
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
     bool fresh = active;  // the lane starts step `it` at the top of the round
     Draw d;
     d.nx = d.ny = d.nz = 0.0f; d.u = 1.0f;
-    float ox = x, oy = y, oz = z, px = x, py = y, pz = z;
+    float px = ox, py = oy, pz = oz;
     uint32_t excluded = 0xFFFFFFFFu, sub = 0;
     float umax = 1.0f, umin = 0.0f;
     while (__any_sync(FULL, active)) {
@@ -82,9 +82,8 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
             } else {
                 d = philox_draw(a.spinBase + id, a.step0 + it, a.stream, k0, k1);
             }
-            ox = x; oy = y; oz = z;
             const float sd = a.sd[comp & 3u];
-            px = x + d.nx * sd; py = y + d.ny * sd; pz = z + d.nz * sd;
+            px = ox + d.nx * sd; py = oy + d.ny * sd; pz = oz + d.nz * sd;
             // the reference's endPos equals the sub-segment target p at the top
             // of every collision round, so p doubles as endPos
             excluded = 0xFFFFFFFFu;
@@ -125,11 +124,11 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
                     if (ex > a.clampHi) ex = a.clampHi; else if (ex < a.clampLo) ex = a.clampLo;
                     if (ey > a.clampHi) ey = a.clampHi; else if (ey < a.clampLo) ey = a.clampLo;
                     if (ez > a.clampHi) ez = a.clampHi; else if (ez < a.clampLo) ez = a.clampLo;
-                    x = ex; y = ey; z = ez;
+                    ox = ex; oy = ey; oz = ez;
                     mag += -mag / a.T2[comp & 3u] * a.dt;
                     float gx = a.gx, gy = a.gy, gz = a.gz;
                     if (a.grad) { float4 G = __ldg(a.grad + it); gx = G.x; gy = G.y; gz = G.z; }
-                    phase += (gx * x + gy * y + gz * z) * a.pc;
+                    phase += (gx * ox + gy * oy + gz * oz) * a.pc;
                     if (++it >= a.iterations) active = false;
                     else fresh = true;
                 }
@@ -142,7 +141,7 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
         }
     }
     if (!valid) return;
-    S.x[i] = x; S.y[i] = y; S.z[i] = z; S.mag[i] = mag; S.phase[i] = phase;
+    S.x[i] = ox; S.y[i] = oy; S.z[i] = oz; S.mag[i] = mag; S.phase[i] = phase;
     S.meta[i] = (comp & 0xFFu) | (fiber << 8);
     if (a.counts) { a.counts[2 * id] += nrefl; a.counts[2 * id + 1] += nperm; }
     if (STATS && a.tested) a.tested[id] += ntested;

@@ -4,13 +4,25 @@
 //
 // Semantics: rfdougherty/dSim dSim3/src/spinKernelCpu.cpp:198-337 (the
 // collision search over the cells of the sub-segment's box, nearest hit of the
-// first reference cell with a hit, last-hit triangle excluded).  The warp
-// concatenates its lanes' fine-cell boxes by a prefix sum and loads 32 cell
-// ranges at once, then concatenates those cells' records and tests record j,
-// j + 32, ... per lane against the owner's sub-segment (segment table in shared
-// memory, owner found by a shuffle binary search).  Hits are filed in the
-// owner's shared-memory slots and each owner replays the reference's rule over
-// its own hits (exact reference-grid scan when the slots overflowed).
+// first reference cell with a hit, last-hit triangle excluded).  The lanes'
+// fine-cell boxes form one flat list of cells (a prefix sum; an element's owner
+// from a mask of starts and a rank table, flat_starts); 32 cells at a time are
+// looked up and those whose slab the sub-segment may meet are kept.  The kept
+// cells' records form flat lists in blocks of 32 cells, tested 64 records at a
+// time against their owners' sub-segments (segment table in shared memory);
+// records past the plane test are queued and finished 32 at a time.  Hits are
+// filed in the owner's shared-memory slots.  An owner with one hit of a triangle
+// that every reference cell it enters lists takes it; others choose by the
+// reference's walk over its cells (exact reference-grid scan when the slots
+// overflowed).
+//
+// Bound by instruction issue and L2 latency together (400,000 spins on 640,000
+// triangles: issue 51 %, long-scoreboard stalls 3.1 of 8.2 cycles an
+// instruction, DRAM idle).  Warp instructions per step of 32 spins went 3031 ->
+// 2513 (slabs) -> 2164 (this layout: owners by mask and rank instead of
+// five-shuffle searches, no integer division, full windows, one copy of the
+// exact test, no walk over cells for nine hits in ten); 6.6e9 -> 9.1e9
+// spin-steps/s there, 6.8e9 -> 9.4e9 for 1M spins on 2.56M triangles.
 #pragma once
 #include "common.cuh"
 #include "engine.h"
@@ -22,14 +34,15 @@ namespace dsim {
 static constexpr int kFlatThreads = 128;
 static constexpr int kFlatWarps = kFlatThreads / 32;
 static constexpr int kFlatSlots = 4;      // hits kept per owner per round
-static constexpr int kFlatMaxItems = 27;  // cells per segment handled by the warp (3 x 3 x 3)
+static constexpr uint32_t kFlatMaxWidth = 4;  // cells per axis of a box the warp handles
 
 struct FlatWarp {
-    // sub-segment table of the current round, by owner lane
-    float ox[32], oy[32], oz[32], dx[32], dy[32], dz[32];
-    uint32_t excl[32];
-    uint32_t box[32];  // fine-cell box origin lo0 | lo1 << 10 | lo2 << 20
-    uint32_t wd[32];   // box widths w0 | w1 << 8 | w2 << 16
+    // the round's sub-segments by owner lane: start and excluded triangle
+    // (bits); end - start and fine-cell box origin lo0 | lo1 << 10 | lo2 << 20
+    // (bits)
+    float4 o[32], d[32];
+    uint32_t src[32];  // by rank among the lanes with cells (flat_box)
+    uint2 cell[64];    // cells with records still to test: first record, owner | count << 5
     // hits filed per owner
     uint32_t n[32];
     uint32_t t[kFlatSlots][32];
@@ -57,33 +70,154 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, uint32_t lane) {
     return v;
 }
 
-// index of the first lane j with incl[j] > r (incl non-decreasing over the
-// lanes); valid for r < incl[31]
-__device__ __forceinline__ uint32_t warp_find(uint32_t incl, uint32_t r) {
-    uint32_t pos = 0;
-#pragma unroll
-    for (uint32_t step = 16; step > 0; step >>= 1) {
-        uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, pos + step - 1);
-        if (v <= r) pos += step;
+// ---- flat lists over the warp -----------------------------------------------
+// Lane k's `count` elements (none or more) occupy [start, start + count) of a
+// flat list.  For the 32 elements from `base` on, the warp's starts among them
+// form one mask (a hardware OR-reduction), and element base + l belongs to the
+// lane whose rank among the lanes with elements is the number of starts up to
+// it, less one; a table in shared memory takes the rank to the lane.  A binary
+// search of the prefix sums by shuffles took five dependent shuffles instead.
+__device__ __forceinline__ uint32_t flat_starts(bool has, uint32_t start, uint32_t base) {
+    const uint32_t k = start - base;
+    return __reduce_or_sync(0xFFFFFFFFu, (has && k < 32u) ? 1u << k : 0u);
+}
+
+// A lane's fine-cell box, from absolute end points: its cells are counted with
+// the y and z widths rounded up to 1, 2 or 4 (so an element's cell needs no
+// division; the cells beyond the box are skipped).  Boxes wider than 4 cells
+// are left to their owner (solo).
+struct FlatBox {
+    uint32_t lo0, lo1, lo2, w0, w1, w2, count, packed;
+    bool solo;
+};
+__device__ __forceinline__ FlatBox flat_box(const AccelDev& acc, bool open, float ox, float oy, float oz, float px,
+                                            float py, float pz) {
+    FlatBox b;
+    b.lo0 = b.lo1 = b.lo2 = b.w0 = b.w1 = b.w2 = b.count = b.packed = 0;
+    b.solo = false;
+    if (open) {
+        const float invLf = acc.invLf;
+        const uint32_t nf = acc.nf;
+        b.lo0 = fine_coord(fminf(ox, px) - kAccelEps, invLf, nf);
+        b.lo1 = fine_coord(fminf(oy, py) - kAccelEps, invLf, nf);
+        b.lo2 = fine_coord(fminf(oz, pz) - kAccelEps, invLf, nf);
+        b.w0 = fine_coord(fmaxf(ox, px) + kAccelEps, invLf, nf) - b.lo0 + 1;
+        b.w1 = fine_coord(fmaxf(oy, py) + kAccelEps, invLf, nf) - b.lo1 + 1;
+        b.w2 = fine_coord(fmaxf(oz, pz) + kAccelEps, invLf, nf) - b.lo2 + 1;
+        b.solo = max(b.w0, max(b.w1, b.w2)) > kFlatMaxWidth;
+        const uint32_t b2 = (b.w2 > 1u) + (b.w2 > 2u), b12 = b2 + (b.w1 > 1u) + (b.w1 > 2u);
+        if (!b.solo) {
+            b.count = b.w0 << b12;
+            b.packed = (b2 << 5) | (b12 << 7) | ((b.w1 - 1u) << 10) | ((b.w2 - 1u) << 12);
+        }
     }
-    return pos;
+    return b;
+}
+
+// fills the rank table of the lanes' boxes; returns the elements in all.  first:
+// the lane's first element
+__device__ __forceinline__ uint32_t flat_items(FlatWarp& H, const FlatBox& b, uint32_t lane, uint32_t& first) {
+    const uint32_t incl = warp_incl_scan(b.count, lane);
+    first = incl - b.count;
+    const uint32_t some = __ballot_sync(0xFFFFFFFFu, b.count > 0);
+    if (b.count > 0) H.src[__popc(some & ((1u << lane) - 1u))] = lane | b.packed | (first << 14);
+    return __shfl_sync(0xFFFFFFFFu, incl, 31);
+}
+
+// element m's owner and cell offset in its box; false beyond the box
+__device__ __forceinline__ bool flat_cell(uint32_t src, uint32_t m, uint32_t& ow, uint32_t& ix, uint32_t& iy,
+                                          uint32_t& iz) {
+    const uint32_t q = m - (src >> 14), b2 = (src >> 5) & 3u, b12 = (src >> 7) & 7u;
+    ow = src & 31u;
+    ix = q >> b12;
+    iy = (q & ((1u << b12) - 1u)) >> b2;
+    iz = q & ((1u << b2) - 1u);
+    return (iy <= ((src >> 10) & 3u)) & (iz <= ((src >> 12) & 3u));
+}
+
+// The round's records, window by window (one per warp; the members are
+// warp-uniform but for first, cells, start, cnt and b0).  Cells are looked up 32
+// at a time (flat_cell, cell_records); those with records left wait in H.cell
+// until 32 of them (or the last) make a block, whose records form one flat
+// list: so windows are full but for a block's last.
+struct FlatList {
+    uint32_t itotal, first, cells;  // elements in all; the lane's first one and their number
+    uint32_t ib, before;            // next element; boxes begun before it
+    uint32_t nq;                    // cells waiting
+    uint32_t rb, total, from;       // next record of the block, records in it, its cells begun before rb
+    uint32_t start, cnt, b0;        // lane's cell of the block: first record in the flat list, count, record index
+};
+__device__ __forceinline__ FlatList flat_list(FlatWarp& H, const FlatBox& b, uint32_t lane) {
+    FlatList l;
+    l.cells = b.count;
+    l.itotal = flat_items(H, b, lane, l.first);
+    l.ib = l.before = l.nq = l.rb = l.total = l.from = l.start = l.cnt = l.b0 = 0;
+    return l;
+}
+// Makes the next block when the current one's records are used up; false when
+// no record is left.  at(owner, O): the owner's absolute start.
+template <class At>
+__device__ __forceinline__ bool flat_next(FlatWarp& H, FlatList& l, const AccelDev& acc, uint32_t lane, At at) {
+    const uint32_t below = (1u << lane) - 1u;
+    while (l.rb >= l.total && (l.ib < l.itotal || l.nq > 0)) {
+        if (l.ib < l.itotal && l.nq < 32) {
+            const uint32_t begun = flat_starts(l.cells > 0, l.first, l.ib);
+            const uint32_t src = H.src[l.before + __popc(begun & (below * 2u + 1u)) - 1u];
+            l.before += __popc(begun);
+            uint32_t b0 = 0, cnt = 0, ow, ix, iy, iz;
+            if (flat_cell(src, l.ib + lane, ow, ix, iy, iz) && l.ib + lane < l.itotal) {
+                const float4 D = H.d[ow];
+                const float4 O = at(ow, H.o[ow]);
+                const uint32_t bx = __float_as_uint(D.w);
+                cell_records(acc, (bx & 1023u) + ix, ((bx >> 10) & 1023u) + iy, (bx >> 20) + iz, O.x, O.y, O.z, D.x,
+                             D.y, D.z, b0, cnt);
+            }
+            const uint32_t some = __ballot_sync(0xFFFFFFFFu, cnt > 0);
+            if (cnt > 0) H.cell[l.nq + __popc(some & below)] = make_uint2(b0, ow | (cnt << 5));
+            l.nq += __popc(some);
+            l.ib += 32;
+            __syncwarp();
+        } else {
+            const uint32_t k = min(l.nq, 32u);
+            l.nq -= k;
+            const uint2 c = lane < k ? H.cell[l.nq + lane] : make_uint2(0u, 0u);
+            l.b0 = c.x;
+            l.cnt = c.y >> 5;
+            const uint32_t incl = warp_incl_scan(l.cnt, lane);
+            l.start = incl - l.cnt;
+            l.total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+            l.rb = l.from = 0;
+            if (lane < k) H.cell[l.nq + lane] = make_uint2(c.x - l.start, c.y & 31u);  // record - flat index, owner
+            __syncwarp();
+        }
+    }
+    return l.rb < l.total;
+}
+// record e and owner o of flat record base + lane (call in ascending order of
+// base; all lanes; meaningless past the block's total)
+__device__ __forceinline__ void flat_pick(const FlatWarp& H, FlatList& l, uint32_t lane, uint32_t base, uint32_t& e,
+                                          uint32_t& o) {
+    const uint32_t begun = flat_starts(l.cnt > 0, l.start, base);
+    const uint2 c = H.cell[l.nq + l.from + __popc(begun & (0xFFFFFFFFu >> (31u - lane))) - 1u];
+    l.from += __popc(begun);
+    e = c.x + base + lane;
+    o = c.y;
 }
 
 // Queue of a warp's 32-byte records that passed the plane test, as (record,
 // owner) pairs: the rest of the exact test (with its dependent loads) runs on
 // 32 of them at a time with every lane busy
-static constexpr uint32_t kFlatQueue = 64;  // at most 31 left over + 32 appended
+static constexpr uint32_t kFlatQueue = 96;  // at most 31 left over + a window of 64
 struct FlatQueue {
-    uint32_t e[kFlatQueue], o[kFlatQueue];
+    uint2 eo[kFlatQueue];
 };
 
 // one 32-byte record already in registers against a sub-segment
-__device__ __forceinline__ bool test_wide_loaded(const MeshDev& g, float4 q, float4 pt, uint32_t excl,
-                                                 float ox, float oy, float oz, float dx, float dy,
-                                                 float dz, FastHit& h) {
-    if (!plane_may_cross(q, ox, oy, oz, dx, dy, dz)) return false;
-    if (__float_as_uint(pt.w) == excl) return false;
-    return test_split(g, q, pt, ox, oy, oz, dx, dy, dz, h);
+__device__ __forceinline__ bool test_wide_loaded(const MeshDev& g, float4 q, float4 pt, float4 O, float4 D,
+                                                 FastHit& h) {
+    if (!plane_may_cross(q, O.x, O.y, O.z, D.x, D.y, D.z)) return false;
+    if (__float_as_uint(pt.w) == __float_as_uint(O.w)) return false;
+    return test_split(g, q, pt, O.x, O.y, O.z, D.x, D.y, D.z, h);
 }
 
 // Staging of 32-byte records in shared memory by bulk copies (the TMA engine,
@@ -150,28 +284,80 @@ __device__ __forceinline__ bool stage_wait(FlatStage* P, uint32_t buf) {
 __device__ __forceinline__ void flat_test_queued(FlatWarp& H, const MeshDev& g, const AccelDev& acc, uint32_t e,
                                                  uint32_t o) {
     const float4 q = __ldg(&acc.recw[e].q), pt = __ldg(&acc.recw[e].pt);
+    const float4 O = H.o[o], D = H.d[o];
     FastHit h;
-    if (test_split(g, q, pt, H.ox[o], H.oy[o], H.oz[o], H.dx[o], H.dy[o], H.dz[o], h)) flat_file_hit(H, o, h);
+    if (__float_as_uint(pt.w) != __float_as_uint(O.w) && test_split(g, q, pt, O.x, O.y, O.z, D.x, D.y, D.z, h))
+        flat_file_hit(H, o, h);
 }
 
-// appends the lanes' surviving (e, o) to the queue (qn: warp-uniform length)
-// and tests full groups of 32 from its top; all lanes call it
+// appends the lanes' surviving pairs to the queue (qn: warp-uniform length) and
+// tests full groups of 32 from its top, with `last` (warp-uniform) the partial
+// group too: one copy of the exact test a round
 __device__ __forceinline__ void flat_enqueue(FlatWarp& H, FlatQueue& Q, const MeshDev& g, const AccelDev& acc,
-                                             uint32_t lane, bool live, uint32_t e, uint32_t o, uint32_t& qn) {
-    const uint32_t b = __ballot_sync(0xFFFFFFFFu, live);
-    if (live) {
-        const uint32_t at = qn + __popc(b & ((1u << lane) - 1u));
-        Q.e[at] = e; Q.o[at] = o;
-    }
-    qn += __popc(b);
+                                             uint32_t lane, bool s0, uint32_t e0, uint32_t o0, bool s1, uint32_t e1,
+                                             uint32_t o1, uint32_t& qn, bool last) {
+    const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, s0), b1 = __ballot_sync(0xFFFFFFFFu, s1);
+    const uint32_t below = (1u << lane) - 1u;
+    if (s0) Q.eo[qn + __popc(b0 & below)] = make_uint2(e0, o0);
+    qn += __popc(b0);
+    if (s1) Q.eo[qn + __popc(b1 & below)] = make_uint2(e1, o1);
+    qn += __popc(b1);
     __syncwarp();
-    while (qn >= 32) {
-        const uint32_t at = qn - 32 + lane;
-        const uint32_t eq = Q.e[at], oq = Q.o[at];
+    while (qn >= 32 || (last && qn > 0)) {
+        const uint32_t k = min(qn, 32u);
+        qn -= k;
+        if (lane < k) flat_test_queued(H, g, acc, Q.eo[qn + lane].x, Q.eo[qn + lane].y);
         __syncwarp();
-        qn -= 32;
-        flat_test_queued(H, g, acc, eq, oq);
     }
+}
+
+// A lane whose box is too wide for the warp's list: its own records, cell by
+// cell (rare, and out of line so that the box's corners need not be kept)
+static __device__ __noinline__ void flat_solo(FlatWarp& H, const MeshDev& g, const AccelDev& acc, uint32_t lane,
+                                              float px, float py, float pz) {
+    const float4 O = H.o[lane], D = H.d[lane];
+    const FlatBox b = flat_box(acc, true, O.x, O.y, O.z, px, py, pz);
+    for (uint32_t ix = 0; ix < b.w0; ix++)
+        for (uint32_t iy = 0; iy < b.w1; iy++)
+            for (uint32_t iz = 0; iz < b.w2; iz++) {
+                const uint32_t key = morton3(b.lo0 + ix, b.lo1 + iy, b.lo2 + iz);
+                const uint32_t b0 = __ldg(acc.start + key), b1 = __ldg(acc.start + key + 1);
+                for (uint32_t k = b0; k < b1; k++) {
+                    FastHit h;
+                    if (test_entry(g, acc, k, __float_as_uint(O.w), O.x, O.y, O.z, D.x, D.y, D.z, h))
+                        flat_file_hit(H, lane, h);
+                }
+            }
+}
+
+// Are the lane's n filed hits one hit (filed once per fine cell that lists its
+// triangle), at (x, y, z), that needs no walk?  Then it is the reference's.
+__device__ __forceinline__ bool flat_only_hit(const FlatWarp& H, uint32_t lane, uint32_t n, uint32_t gn, float x,
+                                              float y, float z) {
+    const uint32_t t = H.t[0][lane];
+    bool one = n <= (uint32_t)kFlatSlots && !(H.type[0][lane] & kHitWalk);
+    if (n > 1) one = one && H.t[1][lane] == t && (n < 3 || H.t[2][lane] == t) && (n < 4 || H.t[3][lane] == t);
+    const float inv = 0.5f * (float)gn, margin = 2.0f * kRegularEps * inv;
+    return one & clear_of_faces(x, inv, margin) & clear_of_faces(y, inv, margin) & clear_of_faces(z, inv, margin);
+}
+// The slot of the reference's hit among several (n <= kFlatSlots) by the walk
+// over its cells, kNoPlace for none.  About one hit in ten needs it: out of
+// line, so that a round keeps neither its registers nor its code.
+static __device__ __noinline__ uint32_t flat_choose(const FlatWarp& H, const MeshDev& g, uint32_t lane, uint32_t n,
+                                                    RefWalk w) {
+    uint32_t bq = kNoPlace, bt = 0, bplace = kNoPlace;
+    for (uint32_t q = 0; q < n; q++) {
+        const uint32_t t = H.t[q][lane];
+        if (bq != kNoPlace && t == bt) continue;  // filed from another fine cell too
+        const uint32_t place = first_place(g, w, __ldg(g.tri_cells + t), t);
+        if (place == kNoPlace) continue;
+        const float d2 = H.d2[q][lane];
+        if (place < bplace ||
+            (place == bplace && (d2 < H.d2[bq][lane] || (d2 == H.d2[bq][lane] && t < bt)))) {
+            bq = q; bplace = place; bt = t;
+        }
+    }
+    return bq;
 }
 
 // One round for every lane of the warp (all 32 lanes call it).  open: the lane
@@ -187,84 +373,55 @@ __device__ __forceinline__ void flat_round_mode(FlatWarp& H, const MeshDev& g, c
                                                 float px, float py, float pz, uint32_t excluded,
                                                 bool& found, FastHit& best, FlatQueue* Q = nullptr,
                                                 FlatStage* P = nullptr) {
-    const uint32_t FULL = 0xFFFFFFFFu;
-    const float invLf = acc.invLf;
-    const uint32_t nf = acc.nf;
-    float dx = px - ox, dy = py - oy, dz = pz - oz;
-    uint32_t lo0 = 0, lo1 = 0, lo2 = 0, w0 = 0, w1 = 0, w2 = 0, nc = 0;
-    if (open) {
-        lo0 = fine_coord(fminf(ox, px) - kAccelEps, invLf, nf);
-        lo1 = fine_coord(fminf(oy, py) - kAccelEps, invLf, nf);
-        lo2 = fine_coord(fminf(oz, pz) - kAccelEps, invLf, nf);
-        w0 = fine_coord(fmaxf(ox, px) + kAccelEps, invLf, nf) - lo0 + 1;
-        w1 = fine_coord(fmaxf(oy, py) + kAccelEps, invLf, nf) - lo1 + 1;
-        w2 = fine_coord(fmaxf(oz, pz) + kAccelEps, invLf, nf) - lo2 + 1;
-        nc = w0 * w1 * w2;
-    }
-    const bool solo = open && nc > (uint32_t)kFlatMaxItems;
-    const uint32_t ncw = (open && !solo) ? nc : 0u;
-    H.ox[lane] = ox; H.oy[lane] = oy; H.oz[lane] = oz;
-    H.dx[lane] = dx; H.dy[lane] = dy; H.dz[lane] = dz;
-    H.excl[lane] = excluded;
-    H.box[lane] = lo0 | (lo1 << 10) | (lo2 << 20);
-    H.wd[lane] = w0 | (w1 << 8) | (w2 << 16);
+    const float dx = px - ox, dy = py - oy, dz = pz - oz;
+    const FlatBox box = flat_box(acc, open, ox, oy, oz, px, py, pz);
+    H.o[lane] = make_float4(ox, oy, oz, __uint_as_float(excluded));
+    H.d[lane] = make_float4(dx, dy, dz, __uint_as_float(box.lo0 | (box.lo1 << 10) | (box.lo2 << 20)));
     H.n[lane] = 0;
-    const uint32_t iincl = warp_incl_scan(ncw, lane);
-    const uint32_t iexcl = iincl - ncw;
-    const uint32_t itotal = __shfl_sync(FULL, iincl, 31);
-    uint32_t qn = 0;  // queue length (warp-uniform)
+    FlatList l = flat_list(H, box, lane);
     __syncwarp();
-    // pass 1: 32 items at a time, one cell-range load per lane
-    for (uint32_t ib = 0; ib < itotal; ib += 32) {
-        const uint32_t m = ib + lane;
-        const uint32_t ow = min(warp_find(iincl, m), 31u);
-        const uint32_t ofs = __shfl_sync(FULL, iexcl, ow);
-        uint32_t b0 = 0, cnt = 0;
-        if (m < itotal) {
-            const uint32_t q = m - ofs;
-            const uint32_t wd = H.wd[ow], bx = H.box[ow];
-            const uint32_t ww1 = (wd >> 8) & 0xFFu, ww2 = wd >> 16;
-            const uint32_t iz = q % ww2, r = q / ww2, iy = r % ww1, ix = r / ww1;
-            cell_records(acc, (bx & 1023u) + ix, ((bx >> 10) & 1023u) + iy, (bx >> 20) + iz, H.ox[ow], H.oy[ow],
-                         H.oz[ow], H.dx[ow], H.dy[ow], H.dz[ow], b0, cnt);
-        }
-        // pass 2: the items' records, concatenated over the warp
-        const uint32_t rincl = warp_incl_scan(cnt, lane);
-        const uint32_t rtotal = __shfl_sync(FULL, rincl, 31);
-        const uint32_t rbase = b0 - (rincl - cnt);  // record index = rbase of its item + flat index
-        if (LAYOUT == 2 || (LAYOUT == 0 && acc.wide == 2)) {
-            for (uint32_t rb = 0; rb < rtotal; rb += 64) {
-                const uint32_t r0 = rb + lane, r1 = rb + 32 + lane;
-                const uint32_t j0 = min(warp_find(rincl, r0), 31u);
-                const uint32_t j1 = min(warp_find(rincl, r1), 31u);
-                const uint32_t e0 = __shfl_sync(FULL, rbase, j0) + r0;
-                const uint32_t e1 = __shfl_sync(FULL, rbase, j1) + r1;
-                const uint32_t o0 = __shfl_sync(FULL, ow, j0);
-                const uint32_t o1 = __shfl_sync(FULL, ow, j1);
-                const bool v0 = r0 < rtotal, v1 = r1 < rtotal;
-                AccelRecFull f0, f1;
-                if (v0) f0 = load_full(acc.recf + e0);
-                if (v1) f1 = load_full(acc.recf + e1);
-                FastHit h;
-                if (v0 && test_full(f0, H.excl[o0], H.ox[o0], H.oy[o0], H.oz[o0], H.dx[o0], H.dy[o0], H.dz[o0], h))
-                    flat_file_hit(H, o0, h);
-                if (v1 && test_full(f1, H.excl[o1], H.ox[o1], H.oy[o1], H.oz[o1], H.dx[o1], H.dy[o1], H.dz[o1], h))
-                    flat_file_hit(H, o1, h);
+    auto at = [](uint32_t, float4 O) { return O; };
+    if (LAYOUT == 1 && Q) {
+        // records past the plane test are queued and finished 32 at a time
+        uint32_t qn = 0;
+        for (;;) {
+            const bool more = flat_next(H, l, acc, lane, at);  // warp-uniform
+            bool s0 = false, s1 = false;
+            uint32_t e0 = 0, e1 = 0, o0 = 0, o1 = 0;
+            if (more) {
+                flat_pick(H, l, lane, l.rb, e0, o0);
+                flat_pick(H, l, lane, l.rb + 32, e1, o1);
+                s0 = l.rb + lane < l.total;
+                s1 = l.rb + 32 + lane < l.total;
+                float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
+                if (s0) q0 = __ldg(&acc.recw[e0].q);
+                if (s1) q1 = __ldg(&acc.recw[e1].q);
+                if (s0) {
+                    const float4 O = H.o[o0], D = H.d[o0];
+                    s0 = plane_may_cross(q0, O.x, O.y, O.z, D.x, D.y, D.z);
+                }
+                if (s1) {
+                    const float4 O = H.o[o1], D = H.d[o1];
+                    s1 = plane_may_cross(q1, O.x, O.y, O.z, D.x, D.y, D.z);
+                }
+                l.rb += 64;
             }
-        } else if (LAYOUT == 1 && P) {
+            flat_enqueue(H, *Q, g, acc, lane, s0, e0, o0, s1, e1, o1, qn, !more);
+            if (!more) break;
+        }
+    } else if (LAYOUT == 1 && P) {
+        while (flat_next(H, l, acc, lane, at)) {
             // windows of kStageRecs records staged by bulk copies, the next one in
-            // flight while this one is tested; lane k's cell holds the flat
-            // records [rincl - cnt, rincl) at global index b0
-            const uint32_t nwin = (rtotal + kStageRecs - 1) / kStageRecs;
-            const uint32_t rexcl = rincl - cnt;
+            // flight while this one is tested
+            const uint32_t nwin = (l.total + kStageRecs - 1) / kStageRecs;
             auto issue = [&](uint32_t w, uint32_t buf) {
-                const uint32_t lo = w * kStageRecs, hi = min(lo + kStageRecs, rtotal);
+                const uint32_t lo = w * kStageRecs, hi = min(lo + kStageRecs, l.total);
                 if (lane == 0) stage_expect(P, buf, (hi - lo) * 32u);
                 __syncwarp();
-                const uint32_t a = max(rexcl, lo), z = min(rincl, hi);
-                if (a < z) stage_copy(P, buf, a - lo, acc.recw + b0 + (a - rexcl), z - a);
+                const uint32_t a = max(l.start, lo), z = min(l.start + l.cnt, hi);
+                if (a < z) stage_copy(P, buf, a - lo, acc.recw + l.b0 + (a - l.start), z - a);
             };
-            if (nwin > 0 && !P->abort) issue(0, 0);
+            if (!P->abort) issue(0, 0);
             for (uint32_t w = 0; w < nwin && !P->abort; w++) {
                 const uint32_t buf = w & 1u;
                 if (w + 1 < nwin) issue(w + 1, buf ^ 1u);
@@ -278,137 +435,67 @@ __device__ __forceinline__ void flat_round_mode(FlatWarp& H, const MeshDev& g, c
                     break;
                 }
                 if (lane == 0) P->parity[buf] ^= 1u;
-                const uint32_t lo = w * kStageRecs;
-                const uint32_t r0 = lo + lane, r1 = lo + 32 + lane;
-                const uint32_t j0 = min(warp_find(rincl, r0), 31u);
-                const uint32_t j1 = min(warp_find(rincl, r1), 31u);
-                const uint32_t o0 = __shfl_sync(FULL, ow, j0);
-                const uint32_t o1 = __shfl_sync(FULL, ow, j1);
-                FastHit h;
-                if (r0 < rtotal && test_wide_loaded(g, P->rec[buf][lane][0], P->rec[buf][lane][1], H.excl[o0],
-                                                    H.ox[o0], H.oy[o0], H.oz[o0], H.dx[o0], H.dy[o0], H.dz[o0], h))
-                    flat_file_hit(H, o0, h);
-                if (r1 < rtotal && test_wide_loaded(g, P->rec[buf][32 + lane][0], P->rec[buf][32 + lane][1],
-                                                    H.excl[o1], H.ox[o1], H.oy[o1], H.oz[o1], H.dx[o1], H.dy[o1],
-                                                    H.dz[o1], h))
-                    flat_file_hit(H, o1, h);
+#pragma unroll
+                for (uint32_t half = 0; half < 64; half += 32) {
+                    const uint32_t at0 = w * kStageRecs + half;
+                    uint32_t e, o;
+                    flat_pick(H, l, lane, at0, e, o);
+                    FastHit h;
+                    if (at0 + lane < l.total && test_wide_loaded(g, P->rec[buf][half + lane][0],
+                                                                 P->rec[buf][half + lane][1], H.o[o], H.d[o], h))
+                        flat_file_hit(H, o, h);
+                }
                 __syncwarp();  // the buffer's reads end before its next copies
             }
-        } else if (LAYOUT == 1 || (LAYOUT == 0 && acc.wide)) {
-            for (uint32_t rb = 0; rb < rtotal; rb += 64) {
-                const uint32_t r0 = rb + lane, r1 = rb + 32 + lane;
-                const uint32_t j0 = min(warp_find(rincl, r0), 31u);
-                const uint32_t j1 = min(warp_find(rincl, r1), 31u);
-                const uint32_t e0 = __shfl_sync(FULL, rbase, j0) + r0;
-                const uint32_t e1 = __shfl_sync(FULL, rbase, j1) + r1;
-                const uint32_t o0 = __shfl_sync(FULL, ow, j0);
-                const uint32_t o1 = __shfl_sync(FULL, ow, j1);
-                const bool v0 = r0 < rtotal, v1 = r1 < rtotal;
-                float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), t0 = q0, q1 = q0, t1 = q0;
-                if (v0) { q0 = __ldg(&acc.recw[e0].q); t0 = __ldg(&acc.recw[e0].pt); }
-                if (v1) { q1 = __ldg(&acc.recw[e1].q); t1 = __ldg(&acc.recw[e1].pt); }
-                if (Q) {
-                    const bool s0 = v0 && __float_as_uint(t0.w) != H.excl[o0] &&
-                                    plane_may_cross(q0, H.ox[o0], H.oy[o0], H.oz[o0], H.dx[o0], H.dy[o0], H.dz[o0]);
-                    const bool s1 = v1 && __float_as_uint(t1.w) != H.excl[o1] &&
-                                    plane_may_cross(q1, H.ox[o1], H.oy[o1], H.oz[o1], H.dx[o1], H.dy[o1], H.dz[o1]);
-                    flat_enqueue(H, *Q, g, acc, lane, s0, e0, o0, qn);
-                    flat_enqueue(H, *Q, g, acc, lane, s1, e1, o1, qn);
-                    continue;
-                }
+            l.rb = l.total;
+        }
+    } else {
+        // tested in place
+        while (flat_next(H, l, acc, lane, at)) {
+            uint32_t e, o;
+            flat_pick(H, l, lane, l.rb, e, o);
+            if (l.rb + lane < l.total) {
+                const float4 O = H.o[o], D = H.d[o];
+                const uint32_t excl = __float_as_uint(O.w);
                 FastHit h;
-                if (v0 && test_wide_loaded(g, q0, t0, H.excl[o0], H.ox[o0], H.oy[o0], H.oz[o0],
-                                           H.dx[o0], H.dy[o0], H.dz[o0], h))
-                    flat_file_hit(H, o0, h);
-                if (v1 && test_wide_loaded(g, q1, t1, H.excl[o1], H.ox[o1], H.oy[o1], H.oz[o1],
-                                           H.dx[o1], H.dy[o1], H.dz[o1], h))
-                    flat_file_hit(H, o1, h);
+                bool hit;
+                if (LAYOUT == 2 || (LAYOUT == 0 && acc.wide == 2))
+                    hit = test_full(load_full(acc.recf + e), excl, O.x, O.y, O.z, D.x, D.y, D.z, h);
+                else if (LAYOUT == 1 || acc.wide == 1)
+                    hit = test_wide_loaded(g, __ldg(&acc.recw[e].q), __ldg(&acc.recw[e].pt), O, D, h);
+                else
+                    hit = test_narrow(g, acc, e, excl, O.x, O.y, O.z, D.x, D.y, D.z, h);
+                if (hit) flat_file_hit(H, o, h);
             }
-        } else if (LAYOUT == 0) {
-            for (uint32_t rb = 0; rb < rtotal; rb += 32) {
-                const uint32_t r0 = rb + lane;
-                const uint32_t j0 = min(warp_find(rincl, r0), 31u);
-                const uint32_t e0 = __shfl_sync(FULL, rbase, j0) + r0;
-                const uint32_t o0 = __shfl_sync(FULL, ow, j0);
-                FastHit h;
-                if (r0 < rtotal && test_narrow(g, acc, e0, H.excl[o0], H.ox[o0], H.oy[o0], H.oz[o0],
-                                               H.dx[o0], H.dy[o0], H.dz[o0], h))
-                    flat_file_hit(H, o0, h);
-            }
+            l.rb += 32;
+            __syncwarp();
         }
     }
-    if (Q && lane < qn) flat_test_queued(H, g, acc, Q->e[lane], Q->o[lane]);  // the queue's remainder
-    // boxes of more than kFlatMaxItems cells (long sub-segments): the owner alone
-    if (solo) {
-        for (uint32_t q = 0; q < nc; q++) {
-            uint32_t iz = q % w2, r = q / w2, iy = r % w1, ix = r / w1;
-            uint32_t key = morton3(lo0 + ix, lo1 + iy, lo2 + iz);
-            uint32_t b0 = __ldg(acc.start + key), b1 = __ldg(acc.start + key + 1);
-            for (uint32_t k = b0; k < b1; k++) {
-                FastHit h;
-                if (test_entry(g, acc, k, excluded, ox, oy, oz, dx, dy, dz, h)) flat_file_hit(H, lane, h);
-            }
-        }
-    }
+    // wider boxes (long sub-segments): the owner alone
+    if (box.solo) flat_solo(H, g, acc, lane, px, py, pz);
     __syncwarp();
     found = false;
     if (!open) return;
     const uint32_t n = H.n[lane];
-    if (n > (uint32_t)kFlatSlots) {
-        ref_scan(g, ox, oy, oz, px, py, pz, excluded, best, found);
-    } else if (n > 0) {
-        // the reference's traversal of its grid over the hits filed in
-        // this lane's slots (a triangle filed twice from two fine cells
-        // is the same hit)
+    if (n == 0) return;
+    uint32_t bq = 0;
+    found = true;
+    if (!flat_only_hit(H, lane, n, g.n, H.x[0][lane], H.y[0][lane], H.z[0][lane])) {
+        if (n > (uint32_t)kFlatSlots) {
+            ref_scan(g, ox, oy, oz, px, py, pz, excluded, best, found);
+            return;
+        }
         const uint32_t gn = g.n;
         const float L = g.L;
-        uint32_t sx = ref_coord(ox, L, gn), sy = ref_coord(oy, L, gn), sz = ref_coord(oz, L, gn);
-        uint32_t tx = ref_coord(px, L, gn), ty = ref_coord(py, L, gn), tz = ref_coord(pz, L, gn);
-        uint32_t ix = (uint32_t)((int)(tx > sx) - (int)(tx < sx));
-        uint32_t iy = (uint32_t)((int)(ty > sy) - (int)(ty < sy));
-        uint32_t iz = (uint32_t)((int)(tz > sz) - (int)(tz < sz));
-        uint32_t bq = 0;
-        // each hit's reference cells, loaded together before the walk
-        uint4 hc[kFlatSlots];
-#pragma unroll
-        for (int q = 0; q < kFlatSlots; q++)
-            hc[q] = ((uint32_t)q < n) ? hit_cells(g, H.t[q][lane]) : make_uint4(kCellNone, kCellNone, kCellNone, kCellNone);
-        uint32_t cx = sx;
-        do {
-            uint32_t cy = sy;
-            do {
-                uint32_t cz = sz;
-                do {
-                    uint32_t c = gn * gn * cz + gn * cy + cx;
-#pragma unroll
-                    for (uint32_t q = 0; q < (uint32_t)kFlatSlots; q++) {
-                        if (q >= n) break;
-                        const uint32_t t = H.t[q][lane];
-                        if (!hit_in_cell(g, hc[q], c, t)) continue;
-                        const float d2 = H.d2[q][lane];
-                        if (!found || d2 < H.d2[bq][lane] || (d2 == H.d2[bq][lane] && t < H.t[bq][lane])) {
-                            bq = q;
-                            found = true;
-                        }
-                    }
-                    cz += iz;
-                } while ((cz != tz + iz) && !found);
-                cy += iy;
-            } while ((cy != ty + iy) && !found);
-            cx += ix;
-        } while ((cx != tx + ix) && !found);
-        if (found) {
-            best.t = H.t[bq][lane]; best.type = H.type[bq][lane]; best.d2 = H.d2[bq][lane];
-            best.x = H.x[bq][lane]; best.y = H.y[bq][lane]; best.z = H.z[bq][lane];
-        }
+        bq = flat_choose(H, g, lane, n,
+                         ref_walk(ref_coord(ox, L, gn), ref_coord(oy, L, gn), ref_coord(oz, L, gn),
+                                  ref_coord(px, L, gn), ref_coord(py, L, gn), ref_coord(pz, L, gn)));
+        found = bq != kNoPlace;
     }
-}
-
-// every record layout
-__device__ __forceinline__ void flat_round(FlatWarp& H, const MeshDev& g, const AccelDev& acc, uint32_t lane,
-                                           bool open, float ox, float oy, float oz, float px, float py, float pz,
-                                           uint32_t excluded, bool& found, FastHit& best) {
-    flat_round_mode<0>(H, g, acc, lane, open, ox, oy, oz, px, py, pz, excluded, found, best);
+    if (found) {
+        best.t = H.t[bq][lane]; best.type = H.type[bq][lane] & ~kHitWalk; best.d2 = H.d2[bq][lane];
+        best.x = H.x[bq][lane]; best.y = H.y[bq][lane]; best.z = H.z[bq][lane];
+    }
 }
 
 // Reflection or permeation at the round's hit `best`: the permeation interval

@@ -60,9 +60,10 @@ __device__ __forceinline__ void record_load(const AccelDev& acc, uint32_t k, boo
 // meet the sub-segment?  (na: n.p1 - n.origin - n.offset; margin as
 // plane_may_cross)
 __device__ __forceinline__ bool local_plane(const FlatWarp& H, const LocalWarp& Lw, float4 q, uint32_t o) {
-    const float den = q.x * H.dx[o] + q.y * H.dy[o] + q.z * H.dz[o];
+    const float4 O = H.o[o], D = H.d[o];
+    const float den = q.x * D.x + q.y * D.y + q.z * D.z;
     const float na = (q.w - (q.x * Lw.gx[o] + q.y * Lw.gy[o] + q.z * Lw.gz[o])) -
-                     (q.x * H.ox[o] + q.y * H.oy[o] + q.z * H.oz[o]);
+                     (q.x * O.x + q.y * O.y + q.z * O.z);
     return (den > 0.0f) ? ((na > -kPlaneMargin) & (na < den + kPlaneMargin))
                         : ((den < 0.0f) & (na < kPlaneMargin) & (na > den - kPlaneMargin)) |
                               ((den == 0.0f) & (fabsf(na) < kPlaneMargin));
@@ -74,8 +75,9 @@ __device__ __forceinline__ bool local_fp64(const FlatWarp& H, const LocalWarp& L
                                            uint32_t o, FastHit& h, PrecCount& pc) {
     pc.exact++;
     const float gx = Lw.gx[o], gy = Lw.gy[o], gz = Lw.gz[o];
-    const float dx = H.dx[o], dy = H.dy[o], dz = H.dz[o];
-    const double Ox = (double)gx + (double)H.ox[o], Oy = (double)gy + (double)H.oy[o], Oz = (double)gz + (double)H.oz[o];
+    const float4 O = H.o[o], D = H.d[o];
+    const float dx = D.x, dy = D.y, dz = D.z;
+    const double Ox = (double)gx + (double)O.x, Oy = (double)gy + (double)O.y, Oz = (double)gz + (double)O.z;
     double r64;
     uint32_t type;
     if (!tri_test64(g.tri64, t, Ox, Oy, Oz, (double)dx, (double)dy, (double)dz, r64, type)) return false;
@@ -84,7 +86,7 @@ __device__ __forceinline__ bool local_fp64(const FlatWarp& H, const LocalWarp& L
     h.t = t;
     h.x = (float)(hx - (double)gx); h.y = (float)(hy - (double)gy); h.z = (float)(hz - (double)gz);
     h.d2 = (float)d2;
-    h.type = type;
+    h.type = type | hit_walk(__ldg(&g.plane[t].vv));
     return true;
 }
 
@@ -96,7 +98,8 @@ __device__ __forceinline__ bool local_test_core(const FlatWarp& H, const LocalWa
                                                 float3 p1, uint32_t t, uint32_t o, FastHit& h, PrecCount& pc,
                                                 bool defer, bool& deferred) {
     const float gx = Lw.gx[o], gy = Lw.gy[o], gz = Lw.gz[o];
-    const float ox = H.ox[o], oy = H.oy[o], oz = H.oz[o], dx = H.dx[o], dy = H.dy[o], dz = H.dz[o];
+    const float4 O = H.o[o], D = H.d[o];
+    const float ox = O.x, oy = O.y, oz = O.z, dx = D.x, dy = D.y, dz = D.z;
     const float ax = p1.x - gx, ay = p1.y - gy, az = p1.z - gz;
     const float bx = ax - ox, by = ay - oy, bz = az - oz;
     const float num = q.x * bx + q.y * by + q.z * bz;
@@ -113,7 +116,7 @@ __device__ __forceinline__ bool local_test_core(const FlatWarp& H, const LocalWa
         r = num / den;
         const float4* bb = reinterpret_cast<const float4*>(g.bary + t);
         const float4 u4 = __ldg(bb), v4 = __ldg(bb + 1);
-        const float vv = __ldg(&g.plane[t].vv);
+        const float vs = __ldg(&g.plane[t].vv), vv = fabsf(vs);
         const float uv = v4.z, uu = v4.w;
         const float wx = ox + r * dx - ax, wy = oy + r * dy - ay, wz = oz + r * dz - az;
         const float wu = wx * u4.x + wy * u4.y + wz * u4.z;
@@ -128,7 +131,7 @@ __device__ __forceinline__ bool local_test_core(const FlatWarp& H, const LocalWa
             h.t = t;
             h.x = ox + dx * r; h.y = oy + dy * r; h.z = oz + dz * r;
             h.d2 = (ox - h.x) * (ox - h.x) + (oy - h.y) * (oy - h.y) + (oz - h.z) * (oz - h.z);
-            h.type = 1u | kLocalRefine;
+            h.type = 1u | kLocalRefine | hit_walk(vs);
             return true;
         }
     }
@@ -322,56 +325,50 @@ __device__ __forceinline__ void local_enqueue(FlatWarp& H, LocalWarp& Lw, const 
 // A lane whose cell box is too large for the warp's flattened pass: its own
 // records, cell by cell.
 __device__ __noinline__ void local_solo(FlatWarp& H, LocalWarp& Lw, const MeshDev& g, const AccelDev& acc, bool full,
-                                        uint32_t lane, uint32_t lo0, uint32_t lo1, uint32_t lo2, uint32_t w1,
-                                        uint32_t w2, uint32_t nc, uint32_t excluded, PrecCount& pc) {
-    for (uint32_t q = 0; q < nc; q++) {
-        const uint32_t iz = q % w2, r = q / w2, iy = r % w1, ix = r / w1;
-        const uint32_t key = morton3(lo0 + ix, lo1 + iy, lo2 + iz);
-        const uint32_t b0 = __ldg(acc.start + key), b1 = __ldg(acc.start + key + 1);
-        for (uint32_t k = b0; k < b1; k++) {
-            float4 qq; float3 p1; uint32_t t;
-            record_load(acc, k, full, qq, p1, t);
-            pc.records++;
-            if (t == excluded || !local_plane(H, Lw, qq, lane)) continue;
-            FastHit h;
-            if (local_test(H, Lw, g, acc, k, full, lane, h, pc)) flat_file_hit(H, lane, h);
-        }
-    }
+                                        uint32_t lane, float apx, float apy, float apz, PrecCount& pc) {
+    const float4 O = H.o[lane];
+    const FlatBox b = flat_box(acc, true, Lw.gx[lane] + O.x, Lw.gy[lane] + O.y, Lw.gz[lane] + O.z, apx, apy, apz);
+    for (uint32_t ix = 0; ix < b.w0; ix++)
+        for (uint32_t iy = 0; iy < b.w1; iy++)
+            for (uint32_t iz = 0; iz < b.w2; iz++) {
+                const uint32_t key = morton3(b.lo0 + ix, b.lo1 + iy, b.lo2 + iz);
+                const uint32_t b0 = __ldg(acc.start + key), b1 = __ldg(acc.start + key + 1);
+                for (uint32_t k = b0; k < b1; k++) {
+                    float4 qq; float3 p1; uint32_t t;
+                    record_load(acc, k, full, qq, p1, t);
+                    pc.records++;
+                    if (t == __float_as_uint(O.w) || !local_plane(H, Lw, qq, lane)) continue;
+                    FastHit h;
+                    if (local_test(H, Lw, g, acc, k, full, lane, h, pc)) flat_file_hit(H, lane, h);
+                }
+            }
 }
 
 // A lane whose hit slots overflowed: every triangle of the reference cells
 // from the start cell s towards the end cell t, in order, stopping at the
 // first cell with a hit (the reference's cell walk); returns found.
-__device__ __noinline__ bool local_overflow(FlatWarp& H, LocalWarp& Lw, const MeshDev& g, uint32_t lane, uint32_t sx,
-                                            uint32_t sy, uint32_t sz, uint32_t tx, uint32_t ty, uint32_t tz,
-                                            uint32_t ix, uint32_t iy, uint32_t iz, uint32_t excluded, FastHit& best,
-                                            PrecCount& pc) {
+__device__ __noinline__ bool local_overflow(FlatWarp& H, LocalWarp& Lw, const MeshDev& g, uint32_t lane, RefWalk w,
+                                            uint32_t excluded, FastHit& best, PrecCount& pc) {
     const uint32_t gn = g.n;
-    bool found = false;
-    uint32_t cx = sx;
-    do {
-        uint32_t cy = sy;
-        do {
-            uint32_t cz = sz;
-            do {
-                const uint32_t c = gn * gn * cz + gn * cy + cx;
+    for (uint32_t ax = 0; ax < w.nx; ax++)
+        for (uint32_t ay = 0; ay < w.ny; ay++)
+            for (uint32_t az = 0; az < w.nz; az++) {
+                const uint32_t c = gn * gn * (w.sz + (uint32_t)w.iz * az) + gn * (w.sy + (uint32_t)w.iy * ay) + w.sx +
+                                   (uint32_t)w.ix * ax;
                 const uint32_t c0 = __ldg(g.cell_start + c), c1 = __ldg(g.cell_start + c + 1);
                 float bd2 = 400000000.0f;
+                bool found = false;
                 for (uint32_t k = c0; k < c1; k++) {
                     const uint32_t t = __ldg(g.cell_tri + k);
                     if (t == excluded) continue;
                     FastHit h;
                     if (local_test_tri(H, Lw, g, t, lane, h, pc) && h.d2 < bd2) {
-                        bd2 = h.d2; best = h; found = true;
+                        bd2 = h.d2; best = h; best.type &= ~kHitWalk; found = true;
                     }
                 }
-                cz += iz;
-            } while ((cz != tz + iz) && !found);
-            cy += iy;
-        } while ((cy != ty + iy) && !found);
-        cx += ix;
-    } while ((cx != tx + ix) && !found);
-    return found;
+                if (found) return true;
+            }
+    return false;
 }
 
 // One collision round of the local form for every lane of the warp (all 32
@@ -384,87 +381,44 @@ __device__ __forceinline__ void local_round(FlatWarp& H, LocalWarp& Lw, const Me
                                             uint32_t lane, bool open, float gx, float gy, float gz, float ox,
                                             float oy, float oz, float px, float py, float pz, uint32_t excluded,
                                             bool& found, FastHit& best, PrecCount& pc) {
-    const uint32_t FULL = 0xFFFFFFFFu;
     const bool full = LAYOUT == 0 ? acc.wide == 2 : LAYOUT == 2;  // LAYOUT 1 / 2: one record path compiled
-    const float invLf = acc.invLf;
-    const uint32_t nf = acc.nf;
     const float dx = px - ox, dy = py - oy, dz = pz - oz;
     // absolute FP32 end points for the grid lookups
     const float aox = gx + ox, aoy = gy + oy, aoz = gz + oz;
     const float apx = gx + px, apy = gy + py, apz = gz + pz;
-    uint32_t lo0 = 0, lo1 = 0, lo2 = 0, w0 = 0, w1 = 0, w2 = 0, nc = 0;
-    if (open) {
-        lo0 = fine_coord(fminf(aox, apx) - kAccelEps, invLf, nf);
-        lo1 = fine_coord(fminf(aoy, apy) - kAccelEps, invLf, nf);
-        lo2 = fine_coord(fminf(aoz, apz) - kAccelEps, invLf, nf);
-        w0 = fine_coord(fmaxf(aox, apx) + kAccelEps, invLf, nf) - lo0 + 1;
-        w1 = fine_coord(fmaxf(aoy, apy) + kAccelEps, invLf, nf) - lo1 + 1;
-        w2 = fine_coord(fmaxf(aoz, apz) + kAccelEps, invLf, nf) - lo2 + 1;
-        nc = w0 * w1 * w2;
-    }
-    const bool solo = open && nc > (uint32_t)kFlatMaxItems;
-    const uint32_t ncw = (open && !solo) ? nc : 0u;
-    H.ox[lane] = ox; H.oy[lane] = oy; H.oz[lane] = oz;
-    H.dx[lane] = dx; H.dy[lane] = dy; H.dz[lane] = dz;
+    const FlatBox box = flat_box(acc, open, aox, aoy, aoz, apx, apy, apz);
+    H.o[lane] = make_float4(ox, oy, oz, __uint_as_float(excluded));
+    H.d[lane] = make_float4(dx, dy, dz, __uint_as_float(box.lo0 | (box.lo1 << 10) | (box.lo2 << 20)));
     Lw.gx[lane] = gx; Lw.gy[lane] = gy; Lw.gz[lane] = gz;
-    H.excl[lane] = excluded;
-    H.box[lane] = lo0 | (lo1 << 10) | (lo2 << 20);
-    H.wd[lane] = w0 | (w1 << 8) | (w2 << 16);
     H.n[lane] = 0;
-    const uint32_t iincl = warp_incl_scan(ncw, lane);
-    const uint32_t iexcl = iincl - ncw;
-    const uint32_t itotal = __shfl_sync(FULL, iincl, 31);
+    FlatList l = flat_list(H, box, lane);
     uint32_t qn = 0, fn = 0;  // queue lengths (warp-uniform)
     __syncwarp();
-    // the warp's records pair by pair, item block after item block, and then
-    // one last pass that tests the record queue's partial group: one inlined
-    // copy of the exact test for the whole round
-    uint32_t ib = 0, rb = 0, rtotal = 0, rincl = 0, rbase = 0, ow = 0;
+    // the warp's records pair by pair and then one last pass that tests the
+    // record queue's partial group: one inlined copy of the exact test for the
+    // whole round
     for (;;) {
-        while (rb >= rtotal && ib < itotal) {  // warp-uniform
-            const uint32_t m = ib + lane;
-            ow = min(warp_find(iincl, m), 31u);
-            const uint32_t ofs = __shfl_sync(FULL, iexcl, ow);
-            uint32_t b0 = 0, cnt = 0;
-            if (m < itotal) {
-                const uint32_t q = m - ofs;
-                const uint32_t wd = H.wd[ow], bx = H.box[ow];
-                const uint32_t ww1 = (wd >> 8) & 0xFFu, ww2 = wd >> 16;
-                const uint32_t iz = q % ww2, r = q / ww2, iy = r % ww1, ix = r / ww1;
-                cell_records(acc, (bx & 1023u) + ix, ((bx >> 10) & 1023u) + iy, (bx >> 20) + iz,
-                             Lw.gx[ow] + H.ox[ow], Lw.gy[ow] + H.oy[ow], Lw.gz[ow] + H.oz[ow], H.dx[ow], H.dy[ow],
-                             H.dz[ow], b0, cnt);
-            }
-            rincl = warp_incl_scan(cnt, lane);
-            rtotal = __shfl_sync(FULL, rincl, 31);
-            rbase = b0 - (rincl - cnt);
-            rb = 0;
-            ib += 32;
-        }
-        const bool more = rb < rtotal;  // warp-uniform
+        const bool more = flat_next(H, l, acc, lane, [&](uint32_t ow, float4 O) {  // warp-uniform
+            return make_float4(Lw.gx[ow] + O.x, Lw.gy[ow] + O.y, Lw.gz[ow] + O.z, 0.0f);
+        });
         bool s0 = false, s1 = false;
         uint32_t e0 = 0, e1 = 0, o0 = 0, o1 = 0;
         if (more) {
-            const uint32_t r0 = rb + lane, r1 = rb + 32 + lane;
-            const uint32_t j0 = min(warp_find(rincl, r0), 31u);
-            const uint32_t j1 = min(warp_find(rincl, r1), 31u);
-            e0 = __shfl_sync(FULL, rbase, j0) + r0;
-            e1 = __shfl_sync(FULL, rbase, j1) + r1;
-            o0 = __shfl_sync(FULL, ow, j0);
-            o1 = __shfl_sync(FULL, ow, j1);
-            if (r0 < rtotal) {
+            flat_pick(H, l, lane, l.rb, e0, o0);
+            flat_pick(H, l, lane, l.rb + 32, e1, o1);
+            if (l.rb + lane < l.total) {
                 float4 q; float3 p1; uint32_t t;
                 record_load(acc, e0, full, q, p1, t);
                 pc.records++;
-                s0 = t != H.excl[o0] && local_plane(H, Lw, q, o0);
+                s0 = t != __float_as_uint(H.o[o0].w) && local_plane(H, Lw, q, o0);
             }
-            if (r1 < rtotal) {
+            if (l.rb + 32 + lane < l.total) {
                 float4 q; float3 p1; uint32_t t;
                 record_load(acc, e1, full, q, p1, t);
                 pc.records++;
-                s1 = t != H.excl[o1] && local_plane(H, Lw, q, o1);
+                s1 = t != __float_as_uint(H.o[o1].w) && local_plane(H, Lw, q, o1);
             }
-            rb += 64;
+            l.rb += 64;
         }
         local_enqueue(H, Lw, g, acc, full, lane, s0, e0, o0, s1, e1, o1, qn, fn, pc, !more);
         if (!more) break;
@@ -474,55 +428,29 @@ __device__ __forceinline__ void local_round(FlatWarp& H, LocalWarp& Lw, const Me
         FastHit h;
         if (lane < fn && local_fp64(H, Lw, g, Lw.ft[lane], Lw.fo[lane], h, pc)) flat_file_hit(H, Lw.fo[lane], h);
     }
-    if (solo) local_solo(H, Lw, g, acc, full, lane, lo0, lo1, lo2, w1, w2, nc, excluded, pc);
+    if (box.solo) local_solo(H, Lw, g, acc, full, lane, apx, apy, apz, pc);
     __syncwarp();
     found = false;
     if (!open) return;
     const uint32_t n = H.n[lane];
-    const uint32_t gn = g.n;
-    const float L = g.L;
-    const uint32_t sx = ref_coord(aox, L, gn), sy = ref_coord(aoy, L, gn), sz = ref_coord(aoz, L, gn);
-    const uint32_t tx = ref_coord(apx, L, gn), ty = ref_coord(apy, L, gn), tz = ref_coord(apz, L, gn);
-    const uint32_t ix = (uint32_t)((int)(tx > sx) - (int)(tx < sx));
-    const uint32_t iy = (uint32_t)((int)(ty > sy) - (int)(ty < sy));
-    const uint32_t iz = (uint32_t)((int)(tz > sz) - (int)(tz < sz));
-    if (n > (uint32_t)kFlatSlots) {
-        found = local_overflow(H, Lw, g, lane, sx, sy, sz, tx, ty, tz, ix, iy, iz, excluded, best, pc);
-        if (found) local_refine(g, gx, gy, gz, ox, oy, oz, dx, dy, dz, best);
-        return;
-    }
     if (n == 0) return;
     uint32_t bq = 0;
-    uint4 hc[kFlatSlots];  // each hit's reference cells, loaded together before the walk
-#pragma unroll
-    for (int q = 0; q < kFlatSlots; q++)
-        hc[q] = ((uint32_t)q < n) ? hit_cells(g, H.t[q][lane]) : make_uint4(kCellNone, kCellNone, kCellNone, kCellNone);
-    uint32_t cx = sx;
-    do {
-        uint32_t cy = sy;
-        do {
-            uint32_t cz = sz;
-            do {
-                const uint32_t c = gn * gn * cz + gn * cy + cx;
-#pragma unroll
-                for (uint32_t q = 0; q < (uint32_t)kFlatSlots; q++) {
-                    if (q >= n) break;
-                    const uint32_t t = H.t[q][lane];
-                    if (!hit_in_cell_compact(g, hc[q], c, t)) continue;
-                    const float d2 = H.d2[q][lane];
-                    if (!found || d2 < H.d2[bq][lane] || (d2 == H.d2[bq][lane] && t < H.t[bq][lane])) {
-                        bq = q;
-                        found = true;
-                    }
-                }
-                cz += iz;
-            } while ((cz != tz + iz) && !found);
-            cy += iy;
-        } while ((cy != ty + iy) && !found);
-        cx += ix;
-    } while ((cx != tx + ix) && !found);
+    found = true;
+    if (!flat_only_hit(H, lane, n, g.n, gx + H.x[0][lane], gy + H.y[0][lane], gz + H.z[0][lane])) {
+        const uint32_t gn = g.n;
+        const float L = g.L;
+        const uint32_t sx = ref_coord(aox, L, gn), sy = ref_coord(aoy, L, gn), sz = ref_coord(aoz, L, gn);
+        const uint32_t tx = ref_coord(apx, L, gn), ty = ref_coord(apy, L, gn), tz = ref_coord(apz, L, gn);
+        if (n > (uint32_t)kFlatSlots) {
+            found = local_overflow(H, Lw, g, lane, ref_walk(sx, sy, sz, tx, ty, tz), excluded, best, pc);
+            if (found) local_refine(g, gx, gy, gz, ox, oy, oz, dx, dy, dz, best);
+            return;
+        }
+        bq = flat_choose(H, g, lane, n, ref_walk(sx, sy, sz, tx, ty, tz));
+        found = bq != kNoPlace;
+    }
     if (found) {
-        best.t = H.t[bq][lane]; best.type = H.type[bq][lane]; best.d2 = H.d2[bq][lane];
+        best.t = H.t[bq][lane]; best.type = H.type[bq][lane] & ~kHitWalk; best.d2 = H.d2[bq][lane];
         best.x = H.x[bq][lane]; best.y = H.y[bq][lane]; best.z = H.z[bq][lane];
         local_refine(g, gx, gy, gz, ox, oy, oz, dx, dy, dz, best);
     }

@@ -36,7 +36,14 @@ struct FastHit {
     float x, y, z, d2;
     uint32_t type;
 };
-static constexpr int kMaxHits = 4;
+// Hit type flag: the reference's walk over its cells decides whether (and when)
+// it meets this triangle.  Without it every reference cell that the triangle
+// enters by more than kRegularEps lists it (k_tri_regular; the sign of its vv
+// carries the flag), so a sub-segment's only hit is the reference's when it
+// lies clear of the cell's faces.
+static constexpr float kRegularEps = 3e-5f;
+static constexpr uint32_t kHitWalk = 0x200u;
+__device__ __forceinline__ uint32_t hit_walk(float vv) { return __float_as_uint(vv) >> 31 << 9; }
 
 // reference-grid membership of triangle t in cell c: binary search of the
 // ascending list
@@ -51,36 +58,65 @@ __device__ __forceinline__ bool in_ref_cell(const MeshDev& g, uint32_t c, uint32
     return false;
 }
 
-// Membership of triangle t in reference cell c from the triangle's own cell
-// record (loaded once per hit): the same answer as in_ref_cell with no
-// dependent loads; a triangle in more than four cells keeps the search.
-__device__ __forceinline__ bool hit_in_cell(const MeshDev& g, uint4 cells, uint32_t c, uint32_t t) {
-    if (cells.x == kCellMany) return in_ref_cell(g, c, t);
-    return (cells.x == c) | (cells.y == c) | (cells.z == c) | (cells.w == c);
-}
-
-// The same with the rare search out of line, for a kernel whose code size
-// limits it (hit resolution tests every hit slot, so an inlined search is
-// copied into each unrolled slot test): the cell-local round measured 1.5 %
-// faster with it, the plain round 0.6 % slower.
-static __device__ __noinline__ bool in_ref_cell_search(const MeshDev& g, uint32_t c, uint32_t t) {
-    return in_ref_cell(g, c, t);
-}
-__device__ __forceinline__ bool hit_in_cell_compact(const MeshDev& g, uint4 cells, uint32_t c, uint32_t t) {
-    if (cells.x == kCellMany) return in_ref_cell_search(g, c, t);
-    return (cells.x == c) | (cells.y == c) | (cells.z == c) | (cells.w == c);
-}
-__device__ __forceinline__ uint4 hit_cells(const MeshDev& g, uint32_t t) {
-    if (!g.tri_cells) return make_uint4(kCellMany, kCellMany, kCellMany, kCellMany);
-    return __ldg(g.tri_cells + t);
-}
-
 __device__ __forceinline__ uint32_t ref_coord(float p, float L, uint32_t n) {
     float f = floorf((p + 1.0f) / L);
     float hi = (float)(n - 1);
     float mn = (hi < f) ? hi : f;
     float mx = (0.0f < mn) ? mn : 0.0f;
     return (uint32_t)mx;
+}
+
+// ---- which of several hits the reference takes ------------------------------
+// cubeCollDetect's loops (dSim3/src/spinKernelCpu.cpp:198-337) walk the
+// reference cells from the start's to the end's, x outermost and z innermost,
+// and stop at the first whose list holds a hit.  A cell's place in that walk is
+// (ax ny + ay) nz + az, ax, ay, az its distances from the start's cell, so the
+// reference's hit is the one of lowest (place of its triangle's first cell,
+// distance, triangle index), found without walking the cells.
+static constexpr uint32_t kNoPlace = 0xFFFFFFFFu;
+struct RefWalk {
+    uint32_t sx, sy, sz;  // the start's cell
+    int ix, iy, iz;       // +1, or -1 where the walk descends
+    uint32_t nx, ny, nz;  // cells on each axis
+};
+__device__ __forceinline__ RefWalk ref_walk(uint32_t sx, uint32_t sy, uint32_t sz, uint32_t tx, uint32_t ty,
+                                            uint32_t tz) {
+    RefWalk w;
+    w.sx = sx; w.sy = sy; w.sz = sz;
+    w.ix = tx < sx ? -1 : 1; w.iy = ty < sy ? -1 : 1; w.iz = tz < sz ? -1 : 1;
+    w.nx = (uint32_t)(w.ix * (int)(tx - sx)) + 1u;
+    w.ny = (uint32_t)(w.iy * (int)(ty - sy)) + 1u;
+    w.nz = (uint32_t)(w.iz * (int)(tz - sz)) + 1u;
+    return w;
+}
+// does p keep 2 kRegularEps from the faces of its reference cell?
+__device__ __forceinline__ bool clear_of_faces(float p, float inv, float margin) {
+    const float e = (p + 1.0f) * inv;
+    const float f = e - floor_small(e);
+    return (f > margin) & (f < 1.0f - margin);
+}
+// the place of packed cell c (pack_cell), kNoPlace when the walk misses it
+__device__ __forceinline__ uint32_t cell_place(const RefWalk& w, uint32_t c) {
+    const uint32_t ax = (uint32_t)(w.ix * (int)((c & 1023u) - w.sx));
+    const uint32_t ay = (uint32_t)(w.iy * (int)(((c >> 10) & 1023u) - w.sy));
+    const uint32_t az = (uint32_t)(w.iz * (int)((c >> 20) - w.sz));  // an unused entry's z is 4095
+    return ((ax < w.nx) & (ay < w.ny) & (az < w.nz)) ? (ax * w.ny + ay) * w.nz + az : kNoPlace;
+}
+// a triangle of more than four cells: walk the cells, searching their lists
+static __device__ __noinline__ uint32_t search_place(const MeshDev& g, RefWalk w, uint32_t t) {
+    for (uint32_t ax = 0; ax < w.nx; ax++)
+        for (uint32_t ay = 0; ay < w.ny; ay++)
+            for (uint32_t az = 0; az < w.nz; az++) {
+                const uint32_t x = w.sx + (uint32_t)w.ix * ax, y = w.sy + (uint32_t)w.iy * ay,
+                               z = w.sz + (uint32_t)w.iz * az;
+                if (in_ref_cell(g, g.n * g.n * z + g.n * y + x, t)) return (ax * w.ny + ay) * w.nz + az;
+            }
+    return kNoPlace;
+}
+// the place of the first of triangle t's cells (its record `c`, loaded ahead)
+__device__ __forceinline__ uint32_t first_place(const MeshDev& g, const RefWalk& w, uint4 c, uint32_t t) {
+    if (c.x == kCellMany) return search_place(g, w, t);
+    return min(min(cell_place(w, c.x), cell_place(w, c.y)), min(cell_place(w, c.z), cell_place(w, c.w)));
 }
 
 // full test of one accel record against the sub-segment (same float
@@ -101,7 +137,7 @@ __device__ __forceinline__ bool test_rec_uv(float4 a, float4 b, float4 u4, float
     float wz = oz + r * dz - b.y;
     float wu = wx * u4.x + wy * u4.y + wz * u4.z;
     float wv = wx * u4.w + wy * v4.x + wz * v4.y;
-    float uv = v4.z, uu = v4.w, vv = b.z;
+    float uv = v4.z, uu = v4.w, vv = fabsf(b.z);
     float s = (uv * wv - vv * wu) / (uv * uv - uu * vv);
     float tt = (uv * wu - uu * wv) / (uv * uv - uu * vv);
     if (!((s >= 0.0f) & (tt >= 0.0f) & (s + tt <= 1.0f))) return false;
@@ -114,7 +150,7 @@ __device__ __forceinline__ bool test_rec_uv(float4 a, float4 b, float4 u4, float
         if (((s == 0.0f) & (tt == 0.0f)) | ((s == 0.0f) & (tt == 1.0f)) | ((s == 1.0f) & (tt == 0.0f)))
             type = 3;
     }
-    h.type = type;
+    h.type = type | hit_walk(b.z);
     return true;
 }
 
@@ -154,8 +190,9 @@ __device__ __forceinline__ AccelRecFull load_full(const AccelRecFull* p) {
 static constexpr float kPlaneMargin = 1e-5f;
 __device__ __forceinline__ bool plane_may_cross(float4 q, float ox, float oy, float oz, float dx,
                                                 float dy, float dz) {
-    float den = q.x * dx + q.y * dy + q.z * dz;
-    float na = q.w - (q.x * ox + q.y * oy + q.z * oz);
+    // fused sums: a bound, tighter than the separate roundings the margin allows for
+    const float den = __fmaf_rn(q.x, dx, __fmaf_rn(q.y, dy, q.z * dz));
+    const float na = __fmaf_rn(-q.x, ox, __fmaf_rn(-q.y, oy, __fmaf_rn(-q.z, oz, q.w)));
     return (den > 0.0f) ? ((na > -kPlaneMargin) & (na < den + kPlaneMargin))
                         : ((den < 0.0f) & (na < kPlaneMargin) & (na > den - kPlaneMargin));
 }
@@ -262,7 +299,7 @@ static __device__ __noinline__ void ref_scan(const MeshDev& g, float ox, float o
                     float4 rb = make_float4(rc.x, rc.y, rc.z, __uint_as_float(t));
                     FastHit h;
                     if (!test_rec(g, ra, rb, ox, oy, oz, dx, dy, dz, h)) continue;
-                    if (h.d2 < bd2) { bd2 = h.d2; best = h; found = true; }
+                    if (h.d2 < bd2) { bd2 = h.d2; best = h; best.type &= ~kHitWalk; found = true; }
                 }
                 cz += iz;
             } while ((cz != tz + iz) && !found);

@@ -143,8 +143,9 @@ __device__ __forceinline__ uint32_t prec_prune(const FlatWarp& H, const AccelDev
     uint32_t t;
     record_plane(acc, k, full, q, t);
     pc.records++;
-    if (t == H.excl[o]) return 0xFFFFFFFFu;
-    if (!plane_near(q.x, q.y, q.z, q.w, H.ox[o], H.oy[o], H.oz[o], H.dx[o], H.dy[o], H.dz[o])) return 0xFFFFFFFFu;
+    const float4 O = H.o[o], D = H.d[o];
+    if (t == __float_as_uint(O.w)) return 0xFFFFFFFFu;
+    if (!plane_near(q.x, q.y, q.z, q.w, O.x, O.y, O.z, D.x, D.y, D.z)) return 0xFFFFFFFFu;
     return t;
 }
 
@@ -155,7 +156,7 @@ __device__ __forceinline__ void prec_test(FlatWarp& H, const PrecWarp& P, const 
     double r;
     uint32_t type;
     if (tri_test64(g.tri64, t, P.ox[o], P.oy[o], P.oz[o], P.dx[o], P.dy[o], P.dz[o], r, type))
-        prec_file_hit(H, o, t, type, r);
+        prec_file_hit(H, o, t, type | hit_walk(__ldg(&g.plane[t].vv)), r);
 }
 
 // FP32 barycentric pre-test: false only when the crossing of t's plane lies
@@ -172,10 +173,11 @@ __device__ __forceinline__ bool prec_pretest(const FlatWarp& H, const MeshDev& g
     const float4 a = __ldg(pp), c = __ldg(pp + 1);  // {n, p1.x}, {p1.y, p1.z, vv, info}
     const float4* bb = reinterpret_cast<const float4*>(g.bary + t);
     const float4 u4 = __ldg(bb), v4 = __ldg(bb + 1);  // {u, v.x}, {v.y, v.z, uv, uu}
-    const float uv = v4.z, uu = v4.w, vv = c.z;
+    const float uv = v4.z, uu = v4.w, vv = fabsf(c.z);
     const float mn = fminf(uu, vv), mx = fmaxf(uu, vv);
     if (!((uv * uv <= 0.82f * uu * vv) & (mx <= 100.0f * mn) & (mn >= 1e-6f))) return true;
-    const float ox = H.ox[o], oy = H.oy[o], oz = H.oz[o], dx = H.dx[o], dy = H.dy[o], dz = H.dz[o];
+    const float4 O = H.o[o], D4 = H.d[o];
+    const float ox = O.x, oy = O.y, oz = O.z, dx = D4.x, dy = D4.y, dz = D4.z;
     const float den = a.x * dx + a.y * dy + a.z * dz;
     if (den == 0.0f) return true;
     const float r = (a.x * (a.w - ox) + a.y * (c.x - oy) + a.z * (c.y - oz)) / den;
@@ -275,6 +277,24 @@ static __device__ __noinline__ void ref_scan64(const MeshDev& g, double ox, doub
     } while ((cx != tx + ix) && !found);
 }
 
+// a lane whose box is too wide for the warp's list: its own records
+static __device__ __noinline__ void prec_solo(FlatWarp& H, PrecWarp& P, const MeshDev& g, const AccelDev& acc,
+                                              bool full, uint32_t lane, float fpx, float fpy, float fpz,
+                                              PrecCount& pc) {
+    const float4 O = H.o[lane];
+    const FlatBox b = flat_box(acc, true, O.x, O.y, O.z, fpx, fpy, fpz);
+    for (uint32_t ix = 0; ix < b.w0; ix++)
+        for (uint32_t iy = 0; iy < b.w1; iy++)
+            for (uint32_t iz = 0; iz < b.w2; iz++) {
+                const uint32_t key = morton3(b.lo0 + ix, b.lo1 + iy, b.lo2 + iz);
+                const uint32_t b0 = __ldg(acc.start + key), b1 = __ldg(acc.start + key + 1);
+                for (uint32_t k = b0; k < b1; k++) {
+                    const uint32_t t = prec_prune(H, acc, k, full, lane, pc);
+                    if (t != 0xFFFFFFFFu) prec_test(H, P, g, t, lane, pc);
+                }
+            }
+}
+
 // One FP64 collision round for every lane of the warp (all 32 lanes call
 // it); the counterpart of flat_round_mode.  On return, for open lanes, found
 // and the hit (triangle ht, type htype, point hx, hy, hz) hold the
@@ -283,67 +303,29 @@ __device__ __forceinline__ void prec_round(FlatWarp& H, PrecWarp& P, const MeshD
                                            uint32_t lane, bool open, double ox, double oy, double oz, double px,
                                            double py, double pz, uint32_t excluded, bool& found, uint32_t& ht,
                                            uint32_t& htype, double& hx, double& hy, double& hz, PrecCount& pc) {
-    const uint32_t FULL = 0xFFFFFFFFu;
     const bool full = acc.wide == 2;
-    const float invLf = acc.invLf;
-    const uint32_t nf = acc.nf;
     const double dx = px - ox, dy = py - oy, dz = pz - oz;
     const float fox = (float)ox, foy = (float)oy, foz = (float)oz;
     const float fpx = (float)px, fpy = (float)py, fpz = (float)pz;
-    uint32_t lo0 = 0, lo1 = 0, lo2 = 0, w0 = 0, w1 = 0, w2 = 0, nc = 0;
-    if (open) {
-        lo0 = fine_coord(fminf(fox, fpx) - kAccelEps, invLf, nf);
-        lo1 = fine_coord(fminf(foy, fpy) - kAccelEps, invLf, nf);
-        lo2 = fine_coord(fminf(foz, fpz) - kAccelEps, invLf, nf);
-        w0 = fine_coord(fmaxf(fox, fpx) + kAccelEps, invLf, nf) - lo0 + 1;
-        w1 = fine_coord(fmaxf(foy, fpy) + kAccelEps, invLf, nf) - lo1 + 1;
-        w2 = fine_coord(fmaxf(foz, fpz) + kAccelEps, invLf, nf) - lo2 + 1;
-        nc = w0 * w1 * w2;
-    }
-    const bool solo = open && nc > (uint32_t)kFlatMaxItems;
-    const uint32_t ncw = (open && !solo) ? nc : 0u;
-    H.ox[lane] = fox; H.oy[lane] = foy; H.oz[lane] = foz;
-    H.dx[lane] = fpx - fox; H.dy[lane] = fpy - foy; H.dz[lane] = fpz - foz;
+    const FlatBox box = flat_box(acc, open, fox, foy, foz, fpx, fpy, fpz);
+    H.o[lane] = make_float4(fox, foy, foz, __uint_as_float(excluded));
+    H.d[lane] = make_float4(fpx - fox, fpy - foy, fpz - foz,
+                            __uint_as_float(box.lo0 | (box.lo1 << 10) | (box.lo2 << 20)));
     P.ox[lane] = ox; P.oy[lane] = oy; P.oz[lane] = oz;
     P.dx[lane] = dx; P.dy[lane] = dy; P.dz[lane] = dz;
-    H.excl[lane] = excluded;
-    H.box[lane] = lo0 | (lo1 << 10) | (lo2 << 20);
-    H.wd[lane] = w0 | (w1 << 8) | (w2 << 16);
     H.n[lane] = 0;
-    const uint32_t iincl = warp_incl_scan(ncw, lane);
-    const uint32_t iexcl = iincl - ncw;
-    const uint32_t itotal = __shfl_sync(FULL, iincl, 31);
+    FlatList l = flat_list(H, box, lane);
     uint32_t qn = 0, fn = 0;  // queue lengths (warp-uniform)
     __syncwarp();
-    for (uint32_t ib = 0; ib < itotal; ib += 32) {
-        const uint32_t m = ib + lane;
-        const uint32_t ow = min(warp_find(iincl, m), 31u);
-        const uint32_t ofs = __shfl_sync(FULL, iexcl, ow);
-        uint32_t b0 = 0, cnt = 0;
-        if (m < itotal) {
-            const uint32_t q = m - ofs;
-            const uint32_t wd = H.wd[ow], bx = H.box[ow];
-            const uint32_t ww1 = (wd >> 8) & 0xFFu, ww2 = wd >> 16;
-            const uint32_t iz = q % ww2, r = q / ww2, iy = r % ww1, ix = r / ww1;
-            cell_records(acc, (bx & 1023u) + ix, ((bx >> 10) & 1023u) + iy, (bx >> 20) + iz, H.ox[ow], H.oy[ow],
-                         H.oz[ow], H.dx[ow], H.dy[ow], H.dz[ow], b0, cnt);
-        }
-        const uint32_t rincl = warp_incl_scan(cnt, lane);
-        const uint32_t rtotal = __shfl_sync(FULL, rincl, 31);
-        const uint32_t rbase = b0 - (rincl - cnt);
-        for (uint32_t rb = 0; rb < rtotal; rb += 64) {
-            const uint32_t r0 = rb + lane, r1 = rb + 32 + lane;
-            const uint32_t j0 = min(warp_find(rincl, r0), 31u);
-            const uint32_t j1 = min(warp_find(rincl, r1), 31u);
-            const uint32_t e0 = __shfl_sync(FULL, rbase, j0) + r0;
-            const uint32_t e1 = __shfl_sync(FULL, rbase, j1) + r1;
-            const uint32_t o0 = __shfl_sync(FULL, ow, j0);
-            const uint32_t o1 = __shfl_sync(FULL, ow, j1);
-            const uint32_t t0 = (r0 < rtotal) ? prec_prune(H, acc, e0, full, o0, pc) : 0xFFFFFFFFu;
-            const uint32_t t1 = (r1 < rtotal) ? prec_prune(H, acc, e1, full, o1, pc) : 0xFFFFFFFFu;
-            prec_enqueue(H, P, g, lane, t0, o0, qn, fn, pc);
-            prec_enqueue(H, P, g, lane, t1, o1, qn, fn, pc);
-        }
+    while (flat_next(H, l, acc, lane, [](uint32_t, float4 O) { return O; })) {
+        uint32_t e0, e1, o0, o1;
+        flat_pick(H, l, lane, l.rb, e0, o0);
+        flat_pick(H, l, lane, l.rb + 32, e1, o1);
+        const uint32_t t0 = (l.rb + lane < l.total) ? prec_prune(H, acc, e0, full, o0, pc) : 0xFFFFFFFFu;
+        const uint32_t t1 = (l.rb + 32 + lane < l.total) ? prec_prune(H, acc, e1, full, o1, pc) : 0xFFFFFFFFu;
+        prec_enqueue(H, P, g, lane, t0, o0, qn, fn, pc);
+        prec_enqueue(H, P, g, lane, t1, o1, qn, fn, pc);
+        l.rb += 64;
     }
     // the queues' remainders (fewer than 32 each)
     {
@@ -352,17 +334,7 @@ __device__ __forceinline__ void prec_round(FlatWarp& H, PrecWarp& P, const MeshD
         prec_enqueue64(H, P, g, lane, pass ? tq : 0xFFFFFFFFu, oq, fn, pc);
         if (lane < fn) prec_test(H, P, g, P.ft[lane], P.fo[lane], pc);
     }
-    if (solo) {
-        for (uint32_t q = 0; q < nc; q++) {
-            const uint32_t iz = q % w2, r = q / w2, iy = r % w1, ix = r / w1;
-            const uint32_t key = morton3(lo0 + ix, lo1 + iy, lo2 + iz);
-            const uint32_t b0 = __ldg(acc.start + key), b1 = __ldg(acc.start + key + 1);
-            for (uint32_t k = b0; k < b1; k++) {
-                const uint32_t t = prec_prune(H, acc, k, full, lane, pc);
-                if (t != 0xFFFFFFFFu) prec_test(H, P, g, t, lane, pc);
-            }
-        }
-    }
+    if (box.solo) prec_solo(H, P, g, acc, full, lane, fpx, fpy, fpz, pc);
     __syncwarp();
     found = false;
     if (!open) return;
@@ -372,49 +344,39 @@ __device__ __forceinline__ void prec_round(FlatWarp& H, PrecWarp& P, const MeshD
         return;
     }
     if (n == 0) return;
-    // the reference's cell order over the filed hits; in a cell, the nearest
-    // hit, the lowest triangle index on ties (its cell lists ascend)
+    {
+        const double r = __hiloint2double(__float_as_int(H.y[0][lane]), __float_as_int(H.x[0][lane]));
+        hit_point64(ox, oy, oz, dx, dy, dz, r, hx, hy, hz);
+    }
+    if (flat_only_hit(H, lane, n, g.n, (float)hx, (float)hy, (float)hz)) {
+        ht = H.t[0][lane];
+        htype = H.type[0][lane];
+        found = true;
+        return;
+    }
+    // the reference's choice among the filed hits
     const uint32_t gn = g.n;
     const double L = (double)g.L;
     const float invL = 1.0f / g.L;
-    const uint32_t sx = ref_coord64_est(ox, fox, L, invL, gn), sy = ref_coord64_est(oy, foy, L, invL, gn),
-                   sz = ref_coord64_est(oz, foz, L, invL, gn);
-    const uint32_t tx = ref_coord64_est(px, fpx, L, invL, gn), ty = ref_coord64_est(py, fpy, L, invL, gn),
-                   tz = ref_coord64_est(pz, fpz, L, invL, gn);
-    const uint32_t ix = (uint32_t)((int)(tx > sx) - (int)(tx < sx));
-    const uint32_t iy = (uint32_t)((int)(ty > sy) - (int)(ty < sy));
-    const uint32_t iz = (uint32_t)((int)(tz > sz) - (int)(tz < sz));
+    const RefWalk w = ref_walk(ref_coord64_est(ox, fox, L, invL, gn), ref_coord64_est(oy, foy, L, invL, gn),
+                               ref_coord64_est(oz, foz, L, invL, gn), ref_coord64_est(px, fpx, L, invL, gn),
+                               ref_coord64_est(py, fpy, L, invL, gn), ref_coord64_est(pz, fpz, L, invL, gn));
+    uint32_t bplace = kNoPlace;
     double bd2 = 0.0;
-    uint4 hc[kFlatSlots];  // each hit's reference cells, loaded together before the walk
-#pragma unroll
-    for (int q = 0; q < kFlatSlots; q++)
-        hc[q] = ((uint32_t)q < n) ? hit_cells(g, H.t[q][lane]) : make_uint4(kCellNone, kCellNone, kCellNone, kCellNone);
-    uint32_t cx = sx;
-    do {
-        uint32_t cy = sy;
-        do {
-            uint32_t cz = sz;
-            do {
-                const uint32_t c = gn * gn * cz + gn * cy + cx;
-#pragma unroll
-                for (uint32_t q = 0; q < (uint32_t)kFlatSlots; q++) {
-                    if (q >= n) break;
-                    const uint32_t t = H.t[q][lane];
-                    if (!hit_in_cell(g, hc[q], c, t)) continue;
-                    const double r = __hiloint2double(__float_as_int(H.y[q][lane]), __float_as_int(H.x[q][lane]));
-                    double x, y, z;
-                    const double d2 = hit_point64(ox, oy, oz, dx, dy, dz, r, x, y, z);
-                    if (!found || d2 < bd2 || (d2 == bd2 && t < ht)) {
-                        found = true; bd2 = d2;
-                        ht = t; htype = H.type[q][lane]; hx = x; hy = y; hz = z;
-                    }
-                }
-                cz += iz;
-            } while ((cz != tz + iz) && !found);
-            cy += iy;
-        } while ((cy != ty + iy) && !found);
-        cx += ix;
-    } while ((cx != tx + ix) && !found);
+    for (uint32_t q = 0; q < n; q++) {
+        const uint32_t t = H.t[q][lane];
+        if (bplace != kNoPlace && t == ht) continue;  // filed from another fine cell too
+        const uint32_t place = first_place(g, w, __ldg(g.tri_cells + t), t);
+        if (place == kNoPlace) continue;
+        const double r = __hiloint2double(__float_as_int(H.y[q][lane]), __float_as_int(H.x[q][lane]));
+        double x, y, z;
+        const double d2 = hit_point64(ox, oy, oz, dx, dy, dz, r, x, y, z);
+        if (place < bplace || (place == bplace && (d2 < bd2 || (d2 == bd2 && t < ht)))) {
+            bplace = place; bd2 = d2;
+            ht = t; htype = H.type[q][lane] & ~kHitWalk; hx = x; hy = y; hz = z;
+        }
+    }
+    found = bplace != kNoPlace;
 }
 
 // Reflection or permeation at a hit, in FP64: the permeation interval, the

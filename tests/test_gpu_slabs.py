@@ -44,9 +44,18 @@ class OddMeshCase(MeshCase):
 @pytest.mark.parametrize("membranes,accel,records", [("G", None, 32), ("AM", None, 32), ("G", 2, 32), ("AM", 5, 64),
                                                      ("G", 30, 16), ("AM", 90, 32), ("G", 190, 64)])
 def test_replay_parity_with_odd_triangles(engine, tmp_path, membranes, accel, records):
+    _replay_parity(OddMeshCase(tmp_path, membranes, N=1200, permeability=0.05), accel, records)
+
+
+@pytest.mark.parametrize("membranes,ring,verts", [("G", 0.4, 16), ("AM", 0.2, 24), ("AM", 0.8, 12)])
+def test_replay_parity_with_rings_on_cell_faces(engine, tmp_path, membranes, ring, verts):
+    """Triangles that end on faces of the reference grid (cells of 0.4 um), whose lists rounding decides: a single hit
+    is taken without the walk over the cells only clear of the faces."""
+    _replay_parity(MeshCase(tmp_path, membranes=membranes, N=4000, ring=ring, verts=verts), None, 32)
+
+
+def _replay_parity(case, accel, records, iters=50):
     from dsim_gb300.engine import Mesh, Spins, mesh_params, mesh_run
-    case = OddMeshCase(tmp_path, membranes, N=1200, permeability=0.05)
-    iters = 50
     d = draws(iters, case.N, seed=3)
     mo = O.Mesh(case.path, case.spaceScale)
     cc, tic, maxtpc = O.populate_cubes(mo.vertices, mo.trgls, 50)
