@@ -161,6 +161,7 @@ struct dsim_cyl {
         CylDev g;
         g.fibers = fibers; g.cube_count = cc; g.cubes = cubes; g.cube_fibers = cubeF;
         g.n = host.numCubes; g.maxFPC = host.maxFPC; g.L = host.cubeLength;
+        g.inv = 1.0f / host.cubeLength; g.inv64 = 1.0 / (double)host.cubeLength;
         g.nF = host.nF;
         g.fine_start = fineK ? fineStart : nullptr; g.fine_rec = fineRec; g.fine_pos = finePos;
         g.fineK = fineK;
@@ -234,6 +235,7 @@ struct dsim_spins {
     bool permuted = false;      // slot i does not hold spin i
     float4* cpos = nullptr;     // cylinder layout (lazy)
     uint32_t* cseed = nullptr;  // cylinder layout (lazy)
+    uint32_t* corder = nullptr; // cylinder runs: the spins by region, and two counters (lazy)
     uint32_t* counts = nullptr;
     uint32_t* tested = nullptr;  // per-spin scanned grid entries (lazy)
     uint32_t* status = nullptr;
@@ -642,7 +644,7 @@ static void spins_release(dsim_spins* s) {
     if (!s) return;
     if (s->st) cudaStreamSynchronize(s->st);
     cudaFree(s->x); cudaFree(s->y); cudaFree(s->z); cudaFree(s->mag); cudaFree(s->phase);
-    cudaFree(s->meta); cudaFree(s->cpos); cudaFree(s->cseed); cudaFree(s->counts);
+    cudaFree(s->meta); cudaFree(s->cpos); cudaFree(s->cseed); cudaFree(s->corder); cudaFree(s->counts);
     cudaFree(s->status); cudaFree(s->tested); cudaFree(s->draws); cudaFree(s->grad); cudaFree(s->partials);
     cudaFree(s->sig); cudaFree(s->flush);
     cudaFree(s->id); cudaFree(s->x2); cudaFree(s->y2); cudaFree(s->z2); cudaFree(s->mag2);
@@ -787,6 +789,7 @@ static int ensure_cyl(dsim_spins* s) {
     int rc;
     if (!s->cpos && (rc = dev_alloc(&s->cpos, s->N, &s->bytes))) return rc;
     if (!s->cseed && (rc = dev_alloc(&s->cseed, (size_t)4 * s->N, &s->bytes))) return rc;
+    if (!s->corder && (rc = dev_alloc(&s->corder, (size_t)s->N + 2, &s->bytes))) return rc;
     return kOk;
 }
 
@@ -1028,8 +1031,11 @@ int dsim_cyl_run(dsim_cyl* c, dsim_spins* s, const dsim_cyl_params* p, const flo
     if (rc) return rc;
     CylSpinsDev S;
     S.pos = s->cpos; S.seed4 = s->cseed; S.mag = s->mag; S.N = s->N;
-    s->launches += 1;
-    return launch_cyl_step(c->dev(), a, S, replayDraws ? kRngReplay : kRngPhilox, s->st);
+    uint32_t launches = 0;
+    rc = launch_cyl_step(c->dev(), a, S, {s->corder, s->corder + s->N}, replayDraws ? kRngReplay : kRngPhilox, s->st,
+                         &launches);
+    s->launches += launches;
+    return rc;
 }
 
 int dsim_signal(dsim_spins* s, double region, double out[15]) {

@@ -199,19 +199,19 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
         }
     } else if (valid) {
         const CylDev& g = sub.c;
-        const float perm = J.perm, inR = J.inR;
+        const float perm = J.perm;
         uint32_t imo = comp, nearest = fiber;
+        Cyl32 form = {J.inR};
+        bool clear = false;
         if (imo < 2 && nearest >= g.nF) imo = 2;
         for (uint32_t it = 0; it < nsteps; it++) {
             const Draw d = philox_draw(id, (uint64_t)(ls0 + it), 0u, k0, k1);
-            const float ox = x, oy = y, oz = z;
             const float sdv = J.sd[imo];
-            float px = x + d.nx * sdv, py = y + d.ny * sdv, pz = z + d.nz * sdv;
-            if (perm < 1.0f) cyl_membranes(g, ox, oy, oz, px, py, pz, d.u, perm, inR, imo, nearest, nrefl, nperm, st);
-            if (px > J.clampHi) px = J.clampHi; else if (px < J.clampLo) px = J.clampLo;
-            if (py > J.clampHi) py = J.clampHi; else if (py < J.clampLo) py = J.clampLo;
-            if (pz > J.clampHi) pz = J.clampHi; else if (pz < J.clampLo) pz = J.clampLo;
-            x = px; y = py; z = pz;
+            const P3<float> o = {x, y, z};
+            P3<float> p = {x + d.nx * sdv, y + d.ny * sdv, z + d.nz * sdv};
+            cyl_membranes(g, form, o, p, d.u, perm, imo, nearest, nrefl, nperm, st, clear);
+            cyl_clamp(p, J.clampLo, J.clampHi, clear);
+            x = p.x; y = p.y; z = p.z;
             const float T2 = J.T2[imo];
             if (T2 > 0.0f) mag += -mag / T2 * J.dt;
             const float w = __ldg(wave + ls0 + it);
@@ -833,7 +833,7 @@ uint64_t chunk_launches(const dsim_batch* b) {
 
 // Precision-form cylinder jobs (DSIM_JOB_PRECISE): the dSim2 step of
 // cpuIntegrate (dSim2/src/spinKernelCpu.cpp:312-641) with positions,
-// distances, clamp, T2 decay and moments in double (cyl_membranes64); the
+// distances, clamp, T2 decay and moments in double (cyl_membranes); the
 // parameters are the job's float values.  Position and magnitude persist in
 // the double fields; the moment is kept as the float pair m - c.
 __global__ void __launch_bounds__(kFlatThreads, 4)
@@ -866,21 +866,21 @@ k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
         const uint32_t meta = S.u[U_META][i];
         uint32_t imo = meta & 0xFFu, nearest = meta >> 8;
         if (imo < 2 && nearest >= g.nF) imo = 2;
-        const double perm = (double)__ldg(&J.perm), inR = (double)__ldg(&J.inR);
+        const double perm = (double)__ldg(&J.perm);
+        Cyl64 form = {(double)__ldg(&J.inR)};
+        bool clear = false;
         const double hiC = 1.0 - (double)__ldg(&J.spinR), loC = -1.0 + (double)__ldg(&J.spinR);
         const double dt = (double)__ldg(&J.dt);
         const uint32_t k0 = __ldg(&J.key0), k1 = __ldg(&J.key1);
         const float* __restrict__ wave = J.wave;
         for (uint32_t it = 0; it < nsteps; it++) {
             const Draw d = philox_draw(id, (uint64_t)(ls0 + it), 0u, k0, k1);
-            const double ox = x, oy = y, oz = z;
             const double sd = (double)__ldg(&J.sd[imo == 0 ? 0 : (imo == 1 ? 1 : 2)]);
-            double px = x + (double)d.nx * sd, py = y + (double)d.ny * sd, pz = z + (double)d.nz * sd;
-            cyl_membranes64(g, ox, oy, oz, px, py, pz, (double)d.u, perm, inR, imo, nearest, nrefl, nperm, st);
-            if (px > hiC) px = hiC; else if (px < loC) px = loC;
-            if (py > hiC) py = hiC; else if (py < loC) py = loC;
-            if (pz > hiC) pz = hiC; else if (pz < loC) pz = loC;
-            x = px; y = py; z = pz;
+            const P3<double> o = {x, y, z};
+            P3<double> p = {x + (double)d.nx * sd, y + (double)d.ny * sd, z + (double)d.nz * sd};
+            cyl_membranes(g, form, o, p, (double)d.u, perm, imo, nearest, nrefl, nperm, st, clear);
+            cyl_clamp(p, loC, hiC, clear);
+            x = p.x; y = p.y; z = p.z;
             if (imo <= 2) {
                 const float T2 = __ldg(&J.T2[imo]);
                 if (T2 > 0.0f) mag += -mag / (double)T2 * dt;
@@ -914,7 +914,7 @@ k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
 // Cell-local FP32 cylinder jobs (DSIM_JOB_LOCAL): the dSim2 step with the
 // position as a lattice origin (multiple of 1/16) plus an FP32 offset in
 // [0, 1/16), membrane decisions near their FP32 error band taken in FP64
-// (cyl_membranes_local), Kahan moments.  Between chunks the position is kept
+// (CylLocal), Kahan moments.  Between chunks the position is kept
 // in the double fields as origin + offset.
 __global__ void __launch_bounds__(kFlatThreads, 4)
 k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S,
@@ -938,11 +938,12 @@ k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
     const bool valid = id != 0xFFFFFFFFu;
-    uint32_t nrefl = 0, nperm = 0, st = 0, ntests = 0, nexact = 0;
+    uint32_t nrefl = 0, nperm = 0, st = 0;
+    CylLocal form = {__ldg(&J.inR), {0.0f, 0.0f, 0.0f}, 0u, 0u};
     if (valid) {
         const CylDev g = sub.c;
         const double X = S.d[D_X][i], Y = S.d[D_Y][i], Z = S.d[D_Z][i];
-        CylOrigin G;
+        CylOrigin& G = form.G;
         G.x = (float)(floor(X * 16.0) * 0.0625);
         G.y = (float)(floor(Y * 16.0) * 0.0625);
         G.z = (float)(floor(Z * 16.0) * 0.0625);
@@ -953,26 +954,28 @@ k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict
         const uint32_t meta = S.u[U_META][i];
         uint32_t imo = meta & 0xFFu, nearest = meta >> 8;
         if (imo < 2 && nearest >= g.nF) imo = 2;
-        const float perm = __ldg(&J.perm), inR = __ldg(&J.inR);
+        const float perm = __ldg(&J.perm);
+        bool clear = false;
         const float clampHi = __ldg(&J.clampHi), clampLo = __ldg(&J.clampLo), dt = __ldg(&J.dt);
         const uint32_t k0 = __ldg(&J.key0), k1 = __ldg(&J.key1);
         const float* __restrict__ wave = J.wave;
         for (uint32_t it = 0; it < nsteps; it++) {
             const Draw d = philox_draw(id, (uint64_t)(ls0 + it), 0u, k0, k1);
-            const float ox = x, oy = y, oz = z;
             const float sd = __ldg(&J.sd[imo < 3 ? imo : 2]);
-            float px = x + d.nx * sd, py = y + d.ny * sd, pz = z + d.nz * sd;
-            cyl_membranes_local(g, G, ox, oy, oz, px, py, pz, d.u, perm, inR, imo, nearest, nrefl, nperm, st, ntests,
-                                nexact);
+            const P3<float> o = {x, y, z};
+            P3<float> p = {x + d.nx * sd, y + d.ny * sd, z + d.nz * sd};
+            cyl_membranes(g, form, o, p, d.u, perm, imo, nearest, nrefl, nperm, st, clear);
             // clamp in absolute coordinates, then move the origin so the
             // offset is back in [0, 1/16)
-            if (G.x + px > clampHi) px = clampHi - G.x; else if (G.x + px < clampLo) px = clampLo - G.x;
-            if (G.y + py > clampHi) py = clampHi - G.y; else if (G.y + py < clampLo) py = clampLo - G.y;
-            if (G.z + pz > clampHi) pz = clampHi - G.z; else if (G.z + pz < clampLo) pz = clampLo - G.z;
-            const float sx = floor_small(px * 16.0f) * kLatticeH, sy = floor_small(py * 16.0f) * kLatticeH,
-                        sz = floor_small(pz * 16.0f) * kLatticeH;
+            const P3<float> q = p;
+            if (G.x + p.x > clampHi) p.x = clampHi - G.x; else if (G.x + p.x < clampLo) p.x = clampLo - G.x;
+            if (G.y + p.y > clampHi) p.y = clampHi - G.y; else if (G.y + p.y < clampLo) p.y = clampLo - G.y;
+            if (G.z + p.z > clampHi) p.z = clampHi - G.z; else if (G.z + p.z < clampLo) p.z = clampLo - G.z;
+            clear = clear & (p.x == q.x) & (p.y == q.y) & (p.z == q.z);
+            const float sx = floor_small(p.x * 16.0f) * kLatticeH, sy = floor_small(p.y * 16.0f) * kLatticeH,
+                        sz = floor_small(p.z * 16.0f) * kLatticeH;
             G.x += sx; G.y += sy; G.z += sz;
-            x = px - sx; y = py - sy; z = pz - sz;
+            x = p.x - sx; y = p.y - sy; z = p.z - sz;
             const float T2 = __ldg(&J.T2[imo < 3 ? imo : 2]);
             if (T2 > 0.0f) mag += -mag / T2 * dt;
             const float w = __ldg(wave + ls0 + it);
@@ -989,7 +992,7 @@ k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict
         S.u[U_META][i] = (imo & 0xFFu) | ((nearest & 0xFFFFFFu) << 8);
     }
     // per-job counters {reflections, permeations, distance tests, FP64 decisions}
-    unsigned long long r = nrefl, p = nperm, te = ntests, ex = nexact;
+    unsigned long long r = nrefl, p = nperm, te = form.ntests, ex = form.nexact;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         r += __shfl_down_sync(FULL, r, o);

@@ -65,6 +65,8 @@ struct State {
     const float4* replay = nullptr;
     uint32_t* counts = nullptr;
     uint32_t* status = nullptr;
+    uint32_t* order = nullptr;  // the spins by region and two counters, for a step call
+    uint32_t orderCap = 0;
 };
 State& S() {
     static State s;
@@ -229,6 +231,8 @@ void integrateSystem(float* pos, unsigned int* randSeed, float deltaTime, float*
     g.n = numCubes;
     g.maxFPC = maxFibersPerCube;
     g.L = cubeLength;
+    g.inv = 1.0f / cubeLength;
+    g.inv64 = 1.0 / (double)cubeLength;
     g.nF = s.nF;
     if (!g.fibers || g.nF == 0) {
         set_last_error(kErrInvalid, "integrateSystem: bindFiberList(fibers, count) must precede the step");
@@ -259,7 +263,14 @@ void integrateSystem(float* pos, unsigned int* randSeed, float deltaTime, float*
     sp.seed4 = randSeed;
     sp.mag = nullptr;
     sp.N = (uint32_t)numBodies;
-    int rc = launch_cyl_step(g, a, sp, s.replay ? kRngReplay : kRngPhiloxPerSpinKey, 0);
+    if (s.orderCap < sp.N) {
+        cudaFree(s.order);
+        s.order = nullptr; s.orderCap = 0;
+        if (cudaMalloc(&s.order, ((size_t)sp.N + 2) * 4) == cudaSuccess) s.orderCap = sp.N;
+        else cudaGetLastError();  // no room: the spins run in the caller's order
+    }
+    const CylOrder order = {s.order, s.order ? s.order + s.orderCap : nullptr};
+    int rc = launch_cyl_step(g, a, sp, order, s.replay ? kRngReplay : kRngPhiloxPerSpinKey, 0, nullptr);
     if (rc) fail(rc);
 }
 

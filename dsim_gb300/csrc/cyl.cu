@@ -110,11 +110,12 @@ __device__ void cyl_fiber_insertions(float4 fr, uint32_t n, float L, float H, Em
     else if (fp[1] == 2.0f) { a = 1; f = 2; s = 0; }
     else return;
     const float start = (float)(-1.0 + 0.002);
+    const float inv = 1.0f / L;
     uint32_t seq = 0;
     auto line = [&](float* cp) {
         cp[a] = start;
         for (uint32_t j = 0; j < n; j++) {
-            emit(cyl_cell(cp[0], cp[1], cp[2], L, n), seq++);
+            emit(cyl_cell(n, inv, cp[0], cp[1], cp[2]).cube, seq++);
             cp[a] += L;
         }
     };
@@ -122,7 +123,6 @@ __device__ void cyl_fiber_insertions(float4 fr, uint32_t n, float L, float H, Em
     line(cp);
     float tp[3] = {fp[0], fp[1], fp[2]};
     tp[a] = start;
-    const float inv = 1.0f / L;
     const float cpos_f = floorf((tp[f] + 1.0f) * inv), cpos_s = floorf((tp[s] + 1.0f) * inv);
     const float dfc_f = tp[f] - cpos_f * L;
     const float dfc_s = tp[s] - cpos_s * L;
@@ -240,44 +240,93 @@ int build_cyl_grid_gpu(const float4* fibers, uint32_t nF, uint32_t n, uint32_t m
     return kOk;
 }
 
-template <int RNG>
-__global__ void __launch_bounds__(256) k_cyl_step(CylDev g, CylStepArgs a, CylSpinsDev S) {
+// the region of spin i as the step takes it (a spin whose fiber is not in the
+// list is outside)
+__device__ __forceinline__ uint32_t cyl_spin_region(uint4 w, uint32_t nF) {
+    const uint32_t imo = dsim2_region(w.z, w.w);
+    return (imo < 2 && w.w >= nF) ? 2u : imo;
+}
+
+// The spins outside every fiber from the front of `order`, those inside from
+// its end (count: two zeroed words), so that warps hold one kind and the kind
+// with the longer steps starts first.  The order within the two is left to the
+// atomics; no result depends on it: a spin's walk is its own.
+__global__ void __launch_bounds__(256) k_cyl_order(uint32_t N, uint32_t nF, const uint4* __restrict__ seed4,
+                                                   uint32_t* order, uint32_t* count) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    const bool out = i < N && cyl_spin_region(seed4[i], nF) >= 2u;
+    const uint32_t outs = __ballot_sync(0xFFFFFFFFu, out), ins = __ballot_sync(0xFFFFFFFFu, i < N && !out);
+    uint32_t at = 0;
+    if (lane == 0 && outs) at = atomicAdd(count, __popc(outs));
+    if (lane == 1 && ins) at = atomicAdd(count + 1, __popc(ins));
+    const uint32_t a0 = __shfl_sync(0xFFFFFFFFu, at, 0), a1 = __shfl_sync(0xFFFFFFFFu, at, 1);
+    const uint32_t below = (1u << lane) - 1u;
+    if (i < N) order[out ? a0 + __popc(outs & below) : N - 1u - (a1 + __popc(ins & below))] = i;
+}
+
+// One thread per spin, all steps with the state in registers.  Bound by
+// instruction issue (300,000 spins among 256 cylinders: issue 77 %), with the
+// lanes a warp's kinds of step leave idle: 1363 warp instructions a step at 11
+// lanes -> 799 at 17 with the spins ordered by region and a rejected step ended
+// at once (cyl_membranes), 16.0 -> 9.8 us a step.  THIN (fewer than
+// 32 spins a warp, a.perWarp): the lanes repeat the warp's spins, so 32 lanes
+// draw for 32 / perWarp steps of each at once and a step takes its draws by
+// shuffles; every copy of a spin computes the same step.  A step is then one
+// warp's chain of about 470 instructions, 160 of them the draws.
+template <int RNG, bool THIN>
+__global__ void __launch_bounds__(128) k_cyl_step(CylDev g, CylStepArgs a, CylSpinsDev S,
+                                                  const uint32_t* __restrict__ order) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * a.perWarp + lane;
-    if (lane >= a.perWarp || i >= S.N) return;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t own = THIN ? lane & (a.perWarp - 1u) : lane;  // the lane's spin in the warp
+    const uint32_t ahead = THIN ? lane / a.perWarp : 0u, batch = THIN ? 32u / a.perWarp : 1u;
+    const uint32_t slot = warp * (THIN ? a.perWarp : 32u) + own;
+    const uint32_t live = THIN ? __ballot_sync(0xFFFFFFFFu, slot < S.N) : 0u;
+    if (slot >= S.N) return;
+    const uint32_t i = order ? order[slot] : slot;
     float4 P = S.pos[i];
     uint4 sd4 = reinterpret_cast<const uint4*>(S.seed4)[i];
     float x = P.x, y = P.y, z = P.z, phase = P.w;
     float mag = S.mag ? S.mag[i] : 1.0f;
     uint32_t nearest = sd4.w;
-    uint32_t imo = dsim2_region(sd4.z, nearest);
-    if (imo < 2 && nearest >= g.nF) imo = 2;  // no valid fiber: treat as outside
+    uint32_t imo = cyl_spin_region(sd4, g.nF);
+    Cyl32 form = {a.inRadPropSq};
+    bool clear = false;
     uint32_t nrej = 0, nperm = 0, status = 0;
     uint32_t k0 = a.key0, k1 = a.key1;
     if (RNG == kRngPhiloxPerSpinKey) { k0 = sd4.x; k1 = sd4.y; }
-    const float perm = a.perm, inR = a.inRadPropSq;
+    const float perm = a.perm;
+    Draw mine;  // THIN: the draw of step (it rounded down to a batch) + ahead
+    mine.nx = mine.ny = mine.nz = mine.u = 0.0f;
     for (uint32_t it = 0; it < a.iterations; it++) {
         Draw d;
         if (RNG == kRngReplay) {
             float4 q = __ldg(a.draws + (size_t)it * S.N + i);
             d.nx = q.x; d.ny = q.y; d.nz = q.z; d.u = q.w;
+        } else if (THIN) {
+            const uint32_t k = it & (batch - 1u);
+            if (k == 0) mine = philox_draw(a.spinBase + i, a.step0 + it + ahead, a.stream, k0, k1);
+            const uint32_t from = k * a.perWarp + own;
+            d.nx = __shfl_sync(live, mine.nx, from);
+            d.ny = __shfl_sync(live, mine.ny, from);
+            d.nz = __shfl_sync(live, mine.nz, from);
+            d.u = __shfl_sync(live, mine.u, from);
         } else {
             d = philox_draw(a.spinBase + i, a.step0 + it, a.stream, k0, k1);
         }
-        float ox = x, oy = y, oz = z;
         float sdv = (imo == 0) ? a.intraSd : ((imo == 1) ? a.myelinSd : a.extraSd);
-        float px = x + d.nx * sdv, py = y + d.ny * sdv, pz = z + d.nz * sdv;
-        cyl_membranes(g, ox, oy, oz, px, py, pz, d.u, perm, inR, imo, nearest, nrej, nperm, status);
-        if (px > a.clampHi) px = a.clampHi; else if (px < a.clampLo) px = a.clampLo;
-        if (py > a.clampHi) py = a.clampHi; else if (py < a.clampLo) py = a.clampLo;
-        if (pz > a.clampHi) pz = a.clampHi; else if (pz < a.clampLo) pz = a.clampLo;
-        x = px; y = py; z = pz;
+        const P3<float> o = {x, y, z};
+        P3<float> p = {x + d.nx * sdv, y + d.ny * sdv, z + d.nz * sdv};
+        cyl_membranes(g, form, o, p, d.u, perm, imo, nearest, nrej, nperm, status, clear);
+        cyl_clamp(p, a.clampLo, a.clampHi, clear);
+        x = p.x; y = p.y; z = p.z;
         float T2 = (imo == 0) ? a.T2fiber : ((imo == 1) ? a.T2myelin : a.T2outside);
         mag += -mag / T2 * a.dt;
         float gx = a.gx, gy = a.gy, gz = a.gz;
         if (a.grad) { float4 G = __ldg(a.grad + it); gx = G.x; gy = G.y; gz = G.z; }
         phase += (gx * x + gy * y + gz * z) * a.pc;
     }
+    if (THIN && ahead > 0) return;
     S.pos[i] = make_float4(x, y, z, phase);
     if (S.mag) S.mag[i] = mag;
     uint4 o4 = sd4;
@@ -292,21 +341,39 @@ __global__ void __launch_bounds__(256) k_cyl_step(CylDev g, CylStepArgs a, CylSp
     if (status) atomicOr(a.status, status);
 }
 
-int launch_cyl_step(const CylDev& g, const CylStepArgs& args, const CylSpinsDev& S, int rng,
-                    cudaStream_t st) {
+int launch_cyl_step(const CylDev& g, const CylStepArgs& args, const CylSpinsDev& S, const CylOrder& scratch, int rng,
+                    cudaStream_t st, uint32_t* launches) {
+    if (launches) *launches = 0;
     if (S.N == 0 || args.iterations == 0) return kOk;
     CylStepArgs a = args;
-    // at most 17 warps per SM below 32 spins a warp.  us per step, 64
-    // cylinders, 32 / 16 / 8 / 4 / 2 / 1 spins a warp: 1000 spins 3.9 / 3.5 /
-    // 2.9 / 2.6 / 2.4 / 2.2; 10,000 spins 4.9 / 4.1 / 3.4 / 3.4 / 4.1 / 5.7;
-    // 40,000 spins 5.1 / 4.6 / 6.4; 80,000 spins 5.8 / 7.2
-    a.perWarp = spins_per_warp(S.N, 17);
+    // at most 33 warps per SM below 32 spins a warp.  us per step, 64
+    // cylinders, 32 / 16 / 8 / 4 / 2 / 1 spins a warp: 1000 spins 3.3 / 2.6 /
+    // 2.1 / 1.8 / 1.7 / 1.5; 4096 spins 3.4 / 3.0 / 2.6 / 2.2 / 2.1 / 1.7;
+    // 10,000 spins 3.7 / 3.1 / 2.7 / 2.3 / 2.3 / 2.5; 40,000 spins 3.9 / 3.4 /
+    // 3.2 / 3.7; 80,000 spins 4.1 / 3.9 / 4.6; 120,000 spins 4.7 / 4.8
+    a.perWarp = spins_per_warp(S.N, 33);
+    const uint32_t* order = nullptr;
+    if (scratch.order) {
+        DSIM_CUDA_TRY(cudaMemsetAsync(scratch.count, 0, 8, st));
+        k_cyl_order<<<(S.N + 255) / 256, 256, 0, st>>>(S.N, g.nF, reinterpret_cast<const uint4*>(S.seed4),
+                                                       scratch.order, scratch.count);
+        order = scratch.order;
+        if (launches) *launches += 1;
+    }
     const uint32_t warps = (S.N + a.perWarp - 1) / a.perWarp;
     dim3 block(128), grid((warps + 3) / 4);
-    if (rng == kRngReplay) k_cyl_step<kRngReplay><<<grid, block, 0, st>>>(g, a, S);
-    else if (rng == kRngPhilox) k_cyl_step<kRngPhilox><<<grid, block, 0, st>>>(g, a, S);
-    else k_cyl_step<kRngPhiloxPerSpinKey><<<grid, block, 0, st>>>(g, a, S);
+    const bool thin = a.perWarp < 32;
+#define DSIM_CYL_STEP(R)                                                        \
+    do {                                                                        \
+        if (thin) k_cyl_step<R, true><<<grid, block, 0, st>>>(g, a, S, order);  \
+        else k_cyl_step<R, false><<<grid, block, 0, st>>>(g, a, S, order);      \
+    } while (0)
+    if (rng == kRngReplay) DSIM_CYL_STEP(kRngReplay);
+    else if (rng == kRngPhilox) DSIM_CYL_STEP(kRngPhilox);
+    else DSIM_CYL_STEP(kRngPhiloxPerSpinKey);
+#undef DSIM_CYL_STEP
     DSIM_CUDA_TRY(cudaGetLastError());
+    if (launches) *launches += 1;
     return kOk;
 }
 

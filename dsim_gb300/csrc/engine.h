@@ -217,6 +217,8 @@ struct CylDev {
     const float4* cube_fibers;  // per grid entry, its fiber's record inline (or null)
     uint32_t n, maxFPC;
     float L;
+    float inv;                  // 1 / cell edge, as the reference rounds it
+    double inv64;               // the same in double (FP64 form)
     uint32_t nF;                // number of fibers (index bound)
     // fine filter grid (or null): each grid cell split fineK^3 ways; a fine
     // cell lists, in list order, the positions of its grid cell's entries
@@ -232,6 +234,10 @@ struct CylSpinsDev {
     uint32_t* seed4;   // s0, s1, imo + 1 (0 = derive from w), inside fiber / nearest
     float* mag;        // or null (no T2 in the dSim2 GPU ABI)
     uint32_t N;
+};
+// scratch of a cylinder run: the spins' order (N words) and two counters, or null
+struct CylOrder {
+    uint32_t *order, *count;
 };
 struct CylStepArgs {
     float intraSd, extraSd, myelinSd;
@@ -251,9 +257,10 @@ struct CylStepArgs {
     uint32_t spinBase;    // added to the spin index in the Philox counter (replica shards)
     uint32_t perWarp;     // spins a warp advances (spins_per_warp; set by the launcher)
 };
-// rng: kRngPhilox (key0/key1), kRngPhiloxPerSpinKey (seed4.x/.y), kRngReplay
-int launch_cyl_step(const CylDev& g, const CylStepArgs& a, const CylSpinsDev& S, int rng,
-                    cudaStream_t st);
+// rng: kRngPhilox (key0/key1), kRngPhiloxPerSpinKey (seed4.x/.y), kRngReplay.
+// *launches: kernels launched
+int launch_cyl_step(const CylDev& g, const CylStepArgs& a, const CylSpinsDev& S, const CylOrder& scratch, int rng,
+                    cudaStream_t st, uint32_t* launches);
 
 // ---- host helpers --------------------------------------------------------
 const char* last_error_message();

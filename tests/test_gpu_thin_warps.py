@@ -1,7 +1,7 @@
 """Few spins: a warp then advances 1 to 16 of them instead of 32.  The spins'
 walks do not depend on how many share a warp: the first n of a large set
 equal, bit for bit, a set of those n alone, at counts around each change of
-the rule (152 SMs x 14 warps for meshes, x 17 for cylinders)."""
+the rule (152 SMs x 14 warps for meshes, x 33 for cylinders)."""
 import numpy as np
 import pytest
 
@@ -31,10 +31,10 @@ def test_mesh_walks_do_not_depend_on_spins_per_warp(engine, tmp_path, n):
         assert np.array_equal(a, b[:n] if a.ndim == 2 else b[:k * n])
 
 
-@pytest.mark.parametrize("n", [1, 31, 2584, 2585, 5169, 10337, 20673, 41345])
+@pytest.mark.parametrize("n", [1, 31, 5016, 5017, 10033, 20065, 40129, 80257])
 def test_cylinder_walks_do_not_depend_on_spins_per_warp(engine, tmp_path, n):
     from dsim_gb300.engine import Cylinders, Spins, cyl_params, cyl_run
-    case = CylCase(tmp_path, N=83000)
+    case = CylCase(tmp_path, N=161000)
     c = Cylinders.load(case.path, case.spaceScale)
     imo = np.full(case.N, 2, np.uint32)
     p = cyl_params(2.0, 2.0, 0.2, case.spaceScale, 70.0, 8.0, 80.0, case.permeability, case.inner, case.dt, case.pc)
