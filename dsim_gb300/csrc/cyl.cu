@@ -351,7 +351,7 @@ int launch_cyl_step(const CylDev& g, const CylStepArgs& args, const CylSpinsDev&
     // 2.1 / 1.8 / 1.7 / 1.5; 4096 spins 3.4 / 3.0 / 2.6 / 2.2 / 2.1 / 1.7;
     // 10,000 spins 3.7 / 3.1 / 2.7 / 2.3 / 2.3 / 2.5; 40,000 spins 3.9 / 3.4 /
     // 3.2 / 3.7; 80,000 spins 4.1 / 3.9 / 4.6; 120,000 spins 4.7 / 4.8
-    a.perWarp = spins_per_warp(S.N, 33);
+    a.perWarp = spins_per_warp(S.N, 33, true);
     const uint32_t* order = nullptr;
     if (scratch.order) {
         DSIM_CUDA_TRY(cudaMemsetAsync(scratch.count, 0, 8, st));

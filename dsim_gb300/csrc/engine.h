@@ -68,14 +68,17 @@ struct MeshStepArgs {
 };
 
 // Spins a warp advances: 32 while the spins give every SM `warpsPerSm` warps
-// or more, else the largest power of two below that still does.  With fewer
-// spins than the chip has lanes a step takes as long as one warp's chain, and
-// a warp's chain is the longer the more spins share it (mesh: their records
-// and reflections add up; cylinders: their branches do).
+// or more, else as few as keep the warps at that number.  With fewer spins than
+// the chip has lanes a step takes as long as one warp's chain, and a warp's
+// chain is the longer the more spins share it (mesh: their records and
+// reflections add up; cylinders: their branches do).  pow2: a power of two.
 static constexpr uint32_t kSmCount = 152;
-inline uint32_t spins_per_warp(uint32_t N, uint32_t warpsPerSm) {
+inline uint32_t spins_per_warp(uint64_t N, uint32_t warpsPerSm, bool pow2) {
+    const uint64_t warps = (uint64_t)kSmCount * warpsPerSm;
+    const uint32_t need = (uint32_t)(N >= 32 * warps ? 32 : (N + warps - 1) / warps);
+    if (!pow2) return need ? need : 1;
     uint32_t p = 1;
-    while (p < 32 && (N + p - 1) / p > kSmCount * warpsPerSm) p *= 2;
+    while (p < need) p *= 2;
     return p;
 }
 

@@ -152,11 +152,12 @@ int launch_mesh_step_flat(const MeshDev& g, const AccelDev& acc, const MeshStepA
                           const SpinsSorted& S, int rng, cudaStream_t st, int occupancy, bool queue, bool stage) {
     if (S.N == 0 || args.iterations == 0) return kOk;
     MeshStepArgs a = args;
-    // at most 14 warps per SM below 32 spins a warp.  us per step, 25 tubes
-    // with myelin, 32 / 16 / 8 / 4 / 2 / 1 spins a warp: 1000 spins 15.8 / 9.5
-    // / 6.6 / 4.9 / 4.1 / 3.9; 8192 spins 17.9 / 11.2 / 7.8 / 6.8 / 8.8 / 10.5;
-    // 32768 spins 19.0 / 13.8 / 14.7; 65536 spins 21.6 / 22.2
-    a.perWarp = spins_per_warp(S.N, 14);
+    // at most 16 warps per SM below 32 spins a warp.  us per step, 25 tubes
+    // with myelin, 32 / 16 / 8 / 4 / 2 / 1 spins a warp: 1000 spins 12.9 / 7.9 /
+    // 5.6 / 4.4 / 3.7 / 3.5; 8192 spins 14.0 / 9.3 / 6.8 / 6.1 / 8.2 / 9.8; 24,576
+    // spins 15.4 / 10.4 / 9.7 / 11.9; 40,960 spins 16.3 / 11.8 / 14.4; 65,536
+    // spins 17.6 / 18.9
+    a.perWarp = spins_per_warp(S.N, 16, false);
     const uint32_t warps = (S.N + a.perWarp - 1) / a.perWarp;
     dim3 block(kFlatThreads), grid((warps + kFlatWarps - 1) / kFlatWarps);
     // one instantiation per record layout keeps each kernel's registers to its own path
@@ -168,9 +169,18 @@ int launch_mesh_step_flat(const MeshDev& g, const AccelDev& acc, const MeshStepA
     } else if (acc.wide == 1 && stage) {
         k_mesh_step_flat<false, 6, 1, false, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
     } else if (acc.wide == 1 && queue) {
-        // 5 blocks per SM: 96 registers with no spills (at 6: 80 registers and
-        // 124 B of spills); 3 % faster on the 1M-spin walk
-        k_mesh_step_flat<false, 5, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
+        // Blocks per SM: 5 (96 registers, 40 B of spills) over many waves, and
+        // whichever of 4 (126 registers, no spills) to 7 (72) takes a small grid
+        // in one wave.  us per step on 100 tubes at 4 / 5 / 6 / 7: 65,536 spins
+        // (512 blocks) 10.3 / 10.9 / 13.1 / 13.7; 90,000 15.8 / 11.4 / 13.5 / 14.3;
+        // 100,000 16.4 / 16.4 / 13.8 / 14.5; 150,000 (two waves of 4) 18.5 / 19.4 /
+        // 22.6 / 23.3; 400,000 46.6 / 44.3 / 46.6 / 44.1; 1M spins on 2.56M
+        // triangles 120.8 / 111.3 / 117.0 / 114.3
+        const uint32_t perSm = (grid.x + kSmCount - 1) / kSmCount;
+        if (perSm <= 4 || perSm == 8) k_mesh_step_flat<false, 4, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
+        else if (perSm == 6) k_mesh_step_flat<false, 6, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
+        else if (perSm == 7) k_mesh_step_flat<false, 7, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
+        else k_mesh_step_flat<false, 5, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
     } else if (acc.wide == 1) {
         if (occupancy >= 8) k_mesh_step_flat<false, 8, 1><<<grid, block, 0, st>>>(g, acc, a, S, rng);
         else if (occupancy >= 6) k_mesh_step_flat<false, 6, 1><<<grid, block, 0, st>>>(g, acc, a, S, rng);

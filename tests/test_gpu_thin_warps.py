@@ -1,7 +1,8 @@
-"""Few spins: a warp then advances 1 to 16 of them instead of 32.  The spins'
-walks do not depend on how many share a warp: the first n of a large set
-equal, bit for bit, a set of those n alone, at counts around each change of
-the rule (152 SMs x 14 warps for meshes, x 33 for cylinders)."""
+"""Launch shapes: with few spins a warp advances fewer than 32 of them, and the
+mesh step picks its blocks per SM by the count.  The spins' walks do not depend
+on either: the first n of a large set equal, bit for bit, a set of those n
+alone, at counts around the changes of the rules (152 SMs x 16 warps for
+meshes, then 4 to 8 blocks of 128 per SM; x 33 warps for cylinders)."""
 import numpy as np
 import pytest
 
@@ -20,10 +21,10 @@ def _mesh(case, m, n):
     return (*s.get(), s.counts())
 
 
-@pytest.mark.parametrize("n", [1, 31, 2128, 2129, 4257, 8513, 17025, 34049])
+@pytest.mark.parametrize("n", [1, 31, 2433, 4865, 40961, 77825, 97281, 116737, 136193])
 def test_mesh_walks_do_not_depend_on_spins_per_warp(engine, tmp_path, n):
     from dsim_gb300.engine import Mesh
-    case = MeshCase(tmp_path, membranes="AM", N=70001)
+    case = MeshCase(tmp_path, membranes="AM", N=165001)
     m = Mesh.load(case.path, case.spaceScale)
     one, all_ = _mesh(case, m, n), _mesh(case, m, case.N)
     for a, b in zip(one, all_):
