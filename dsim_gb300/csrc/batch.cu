@@ -80,6 +80,35 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
     s = t;
 }
 
+// The warps of one kind of step kernel: first slot and number of slots (of one
+// job) of each, at most `per` (spins_per_warp over the kind's spins).  A launch
+// covers the kind's unfinished jobs only, whatever else the batch holds.
+struct StepWarps {
+    const uint2* warp;
+    uint32_t count, per;
+};
+
+// Draws for a warp whose lanes repeat its `per` spins (a power of two; lane l
+// holds spin l mod per): every 32 / per steps all lanes draw at once, lane l for
+// its spin's step number l / per of the coming ones, and a step takes its draw
+// by shuffles.  live: the lanes with a spin.
+struct ThinDraws {
+    Draw drawn;
+    __device__ __forceinline__ Draw step(uint32_t it, uint32_t per, uint32_t lane, uint32_t live, uint32_t id,
+                                         uint32_t step0, uint32_t k0, uint32_t k1) {
+        const uint32_t lg = 31u - __clz(per), k = it & ((32u >> lg) - 1u);
+        if (k == 0) drawn = philox_draw(id, (uint64_t)(step0 + it + (lane >> lg)), 0u, k0, k1);
+        if (per == 32) return drawn;
+        const uint32_t from = (k << lg) + (lane & (per - 1u));
+        Draw d;
+        d.nx = __shfl_sync(live, drawn.nx, from);
+        d.ny = __shfl_sync(live, drawn.ny, from);
+        d.nz = __shfl_sync(live, drawn.nz, from);
+        d.u = __shfl_sync(live, drawn.u, from);
+        return d;
+    }
+};
+
 // The plain form has one instantiation per fine-grid record layout (LAYOUT 1:
 // 32-byte, 2: 64-byte records), each advancing only the mesh jobs whose
 // substrate uses it, and one for cylinder jobs (LAYOUT 3), so no kernel
@@ -89,7 +118,7 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
 // block shape of one occupancy has the same register budget per thread.
 template <int MINB, int LAYOUT, int THREADS = kFlatThreads>
 __global__ void __launch_bounds__(THREADS, MINB * kFlatThreads / THREADS)
-k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S,
+k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
              const uint32_t* __restrict__ stepNow, uint32_t chunk, uint32_t* status,
              unsigned long long* jobCounts) {
     constexpr int MESH = LAYOUT == 3 ? 1 : LAYOUT;  // the record path of the mesh instantiations
@@ -101,9 +130,14 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t tx = threadIdx.x;
     FlatWarp& H = wh[LAYOUT == 3 ? 0u : (threadIdx.x >> 5)];  // the cylinder path uses no table
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((i & ~31u) >= S.N) return;  // whole warp: N is a multiple of 32
-    const uint32_t jb = S.u[U_JOB][i & ~31u];
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= W.count) return;  // whole warp
+    // mesh: the lanes past the warp's spins help with the records; cylinders:
+    // they repeat the spins (ThinDraws)
+    const uint2 mine = __ldg(W.warp + w);
+    const uint32_t at = LAYOUT == 3 ? lane & (W.per - 1u) : lane;
+    const uint32_t i = mine.x + min(at, mine.y - 1u);
+    const uint32_t jb = S.u[U_JOB][mine.x];
     // the warp's job and substrate records, copied to shared memory once and
     // read from there (kept out of the collision loop's registers)
     __shared__ JobDev jobS[THREADS / 32];
@@ -120,16 +154,13 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
         __syncwarp();
     }
     const JobDev& J = jobS[wi];
-    if (J.flags & (DSIM_JOB_PRECISE | DSIM_JOB_LOCAL)) return;  // warp-uniform
-    if (LAYOUT == 3 ? subS[wi].kind != kSubCyl
-                    : (subS[wi].kind != kSubMesh || subS[wi].acc.wide != (uint32_t)LAYOUT)) return;
     const uint32_t now = *stepNow;
     const uint32_t start = J.start, steps = J.steps;
     if (now < start || now - start >= steps) return;  // not started or finished (warp-uniform)
     const uint32_t ls0 = now - start;
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
-    const bool valid = id != 0xFFFFFFFFu;
+    const bool valid = id != 0xFFFFFFFFu && at < mine.y;
     float x = S.f[F_X][i], y = S.f[F_Y][i], z = S.f[F_Z][i];
     mom[0][tx] = S.f[F_MX][i]; mom[1][tx] = S.f[F_MY][i]; mom[2][tx] = S.f[F_MZ][i];
     mom[3][tx] = S.f[F_CX][i]; mom[4][tx] = S.f[F_CY][i]; mom[5][tx] = S.f[F_CZ][i];
@@ -198,6 +229,8 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
             __syncwarp();
         }
     } else if (valid) {
+        const uint32_t live = __activemask();  // converged: the lanes with a spin
+        ThinDraws draws;
         const CylDev& g = sub.c;
         const float perm = J.perm;
         uint32_t imo = comp, nearest = fiber;
@@ -205,7 +238,7 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
         bool clear = false;
         if (imo < 2 && nearest >= g.nF) imo = 2;
         for (uint32_t it = 0; it < nsteps; it++) {
-            const Draw d = philox_draw(id, (uint64_t)(ls0 + it), 0u, k0, k1);
+            const Draw d = draws.step(it, W.per, lane, live, id, ls0, k0, k1);
             const float sdv = J.sd[imo];
             const P3<float> o = {x, y, z};
             P3<float> p = {x + d.nx * sdv, y + d.ny * sdv, z + d.nz * sdv};
@@ -222,7 +255,8 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
         comp = imo;
         fiber = nearest & 0xFFFFFFu;
     }
-    if (valid) {
+    const bool own = valid && lane == at;
+    if (own) {
         S.f[F_X][i] = x; S.f[F_Y][i] = y; S.f[F_Z][i] = z;
         S.f[F_MX][i] = mom[0][tx]; S.f[F_MY][i] = mom[1][tx]; S.f[F_MZ][i] = mom[2][tx];
         S.f[F_CX][i] = mom[3][tx]; S.f[F_CY][i] = mom[4][tx]; S.f[F_CZ][i] = mom[5][tx];
@@ -230,7 +264,7 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
         S.u[U_META][i] = (comp & 0xFFu) | (fiber << 8);
     }
     // per-job counters {reflections, permeations}: one atomic per warp
-    unsigned long long r = nrefl, p = nperm;
+    unsigned long long r = own ? nrefl : 0u, p = own ? nperm : 0u;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         r += __shfl_down_sync(FULL, r, o);
@@ -250,7 +284,7 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
 // rounded value (sort keys, float readers).
 template <int LAYOUT>
 __global__ void __launch_bounds__(kFlatThreads, 4)
-k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S,
+k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
                    const uint32_t* __restrict__ stepNow, uint32_t chunk, uint32_t* status,
                    unsigned long long* jobCounts) {
     __shared__ FlatWarp wh[kFlatWarps];
@@ -264,9 +298,11 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
     const uint32_t wi = threadIdx.x >> 5;
     FlatWarp& H = wh[wi];
     LocalWarp& Lw = wl[wi];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((i & ~31u) >= S.N) return;  // whole warp: N is a multiple of 32
-    const uint32_t jb = S.u[U_JOB][i & ~31u];
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= W.count) return;  // whole warp
+    const uint2 mine = __ldg(W.warp + w);
+    const uint32_t i = mine.x + min(lane, mine.y - 1u);
+    const uint32_t jb = S.u[U_JOB][mine.x];
     {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(jobs + jb);
         uint32_t* dst = reinterpret_cast<uint32_t*>(jobS + wi);
@@ -278,15 +314,13 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
         __syncwarp();
     }
     const JobDev& J = jobS[wi];
-    if (!(J.flags & DSIM_JOB_LOCAL) || subS[wi].kind != kSubMesh || subS[wi].acc.wide != (uint32_t)LAYOUT)
-        return;  // warp-uniform
     const uint32_t now = *stepNow;
     const uint32_t start = J.start, steps = J.steps;
     if (now < start || now - start >= steps) return;
     const uint32_t ls0 = now - start;
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
-    const bool valid = id != 0xFFFFFFFFu;
+    const bool valid = id != 0xFFFFFFFFu && lane < mine.y;
     // position = lattice origin (multiple of 1/16) + FP32 offset in [0, 1/16)
     float gx = 0.0f, gy = 0.0f, gz = 0.0f, x = 0.0f, y = 0.0f, z = 0.0f, mag = 0.0f;
     uint32_t comp = 0, fiber = 0;
@@ -401,7 +435,7 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
 // fields; the float fields receive their rounded values (sort keys, float
 // readers) and the moment pair (m, c) holds M as m - c.
 __global__ void __launch_bounds__(kFlatThreads, 2)
-k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S,
+k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
                const uint32_t* __restrict__ stepNow, uint32_t chunk, uint32_t* status,
                unsigned long long* jobCounts) {
     __shared__ FlatWarp wh[kFlatWarps];
@@ -413,9 +447,11 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
     const uint32_t wi = threadIdx.x >> 5;
     FlatWarp& H = wh[wi];
     PrecWarp& P = wp[wi];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((i & ~31u) >= S.N) return;  // whole warp: N is a multiple of 32
-    const uint32_t jb = S.u[U_JOB][i & ~31u];
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= W.count) return;  // whole warp
+    const uint2 mine = __ldg(W.warp + w);
+    const uint32_t i = mine.x + min(lane, mine.y - 1u);
+    const uint32_t jb = S.u[U_JOB][mine.x];
     {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(jobs + jb);
         uint32_t* dst = reinterpret_cast<uint32_t*>(jobS + wi);
@@ -427,14 +463,13 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
         __syncwarp();
     }
     const JobDev& J = jobS[wi];
-    if (!(J.flags & DSIM_JOB_PRECISE) || subS[wi].kind != kSubMesh) return;  // warp-uniform
     const uint32_t now = *stepNow;
     const uint32_t start = J.start, steps = J.steps;
     if (now < start || now - start >= steps) return;
     const uint32_t ls0 = now - start;
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
-    const bool valid = id != 0xFFFFFFFFu;
+    const bool valid = id != 0xFFFFFFFFu && lane < mine.y;
     double x = 0.0, y = 0.0, z = 0.0, mag = 0.0, Mx = 0.0, My = 0.0, Mz = 0.0;
     uint32_t comp = 0, fiber = 0;
     if (valid) {
@@ -703,6 +738,12 @@ struct BatchJob {
     uint64_t counts[2] = {0, 0};
 };
 
+// the step kernels: one per form and fine-grid record layout
+enum StepKind {
+    kStepMesh, kStepMeshFull, kStepCyl, kStepMeshLocal, kStepMeshLocalFull, kStepMesh64, kStepCyl64, kStepCylLocal,
+    kStepKinds
+};
+
 struct dsim_batch {
     cudaStream_t st = nullptr;
     // the step kernels of a chunk (one per record layout and form) advance
@@ -732,10 +773,15 @@ struct dsim_batch {
     uint32_t *hist = nullptr, *hstart = nullptr, *scratch = nullptr;
     uint64_t keyCap = 0, K = 0;
     uint32_t chunk = 20, occupancy = 4, graphChunks = 8;
+    bool chunkSet = false;  // dsim_batch_configure or the autotuner chose the chunk
     uint32_t blockThreads = kFlatThreads;  // block size of the plain step kernels (64, 128, 256)
-    bool anyPrecise = false, anyLocal = false;  // precision-form / cell-local mesh jobs
-    bool anyPreciseCyl = false;                 // precision-form cylinder jobs
-    bool anyLocalCyl = false;                   // cell-local cylinder jobs
+    // the warps of each kind of step kernel, as uploaded: built from the
+    // unfinished jobs
+    uint2* d_warps = nullptr;
+    size_t warpCap = 0;
+    StepWarps kinds[kStepKinds] = {};
+    uint32_t warpsAt = 0;     // stepNow when they were built
+    bool warpsValid = false;
     cudaGraphExec_t exec = nullptr;
     bool graphValid = false;
     int graphCur = -1;
@@ -809,26 +855,92 @@ int upload_jobs(dsim_batch* b) {
     return kOk;
 }
 
-// which plain step instantiations a chunk launches: bit 1 / 2 for mesh jobs
-// on 32- / 64-byte fine-grid records, bit 3 for cylinder jobs; bits 5 / 6 for
-// cell-local mesh jobs on 32- / 64-byte records
-uint32_t step_layouts(const dsim_batch* b) {
-    uint32_t mask = 0;
-    for (const auto& j : b->jobs) {
-        const SubDev& s = b->subs[j.d.sub];
-        if (s.kind == kSubCyl) { if (!j.d.flags) mask |= 1u << 3; }
-        else if (!j.d.flags) mask |= 1u << (s.acc.wide == 2 ? 2u : 1u);
-        else if (j.d.flags & DSIM_JOB_LOCAL) mask |= 1u << (s.acc.wide == 2 ? 6u : 5u);
-    }
-    return mask;
+StepKind kind_of(const dsim_batch* b, const BatchJob& j) {
+    const SubDev& s = b->subs[j.d.sub];
+    const bool cyl = s.kind == kSubCyl, full = s.acc.wide == 2;
+    if (j.d.flags & DSIM_JOB_PRECISE) return cyl ? kStepCyl64 : kStepMesh64;
+    if (j.d.flags & DSIM_JOB_LOCAL) return cyl ? kStepCylLocal : (full ? kStepMeshLocalFull : kStepMeshLocal);
+    return cyl ? kStepCyl : (full ? kStepMeshFull : kStepMesh);
 }
 
-// kernels one chunk launches: keys, scan (3), scatter, the step
-// instantiations, advance
+bool job_finished(const dsim_batch* b, const BatchJob& j) {
+    return b->stepNow >= j.d.start && b->stepNow - j.d.start >= j.d.steps;
+}
+
+// Warps per SM below which a kind's warps hold fewer than 32 spins.  us per step
+// at 32 / 16 / 8 / 4 / 2 spins a warp: FP32 mesh 16,384 spins 12.2 / 8.4 / 6.5 /
+// 7.9 / 11.2, 32,768 13.7 / 9.2 / 10.2; cell-local mesh 16,384 17.0 / 13.0 / 10.4 /
+// 13.1, 32,768 18.8 / 14.7 / 18.5; FP64 mesh 4096 26.8 / 19.8 / 15.8 / 14.5 / 17.7,
+// 16,384 32.3 / 28.7 / 31.6; FP32 cylinders 16,384 6.3 / 5.7 / 4.0 / 3.4 / 3.9,
+// 49,152 8.5 / 6.7 / 5.8 / 6.3; cell-local cylinders 32,768 11.4 / 8.6 / 7.3 / 7.4;
+// FP64 cylinders 4096 28.9 / 20.2 / 17.9 / 16.2 / 20.6, 32,768 48.5 / 46.7 / 52.3
+uint32_t warps_per_sm(StepKind k) {
+    switch (k) {
+        case kStepCyl: case kStepCylLocal: return 41;
+        case kStepMesh64: case kStepCyl64: return 8;
+        default: return 16;
+    }
+}
+uint32_t spins_per_warp_of(StepKind k, uint64_t spins) {
+    return spins_per_warp(spins, warps_per_sm(k), k == kStepCyl || k == kStepCylLocal || k == kStepCyl64);
+}
+
+// lists the warps of the unfinished jobs by kind
+int build_warps(dsim_batch* b) {
+    std::vector<uint2> list;
+    size_t first[kStepKinds];
+    uint64_t spins[kStepKinds] = {};
+    for (const auto& j : b->jobs)
+        if (!job_finished(b, j)) spins[kind_of(b, j)] += j.nSpins;
+    for (int k = 0; k < kStepKinds; k++) {
+        first[k] = list.size();
+        const uint32_t per = spins_per_warp_of((StepKind)k, spins[k]);
+        for (const auto& j : b->jobs) {
+            if (job_finished(b, j) || kind_of(b, j) != (StepKind)k) continue;
+            for (uint32_t q = 0; q < j.pad; q += per)
+                list.push_back(make_uint2((uint32_t)j.slot0 + q, std::min(per, j.pad - q)));
+        }
+        b->kinds[k].count = (uint32_t)(list.size() - first[k]);
+        b->kinds[k].per = per;
+    }
+    if (list.size() > b->warpCap) {
+        cudaFree(b->d_warps);
+        b->bytes -= b->warpCap * sizeof(uint2);
+        b->d_warps = nullptr; b->warpCap = 0;
+        const size_t cap = std::max<size_t>(list.size() * 2, 1024);
+        int rc = balloc(b, (void**)&b->d_warps, cap * sizeof(uint2));
+        if (rc) return rc;
+        b->warpCap = cap;
+    }
+    for (int k = 0; k < kStepKinds; k++) b->kinds[k].warp = b->d_warps + first[k];
+    if (!list.empty())
+        DSIM_CUDA_TRY(cudaMemcpyAsync(b->d_warps, list.data(), list.size() * sizeof(uint2), cudaMemcpyHostToDevice, b->st));
+    b->warpsAt = b->stepNow;
+    b->warpsValid = true;
+    invalidate_graph(b);
+    return kOk;
+}
+
+// builds them when jobs came or went, or when so many have finished that a
+// kind's warps should hold at most three quarters of the spins they do
+int ensure_warps(dsim_batch* b) {
+    bool stale = !b->warpsValid;
+    if (!stale && b->warpsAt != b->stepNow) {
+        uint64_t left[kStepKinds] = {};
+        for (const auto& j : b->jobs)
+            if (!job_finished(b, j)) left[kind_of(b, j)] += j.nSpins;
+        for (int k = 0; k < kStepKinds; k++)
+            stale = stale || (b->kinds[k].count > 0 &&
+                              (left[k] == 0 || 4 * spins_per_warp_of((StepKind)k, left[k]) <= 3 * b->kinds[k].per));
+    }
+    return stale ? build_warps(b) : kOk;
+}
+
+// kernels one chunk launches: keys, scan (3), scatter, the step kernels, advance
 uint64_t chunk_launches(const dsim_batch* b) {
-    const uint32_t mask = step_layouts(b);
-    return 5ull + (uint64_t)__builtin_popcount(mask & 0x6Eu) + (b->anyPrecise ? 1ull : 0ull) +
-           (b->anyPreciseCyl ? 1ull : 0ull) + (b->anyLocalCyl ? 1ull : 0ull) + 1ull;
+    uint64_t n = 6;
+    for (const StepWarps& W : b->kinds) n += W.count > 0;
+    return n;
 }
 
 // Precision-form cylinder jobs (DSIM_JOB_PRECISE): the dSim2 step of
@@ -837,27 +949,29 @@ uint64_t chunk_launches(const dsim_batch* b) {
 // parameters are the job's float values.  Position and magnitude persist in
 // the double fields; the moment is kept as the float pair m - c.
 __global__ void __launch_bounds__(kFlatThreads, 4)
-k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S,
+k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
                    const uint32_t* __restrict__ stepNow, uint32_t chunk, uint32_t* status,
                    unsigned long long* jobCounts) {
     const uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((i & ~31u) >= S.N) return;  // whole warp: N is a multiple of 32
-    const uint32_t jb = S.u[U_JOB][i & ~31u];
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= W.count) return;  // whole warp
+    const uint2 mine = __ldg(W.warp + w);
+    const uint32_t at = lane & (W.per - 1u), i = mine.x + min(at, mine.y - 1u);  // the lanes repeat the spins
+    const uint32_t jb = S.u[U_JOB][mine.x];
     const JobDev& J = jobs[jb];
-    if (!(__ldg(&J.flags) & DSIM_JOB_PRECISE)) return;  // warp-uniform
     const SubDev& sub = subs[__ldg(&J.sub)];
-    if (__ldg(&sub.kind) != kSubCyl) return;
     const uint32_t now = *stepNow;
     const uint32_t start = __ldg(&J.start), steps = __ldg(&J.steps);
     if (now < start || now - start >= steps) return;
     const uint32_t ls0 = now - start;
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
-    const bool valid = id != 0xFFFFFFFFu;
+    const bool valid = id != 0xFFFFFFFFu && at < mine.y;
     uint32_t nrefl = 0, nperm = 0, st = 0;
     if (valid) {
+        const uint32_t live = __activemask();  // converged: the lanes with a spin
+        ThinDraws draws;
         const CylDev g = sub.c;
         double x = S.d[D_X][i], y = S.d[D_Y][i], z = S.d[D_Z][i], mag = S.d[D_MAG][i];
         double Mx = (double)S.f[F_MX][i] - (double)S.f[F_CX][i];
@@ -874,7 +988,7 @@ k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
         const uint32_t k0 = __ldg(&J.key0), k1 = __ldg(&J.key1);
         const float* __restrict__ wave = J.wave;
         for (uint32_t it = 0; it < nsteps; it++) {
-            const Draw d = philox_draw(id, (uint64_t)(ls0 + it), 0u, k0, k1);
+            const Draw d = draws.step(it, W.per, lane, live, id, ls0, k0, k1);
             const double sd = (double)__ldg(&J.sd[imo == 0 ? 0 : (imo == 1 ? 1 : 2)]);
             const P3<double> o = {x, y, z};
             P3<double> p = {x + (double)d.nx * sd, y + (double)d.ny * sd, z + (double)d.nz * sd};
@@ -888,15 +1002,19 @@ k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
             const double w = (double)__ldg(wave + ls0 + it);
             Mx += w * x; My += w * y; Mz += w * z;
         }
-        S.d[D_X][i] = x; S.d[D_Y][i] = y; S.d[D_Z][i] = z; S.d[D_MAG][i] = mag;
-        S.f[F_X][i] = (float)x; S.f[F_Y][i] = (float)y; S.f[F_Z][i] = (float)z;
-        S.f[F_MAG][i] = (float)mag;
-        const float mx = (float)Mx, my = (float)My, mz = (float)Mz;
-        S.f[F_MX][i] = mx; S.f[F_MY][i] = my; S.f[F_MZ][i] = mz;
-        S.f[F_CX][i] = (float)((double)mx - Mx);
-        S.f[F_CY][i] = (float)((double)my - My);
-        S.f[F_CZ][i] = (float)((double)mz - Mz);
-        S.u[U_META][i] = (imo & 0xFFu) | ((nearest & 0xFFFFFFu) << 8);
+        if (lane == at) {
+            S.d[D_X][i] = x; S.d[D_Y][i] = y; S.d[D_Z][i] = z; S.d[D_MAG][i] = mag;
+            S.f[F_X][i] = (float)x; S.f[F_Y][i] = (float)y; S.f[F_Z][i] = (float)z;
+            S.f[F_MAG][i] = (float)mag;
+            const float mx = (float)Mx, my = (float)My, mz = (float)Mz;
+            S.f[F_MX][i] = mx; S.f[F_MY][i] = my; S.f[F_MZ][i] = mz;
+            S.f[F_CX][i] = (float)((double)mx - Mx);
+            S.f[F_CY][i] = (float)((double)my - My);
+            S.f[F_CZ][i] = (float)((double)mz - Mz);
+            S.u[U_META][i] = (imo & 0xFFu) | ((nearest & 0xFFFFFFu) << 8);
+        } else {
+            nrefl = nperm = 0;  // counted once
+        }
     }
     unsigned long long r = nrefl, p = nperm;
 #pragma unroll
@@ -917,30 +1035,32 @@ k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
 // (CylLocal), Kahan moments.  Between chunks the position is kept
 // in the double fields as origin + offset.
 __global__ void __launch_bounds__(kFlatThreads, 4)
-k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S,
+k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
                        const uint32_t* __restrict__ stepNow, uint32_t chunk, uint32_t* status,
                        unsigned long long* jobCounts) {
     __shared__ float mom[6][kFlatThreads];
     const uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t tx = threadIdx.x;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((i & ~31u) >= S.N) return;  // whole warp: N is a multiple of 32
-    const uint32_t jb = S.u[U_JOB][i & ~31u];
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= W.count) return;  // whole warp
+    const uint2 mine = __ldg(W.warp + w);
+    const uint32_t at = lane & (W.per - 1u), i = mine.x + min(at, mine.y - 1u);  // the lanes repeat the spins
+    const uint32_t jb = S.u[U_JOB][mine.x];
     const JobDev& J = jobs[jb];
-    if (!(__ldg(&J.flags) & DSIM_JOB_LOCAL)) return;  // warp-uniform
     const SubDev& sub = subs[__ldg(&J.sub)];
-    if (__ldg(&sub.kind) != kSubCyl) return;
     const uint32_t now = *stepNow;
     const uint32_t start = __ldg(&J.start), steps = __ldg(&J.steps);
     if (now < start || now - start >= steps) return;
     const uint32_t ls0 = now - start;
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
-    const bool valid = id != 0xFFFFFFFFu;
+    const bool valid = id != 0xFFFFFFFFu && at < mine.y;
     uint32_t nrefl = 0, nperm = 0, st = 0;
     CylLocal form = {__ldg(&J.inR), {0.0f, 0.0f, 0.0f}, 0u, 0u};
     if (valid) {
+        const uint32_t live = __activemask();  // converged: the lanes with a spin
+        ThinDraws draws;
         const CylDev g = sub.c;
         const double X = S.d[D_X][i], Y = S.d[D_Y][i], Z = S.d[D_Z][i];
         CylOrigin& G = form.G;
@@ -960,7 +1080,7 @@ k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict
         const uint32_t k0 = __ldg(&J.key0), k1 = __ldg(&J.key1);
         const float* __restrict__ wave = J.wave;
         for (uint32_t it = 0; it < nsteps; it++) {
-            const Draw d = philox_draw(id, (uint64_t)(ls0 + it), 0u, k0, k1);
+            const Draw d = draws.step(it, W.per, lane, live, id, ls0, k0, k1);
             const float sd = __ldg(&J.sd[imo < 3 ? imo : 2]);
             const P3<float> o = {x, y, z};
             P3<float> p = {x + d.nx * sd, y + d.ny * sd, z + d.nz * sd};
@@ -984,12 +1104,16 @@ k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict
             kahan_add(mom[2][tx], mom[5][tx], w * (G.z + z));
         }
         const double Xn = (double)G.x + (double)x, Yn = (double)G.y + (double)y, Zn = (double)G.z + (double)z;
-        S.d[D_X][i] = Xn; S.d[D_Y][i] = Yn; S.d[D_Z][i] = Zn; S.d[D_MAG][i] = (double)mag;
-        S.f[F_X][i] = (float)Xn; S.f[F_Y][i] = (float)Yn; S.f[F_Z][i] = (float)Zn;
-        S.f[F_MAG][i] = mag;
-        S.f[F_MX][i] = mom[0][tx]; S.f[F_MY][i] = mom[1][tx]; S.f[F_MZ][i] = mom[2][tx];
-        S.f[F_CX][i] = mom[3][tx]; S.f[F_CY][i] = mom[4][tx]; S.f[F_CZ][i] = mom[5][tx];
-        S.u[U_META][i] = (imo & 0xFFu) | ((nearest & 0xFFFFFFu) << 8);
+        if (lane == at) {
+            S.d[D_X][i] = Xn; S.d[D_Y][i] = Yn; S.d[D_Z][i] = Zn; S.d[D_MAG][i] = (double)mag;
+            S.f[F_X][i] = (float)Xn; S.f[F_Y][i] = (float)Yn; S.f[F_Z][i] = (float)Zn;
+            S.f[F_MAG][i] = mag;
+            S.f[F_MX][i] = mom[0][tx]; S.f[F_MY][i] = mom[1][tx]; S.f[F_MZ][i] = mom[2][tx];
+            S.f[F_CX][i] = mom[3][tx]; S.f[F_CY][i] = mom[4][tx]; S.f[F_CZ][i] = mom[5][tx];
+            S.u[U_META][i] = (imo & 0xFFu) | ((nearest & 0xFFFFFFu) << 8);
+        } else {
+            nrefl = nperm = form.ntests = form.nexact = 0;  // counted once
+        }
     }
     // per-job counters {reflections, permeations, distance tests, FP64 decisions}
     unsigned long long r = nrefl, p = nperm, te = form.ntests, ex = form.nexact;
@@ -1009,32 +1133,37 @@ k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict
     if (st) atomicOr(status, st);
 }
 
+uint32_t step_grid(const StepWarps& W, int threads) {
+    return (uint32_t)(((uint64_t)W.count * 32 + threads - 1) / threads);
+}
+
 template <int LAYOUT, int THREADS>
-void launch_step_shape(dsim_batch* b, const BatchSpins& D, cudaStream_t st) {
-    const uint32_t grid = (uint32_t)((b->N + THREADS - 1) / THREADS);
+void launch_step_shape(dsim_batch* b, const BatchSpins& D, const StepWarps& W, uint32_t steps, cudaStream_t st) {
+    const uint32_t grid = step_grid(W, THREADS);
     if (b->occupancy >= 8)
-        k_batch_step<8, LAYOUT, THREADS><<<grid, THREADS, 0, st>>>(b->d_subs, b->d_jobs, D, b->d_stepNow, b->chunk,
+        k_batch_step<8, LAYOUT, THREADS><<<grid, THREADS, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
                                                                   b->d_status, b->d_counts);
     else if (b->occupancy >= 6)
-        k_batch_step<6, LAYOUT, THREADS><<<grid, THREADS, 0, st>>>(b->d_subs, b->d_jobs, D, b->d_stepNow, b->chunk,
+        k_batch_step<6, LAYOUT, THREADS><<<grid, THREADS, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
                                                                   b->d_status, b->d_counts);
     else if (b->occupancy == 5)
-        k_batch_step<5, LAYOUT, THREADS><<<grid, THREADS, 0, st>>>(b->d_subs, b->d_jobs, D, b->d_stepNow, b->chunk,
+        k_batch_step<5, LAYOUT, THREADS><<<grid, THREADS, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
                                                                   b->d_status, b->d_counts);
     else
-        k_batch_step<4, LAYOUT, THREADS><<<grid, THREADS, 0, st>>>(b->d_subs, b->d_jobs, D, b->d_stepNow, b->chunk,
+        k_batch_step<4, LAYOUT, THREADS><<<grid, THREADS, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
                                                                   b->d_status, b->d_counts);
 }
 
 template <int LAYOUT>
-void launch_step_layout(dsim_batch* b, const BatchSpins& D, cudaStream_t st) {
-    if (b->blockThreads == 64) launch_step_shape<LAYOUT, 64>(b, D, st);
-    else if (b->blockThreads == 256) launch_step_shape<LAYOUT, 256>(b, D, st);
-    else launch_step_shape<LAYOUT, kFlatThreads>(b, D, st);
+void launch_step_layout(dsim_batch* b, const BatchSpins& D, const StepWarps& W, uint32_t steps, cudaStream_t st) {
+    if (b->blockThreads == 64) launch_step_shape<LAYOUT, 64>(b, D, W, steps, st);
+    else if (b->blockThreads == 256) launch_step_shape<LAYOUT, 256>(b, D, W, steps, st);
+    else launch_step_shape<LAYOUT, kFlatThreads>(b, D, W, steps, st);
 }
 
-// one chunk: sort into the other buffer, step, advance the step counter
-int enqueue_chunk(dsim_batch* b) {
+// sort into the other buffer, `steps` steps, advance the step counter; the
+// warps are current (ensure_warps)
+int enqueue_chunk(dsim_batch* b, uint32_t steps) {
     const uint32_t N = (uint32_t)b->N;
     const uint32_t nb = (N + 255) / 256;
     BatchSpins S = view(b, b->cur), D = view(b, 1 - b->cur);
@@ -1045,46 +1174,41 @@ int enqueue_chunk(dsim_batch* b) {
     DSIM_CUDA_TRY(cudaMemsetAsync(b->hist, 0, b->K * 4, b->st));
     k_batch_scatter<<<nb, 256, 0, b->st>>>(S, D, b->keys, b->hstart, b->hist);
     b->cur = 1 - b->cur;
-    const uint32_t grid = (N + kFlatThreads - 1) / kFlatThreads;
-    const uint32_t mask = step_layouts(b);
     // the step kernels this chunk needs, each on its own stream when there
     // are several (they advance disjoint jobs)
-    int kinds[8], nk = 0;
-    for (int L = 1; L <= 3; L++)
-        if (mask & (1u << L)) kinds[nk++] = L;
-    for (int L = 5; L <= 6; L++)
-        if (mask & (1u << L)) kinds[nk++] = 4 + 4 * (L - 5);  // 4, 8: cell-local mesh, 32- / 64-byte records
-    if (b->anyPrecise) kinds[nk++] = 5;
-    if (b->anyPreciseCyl) kinds[nk++] = 6;
-    if (b->anyLocalCyl) kinds[nk++] = 7;
+    int kinds[kStepKinds], nk = 0;
+    for (int k = 0; k < kStepKinds; k++)
+        if (b->kinds[k].count > 0) kinds[nk++] = k;
     const bool fork = nk > 1;
     if (fork) DSIM_CUDA_TRY(cudaEventRecord(b->forkEv, b->st));
     for (int q = 0; q < nk; q++) {
         cudaStream_t st = fork ? b->side[q % dsim_batch::kSide] : b->st;
         if (fork) DSIM_CUDA_TRY(cudaStreamWaitEvent(st, b->forkEv, 0));
+        const StepWarps& W = b->kinds[kinds[q]];
+        const uint32_t grid = step_grid(W, kFlatThreads);
         switch (kinds[q]) {
-            case 1: launch_step_layout<1>(b, D, st); break;
-            case 2: launch_step_layout<2>(b, D, st); break;
-            case 3: launch_step_layout<3>(b, D, st); break;
-            case 4:
-                k_batch_step_local<1><<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, b->d_stepNow,
-                                                                     b->chunk, b->d_status, b->d_counts);
+            case kStepMesh: launch_step_layout<1>(b, D, W, steps, st); break;
+            case kStepMeshFull: launch_step_layout<2>(b, D, W, steps, st); break;
+            case kStepCyl: launch_step_layout<3>(b, D, W, steps, st); break;
+            case kStepMeshLocal:
+                k_batch_step_local<1><<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
+                                                                     b->d_status, b->d_counts);
                 break;
-            case 8:
-                k_batch_step_local<2><<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, b->d_stepNow,
-                                                                     b->chunk, b->d_status, b->d_counts);
+            case kStepMeshLocalFull:
+                k_batch_step_local<2><<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
+                                                                     b->d_status, b->d_counts);
                 break;
-            case 5:
-                k_batch_step64<<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, b->d_stepNow, b->chunk,
+            case kStepMesh64:
+                k_batch_step64<<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
                                                               b->d_status, b->d_counts);
                 break;
-            case 6:
-                k_batch_step_cyl64<<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, b->d_stepNow, b->chunk,
+            case kStepCyl64:
+                k_batch_step_cyl64<<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
                                                                   b->d_status, b->d_counts);
                 break;
             default:
-                k_batch_step_cyl_local<<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, b->d_stepNow,
-                                                                      b->chunk, b->d_status, b->d_counts);
+                k_batch_step_cyl_local<<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
+                                                                      b->d_status, b->d_counts);
                 break;
         }
         if (fork) {
@@ -1092,9 +1216,9 @@ int enqueue_chunk(dsim_batch* b) {
             DSIM_CUDA_TRY(cudaStreamWaitEvent(b->st, b->joinEv[q % dsim_batch::kSide], 0));
         }
     }
-    k_batch_advance<<<1, 1, 0, b->st>>>(b->d_stepNow, b->chunk);
+    k_batch_advance<<<1, 1, 0, b->st>>>(b->d_stepNow, steps);
     DSIM_CUDA_TRY(cudaGetLastError());
-    b->launches += chunk_launches(b);  // keys, scan (3), scatter, step (per layout), advance
+    b->launches += chunk_launches(b);
     return kOk;
 }
 
@@ -1107,7 +1231,7 @@ int capture_graph(dsim_batch* b) {
     cudaGraph_t graph = nullptr;
     DSIM_CUDA_TRY(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
     int rc = kOk;
-    for (uint32_t c = 0; c < G && !rc; c++) rc = enqueue_chunk(b);
+    for (uint32_t c = 0; c < G && !rc; c++) rc = enqueue_chunk(b, b->chunk);
     cudaError_t e = cudaStreamEndCapture(b->st, &graph);
     b->cur = cur0;
     b->launches = launches0;
@@ -1119,10 +1243,6 @@ int capture_graph(dsim_batch* b) {
     b->graphValid = true;
     b->graphCur = cur0;
     return kOk;
-}
-
-bool job_finished(const dsim_batch* b, const BatchJob& j) {
-    return b->stepNow >= j.d.start && b->stepNow - j.d.start >= j.d.steps;
 }
 
 BatchJob* find_job(dsim_batch* b, uint32_t id) {
@@ -1205,7 +1325,7 @@ void dsim_batch_free(dsim_batch* b) {
     }
     for (auto& j : b->jobs) cudaFree(j.wave);
     cudaFree(b->keys); cudaFree(b->hist); cudaFree(b->hstart); cudaFree(b->scratch);
-    cudaFree(b->d_jobs); cudaFree(b->d_subs); cudaFree(b->d_counts); cudaFree(b->d_status);
+    cudaFree(b->d_jobs); cudaFree(b->d_warps); cudaFree(b->d_subs); cudaFree(b->d_counts); cudaFree(b->d_status);
     cudaFree(b->d_stepNow);
     if (b->st) cudaStreamDestroy(b->st);
     for (int k = 0; k < dsim_batch::kSide; k++) {
@@ -1375,9 +1495,7 @@ int dsim_batch_submit(dsim_batch* b, const dsim_job_desc* d, const float* pos3, 
     if ((rc = layout_keys(b)) || (rc = upload_jobs(b))) return rc;
     DSIM_CUDA_TRY(cudaMemsetAsync(b->d_counts + 4 * jobIndex, 0, 32, b->st));
     DSIM_CUDA_TRY(cudaStreamSynchronize(b->st));
-    if (J.flags & DSIM_JOB_PRECISE) (cyl ? b->anyPreciseCyl : b->anyPrecise) = true;
-    if (J.flags & DSIM_JOB_LOCAL) (cyl ? b->anyLocalCyl : b->anyLocal) = true;
-    invalidate_graph(b);
+    b->warpsValid = false;
     *jobId = j.id;
     return kOk;
 }
@@ -1388,6 +1506,7 @@ int dsim_batch_configure(dsim_batch* b, uint32_t chunk, uint32_t occupancy, uint
         return kErrInvalid;
     }
     b->chunk = chunk;
+    b->chunkSet = true;
     b->occupancy = occupancy;
     b->graphChunks = graphChunks;
     invalidate_graph(b);
@@ -1420,16 +1539,45 @@ static uint32_t remaining_steps(const dsim_batch* b) {
     return r;
 }
 
+// Steps of the next launch when the caller left the chunk to the batch: up to
+// kLongChunk (a sort and a launch cost as much as a few steps, and a launch's
+// wait for its slowest warp is paid once), but not far past the end of a job,
+// so that the others' warps are listed again without it.
+static uint32_t long_chunk(const dsim_batch* b, uint32_t steps) {
+    constexpr uint32_t kLongChunk = 1000, kShortest = 100;
+    uint32_t n = std::min(steps, kLongChunk);
+    for (const auto& j : b->jobs) {
+        if (job_finished(b, j)) continue;
+        const uint32_t left = j.d.steps - (b->stepNow - j.d.start);
+        if (left >= kShortest && left < n) n = left;
+    }
+    n = std::max(n, std::min(steps, kShortest));
+    return n;
+}
+
 int dsim_batch_advance(dsim_batch* b, uint32_t steps) {
     if (!b) return kErrInvalid;
     if (b->N == 0 || steps == 0) return kOk;
     uint32_t chunks = (steps + b->chunk - 1) / b->chunk;
+    if (!b->chunkSet) {
+        uint32_t left = chunks * b->chunk;  // whole default chunks, as documented
+        while (left > 0) {
+            int rc = ensure_warps(b);
+            if (rc) return rc;
+            const uint32_t n = long_chunk(b, left);
+            if ((rc = enqueue_chunk(b, n))) return rc;
+            b->stepNow += n;
+            left -= n;
+        }
+        return kOk;
+    }
     const uint32_t G = b->graphChunks & ~1u;
     while (chunks > 0) {
+        int rc = ensure_warps(b);
+        if (rc) return rc;
         if (G > 0 && chunks >= G) {
             if (!b->graphValid || b->graphCur != b->cur) {
-                int rc = capture_graph(b);
-                if (rc) return rc;
+                if ((rc = capture_graph(b))) return rc;
             }
             DSIM_CUDA_TRY(cudaGraphLaunch(b->exec, b->st));
             b->graphLaunches++;
@@ -1437,8 +1585,7 @@ int dsim_batch_advance(dsim_batch* b, uint32_t steps) {
             b->stepNow += G * b->chunk;
             chunks -= G;
         } else {
-            int rc = enqueue_chunk(b);
-            if (rc) return rc;
+            if ((rc = enqueue_chunk(b, b->chunk))) return rc;
             b->stepNow += b->chunk;
             chunks--;
         }
@@ -1658,12 +1805,7 @@ int dsim_batch_compact(dsim_batch* b) {
     b->cur = 1 - b->cur;
     b->jobs = kept;
     b->N = slot;
-    b->anyPrecise = b->anyLocal = b->anyPreciseCyl = b->anyLocalCyl = false;
-    for (const auto& j : b->jobs) {
-        const bool jc = b->subs[j.d.sub].kind == kSubCyl;
-        (jc ? b->anyPreciseCyl : b->anyPrecise) |= (j.d.flags & DSIM_JOB_PRECISE) != 0;
-        (jc ? b->anyLocalCyl : b->anyLocal) |= (j.d.flags & DSIM_JOB_LOCAL) != 0;
-    }
+    b->warpsValid = false;
     if ((rc = layout_keys(b)) || (rc = upload_jobs(b))) return rc;
     if (!newCounts.empty())
         DSIM_CUDA_TRY(cudaMemcpyAsync(b->d_counts, newCounts.data(), newCounts.size() * 8, cudaMemcpyHostToDevice, b->st));
@@ -1714,6 +1856,7 @@ int dsim_batch_autotune(dsim_batch* b, uint32_t trialSteps, uint32_t best[3], fl
             e = cudaMemcpyAsync(b->buf[b->cur].d[f], snap + (size_t)(kBF + kBU + 2 * f) * b->N, b->N * 8,
                                 cudaMemcpyDeviceToDevice, b->st);
         b->stepNow = step0;
+        b->warpsValid = false;  // jobs that finished in the trial run again
         if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_stepNow, &b->stepNow, 4, cudaMemcpyHostToDevice, b->st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_counts, counts0.data(), 32 * nj, cudaMemcpyHostToDevice, b->st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);
@@ -1733,6 +1876,7 @@ int dsim_batch_autotune(dsim_batch* b, uint32_t trialSteps, uint32_t best[3], fl
     float bestT = 3.4e38f;
     uint32_t bg = 0, bo = b->occupancy, bc = b->chunk;
     const uint32_t graph0 = b->graphChunks;
+    b->chunkSet = true;  // the candidates' chunks, and then the best one
     cudaError_t e = save();
     auto set_grid = [&](uint32_t halves) -> int {
         for (size_t k = 0; k < b->meshes.size(); k++) {
