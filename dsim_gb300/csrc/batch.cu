@@ -655,65 +655,139 @@ __global__ void k_batch_gather64(BatchSpins S, uint32_t slot0, uint32_t len, dou
     mag[id] = S.d[D_MAG][i];
 }
 
-// FP64 signal of one job for nG gradients: partial records per (block, g)
+// ---- readout -------------------------------------------------------------------
+// sin and cos of 2 pi k / kTrig, each in two parts (trig_table)
+static constexpr uint32_t kTrig = 1024;
+struct __align__(16) Trig {
+    double s, c, sLo, cLo;
+};
+
+// sin and cos of the angle p.  n is the integer nearest p kTrig / 2 pi (adding
+// and subtracting 1.5 * 2^52 rounds, and leaves n's low bits in the sum's), and
+// r = p - n 2 pi / kTrig with the step in two parts, at most pi / kTrig: the
+// angle's table entry for n and the Taylor polynomials of sin r to r^5 and
+// cos r - 1 to r^4 (next terms below 6e-22 and 2e-18), joined by the addition
+// theorem with the table's value added last.  With the phase's fused sum the
+// error against 128 bits is no larger than that of sincos() of the separately
+// rounded phase (phases to 0.1, 1, 10, 1000, rms: 3.2e-17, 3.8e-17, 1.8e-16,
+// 1.7e-14 against 3.2e-17, 3.8e-17, 2.1e-16, 2.1e-14).  18 FP64 operations; sincos() takes about
+// 30, and the FP64 pipe (1/64 of the FP32 rate) is the readout's bound.
+// Beyond 2^40 (and for no number) sincos() itself.
+__device__ __forceinline__ void sincos_table(double p, const Trig* __restrict__ table, double& s, double& c) {
+    constexpr double kHi = 6.283185307179586232 / (double)kTrig, kLo = 2.4492935982947064e-16 / (double)kTrig;
+    constexpr double kMagic = 6755399441055744.0;
+    if (((uint32_t)__double2hiint(p) & 0x7FFFFFFFu) >= 0x42700000u) {
+        sincos(p, &s, &c);
+        return;
+    }
+    const double q = __fma_rn(p, 1.0 / kHi, kMagic);
+    const Trig T = table[(uint32_t)__double2loint(q) & (kTrig - 1u)];
+    const double n = __dsub_rn(q, kMagic);
+    const double r = __fma_rn(-n, kLo, __fma_rn(-n, kHi, p));
+    const double z = __dmul_rn(r, r);
+    const double sr = __fma_rn(__fma_rn(z, 1.0 / 120.0, -1.0 / 6.0), __dmul_rn(r, z), r);
+    const double cr = __dmul_rn(z, __fma_rn(z, 1.0 / 24.0, -0.5));  // cos r - 1
+    s = __dadd_rn(T.s, __fma_rn(T.c, sr, __fma_rn(T.s, cr, T.sLo)));
+    c = __dadd_rn(T.c, __fma_rn(-T.s, sr, __fma_rn(T.c, cr, T.cLo)));
+}
+
+// Readout of one job for nG gradients sharing its waveform.  Warp w takes the
+// 32 gradients [32 (w % gw), 32 (w % gw) + 32) and the spins of segment w / gw
+// (contiguous slots): each lane keeps its own gradient's sums in registers, so
+// no per-gradient reduction across threads is needed.  32 spins at a time, each
+// lane fetches one and puts its FP64 moments and magnitude in shared memory
+// (one conversion per spin and warp), then all lanes take them in turn.
+// partials[segment][gradient][15] = {X, Y, n} for all spins and per compartment,
+// each summed in slot order; k_batch_signal_final adds the segments in a fixed
+// order, so the result does not depend on the launch.  kg: gradients in units of
+// the table's angle.  fp64: the job keeps FP64 positions and magnitudes
+// (precision and cell-local forms), which the readout then uses.
+//
+// Bound by the FP64 pipe: 23 operations per spin and gradient where the first
+// form took about 48 (the spin's conversions on every lane, sincos, two sums).
+// 65,537 spins x 384 gradients: 2.43 -> 1.10 ms a call.
 static constexpr int kSigThreads = 128;
-// Readout of one job for nG gradients sharing its waveform.  Warp w takes
-// the 32 gradients [32 (w % gw), 32 (w % gw) + 32) and the spins of segment
-// w / gw (contiguous slots): its lanes read each spin once (one address: a
-// broadcast load) and each lane keeps its own gradient's sums in registers,
-// so no per-gradient reduction across threads is needed.  partials[segment]
-// [gradient][15] = {X, Y, n} for all spins and per compartment, each summed in
-// slot order; k_batch_signal_final adds the segments in order, so the result
-// does not depend on the launch.  fp64: the job keeps FP64 positions and
-// magnitudes (precision and cell-local forms), which the readout then uses.
+struct SigWarp {
+    double x[32], y[32], z[32], m[32];
+    uint32_t comp[32];
+};
 __global__ void __launch_bounds__(kSigThreads) k_batch_signal(BatchSpins S, uint32_t slot0, uint32_t len,
                                                               const double* __restrict__ kg, uint32_t nG,
                                                               uint32_t gw, uint32_t nseg, uint32_t segLen,
-                                                              double region, bool fp64, double* partials) {
+                                                              double region, bool fp64,
+                                                              const Trig* __restrict__ trig, double* partials) {
+    __shared__ Trig table[kTrig];
+    __shared__ SigWarp sw[kSigThreads / 32];
+    for (uint32_t k = threadIdx.x; k < 2 * kTrig; k += kSigThreads)
+        reinterpret_cast<double2*>(table)[k] = __ldg(reinterpret_cast<const double2*>(trig) + k);
+    __syncthreads();
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     if (warp >= gw * nseg) return;  // whole warps
+    SigWarp& W = sw[threadIdx.x >> 5];
     const uint32_t gi = (warp % gw) * 32u + lane, sg = warp / gw;
     const bool live = gi < nG;
     const double gx = live ? kg[3 * gi] : 0.0, gy = live ? kg[3 * gi + 1] : 0.0, gz = live ? kg[3 * gi + 2] : 0.0;
-    double X = 0.0, Y = 0.0, cX[4] = {0.0, 0.0, 0.0, 0.0}, cY[4] = {0.0, 0.0, 0.0, 0.0};
-    uint32_t n = 0, cn[4] = {0u, 0u, 0u, 0u};
+    double cX[4] = {0.0, 0.0, 0.0, 0.0}, cY[4] = {0.0, 0.0, 0.0, 0.0};
+    uint32_t cn[4] = {0u, 0u, 0u, 0u};
     const uint32_t k0 = sg * segLen, k1 = min(len, k0 + segLen);
-    for (uint32_t k = k0; k < k1; k++) {  // the same spin on every lane: warp-uniform branches
-        const uint32_t i = slot0 + k;
-        if (S.u[U_ID][i] == 0xFFFFFFFFu) continue;
-        if (region > 0.0) {  // dSim2's readout box (dSim2/src/spinSystem.cpp:944-978)
+    for (uint32_t kb = k0; kb < k1; kb += 32) {
+        const uint32_t i = slot0 + min(kb + lane, k1 - 1u);
+        bool in = kb + lane < k1 && S.u[U_ID][i] != 0xFFFFFFFFu;
+        if (in && region > 0.0) {  // dSim2's readout box (dSim2/src/spinSystem.cpp:944-978)
             const double x = fp64 ? S.d[D_X][i] : (double)S.f[F_X][i];
             const double y = fp64 ? S.d[D_Y][i] : (double)S.f[F_Y][i];
             const double z = fp64 ? S.d[D_Z][i] : (double)S.f[F_Z][i];
-            if (!(x > -region && x < region && y > -region && y < region && z > -region && z < region)) continue;
+            in = x > -region && x < region && y > -region && y < region && z > -region && z < region;
         }
-        const double Mx = (double)S.f[F_MX][i] - (double)S.f[F_CX][i];
-        const double My = (double)S.f[F_MY][i] - (double)S.f[F_CY][i];
-        const double Mz = (double)S.f[F_MZ][i] - (double)S.f[F_CZ][i];
-        const double m = fp64 ? S.d[D_MAG][i] : (double)S.f[F_MAG][i];
-        const uint32_t comp = S.u[U_META][i] & 3u;
-        double sn, cs;
-        sincos(gx * Mx + gy * My + gz * Mz, &sn, &cs);
-        const double xs = m * cs, ys = m * sn;
-        X += xs; Y += ys; n++;
-        if (comp == 0) { cX[0] += xs; cY[0] += ys; cn[0]++; }
-        else if (comp == 1) { cX[1] += xs; cY[1] += ys; cn[1]++; }
-        else if (comp == 2) { cX[2] += xs; cY[2] += ys; cn[2]++; }
-        else { cX[3] += xs; cY[3] += ys; cn[3]++; }
+        const uint32_t some = __ballot_sync(0xFFFFFFFFu, in);
+        __syncwarp();  // the previous spins have been read
+        if (in) {
+            const uint32_t at = __popc(some & ((1u << lane) - 1u));
+            W.x[at] = (double)S.f[F_MX][i] - (double)S.f[F_CX][i];
+            W.y[at] = (double)S.f[F_MY][i] - (double)S.f[F_CY][i];
+            W.z[at] = (double)S.f[F_MZ][i] - (double)S.f[F_CZ][i];
+            W.m[at] = fp64 ? S.d[D_MAG][i] : (double)S.f[F_MAG][i];
+            W.comp[at] = S.u[U_META][i] & 3u;
+        }
+        __syncwarp();
+        const uint32_t n = __popc(some);
+        for (uint32_t k = 0; k < n; k++) {  // the same spin on every lane: warp-uniform branches
+            const double m = W.m[k];
+            const uint32_t comp = W.comp[k];
+            double sn, cs;
+            sincos_table(__fma_rn(gx, W.x[k], __fma_rn(gy, W.y[k], __dmul_rn(gz, W.z[k]))), table, sn, cs);
+#pragma unroll
+            for (uint32_t q = 0; q < 4; q++)
+                if (comp == q) {
+                    cX[q] = __fma_rn(m, cs, cX[q]);
+                    cY[q] = __fma_rn(m, sn, cY[q]);
+                    cn[q]++;
+                }
+        }
     }
     if (!live) return;
     double* o = partials + ((size_t)sg * nG + gi) * 15;
-    o[0] = X; o[1] = Y; o[2] = (double)n;
+    o[0] = (cX[0] + cX[1]) + (cX[2] + cX[3]);
+    o[1] = (cY[0] + cY[1]) + (cY[2] + cY[3]);
+    o[2] = (double)(cn[0] + cn[1] + cn[2] + cn[3]);
 #pragma unroll
     for (int q = 0; q < 4; q++) { o[3 + 3 * q] = cX[q]; o[4 + 3 * q] = cY[q]; o[5 + 3 * q] = (double)cn[q]; }
 }
 
-__global__ void k_batch_signal_final(const double* __restrict__ partials, uint32_t nb, uint32_t nG,
-                                     double* out) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nG * 15) return;
+// Adds the segments: 32 consecutive values a block (coalesced), 16 slices of the
+// segments added side by side and then in slice order.  One thread per value
+// over all segments took 26 us a call.
+__global__ void __launch_bounds__(512) k_batch_signal_final(const double* __restrict__ partials, uint32_t nb,
+                                                            uint32_t nG, double* out) {
+    __shared__ double sh[16][33];
+    const uint32_t t = blockIdx.x * 32 + threadIdx.x;
     double v = 0.0;
-    for (uint32_t b = 0; b < nb; b++) v += partials[(size_t)b * nG * 15 + t];
+    if (t < nG * 15)
+        for (uint32_t b = threadIdx.y; b < nb; b += 16) v += partials[(size_t)b * nG * 15 + t];
+    sh[threadIdx.y][threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.y > 0 || t >= nG * 15) return;
+    for (int k = 1; k < 16; k++) v += sh[k][threadIdx.x];
     out[t] = v;
 }
 
@@ -767,6 +841,9 @@ struct dsim_batch {
     JobDev* d_jobs = nullptr;
     unsigned long long* d_counts = nullptr;
     uint32_t* d_status = nullptr;
+    Trig* d_trig = nullptr;             // readout: sin and cos table
+    double* d_sig = nullptr;               // readout scratch: gradients, partial sums, result (grows)
+    size_t sigCap = 0;
     uint32_t* d_stepNow = nullptr;
     uint32_t stepNow = 0;                  // host mirror of *d_stepNow
     uint32_t* keys = nullptr;
@@ -1253,6 +1330,22 @@ BatchJob* find_job(dsim_batch* b, uint32_t id) {
 
 constexpr double kPi = 3.14159265358979323846;
 
+// the readout's table, made once: the nearest doubles and what they leave
+// (long double has 64 bits of significand or more here)
+const Trig* trig_table() {
+    static const std::vector<Trig> table = [] {
+        std::vector<Trig> t(kTrig);
+        for (uint32_t k = 0; k < kTrig; k++) {
+            const long double a = 6.283185307179586476925286766559L * (long double)k / (long double)kTrig;
+            const long double s = sinl(a), c = cosl(a);
+            t[k].s = (double)s; t[k].c = (double)c;
+            t[k].sLo = (double)(s - (long double)t[k].s); t[k].cLo = (double)(c - (long double)t[k].c);
+        }
+        return t;
+    }();
+    return table.data();
+}
+
 std::vector<float> make_wave(const dsim_job_desc* d) {
     std::vector<float> w(d->steps, 0.0f);
     if (d->waveform == DSIM_WAVE_TABLE) {
@@ -1306,6 +1399,8 @@ int dsim_batch_create(uint64_t spinCapacity, uint32_t jobCapacity, dsim_batch** 
     if (!rc) rc = balloc(b, (void**)&b->d_counts, (size_t)4 * jobCapacity * 8);
     if (!rc) rc = balloc(b, (void**)&b->d_status, 4);
     if (!rc) rc = balloc(b, (void**)&b->d_stepNow, 4);
+    if (!rc) rc = balloc(b, (void**)&b->d_trig, kTrig * sizeof(Trig));
+    if (!rc && cudaMemcpy(b->d_trig, trig_table(), kTrig * sizeof(Trig), cudaMemcpyHostToDevice) != cudaSuccess) rc = kErrCuda;
     if (!rc && (cudaMemset(b->d_status, 0, 4) != cudaSuccess || cudaMemset(b->d_stepNow, 0, 4) != cudaSuccess ||
                 cudaMemset(b->d_counts, 0, (size_t)4 * jobCapacity * 8) != cudaSuccess))
         rc = kErrCuda;
@@ -1326,7 +1421,7 @@ void dsim_batch_free(dsim_batch* b) {
     for (auto& j : b->jobs) cudaFree(j.wave);
     cudaFree(b->keys); cudaFree(b->hist); cudaFree(b->hstart); cudaFree(b->scratch);
     cudaFree(b->d_jobs); cudaFree(b->d_warps); cudaFree(b->d_subs); cudaFree(b->d_counts); cudaFree(b->d_status);
-    cudaFree(b->d_stepNow);
+    cudaFree(b->d_stepNow); cudaFree(b->d_trig); cudaFree(b->d_sig);
     if (b->st) cudaStreamDestroy(b->st);
     for (int k = 0; k < dsim_batch::kSide; k++) {
         if (b->side[k]) cudaStreamDestroy(b->side[k]);
@@ -1622,35 +1717,36 @@ int dsim_batch_signal_region(dsim_batch* b, uint32_t jobId, const float* gradSca
         set_last_error(kErrInvalid, "dsim_batch_signal: bad argument");
         return kErrInvalid;
     }
-    // warps: 32 gradients x one spin segment each, about 16 warps per SM in all
+    // warps: 32 gradients x one spin segment each, about 16 warps per SM in all,
+    // segments of whole windows of 32 spins
     const uint32_t gw = (nG + 31u) / 32u;
-    const uint32_t nseg = std::max<uint32_t>(1u, std::min<uint32_t>((j->pad + 63u) / 64u, std::max<uint32_t>(1u, 2432u / gw)));
-    const uint32_t segLen = (j->pad + nseg - 1u) / nseg;
-    const uint32_t nb = nseg;  // partial records per gradient
+    const uint32_t most = std::max<uint32_t>(1u, std::min<uint32_t>((j->pad + 63u) / 64u, std::max<uint32_t>(1u, 2432u / gw)));
+    const uint32_t segLen = ((j->pad + most - 1u) / most + 31u) & ~31u;
+    const uint32_t nseg = (j->pad + segLen - 1u) / segLen;
+    // phase = phaseConstant * (g . M)
     std::vector<double> kg(3 * (size_t)nG);
-    // phase = phaseConstant * (g . M); the job keeps phaseConstant in its descriptor
-    for (uint32_t g = 0; g < nG; g++)
-        for (int c = 0; c < 3; c++) kg[3 * g + c] = j->pc * (double)gradScaled[3 * g + c];
-    double *dk = nullptr, *dp = nullptr, *dout = nullptr;
-    int rc;
-    if ((rc = balloc(b, (void**)&dk, kg.size() * 8)) || (rc = balloc(b, (void**)&dp, (size_t)nb * nG * 15 * 8)) ||
-        (rc = balloc(b, (void**)&dout, (size_t)nG * 15 * 8))) {
-        cudaFree(dk); cudaFree(dp); cudaFree(dout);
-        return rc;
+    for (size_t k = 0; k < kg.size(); k++) kg[k] = j->pc * (double)gradScaled[k];
+    const size_t np = (size_t)nseg * nG * 15, need = kg.size() + np + (size_t)nG * 15;
+    if (need > b->sigCap) {
+        cudaFree(b->d_sig);
+        b->bytes -= b->sigCap * 8;
+        b->d_sig = nullptr; b->sigCap = 0;
+        int rc = balloc(b, (void**)&b->d_sig, need * 8);
+        if (rc) return rc;
+        b->sigCap = need;
     }
-    b->bytes -= kg.size() * 8 + (size_t)nb * nG * 15 * 8 + (size_t)nG * 15 * 8;
+    double *dk = b->d_sig, *dp = dk + kg.size(), *dout = dp + np;
     cudaError_t e = cudaMemcpyAsync(dk, kg.data(), kg.size() * 8, cudaMemcpyHostToDevice, b->st);
     if (e == cudaSuccess) {
         const uint32_t warps = gw * nseg;
         k_batch_signal<<<(warps * 32u + kSigThreads - 1) / kSigThreads, kSigThreads, 0, b->st>>>(
             view(b, b->cur), (uint32_t)j->slot0, j->pad, dk, nG, gw, nseg, segLen, region,
-            j->d.flags != 0 && b->buf[b->cur].d[0] != nullptr, dp);
-        k_batch_signal_final<<<(nG * 15 + 127) / 128, 128, 0, b->st>>>(dp, nb, nG, dout);
+            j->d.flags != 0 && b->buf[b->cur].d[0] != nullptr, b->d_trig, dp);
+        k_batch_signal_final<<<(nG * 15 + 31) / 32, dim3(32, 16), 0, b->st>>>(dp, nseg, nG, dout);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, dout, (size_t)nG * 15 * 8, cudaMemcpyDeviceToHost, b->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);
-    cudaFree(dk); cudaFree(dp); cudaFree(dout);
     if (e != cudaSuccess) { set_last_cuda_error(e, "dsim_batch_signal", __FILE__, __LINE__); return kErrCuda; }
     return kOk;
 }

@@ -89,14 +89,6 @@ __global__ void __launch_bounds__(kRedThreads) k_signal_partial(SpinsDev S, doub
     }
 }
 
-__global__ void k_signal_final(const double* __restrict__ partials, int nblocks, double* out) {
-    int k = threadIdx.x;
-    if (k >= kRedVals) return;
-    double v = 0.0;
-    for (int b = 0; b < nblocks; b++) v += partials[(size_t)b * kRedVals + k];
-    out[k] = v;
-}
-
 // final pass over nb partial records: warp k adds field k with lane-strided
 // partial sums and a shuffle tree (fixed order, deterministic)
 __global__ void k_signal_final_warps(const double* __restrict__ partials, int nb, double* out) {
@@ -120,15 +112,13 @@ int launch_signal_blocks(const SpinsDev& S, int layout, double region, double* p
     return kOk;
 }
 
+// as many blocks as the spins fill (their FP64 block reductions cost more than
+// a few spins' sums: 608 blocks for 1000 spins took 29 us, 4 take 8), the final
+// pass a warp per field (one thread per field over 608 records took 50 us)
 int launch_signal(const SpinsDev& S, int layout, double region, double* partials, double* out15,
                   cudaStream_t st) {
-    int nb = kRedBlocks;
-    if (layout == kLayoutSoA) k_signal_partial<kLayoutSoA><<<nb, kRedThreads, 0, st>>>(S, region, partials);
-    else if (layout == kLayoutAoS) k_signal_partial<kLayoutAoS><<<nb, kRedThreads, 0, st>>>(S, region, partials);
-    else k_signal_partial<2><<<nb, kRedThreads, 0, st>>>(S, region, partials);
-    k_signal_final<<<1, 32, 0, st>>>(partials, nb, out15);
-    DSIM_CUDA_TRY(cudaGetLastError());
-    return kOk;
+    const uint32_t fill = (S.N + kRedThreads - 1) / kRedThreads;
+    return launch_signal_blocks(S, layout, region, partials, (int)(fill < kRedBlocks ? fill : kRedBlocks), out15, st);
 }
 
 }  // namespace dsim
