@@ -361,6 +361,12 @@ __global__ void k_sort_scatter(SpinsSorted S, SpinsSorted D, const uint32_t* __r
     D.meta[j] = S.meta[i]; D.id[j] = S.id[i];
 }
 
+uint32_t sort_grid(uint32_t N, uint32_t nf) {
+    uint32_t nb = 8;
+    while (nb < nf && (uint64_t)nb * nb * nb < 2ull * N) nb++;
+    return nb < nf ? nb : nf;
+}
+
 int launch_sort_spins(const SpinsSorted& S, const SpinsSorted& D, uint32_t nb, uint32_t* keys,
                       uint32_t* hist, uint32_t* start, uint32_t* scratch, cudaStream_t st) {
     if (S.N == 0) return kOk;

@@ -942,14 +942,15 @@ int dsim_mesh_run(dsim_mesh* m, dsim_spins* s, const dsim_mesh_params* p, const 
         set_last_error(kErrInvalid, "dsim_mesh_run: the mesh has no fine grid (dsim_mesh_set_accel failed)");
         return kErrInvalid;
     }
-    // reorder by fine cell every sortEvery steps
+    // reorder by cell every sortEvery steps, unless each spin has a warp of its own
+    const bool sort = s->sortEvery && mesh_spins_per_warp(s->N) > 1;
     uint32_t chunk = s->sortEvery ? s->sortEvery : iterations;
-    if (s->sortEvery && (rc = ensure_sort_buffers(s, m->nf))) return rc;
+    if (sort && (rc = ensure_sort_buffers(s, sort_grid(s->N, m->nf)))) return rc;
     const float4* grad0 = a.grad;
     const float4* draws0 = a.draws;
     for (uint32_t done = 0; done < iterations; done += chunk) {
         uint32_t n = iterations - done < chunk ? iterations - done : chunk;
-        if (s->sortEvery) {
+        if (sort) {
             if ((rc = launch_sort_spins(s->sorted(), s->sorted2(), s->sortNb, s->keys, s->hist,
                                         s->hstart, s->hscratch, s->st)))
                 return rc;

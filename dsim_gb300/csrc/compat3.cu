@@ -215,14 +215,15 @@ int ensure_work(State& s, uint32_t N) {
         DSIM_CUDA_TRY(cudaMalloc(&s.keys, (size_t)N * 4));
         s.cap = N;
     }
-    if (s.histNf != s.nf) {
+    const uint32_t nb = sort_grid(N, s.nf);
+    if (s.histNf != nb) {
         cudaFree(s.hist); cudaFree(s.hstart); cudaFree(s.hscratch);
         s.hist = s.hstart = s.hscratch = nullptr;
-        uint32_t nkeys = accel_keys(s.nf);
+        uint32_t nkeys = accel_keys(nb);
         DSIM_CUDA_TRY(cudaMalloc(&s.hist, (size_t)nkeys * 4));
         DSIM_CUDA_TRY(cudaMalloc(&s.hstart, ((size_t)nkeys + 1) * 4));
         DSIM_CUDA_TRY(cudaMalloc(&s.hscratch, scan_scratch_words(nkeys) * 4));
-        s.histNf = s.nf;
+        s.histNf = nb;
     }
     return kOk;
 }
@@ -374,8 +375,8 @@ void integrateSystem(float* pos, unsigned int* randSeed, dsim_spinData* spinInfo
     uint32_t chunk = s.sortEvery ? s.sortEvery : iterations;
     for (uint32_t done = 0; done < iterations; done += chunk) {
         uint32_t n = iterations - done < chunk ? iterations - done : chunk;
-        if (s.sortEvery) {
-            rc = launch_sort_spins(s.set(cur, N), s.set(1 - cur, N), s.nf, s.keys, s.hist, s.hstart,
+        if (s.sortEvery && mesh_spins_per_warp(N) > 1) {
+            rc = launch_sort_spins(s.set(cur, N), s.set(1 - cur, N), s.histNf, s.keys, s.hist, s.hstart,
                                    s.hscratch, 0);
             if (rc) { fail(rc); return; }
             cur = 1 - cur;

@@ -141,10 +141,15 @@ int launch_accel_slabs(uint32_t nf, const TriPlane* plane, const TriBary* bary, 
                        cudaStream_t st);
 int launch_sort_spins(const SpinsSorted& S, const SpinsSorted& D, uint32_t nb, uint32_t* keys,
                       uint32_t* hist, uint32_t* start, uint32_t* scratch, cudaStream_t st);
+// cells per axis of the sort's key grid: about two cells a spin, at most the fine
+// grid's (a histogram of the fine grid's 2M keys cost a small set more than its
+// sort: 1000 spins 35 us)
+uint32_t sort_grid(uint32_t N, uint32_t nf);
 int launch_unpermute(const SpinsSorted& S, const SpinsSorted& D, cudaStream_t st);
 // flat.cu: the mesh step (warp-flattened candidate lists); occupancy 4, 6 or
 // 8 blocks per SM; queue: plane-test survivors finished 32 at a time; stage:
 // each cell's records staged in shared memory by bulk (TMA) copies
+uint32_t mesh_spins_per_warp(uint32_t N);
 int launch_mesh_step_flat(const MeshDev& g, const AccelDev& acc, const MeshStepArgs& a,
                           const SpinsSorted& S, int rng, cudaStream_t st, int occupancy = 8,
                           bool queue = false, bool stage = false);

@@ -148,16 +148,18 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
     if (status) atomicOr(a.status, status);
 }
 
+// Spins per warp: at most 16 warps per SM below 32 spins a warp.  us per step, 25 tubes
+// with myelin, 32 / 16 / 8 / 4 / 2 / 1 spins a warp: 1000 spins 12.9 / 7.9 /
+// 5.6 / 4.4 / 3.7 / 3.5; 8192 spins 14.0 / 9.3 / 6.8 / 6.1 / 8.2 / 9.8; 24,576
+// spins 15.4 / 10.4 / 9.7 / 11.9; 40,960 spins 16.3 / 11.8 / 14.4; 65,536
+// spins 17.6 / 18.9
+uint32_t mesh_spins_per_warp(uint32_t N) { return spins_per_warp(N, 16, false); }
+
 int launch_mesh_step_flat(const MeshDev& g, const AccelDev& acc, const MeshStepArgs& args,
                           const SpinsSorted& S, int rng, cudaStream_t st, int occupancy, bool queue, bool stage) {
     if (S.N == 0 || args.iterations == 0) return kOk;
     MeshStepArgs a = args;
-    // at most 16 warps per SM below 32 spins a warp.  us per step, 25 tubes
-    // with myelin, 32 / 16 / 8 / 4 / 2 / 1 spins a warp: 1000 spins 12.9 / 7.9 /
-    // 5.6 / 4.4 / 3.7 / 3.5; 8192 spins 14.0 / 9.3 / 6.8 / 6.1 / 8.2 / 9.8; 24,576
-    // spins 15.4 / 10.4 / 9.7 / 11.9; 40,960 spins 16.3 / 11.8 / 14.4; 65,536
-    // spins 17.6 / 18.9
-    a.perWarp = spins_per_warp(S.N, 16, false);
+    a.perWarp = mesh_spins_per_warp(S.N);
     const uint32_t warps = (S.N + a.perWarp - 1) / a.perWarp;
     dim3 block(kFlatThreads), grid((warps + kFlatWarps - 1) / kFlatWarps);
     // one instantiation per record layout keeps each kernel's registers to its own path
