@@ -454,3 +454,76 @@ int launch_soa_to_aos(const SpinsSorted& S, float* pos, void* spin, uint32_t* sp
     return kOk;
 }
 }  // namespace dsim
+
+namespace dsim {
+// The host's arrays as they come (StageArrays, one buffer on the device) <->
+// the work buffers.  Interleaving, widening and the reordering by id were host
+// loops over every spin and six copies either way; a null array is left out.
+__global__ void k_stage_load(StageArrays A, SpinsSorted D) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= D.N) return;
+    if (A.pos) { D.x[i] = A.pos[3 * i]; D.y[i] = A.pos[3 * i + 1]; D.z[i] = A.pos[3 * i + 2]; }
+    if (A.mag) D.mag[i] = A.mag[i];
+    if (A.phase) D.phase[i] = A.phase[i];
+    if (A.comp || A.fiber16)
+        D.meta[i] = (A.comp ? (uint32_t)A.comp[i] : 0u) | ((A.fiber16 ? (uint32_t)A.fiber16[i] : 0xFFFFu) << 8);
+    D.id[i] = i;
+}
+__global__ void k_stage_store(SpinsSorted S, StageArrays A) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= S.N) return;
+    const uint32_t j = S.id[i];
+    if (j >= S.N) return;
+    if (A.pos) { A.pos[3 * j] = S.x[i]; A.pos[3 * j + 1] = S.y[i]; A.pos[3 * j + 2] = S.z[i]; }
+    if (A.mag) A.mag[j] = S.mag[i];
+    if (A.phase) A.phase[j] = S.phase[i];
+    if (A.comp) A.comp[j] = (uint8_t)(S.meta[i] & 0xFFu);
+    if (A.fiber16) A.fiber16[j] = (uint16_t)(S.meta[i] >> 8);
+}
+// cylinder spins: word 2 of a seed record is imo + 1 (set: 2 when not given; get:
+// a record of 0 reads as outside), word 3 the nearest fiber
+__global__ void k_stage_load_cyl(StageArrays A, CylSpinsDev D) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= D.N) return;
+    D.pos[i] = make_float4(A.pos[3 * i], A.pos[3 * i + 1], A.pos[3 * i + 2], A.phase ? A.phase[i] : 0.0f);
+    reinterpret_cast<uint4*>(D.seed4)[i] =
+        make_uint4(0u, 0u, (A.imo ? A.imo[i] : 2u) + 1u, A.nearest ? A.nearest[i] : 0xFFFFFFFFu);
+    D.mag[i] = A.mag ? A.mag[i] : 1.0f;
+}
+__global__ void k_stage_store_cyl(CylSpinsDev S, StageArrays A) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= S.N) return;
+    const float4 p = S.pos[i];
+    const uint4 w = reinterpret_cast<const uint4*>(S.seed4)[i];
+    if (A.pos) { A.pos[3 * i] = p.x; A.pos[3 * i + 1] = p.y; A.pos[3 * i + 2] = p.z; }
+    if (A.mag) A.mag[i] = S.mag[i];
+    if (A.phase) A.phase[i] = p.w;
+    if (A.imo) A.imo[i] = w.z ? w.z - 1u : 2u;
+    if (A.nearest) A.nearest[i] = w.w;
+}
+
+int launch_stage_load(const StageArrays& A, const SpinsSorted& D, cudaStream_t st) {
+    if (D.N == 0) return kOk;
+    k_stage_load<<<(D.N + 255) / 256, 256, 0, st>>>(A, D);
+    DSIM_CUDA_TRY(cudaGetLastError());
+    return kOk;
+}
+int launch_stage_store(const SpinsSorted& S, const StageArrays& A, cudaStream_t st) {
+    if (S.N == 0) return kOk;
+    k_stage_store<<<(S.N + 255) / 256, 256, 0, st>>>(S, A);
+    DSIM_CUDA_TRY(cudaGetLastError());
+    return kOk;
+}
+int launch_stage_load_cyl(const StageArrays& A, const CylSpinsDev& D, cudaStream_t st) {
+    if (D.N == 0) return kOk;
+    k_stage_load_cyl<<<(D.N + 255) / 256, 256, 0, st>>>(A, D);
+    DSIM_CUDA_TRY(cudaGetLastError());
+    return kOk;
+}
+int launch_stage_store_cyl(const CylSpinsDev& S, const StageArrays& A, cudaStream_t st) {
+    if (S.N == 0) return kOk;
+    k_stage_store_cyl<<<(S.N + 255) / 256, 256, 0, st>>>(S, A);
+    DSIM_CUDA_TRY(cudaGetLastError());
+    return kOk;
+}
+}  // namespace dsim

@@ -218,6 +218,9 @@ void cyl_hold(const dsim_cyl* c, int delta) {
 int mesh_rebuild_accel(dsim_mesh* m, uint32_t nf) { return accel_build(m, nf); }
 }  // namespace dsim
 
+// staging bytes per spin: position, magnitude, phase and two words (cylinders)
+static constexpr size_t kStageBytes = 28;
+
 struct dsim_spins {
     uint32_t N = 0;
     cudaStream_t st = nullptr;
@@ -243,6 +246,8 @@ struct dsim_spins {
     size_t drawsCap = 0;
     float4* grad = nullptr;     // per-step gradient table (lazy, grows)
     size_t gradCap = 0;
+    unsigned char* stage = nullptr;  // the host's arrays on the device (kStageBytes per spin)
+    uint32_t* moved = nullptr;  // spins the compartment search moved
     double* partials = nullptr; // signal scratch
     double* sig = nullptr;      // 15 doubles
     void* flush = nullptr;
@@ -646,7 +651,7 @@ static void spins_release(dsim_spins* s) {
     cudaFree(s->x); cudaFree(s->y); cudaFree(s->z); cudaFree(s->mag); cudaFree(s->phase);
     cudaFree(s->meta); cudaFree(s->cpos); cudaFree(s->cseed); cudaFree(s->corder); cudaFree(s->counts);
     cudaFree(s->status); cudaFree(s->tested); cudaFree(s->draws); cudaFree(s->grad); cudaFree(s->partials);
-    cudaFree(s->sig); cudaFree(s->flush);
+    cudaFree(s->sig); cudaFree(s->flush); cudaFree(s->stage); cudaFree(s->moved);
     cudaFree(s->id); cudaFree(s->x2); cudaFree(s->y2); cudaFree(s->z2); cudaFree(s->mag2);
     cudaFree(s->phase2); cudaFree(s->meta2); cudaFree(s->id2); cudaFree(s->keys); cudaFree(s->hist);
     cudaFree(s->hstart); cudaFree(s->hscratch);
@@ -670,14 +675,14 @@ int dsim_spins_create(uint32_t N, dsim_spins** out) {
             (rc = dev_alloc(&s->phase, N, &s->bytes)) || (rc = dev_alloc(&s->meta, N, &s->bytes)) ||
             (rc = dev_alloc(&s->counts, (size_t)2 * N, &s->bytes)) || (rc = dev_alloc(&s->status, 1, &s->bytes)) ||
             (rc = dev_alloc(&s->partials, reduce_scratch_doubles(N), &s->bytes)) ||
-            (rc = dev_alloc(&s->sig, 15, &s->bytes)) || (rc = dev_alloc(&s->id, N, &s->bytes)))
+            (rc = dev_alloc(&s->sig, 15, &s->bytes)) || (rc = dev_alloc(&s->id, N, &s->bytes)) ||
+            (rc = dev_alloc(&s->moved, 1, &s->bytes)) ||
+            (rc = dev_alloc(&s->stage, (size_t)N * kStageBytes, &s->bytes)))
             break;
         if (cudaMemsetAsync(s->counts, 0, (size_t)8 * N, s->st) != cudaSuccess ||
             cudaMemsetAsync(s->status, 0, 4, s->st) != cudaSuccess) { rc = kErrCuda; break; }
-        std::vector<uint32_t> iota(N);
-        for (uint32_t i = 0; i < N; i++) iota[i] = i;
-        if (cudaMemcpyAsync(s->id, iota.data(), (size_t)4 * N, cudaMemcpyHostToDevice, s->st) != cudaSuccess ||
-            cudaStreamSynchronize(s->st) != cudaSuccess) { rc = kErrCuda; break; }
+        if ((rc = launch_stage_load(StageArrays(), s->sorted(), s->st))) break;  // ids 0, 1, ...
+        if (cudaStreamSynchronize(s->st) != cudaSuccess) { rc = kErrCuda; break; }
     } while (0);
     if (rc == kErrCuda) set_last_error(kErrCuda, "dsim_spins_create: %s", cudaGetErrorString(cudaGetLastError()));
     if (rc) { spins_release(s); return rc; }
@@ -687,15 +692,6 @@ int dsim_spins_create(uint32_t N, dsim_spins** out) {
 
 uint32_t dsim_spins_count(const dsim_spins* s) { return s ? s->N : 0; }
 uint64_t dsim_spins_bytes(const dsim_spins* s) { return s ? s->bytes : 0; }
-
-static int spins_identity(dsim_spins* s) {
-    std::vector<uint32_t> iota(s->N);
-    for (uint32_t i = 0; i < s->N; i++) iota[i] = i;
-    DSIM_CUDA_TRY(cudaMemcpyAsync(s->id, iota.data(), (size_t)4 * s->N, cudaMemcpyHostToDevice, s->st));
-    DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
-    s->permuted = false;
-    return kOk;
-}
 
 // bring slot order back to spin order (slot i holds spin i)
 static int spins_unpermute(dsim_spins* s) {
@@ -729,29 +725,68 @@ static int ensure_sort_buffers(dsim_spins* s, uint32_t nb) {
     return kOk;
 }
 
+// ---- the host's arrays --------------------------------------------------------
+// One host array and its section of the staging buffer.
+struct HostSection {
+    void* host;
+    size_t elem;  // bytes per spin
+    void** dev;
+};
+// Where all the given arrays together are at most this they travel as one copy
+// through a host buffer: a pageable copy takes about 12 us however short, a
+// host memcpy of this size as much.
+static constexpr size_t kOneCopyBytes = 256 << 10;
+
+static size_t stage_layout(dsim_spins* s, HostSection* sec, int n) {
+    size_t at = 0;  // widest elements first: every section is aligned
+    for (int k = 0; k < n; k++) {
+        *sec[k].dev = sec[k].host ? s->stage + at : nullptr;
+        if (sec[k].host) at += sec[k].elem * s->N;
+    }
+    return at;
+}
+static int stage_in(dsim_spins* s, HostSection* sec, int n) {
+    const size_t total = stage_layout(s, sec, n);
+    if (total <= kOneCopyBytes) {
+        std::vector<unsigned char> buf(total);
+        for (int k = 0; k < n; k++)
+            if (sec[k].host) memcpy(buf.data() + ((unsigned char*)*sec[k].dev - s->stage), sec[k].host, sec[k].elem * s->N);
+        if (total) DSIM_CUDA_TRY(cudaMemcpyAsync(s->stage, buf.data(), total, cudaMemcpyHostToDevice, s->st));
+        DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
+        return kOk;
+    }
+    for (int k = 0; k < n; k++)
+        if (sec[k].host)
+            DSIM_CUDA_TRY(cudaMemcpyAsync(*sec[k].dev, sec[k].host, sec[k].elem * s->N, cudaMemcpyHostToDevice, s->st));
+    return kOk;
+}
+static int stage_out(dsim_spins* s, const HostSection* sec, int n, size_t total) {
+    if (total <= kOneCopyBytes) {
+        std::vector<unsigned char> buf(total);
+        if (total) DSIM_CUDA_TRY(cudaMemcpyAsync(buf.data(), s->stage, total, cudaMemcpyDeviceToHost, s->st));
+        DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
+        for (int k = 0; k < n; k++)
+            if (sec[k].host) memcpy(sec[k].host, buf.data() + ((unsigned char*)*sec[k].dev - s->stage), sec[k].elem * s->N);
+        return kOk;
+    }
+    for (int k = 0; k < n; k++)
+        if (sec[k].host)
+            DSIM_CUDA_TRY(cudaMemcpyAsync(sec[k].host, *sec[k].dev, sec[k].elem * s->N, cudaMemcpyDeviceToHost, s->st));
+    DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
+    return kOk;
+}
+
 int dsim_spins_set(dsim_spins* s, const float* pos3, const float* mag, const float* phase,
                    const uint8_t* comp, const uint16_t* fiber) {
     if (!s) return kErrInvalid;
-    uint32_t N = s->N;
-    int rc0 = spins_unpermute(s);
-    if (rc0) return rc0;
-    std::vector<float> a(N), b(N), c(N);
-    if (pos3) {
-        for (uint32_t i = 0; i < N; i++) { a[i] = pos3[3 * i]; b[i] = pos3[3 * i + 1]; c[i] = pos3[3 * i + 2]; }
-        DSIM_CUDA_TRY(cudaMemcpyAsync(s->x, a.data(), N * 4, cudaMemcpyHostToDevice, s->st));
-        DSIM_CUDA_TRY(cudaMemcpyAsync(s->y, b.data(), N * 4, cudaMemcpyHostToDevice, s->st));
-        DSIM_CUDA_TRY(cudaMemcpyAsync(s->z, c.data(), N * 4, cudaMemcpyHostToDevice, s->st));
-        DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
-    }
-    if (mag) DSIM_CUDA_TRY(cudaMemcpyAsync(s->mag, mag, N * 4, cudaMemcpyHostToDevice, s->st));
-    if (phase) DSIM_CUDA_TRY(cudaMemcpyAsync(s->phase, phase, N * 4, cudaMemcpyHostToDevice, s->st));
-    if (comp || fiber) {
-        std::vector<uint32_t> m(N);
-        for (uint32_t i = 0; i < N; i++)
-            m[i] = (comp ? (uint32_t)comp[i] : 0u) | ((fiber ? (uint32_t)fiber[i] : 0xFFFFu) << 8);
-        DSIM_CUDA_TRY(cudaMemcpyAsync(s->meta, m.data(), N * 4, cudaMemcpyHostToDevice, s->st));
-        DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
-    }
+    int rc = spins_unpermute(s);  // what is not given stays with its spin
+    if (rc) return rc;
+    StageArrays A = {};
+    HostSection sec[] = {{const_cast<float*>(pos3), 12, (void**)&A.pos}, {const_cast<float*>(mag), 4, (void**)&A.mag},
+                         {const_cast<float*>(phase), 4, (void**)&A.phase},
+                         {const_cast<uint16_t*>(fiber), 2, (void**)&A.fiber16},
+                         {const_cast<uint8_t*>(comp), 1, (void**)&A.comp}};
+    if ((rc = stage_in(s, sec, 5)) || (rc = launch_stage_load(A, s->sorted(), s->st))) return rc;
     DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
     return kOk;
 }
@@ -759,30 +794,12 @@ int dsim_spins_set(dsim_spins* s, const float* pos3, const float* mag, const flo
 int dsim_spins_get(dsim_spins* s, float* pos3, float* mag, float* phase, uint8_t* comp,
                    uint16_t* fiber) {
     if (!s) return kErrInvalid;
-    uint32_t N = s->N;
-    int rc0 = spins_unpermute(s);
-    if (rc0) return rc0;
-    if (pos3) {
-        std::vector<float> a(N), b(N), c(N);
-        DSIM_CUDA_TRY(cudaMemcpyAsync(a.data(), s->x, N * 4, cudaMemcpyDeviceToHost, s->st));
-        DSIM_CUDA_TRY(cudaMemcpyAsync(b.data(), s->y, N * 4, cudaMemcpyDeviceToHost, s->st));
-        DSIM_CUDA_TRY(cudaMemcpyAsync(c.data(), s->z, N * 4, cudaMemcpyDeviceToHost, s->st));
-        DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
-        for (uint32_t i = 0; i < N; i++) { pos3[3 * i] = a[i]; pos3[3 * i + 1] = b[i]; pos3[3 * i + 2] = c[i]; }
-    }
-    if (mag) DSIM_CUDA_TRY(cudaMemcpyAsync(mag, s->mag, N * 4, cudaMemcpyDeviceToHost, s->st));
-    if (phase) DSIM_CUDA_TRY(cudaMemcpyAsync(phase, s->phase, N * 4, cudaMemcpyDeviceToHost, s->st));
-    if (comp || fiber) {
-        std::vector<uint32_t> m(N);
-        DSIM_CUDA_TRY(cudaMemcpyAsync(m.data(), s->meta, N * 4, cudaMemcpyDeviceToHost, s->st));
-        DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
-        for (uint32_t i = 0; i < N; i++) {
-            if (comp) comp[i] = (uint8_t)(m[i] & 0xFFu);
-            if (fiber) fiber[i] = (uint16_t)(m[i] >> 8);
-        }
-    }
-    DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
-    return kOk;
+    StageArrays A = {};
+    HostSection sec[] = {{pos3, 12, (void**)&A.pos}, {mag, 4, (void**)&A.mag}, {phase, 4, (void**)&A.phase},
+                         {fiber, 2, (void**)&A.fiber16}, {comp, 1, (void**)&A.comp}};
+    const size_t total = stage_layout(s, sec, 5);
+    int rc = launch_stage_store(s->sorted(), A, s->st);
+    return rc ? rc : stage_out(s, sec, 5, total);
 }
 
 static int ensure_cyl(dsim_spins* s) {
@@ -798,22 +815,13 @@ int dsim_spins_set_cyl(dsim_spins* s, const float* pos3, const float* mag, const
     if (!s || !pos3) return kErrInvalid;
     int rc = ensure_cyl(s);
     if (rc) return rc;
-    uint32_t N = s->N;
-    std::vector<float4> p(N);
-    std::vector<uint32_t> sd((size_t)4 * N, 0u);
-    for (uint32_t i = 0; i < N; i++) {
-        p[i] = make_float4(pos3[3 * i], pos3[3 * i + 1], pos3[3 * i + 2], phase ? phase[i] : 0.0f);
-        sd[4 * i + 2] = (imo ? imo[i] : 2u) + 1u;
-        sd[4 * i + 3] = nearest ? nearest[i] : 0xFFFFFFFFu;
-    }
-    DSIM_CUDA_TRY(cudaMemcpyAsync(s->cpos, p.data(), (size_t)N * 16, cudaMemcpyHostToDevice, s->st));
-    DSIM_CUDA_TRY(cudaMemcpyAsync(s->cseed, sd.data(), (size_t)N * 16, cudaMemcpyHostToDevice, s->st));
-    if (mag) DSIM_CUDA_TRY(cudaMemcpyAsync(s->mag, mag, N * 4, cudaMemcpyHostToDevice, s->st));
-    else {
-        std::vector<float> one(N, 1.0f);
-        DSIM_CUDA_TRY(cudaMemcpyAsync(s->mag, one.data(), N * 4, cudaMemcpyHostToDevice, s->st));
-        DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
-    }
+    StageArrays A = {};
+    HostSection sec[] = {{const_cast<float*>(pos3), 12, (void**)&A.pos}, {const_cast<float*>(mag), 4, (void**)&A.mag},
+                         {const_cast<float*>(phase), 4, (void**)&A.phase},
+                         {const_cast<uint32_t*>(imo), 4, (void**)&A.imo},
+                         {const_cast<uint32_t*>(nearest), 4, (void**)&A.nearest}};
+    const CylSpinsDev D = {s->cpos, s->cseed, s->mag, s->N};
+    if ((rc = stage_in(s, sec, 5)) || (rc = launch_stage_load_cyl(A, D, s->st))) return rc;
     DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
     return kOk;
 }
@@ -821,20 +829,13 @@ int dsim_spins_set_cyl(dsim_spins* s, const float* pos3, const float* mag, const
 int dsim_spins_get_cyl(dsim_spins* s, float* pos3, float* mag, float* phase, uint32_t* imo,
                        uint32_t* nearest) {
     if (!s || !s->cpos) return kErrInvalid;
-    uint32_t N = s->N;
-    std::vector<float4> p(N);
-    std::vector<uint32_t> sd((size_t)4 * N);
-    DSIM_CUDA_TRY(cudaMemcpyAsync(p.data(), s->cpos, (size_t)N * 16, cudaMemcpyDeviceToHost, s->st));
-    DSIM_CUDA_TRY(cudaMemcpyAsync(sd.data(), s->cseed, (size_t)N * 16, cudaMemcpyDeviceToHost, s->st));
-    if (mag) DSIM_CUDA_TRY(cudaMemcpyAsync(mag, s->mag, N * 4, cudaMemcpyDeviceToHost, s->st));
-    DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
-    for (uint32_t i = 0; i < N; i++) {
-        if (pos3) { pos3[3 * i] = p[i].x; pos3[3 * i + 1] = p[i].y; pos3[3 * i + 2] = p[i].z; }
-        if (phase) phase[i] = p[i].w;
-        if (imo) imo[i] = sd[4 * i + 2] ? sd[4 * i + 2] - 1u : 2u;
-        if (nearest) nearest[i] = sd[4 * i + 3];
-    }
-    return kOk;
+    StageArrays A = {};
+    HostSection sec[] = {{pos3, 12, (void**)&A.pos}, {mag, 4, (void**)&A.mag}, {phase, 4, (void**)&A.phase},
+                         {imo, 4, (void**)&A.imo}, {nearest, 4, (void**)&A.nearest}};
+    const size_t total = stage_layout(s, sec, 5);
+    const CylSpinsDev S = {s->cpos, s->cseed, s->mag, s->N};
+    int rc = launch_stage_store_cyl(S, A, s->st);
+    return rc ? rc : stage_out(s, sec, 5, total);
 }
 
 int dsim_spins_counts(dsim_spins* s, uint32_t* counts2N, int reset) {
@@ -1084,21 +1085,14 @@ int dsim_mesh_compartments(dsim_mesh* m, dsim_spins* s, uint64_t seed, float sta
         set_last_error(kErrInvalid, "dsim_mesh_compartments: needs the fine grid");
         return kErrInvalid;
     }
-    uint32_t* dmoved = nullptr;
-    int rc = dev_alloc(&dmoved, 1);
+    DSIM_CUDA_TRY(cudaMemsetAsync(s->moved, 0, 4, s->st));
+    int rc = launch_compartments(m->dev(), m->acc(), s->sorted(), m->maxabs, startBoxSize, seed, 20, 8, s->status,
+                                 s->moved, s->st);
     if (rc) return rc;
-    cudaError_t e = cudaMemsetAsync(dmoved, 0, 4, s->st);
-    if (e == cudaSuccess) {
-        rc = launch_compartments(m->dev(), m->acc(), s->sorted(), m->maxabs, startBoxSize, seed, 20, 8, s->status,
-                                 dmoved, s->st);
-        uint32_t h = 0;
-        if (!rc) e = cudaMemcpyAsync(&h, dmoved, 4, cudaMemcpyDeviceToHost, s->st);
-        if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(s->st);
-        if (moved) *moved = h;
-    }
-    cudaFree(dmoved);
-    if (rc) return rc;
-    if (e != cudaSuccess) { set_last_cuda_error(e, "dsim_mesh_compartments", __FILE__, __LINE__); return kErrCuda; }
+    uint32_t h = 0;
+    DSIM_CUDA_TRY(cudaMemcpyAsync(&h, s->moved, 4, cudaMemcpyDeviceToHost, s->st));
+    DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
+    if (moved) *moved = h;
     return kOk;
 }
 

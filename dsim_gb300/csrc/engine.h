@@ -270,6 +270,19 @@ struct CylStepArgs {
 int launch_cyl_step(const CylDev& g, const CylStepArgs& a, const CylSpinsDev& S, const CylOrder& scratch, int rng,
                     cudaStream_t st, uint32_t* launches);
 
+// ---- accel.cu: the host's spin arrays on the device --------------------------
+// sections of a spin object's staging buffer, null when not given
+struct StageArrays {
+    float *pos, *mag, *phase;
+    uint32_t *imo, *nearest;  // cylinder spins
+    uint16_t* fiber16;        // mesh spins
+    uint8_t* comp;
+};
+int launch_stage_load(const StageArrays& A, const SpinsSorted& D, cudaStream_t st);
+int launch_stage_store(const SpinsSorted& S, const StageArrays& A, cudaStream_t st);
+int launch_stage_load_cyl(const StageArrays& A, const CylSpinsDev& D, cudaStream_t st);
+int launch_stage_store_cyl(const CylSpinsDev& S, const StageArrays& A, cudaStream_t st);
+
 // ---- host helpers --------------------------------------------------------
 const char* last_error_message();
 // api.cu: device views of native substrate handles (for batch.cu)
