@@ -213,9 +213,10 @@ int launch_accel_cells(bool fill, uint32_t nT, const TriPlane* plane, const TriB
 // Gram system is nearly singular.
 static constexpr float kSlabEps = 2.5e-5f;
 __device__ __forceinline__ float slab_margin(const TriBary& B, float vv) {
-    const float s2 = 1.0f - (B.uv / B.uu) * (B.uv / vv);
-    if (!(s2 > 1e-5f) || !(B.uu > 0.0f) || !(vv > 0.0f)) return 1e30f;
-    return kSlabEps + 64.0f * 5.9604645e-08f * sqrtf(fmaxf(B.uu, vv)) / s2;
+    const float uu = fabsf(B.uu);
+    const float s2 = 1.0f - (B.uv / uu) * (B.uv / vv);
+    if (!(s2 > 1e-5f) || !(uu > 0.0f) || !(vv > 0.0f)) return 1e30f;
+    return kSlabEps + 64.0f * 5.9604645e-08f * sqrtf(fmaxf(uu, vv)) / s2;
 }
 
 // Marks (by the sign of vv) the triangles whose hits need the reference's walk
@@ -225,9 +226,10 @@ __device__ __forceinline__ float slab_margin(const TriBary& B, float vv) {
 // triangle is listed by the cell of a hit point that keeps 2 kRegularEps from
 // the cell's faces (flat_only_hit).  The reference's overlap test is decided by
 // rounding where a triangle ends on a face, as the rings of a tessellated tube
-// often do, so touching a face alone says nothing.
+// often do, so touching a face alone says nothing.  The sign of uu tells a test
+// to look vv up: it is flagged, or not v . v to the last bit (tri_vv).
 __global__ void k_tri_regular(uint32_t nT, uint32_t n, const uint4* __restrict__ cells,
-                              const TriBary* __restrict__ bary, TriPlane* plane) {
+                              TriBary* bary, TriPlane* plane) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nT) return;
     const float eps = kRegularEps;
@@ -272,9 +274,10 @@ __global__ void k_tri_regular(uint32_t nT, uint32_t n, const uint4* __restrict__
                 regular = apart || tri_box_overlap32(v, h) == 0;
             }
     plane[t].vv = regular ? vv : -vv;
+    if (!regular || vv != B.vx * B.vx + B.vy * B.vy + B.vz * B.vz) bary[t].uu = -fabsf(B.uu);
 }
 
-int launch_tri_regular(uint32_t nT, uint32_t n, const uint4* cells, const TriBary* bary, TriPlane* plane,
+int launch_tri_regular(uint32_t nT, uint32_t n, const uint4* cells, TriBary* bary, TriPlane* plane,
                        cudaStream_t st) {
     if (nT == 0) return kOk;
     k_tri_regular<<<(nT + 127) / 128, 128, 0, st>>>(nT, n, cells, bary, plane);

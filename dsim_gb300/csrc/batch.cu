@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kFlatThreads, 4)
 k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
                    const uint32_t* __restrict__ stepNow, uint32_t chunk, uint32_t* status,
                    unsigned long long* jobCounts) {
-    __shared__ FlatWarp wh[kFlatWarps];
+    __shared__ HitWarp wh[kFlatWarps];
     __shared__ LocalWarp wl[kFlatWarps];
     __shared__ float mom[6][kFlatThreads];
     __shared__ JobDev jobS[kFlatWarps];
@@ -296,7 +296,7 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t tx = threadIdx.x;
     const uint32_t wi = threadIdx.x >> 5;
-    FlatWarp& H = wh[wi];
+    HitWarp& H = wh[wi];
     LocalWarp& Lw = wl[wi];
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (w >= W.count) return;  // whole warp
@@ -438,14 +438,14 @@ __global__ void __launch_bounds__(kFlatThreads, 2)
 k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
                const uint32_t* __restrict__ stepNow, uint32_t chunk, uint32_t* status,
                unsigned long long* jobCounts) {
-    __shared__ FlatWarp wh[kFlatWarps];
+    __shared__ HitWarp wh[kFlatWarps];
     __shared__ PrecWarp wp[kFlatWarps];
     __shared__ JobDev jobS[kFlatWarps];
     __shared__ SubDev subS[kFlatWarps];
     const uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t wi = threadIdx.x >> 5;
-    FlatWarp& H = wh[wi];
+    HitWarp& H = wh[wi];
     PrecWarp& P = wp[wi];
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (w >= W.count) return;  // whole warp

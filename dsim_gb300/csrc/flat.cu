@@ -31,6 +31,18 @@
 
 namespace dsim {
 
+// A lane's state that only the ends of steps and the hits read, kept in shared
+// memory: a round's lists and tests hold nearly every register, and what does
+// not fit is spilled around them.  The 14 words take the 7-block form from 204
+// B of spills to 32 and make it the fastest over many waves (us per step at 4 /
+// 5 / 6 / 7 / 8 / 9 blocks per SM: 400,000 spins on 100 tubes 46.6 / 40.8 /
+// 39.0 / 37.0 / 38.7 / 41.7, 1M spins on 400 tubes 119.4 / 103.0 / 98.3 / 97.8
+// / 98.5 / 102.4; in registers, at 5: 41.7 and 105.6).
+struct LaneState {
+    float mag[32], phase[32], umax[32], umin[32], u[32];
+    uint32_t comp[32], fiber[32], id[32], nrefl[32], nperm[32], status[32], it[32], sub[32];
+};
+
 // QUEUE (32-byte records): records past the plane test are finished 32 at a
 // time from a per-warp queue (flat_round_mode's Q); STAGE: each cell's records
 // staged in shared memory by bulk (TMA) copies, double-buffered
@@ -40,6 +52,7 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
                                                                        MeshStepArgs a, SpinsSorted S,
                                                                        int rng) {
     __shared__ FlatWarp wh[kFlatWarps];
+    __shared__ LaneState wc[kFlatWarps];
     __shared__ FlatQueue wq[QUEUE ? kFlatWarps : 1];
     __shared__ FlatStage ws[STAGE ? kFlatWarps : 1];
     const uint32_t FULL = 0xFFFFFFFFu;
@@ -52,8 +65,15 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
     const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * a.perWarp + lane;
     const bool valid = lane < a.perWarp && i < S.N;
     // the position is o at the top of a step, the start of its current sub-segment within one
-    float ox = 0.0f, oy = 0.0f, oz = 0.0f, mag = 0.0f, phase = 0.0f;
-    uint32_t comp = 0, fiber = 0, id = 0;
+    float ox = 0.0f, oy = 0.0f, oz = 0.0f;
+    LaneState& C = wc[threadIdx.x >> 5];
+    float &mag = C.mag[lane], &phase = C.phase[lane], &umax = C.umax[lane], &umin = C.umin[lane], &u = C.u[lane];
+    uint32_t &comp = C.comp[lane], &fiber = C.fiber[lane], &id = C.id[lane], &nrefl = C.nrefl[lane],
+             &nperm = C.nperm[lane], &status = C.status[lane], &it = C.it[lane], &sub = C.sub[lane];
+    mag = phase = umin = 0.0f;
+    umax = u = 1.0f;
+    comp = fiber = id = nrefl = nperm = status = it = sub = 0;
+    uint32_t ntested = 0;
     if (valid) {
         ox = S.x[i]; oy = S.y[i]; oz = S.z[i]; mag = S.mag[i]; phase = S.phase[i];
         uint32_t meta = S.meta[i];
@@ -62,26 +82,23 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
     }
     uint32_t k0 = a.key0, k1 = a.key1;
     if (valid && rng == kRngPhiloxPerSpinKey) { k0 = a.spinKeys[2 * id]; k1 = a.spinKeys[2 * id + 1]; }
-    uint32_t nrefl = 0, nperm = 0, ntested = 0, status = 0;
     // Each lane runs its own step counter: a lane whose step ends in a round
     // starts its next step in the following round, so the warp's rounds are
     // not held back by the lane with the longest reflection chain of a step.
-    uint32_t it = 0;
     bool active = valid && a.iterations > 0;
     bool fresh = active;  // the lane starts step `it` at the top of the round
-    Draw d;
-    d.nx = d.ny = d.nz = 0.0f; d.u = 1.0f;
     float px = ox, py = oy, pz = oz;
-    uint32_t excluded = 0xFFFFFFFFu, sub = 0;
-    float umax = 1.0f, umin = 0.0f;
+    uint32_t excluded = 0xFFFFFFFFu;
     while (__any_sync(FULL, active)) {
         if (fresh) {
+            Draw d;
             if (rng == kRngReplay) {
                 float4 q = __ldg(a.draws + (size_t)it * S.N + id);
                 d.nx = q.x; d.ny = q.y; d.nz = q.z; d.u = q.w;
             } else {
                 d = philox_draw(a.spinBase + id, a.step0 + it, a.stream, k0, k1);
             }
+            u = d.u;
             const float sd = a.sd[comp & 3u];
             px = ox + d.nx * sd; py = oy + d.ny * sd; pz = oz + d.nz * sd;
             // the reference's endPos equals the sub-segment target p at the top
@@ -110,7 +127,7 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
             if (open) {
                 bool finish = !found;
                 if (found) {
-                    apply_hit(g, best, d.u, a.perm, a.reflType, umax, umin, ox, oy, oz, px, py, pz, comp, fiber,
+                    apply_hit(g, best, u, a.perm, a.reflType, umax, umin, ox, oy, oz, px, py, pz, comp, fiber,
                               excluded, nrefl, nperm);
                     if (++sub >= a.maxSub) {
                         status |= kStatusSubsegCap;
@@ -171,18 +188,19 @@ int launch_mesh_step_flat(const MeshDev& g, const AccelDev& acc, const MeshStepA
     } else if (acc.wide == 1 && stage) {
         k_mesh_step_flat<false, 6, 1, false, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
     } else if (acc.wide == 1 && queue) {
-        // Blocks per SM: 5 (96 registers, 40 B of spills) over many waves, and
-        // whichever of 4 (126 registers, no spills) to 7 (72) takes a small grid
-        // in one wave.  us per step on 100 tubes at 4 / 5 / 6 / 7: 65,536 spins
-        // (512 blocks) 10.3 / 10.9 / 13.1 / 13.7; 90,000 15.8 / 11.4 / 13.5 / 14.3;
-        // 100,000 16.4 / 16.4 / 13.8 / 14.5; 150,000 (two waves of 4) 18.5 / 19.4 /
-        // 22.6 / 23.3; 400,000 46.6 / 44.3 / 46.6 / 44.1; 1M spins on 2.56M
-        // triangles 120.8 / 111.3 / 117.0 / 114.3
-        const uint32_t perSm = (grid.x + kSmCount - 1) / kSmCount;
-        if (perSm <= 4 || perSm == 8) k_mesh_step_flat<false, 4, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
-        else if (perSm == 6) k_mesh_step_flat<false, 6, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
-        else if (perSm == 7) k_mesh_step_flat<false, 7, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
-        else k_mesh_step_flat<false, 5, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
+        // Blocks per SM: as few of 4 (118 registers) to 7 (72, 32 B of spills) as
+        // reach the fewest waves.  us per step on 100 tubes at 4 / 5 / 6 / 7, the
+        // rule's marked: 70,000 spins 10.5* / 10.5 / 11.1 / 11.9; 90,000 16.0 /
+        // 11.2* / 11.8 / 12.7; 100,000 16.8 / 15.5 / 12.2* / 13.0; 125,000 17.4 /
+        // 17.1 / 17.7 / 13.7*; 150,000 19.1* / 18.6 / 19.5 / 20.4; 220,000 26.6 /
+        // 25.2 / 22.4* / 23.9; 400,000 46.6 / 40.6 / 38.8 / 37.0*; 600,000 66.2 /
+        // 57.7 / 55.5 / 55.4*
+        const uint32_t perSm = (grid.x + kSmCount - 1) / kSmCount, waves = (perSm + 6) / 7;
+        const uint32_t k = (perSm + waves - 1) / waves;
+        if (k <= 4) k_mesh_step_flat<false, 4, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
+        else if (k == 5) k_mesh_step_flat<false, 5, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
+        else if (k == 6) k_mesh_step_flat<false, 6, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
+        else k_mesh_step_flat<false, 7, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
     } else if (acc.wide == 1) {
         if (occupancy >= 8) k_mesh_step_flat<false, 8, 1><<<grid, block, 0, st>>>(g, acc, a, S, rng);
         else if (occupancy >= 6) k_mesh_step_flat<false, 6, 1><<<grid, block, 0, st>>>(g, acc, a, S, rng);

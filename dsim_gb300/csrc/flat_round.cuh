@@ -36,15 +36,28 @@ static constexpr int kFlatWarps = kFlatThreads / 32;
 static constexpr int kFlatSlots = 4;      // hits kept per owner per round
 static constexpr uint32_t kFlatMaxWidth = 4;  // cells per axis of a box the warp handles
 
-struct FlatWarp {
+// A warp's lists
+struct FlatLists {
     // the round's sub-segments by owner lane: start and excluded triangle
     // (bits); end - start and fine-cell box origin lo0 | lo1 << 10 | lo2 << 20
     // (bits)
     float4 o[32], d[32];
     uint32_t src[32];  // by rank among the lanes with cells (flat_box)
     uint2 cell[64];    // cells with records still to test: first record, owner | count << 5
-    // hits filed per owner
-    uint32_t n[32];
+    uint32_t n[32];    // hits filed per owner
+};
+
+// Hits filed by owner.  FlatWarp keeps a hit as its triangle and the fraction r
+// of the sub-segment with two flags in its top bits (0 < r < 1 leaves them
+// free), and works the point and its distance out again, by the test's own
+// expressions, for the hit it wants: 1 KB a warp instead of 3, which is L1 that
+// a step's records can stay in.  HitWarp keeps all of a hit, for the forms whose
+// points come by other ways.
+struct FlatWarp : FlatLists {
+    uint32_t t[kFlatSlots][32];
+    uint32_t r[kFlatSlots][32];
+};
+struct HitWarp : FlatLists {
     uint32_t t[kFlatSlots][32];
     uint32_t type[kFlatSlots][32];
     float d2[kFlatSlots][32];
@@ -53,12 +66,43 @@ struct FlatWarp {
     float z[kFlatSlots][32];
 };
 
-__device__ __forceinline__ void flat_file_hit(FlatWarp& H, uint32_t owner, const FastHit& h) {
+__device__ __forceinline__ void file_hit(FlatWarp& H, uint32_t owner, const FastHit& h) {
+    const uint32_t slot = atomicAdd(&H.n[owner], 1u);
+    if (slot < (uint32_t)kFlatSlots) {
+        H.t[slot][owner] = h.t;
+        H.r[slot][owner] = __float_as_uint(h.r) | ((h.type & kHitWalk) ? 0x80000000u : 0u) |
+                           ((h.type & ~kHitWalk) > 1u ? 0x40000000u : 0u);
+    }
+}
+__device__ __forceinline__ void file_hit(HitWarp& H, uint32_t owner, const FastHit& h) {
     uint32_t slot = atomicAdd(&H.n[owner], 1u);
     if (slot < (uint32_t)kFlatSlots) {
         H.t[slot][owner] = h.t; H.type[slot][owner] = h.type; H.d2[slot][owner] = h.d2;
         H.x[slot][owner] = h.x; H.y[slot][owner] = h.y; H.z[slot][owner] = h.z;
     }
+}
+// the lane's own hit q (without its walk flag; an edge's and a vertex's type
+// count the same), and whether it has that flag
+__device__ __forceinline__ FastHit filed_hit(const FlatWarp& H, uint32_t q, uint32_t lane) {
+    const uint32_t bits = H.r[q][lane];
+    const float4 O = H.o[lane], D = H.d[lane];
+    FastHit h;
+    h.t = H.t[q][lane];
+    h.type = 1u + ((bits >> 30) & 1u);
+    h.r = __uint_as_float(bits & 0x3FFFFFFFu);
+    h.x = O.x + D.x * h.r; h.y = O.y + D.y * h.r; h.z = O.z + D.z * h.r;
+    h.d2 = (O.x - h.x) * (O.x - h.x) + (O.y - h.y) * (O.y - h.y) + (O.z - h.z) * (O.z - h.z);
+    return h;
+}
+__device__ __forceinline__ bool filed_walk(const FlatWarp& H, uint32_t q, uint32_t lane) { return H.r[q][lane] >> 31; }
+__device__ __forceinline__ FastHit filed_hit(const HitWarp& H, uint32_t q, uint32_t lane) {
+    FastHit h;
+    h.t = H.t[q][lane]; h.type = H.type[q][lane] & ~kHitWalk; h.d2 = H.d2[q][lane]; h.r = 0.0f;
+    h.x = H.x[q][lane]; h.y = H.y[q][lane]; h.z = H.z[q][lane];
+    return h;
+}
+__device__ __forceinline__ bool filed_walk(const HitWarp& H, uint32_t q, uint32_t lane) {
+    return H.type[q][lane] & kHitWalk;
 }
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, uint32_t lane) {
@@ -116,7 +160,7 @@ __device__ __forceinline__ FlatBox flat_box(const AccelDev& acc, bool open, floa
 
 // fills the rank table of the lanes' boxes; returns the elements in all.  first:
 // the lane's first element
-__device__ __forceinline__ uint32_t flat_items(FlatWarp& H, const FlatBox& b, uint32_t lane, uint32_t& first) {
+__device__ __forceinline__ uint32_t flat_items(FlatLists& H, const FlatBox& b, uint32_t lane, uint32_t& first) {
     const uint32_t incl = warp_incl_scan(b.count, lane);
     first = incl - b.count;
     const uint32_t some = __ballot_sync(0xFFFFFFFFu, b.count > 0);
@@ -147,7 +191,7 @@ struct FlatList {
     uint32_t rb, total, from;       // next record of the block, records in it, its cells begun before rb
     uint32_t start, cnt, b0;        // lane's cell of the block: first record in the flat list, count, record index
 };
-__device__ __forceinline__ FlatList flat_list(FlatWarp& H, const FlatBox& b, uint32_t lane) {
+__device__ __forceinline__ FlatList flat_list(FlatLists& H, const FlatBox& b, uint32_t lane) {
     FlatList l;
     l.cells = b.count;
     l.itotal = flat_items(H, b, lane, l.first);
@@ -157,7 +201,7 @@ __device__ __forceinline__ FlatList flat_list(FlatWarp& H, const FlatBox& b, uin
 // Makes the next block when the current one's records are used up; false when
 // no record is left.  at(owner, O): the owner's absolute start.
 template <class At>
-__device__ __forceinline__ bool flat_next(FlatWarp& H, FlatList& l, const AccelDev& acc, uint32_t lane, At at) {
+__device__ __forceinline__ bool flat_next(FlatLists& H, FlatList& l, const AccelDev& acc, uint32_t lane, At at) {
     const uint32_t below = (1u << lane) - 1u;
     while (l.rb >= l.total && (l.ib < l.itotal || l.nq > 0)) {
         if (l.ib < l.itotal && l.nq < 32) {
@@ -195,7 +239,7 @@ __device__ __forceinline__ bool flat_next(FlatWarp& H, FlatList& l, const AccelD
 }
 // record e and owner o of flat record base + lane (call in ascending order of
 // base; all lanes; meaningless past the block's total)
-__device__ __forceinline__ void flat_pick(const FlatWarp& H, FlatList& l, uint32_t lane, uint32_t base, uint32_t& e,
+__device__ __forceinline__ void flat_pick(const FlatLists& H, FlatList& l, uint32_t lane, uint32_t base, uint32_t& e,
                                           uint32_t& o) {
     const uint32_t begun = flat_starts(l.cnt > 0, l.start, base);
     const uint2 c = H.cell[l.nq + l.from + __popc(begun & (0xFFFFFFFFu >> (31u - lane))) - 1u];
@@ -287,7 +331,7 @@ __device__ __forceinline__ void flat_test_queued(FlatWarp& H, const MeshDev& g, 
     const float4 O = H.o[o], D = H.d[o];
     FastHit h;
     if (__float_as_uint(pt.w) != __float_as_uint(O.w) && test_split(g, q, pt, O.x, O.y, O.z, D.x, D.y, D.z, h))
-        flat_file_hit(H, o, h);
+        file_hit(H, o, h);
 }
 
 // appends the lanes' surviving pairs to the queue (qn: warp-uniform length) and
@@ -325,17 +369,18 @@ static __device__ __noinline__ void flat_solo(FlatWarp& H, const MeshDev& g, con
                 for (uint32_t k = b0; k < b1; k++) {
                     FastHit h;
                     if (test_entry(g, acc, k, __float_as_uint(O.w), O.x, O.y, O.z, D.x, D.y, D.z, h))
-                        flat_file_hit(H, lane, h);
+                        file_hit(H, lane, h);
                 }
             }
 }
 
 // Are the lane's n filed hits one hit (filed once per fine cell that lists its
 // triangle), at (x, y, z), that needs no walk?  Then it is the reference's.
-__device__ __forceinline__ bool flat_only_hit(const FlatWarp& H, uint32_t lane, uint32_t n, uint32_t gn, float x,
-                                              float y, float z) {
+template <class Hits>
+__device__ __forceinline__ bool flat_only_hit(const Hits& H, uint32_t lane, uint32_t n, uint32_t gn, float x, float y,
+                                              float z) {
     const uint32_t t = H.t[0][lane];
-    bool one = n <= (uint32_t)kFlatSlots && !(H.type[0][lane] & kHitWalk);
+    bool one = n <= (uint32_t)kFlatSlots && !filed_walk(H, 0, lane);
     if (n > 1) one = one && H.t[1][lane] == t && (n < 3 || H.t[2][lane] == t) && (n < 4 || H.t[3][lane] == t);
     const float inv = 0.5f * (float)gn, margin = 2.0f * kRegularEps * inv;
     return one & clear_of_faces(x, inv, margin) & clear_of_faces(y, inv, margin) & clear_of_faces(z, inv, margin);
@@ -343,18 +388,19 @@ __device__ __forceinline__ bool flat_only_hit(const FlatWarp& H, uint32_t lane, 
 // The slot of the reference's hit among several (n <= kFlatSlots) by the walk
 // over its cells, kNoPlace for none.  About one hit in ten needs it: out of
 // line, so that a round keeps neither its registers nor its code.
-static __device__ __noinline__ uint32_t flat_choose(const FlatWarp& H, const MeshDev& g, uint32_t lane, uint32_t n,
+template <class Hits>
+static __device__ __noinline__ uint32_t flat_choose(const Hits& H, const MeshDev& g, uint32_t lane, uint32_t n,
                                                     RefWalk w) {
     uint32_t bq = kNoPlace, bt = 0, bplace = kNoPlace;
+    float bd2 = 0.0f;
     for (uint32_t q = 0; q < n; q++) {
         const uint32_t t = H.t[q][lane];
         if (bq != kNoPlace && t == bt) continue;  // filed from another fine cell too
         const uint32_t place = first_place(g, w, __ldg(g.tri_cells + t), t);
         if (place == kNoPlace) continue;
-        const float d2 = H.d2[q][lane];
-        if (place < bplace ||
-            (place == bplace && (d2 < H.d2[bq][lane] || (d2 == H.d2[bq][lane] && t < bt)))) {
-            bq = q; bplace = place; bt = t;
+        const float d2 = filed_hit(H, q, lane).d2;
+        if (place < bplace || (place == bplace && (d2 < bd2 || (d2 == bd2 && t < bt)))) {
+            bq = q; bplace = place; bt = t; bd2 = d2;
         }
     }
     return bq;
@@ -443,7 +489,7 @@ __device__ __forceinline__ void flat_round_mode(FlatWarp& H, const MeshDev& g, c
                     FastHit h;
                     if (at0 + lane < l.total && test_wide_loaded(g, P->rec[buf][half + lane][0],
                                                                  P->rec[buf][half + lane][1], H.o[o], H.d[o], h))
-                        flat_file_hit(H, o, h);
+                        file_hit(H, o, h);
                 }
                 __syncwarp();  // the buffer's reads end before its next copies
             }
@@ -465,7 +511,7 @@ __device__ __forceinline__ void flat_round_mode(FlatWarp& H, const MeshDev& g, c
                     hit = test_wide_loaded(g, __ldg(&acc.recw[e].q), __ldg(&acc.recw[e].pt), O, D, h);
                 else
                     hit = test_narrow(g, acc, e, excl, O.x, O.y, O.z, D.x, D.y, D.z, h);
-                if (hit) flat_file_hit(H, o, h);
+                if (hit) file_hit(H, o, h);
             }
             l.rb += 32;
             __syncwarp();
@@ -478,23 +524,25 @@ __device__ __forceinline__ void flat_round_mode(FlatWarp& H, const MeshDev& g, c
     if (!open) return;
     const uint32_t n = H.n[lane];
     if (n == 0) return;
-    uint32_t bq = 0;
     found = true;
-    if (!flat_only_hit(H, lane, n, g.n, H.x[0][lane], H.y[0][lane], H.z[0][lane])) {
+    best = filed_hit(H, 0, lane);
+    if (!flat_only_hit(H, lane, n, g.n, best.x, best.y, best.z)) {
         if (n > (uint32_t)kFlatSlots) {
-            ref_scan(g, ox, oy, oz, px, py, pz, excluded, best, found);
+            FastHit h;  // (best itself stays in registers)
+            bool any;
+            ref_scan(g, ox, oy, oz, px, py, pz, excluded, h, any);
+            found = any;
+            if (any) best = h;
             return;
         }
         const uint32_t gn = g.n;
         const float L = g.L;
-        bq = flat_choose(H, g, lane, n,
-                         ref_walk(ref_coord(ox, L, gn), ref_coord(oy, L, gn), ref_coord(oz, L, gn),
-                                  ref_coord(px, L, gn), ref_coord(py, L, gn), ref_coord(pz, L, gn)));
+        const uint32_t bq =
+            flat_choose(H, g, lane, n,
+                        ref_walk(ref_coord(ox, L, gn), ref_coord(oy, L, gn), ref_coord(oz, L, gn),
+                                 ref_coord(px, L, gn), ref_coord(py, L, gn), ref_coord(pz, L, gn)));
         found = bq != kNoPlace;
-    }
-    if (found) {
-        best.t = H.t[bq][lane]; best.type = H.type[bq][lane] & ~kHitWalk; best.d2 = H.d2[bq][lane];
-        best.x = H.x[bq][lane]; best.y = H.y[bq][lane]; best.z = H.z[bq][lane];
+        if (found) best = filed_hit(H, bq, lane);
     }
 }
 

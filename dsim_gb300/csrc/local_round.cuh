@@ -59,7 +59,7 @@ __device__ __forceinline__ void record_load(const AccelDev& acc, uint32_t k, boo
 // the plane test of record k for owner o in o's local frame: may the plane
 // meet the sub-segment?  (na: n.p1 - n.origin - n.offset; margin as
 // plane_may_cross)
-__device__ __forceinline__ bool local_plane(const FlatWarp& H, const LocalWarp& Lw, float4 q, uint32_t o) {
+__device__ __forceinline__ bool local_plane(const HitWarp& H, const LocalWarp& Lw, float4 q, uint32_t o) {
     const float4 O = H.o[o], D = H.d[o];
     const float den = q.x * D.x + q.y * D.y + q.z * D.z;
     const float na = (q.w - (q.x * Lw.gx[o] + q.y * Lw.gy[o] + q.z * Lw.gz[o])) -
@@ -71,7 +71,7 @@ __device__ __forceinline__ bool local_plane(const FlatWarp& H, const LocalWarp& 
 
 // the FP64 re-test of triangle t for owner o from the exact position origin +
 // offset; a hit point is local to o's origin
-__device__ __forceinline__ bool local_fp64(const FlatWarp& H, const LocalWarp& Lw, const MeshDev& g, uint32_t t,
+__device__ __forceinline__ bool local_fp64(const HitWarp& H, const LocalWarp& Lw, const MeshDev& g, uint32_t t,
                                            uint32_t o, FastHit& h, PrecCount& pc) {
     pc.exact++;
     const float gx = Lw.gx[o], gy = Lw.gy[o], gz = Lw.gz[o];
@@ -94,7 +94,7 @@ __device__ __forceinline__ bool local_fp64(const FlatWarp& H, const LocalWarp& L
 // o in o's local frame; a hit point is local to o's origin.  A case near a
 // decision boundary is decided by local_fp64 here, or (defer) left to the
 // caller with `deferred` set.
-__device__ __forceinline__ bool local_test_core(const FlatWarp& H, const LocalWarp& Lw, const MeshDev& g, float4 q,
+__device__ __forceinline__ bool local_test_core(const HitWarp& H, const LocalWarp& Lw, const MeshDev& g, float4 q,
                                                 float3 p1, uint32_t t, uint32_t o, FastHit& h, PrecCount& pc,
                                                 bool defer, bool& deferred) {
     const float gx = Lw.gx[o], gy = Lw.gy[o], gz = Lw.gz[o];
@@ -116,8 +116,8 @@ __device__ __forceinline__ bool local_test_core(const FlatWarp& H, const LocalWa
         r = num / den;
         const float4* bb = reinterpret_cast<const float4*>(g.bary + t);
         const float4 u4 = __ldg(bb), v4 = __ldg(bb + 1);
-        const float vs = __ldg(&g.plane[t].vv), vv = fabsf(vs);
-        const float uv = v4.z, uu = v4.w;
+        const float vs = tri_vv(g, t, u4, v4), vv = fabsf(vs);
+        const float uv = v4.z, uu = fabsf(v4.w);
         const float wx = ox + r * dx - ax, wy = oy + r * dy - ay, wz = oz + r * dz - az;
         const float wu = wx * u4.x + wy * u4.y + wz * u4.z;
         const float wv = wx * u4.w + wy * v4.x + wz * v4.y;
@@ -219,7 +219,7 @@ __device__ __forceinline__ void local_refine(const MeshDev& g, float gx, float g
 }
 
 // record k of the fine grid
-__device__ __forceinline__ bool local_test(const FlatWarp& H, const LocalWarp& Lw, const MeshDev& g,
+__device__ __forceinline__ bool local_test(const HitWarp& H, const LocalWarp& Lw, const MeshDev& g,
                                            const AccelDev& acc, uint32_t k, bool full, uint32_t o, FastHit& h,
                                            PrecCount& pc) {
     float4 q;
@@ -232,7 +232,7 @@ __device__ __forceinline__ bool local_test(const FlatWarp& H, const LocalWarp& L
 
 // the same, leaving a near case to the FP64 queue: returns its triangle in
 // *tdef (else 0xFFFFFFFF)
-__device__ __forceinline__ bool local_test_defer(const FlatWarp& H, const LocalWarp& Lw, const MeshDev& g,
+__device__ __forceinline__ bool local_test_defer(const HitWarp& H, const LocalWarp& Lw, const MeshDev& g,
                                                  const AccelDev& acc, uint32_t k, bool full, uint32_t o, FastHit& h,
                                                  PrecCount& pc, uint32_t& tdef) {
     float4 q;
@@ -246,7 +246,7 @@ __device__ __forceinline__ bool local_test_defer(const FlatWarp& H, const LocalW
 }
 
 // triangle t from its per-triangle records
-__device__ __forceinline__ bool local_test_tri(const FlatWarp& H, const LocalWarp& Lw, const MeshDev& g,
+__device__ __forceinline__ bool local_test_tri(const HitWarp& H, const LocalWarp& Lw, const MeshDev& g,
                                                uint32_t t, uint32_t o, FastHit& h, PrecCount& pc) {
     const float4* pp = reinterpret_cast<const float4*>(g.plane + t);
     const float4 a = __ldg(pp), c = __ldg(pp + 1);  // {n, p1.x}, {p1.y, p1.z, vv, info}
@@ -259,7 +259,7 @@ __device__ __forceinline__ bool local_test_tri(const FlatWarp& H, const LocalWar
 // length) and re-tests full groups of 32 in FP64; all lanes call it
 // full groups of 32 from the top of the FP64 queue (rare within a round: out
 // of line, so the record loop's code stays small)
-__device__ __noinline__ void local_flush64(FlatWarp& H, LocalWarp& Lw, const MeshDev& g, uint32_t lane, uint32_t& fn,
+__device__ __noinline__ void local_flush64(HitWarp& H, LocalWarp& Lw, const MeshDev& g, uint32_t lane, uint32_t& fn,
                                            PrecCount& pc) {
     while (fn >= 32) {
         const uint32_t at = fn - 32 + lane;
@@ -267,11 +267,11 @@ __device__ __noinline__ void local_flush64(FlatWarp& H, LocalWarp& Lw, const Mes
         __syncwarp();
         fn -= 32;
         FastHit h;
-        if (local_fp64(H, Lw, g, tq, oq, h, pc)) flat_file_hit(H, oq, h);
+        if (local_fp64(H, Lw, g, tq, oq, h, pc)) file_hit(H, oq, h);
     }
 }
 
-__device__ __forceinline__ void local_enqueue64(FlatWarp& H, LocalWarp& Lw, const MeshDev& g, uint32_t lane,
+__device__ __forceinline__ void local_enqueue64(HitWarp& H, LocalWarp& Lw, const MeshDev& g, uint32_t lane,
                                                 uint32_t t, uint32_t o, uint32_t& fn, PrecCount& pc) {
     const bool live = t != 0xFFFFFFFFu;
     const uint32_t b = __ballot_sync(0xFFFFFFFFu, live);
@@ -287,7 +287,7 @@ __device__ __forceinline__ void local_enqueue64(FlatWarp& H, LocalWarp& Lw, cons
 // appends the lanes' surviving (k, o) to the warp's queue (qn: warp-uniform
 // length) and tests full groups of 32 from its top, their near cases going to
 // the FP64 queue; all lanes call it
-__device__ __forceinline__ void local_enqueue(FlatWarp& H, LocalWarp& Lw, const MeshDev& g, const AccelDev& acc,
+__device__ __forceinline__ void local_enqueue(HitWarp& H, LocalWarp& Lw, const MeshDev& g, const AccelDev& acc,
                                               bool full, uint32_t lane, bool live0, uint32_t k0, uint32_t o0,
                                               bool live1, uint32_t k1, uint32_t o1, uint32_t& qn, uint32_t& fn,
                                               PrecCount& pc, bool last) {
@@ -315,7 +315,7 @@ __device__ __forceinline__ void local_enqueue(FlatWarp& H, LocalWarp& Lw, const 
         qn -= cnt;
         FastHit h;
         uint32_t tdef = 0xFFFFFFFFu;
-        if (act && local_test_defer(H, Lw, g, acc, kq, full, oq, h, pc, tdef)) flat_file_hit(H, oq, h);
+        if (act && local_test_defer(H, Lw, g, acc, kq, full, oq, h, pc, tdef)) file_hit(H, oq, h);
         local_enqueue64(H, Lw, g, lane, act ? tdef : 0xFFFFFFFFu, oq, fn, pc);
     }
 }
@@ -324,7 +324,7 @@ __device__ __forceinline__ void local_enqueue(FlatWarp& H, LocalWarp& Lw, const 
 // small (each holds its own copy of the exact test and the FP64 re-test).
 // A lane whose cell box is too large for the warp's flattened pass: its own
 // records, cell by cell.
-__device__ __noinline__ void local_solo(FlatWarp& H, LocalWarp& Lw, const MeshDev& g, const AccelDev& acc, bool full,
+__device__ __noinline__ void local_solo(HitWarp& H, LocalWarp& Lw, const MeshDev& g, const AccelDev& acc, bool full,
                                         uint32_t lane, float apx, float apy, float apz, PrecCount& pc) {
     const float4 O = H.o[lane];
     const FlatBox b = flat_box(acc, true, Lw.gx[lane] + O.x, Lw.gy[lane] + O.y, Lw.gz[lane] + O.z, apx, apy, apz);
@@ -339,7 +339,7 @@ __device__ __noinline__ void local_solo(FlatWarp& H, LocalWarp& Lw, const MeshDe
                     pc.records++;
                     if (t == __float_as_uint(O.w) || !local_plane(H, Lw, qq, lane)) continue;
                     FastHit h;
-                    if (local_test(H, Lw, g, acc, k, full, lane, h, pc)) flat_file_hit(H, lane, h);
+                    if (local_test(H, Lw, g, acc, k, full, lane, h, pc)) file_hit(H, lane, h);
                 }
             }
 }
@@ -347,7 +347,7 @@ __device__ __noinline__ void local_solo(FlatWarp& H, LocalWarp& Lw, const MeshDe
 // A lane whose hit slots overflowed: every triangle of the reference cells
 // from the start cell s towards the end cell t, in order, stopping at the
 // first cell with a hit (the reference's cell walk); returns found.
-__device__ __noinline__ bool local_overflow(FlatWarp& H, LocalWarp& Lw, const MeshDev& g, uint32_t lane, RefWalk w,
+__device__ __noinline__ bool local_overflow(HitWarp& H, LocalWarp& Lw, const MeshDev& g, uint32_t lane, RefWalk w,
                                             uint32_t excluded, FastHit& best, PrecCount& pc) {
     const uint32_t gn = g.n;
     for (uint32_t ax = 0; ax < w.nx; ax++)
@@ -377,7 +377,7 @@ __device__ __noinline__ bool local_overflow(FlatWarp& H, LocalWarp& Lw, const Me
 // collision result with the hit point in the same frame.  LAYOUT 1 or 2
 // compiles only the 32- or 64-byte record path; 0 dispatches on acc.wide.
 template <int LAYOUT = 0>
-__device__ __forceinline__ void local_round(FlatWarp& H, LocalWarp& Lw, const MeshDev& g, const AccelDev& acc,
+__device__ __forceinline__ void local_round(HitWarp& H, LocalWarp& Lw, const MeshDev& g, const AccelDev& acc,
                                             uint32_t lane, bool open, float gx, float gy, float gz, float ox,
                                             float oy, float oz, float px, float py, float pz, uint32_t excluded,
                                             bool& found, FastHit& best, PrecCount& pc) {
@@ -426,7 +426,7 @@ __device__ __forceinline__ void local_round(FlatWarp& H, LocalWarp& Lw, const Me
     {
         // the FP64 queue's remainder
         FastHit h;
-        if (lane < fn && local_fp64(H, Lw, g, Lw.ft[lane], Lw.fo[lane], h, pc)) flat_file_hit(H, Lw.fo[lane], h);
+        if (lane < fn && local_fp64(H, Lw, g, Lw.ft[lane], Lw.fo[lane], h, pc)) file_hit(H, Lw.fo[lane], h);
     }
     if (box.solo) local_solo(H, Lw, g, acc, full, lane, apx, apy, apz, pc);
     __syncwarp();
@@ -450,8 +450,7 @@ __device__ __forceinline__ void local_round(FlatWarp& H, LocalWarp& Lw, const Me
         found = bq != kNoPlace;
     }
     if (found) {
-        best.t = H.t[bq][lane]; best.type = H.type[bq][lane] & ~kHitWalk; best.d2 = H.d2[bq][lane];
-        best.x = H.x[bq][lane]; best.y = H.y[bq][lane]; best.z = H.z[bq][lane];
+        best = filed_hit(H, bq, lane);
         local_refine(g, gx, gy, gz, ox, oy, oz, dx, dy, dz, best);
     }
 }

@@ -34,6 +34,7 @@ __host__ __device__ __forceinline__ uint32_t morton3(uint32_t x, uint32_t y, uin
 struct FastHit {
     uint32_t t;
     float x, y, z, d2;
+    float r;  // the point's fraction of the sub-segment
     uint32_t type;
 };
 // Hit type flag: the reference's walk over its cells decides whether (and when)
@@ -137,11 +138,12 @@ __device__ __forceinline__ bool test_rec_uv(float4 a, float4 b, float4 u4, float
     float wz = oz + r * dz - b.y;
     float wu = wx * u4.x + wy * u4.y + wz * u4.z;
     float wv = wx * u4.w + wy * v4.x + wz * v4.y;
-    float uv = v4.z, uu = v4.w, vv = fabsf(b.z);
+    float uv = v4.z, uu = fabsf(v4.w), vv = fabsf(b.z);
     float s = (uv * wv - vv * wu) / (uv * uv - uu * vv);
     float tt = (uv * wu - uu * wv) / (uv * uv - uu * vv);
     if (!((s >= 0.0f) & (tt >= 0.0f) & (s + tt <= 1.0f))) return false;
     h.t = t;
+    h.r = r;
     h.x = ox + dx * r; h.y = oy + dy * r; h.z = oz + dz * r;
     h.d2 = (ox - h.x) * (ox - h.x) + (oy - h.y) * (oy - h.y) + (oz - h.z) * (oz - h.z);
     uint32_t type = 1;
@@ -228,8 +230,16 @@ __device__ __forceinline__ bool test_tri(const MeshDev& g, uint32_t t, float ox,
     return test_rec(g, a, make_float4(c.x, c.y, c.z, __uint_as_float(t)), ox, oy, oz, dx, dy, dz, h);
 }
 
+// vv of triangle t with its flag (hit_walk): v . v, and from the triangle's
+// plane record only where the sign of uu says that it is flagged or given
+// otherwise (k_tri_regular): a sector a triangle less to fetch
+__device__ __forceinline__ float tri_vv(const MeshDev& g, uint32_t t, float4 u4, float4 v4) {
+    if (__float_as_uint(v4.w) >> 31) return __ldg(&g.plane[t].vv);
+    return u4.w * u4.w + v4.x * v4.x + v4.y * v4.y;
+}
+
 // exact test with the plane data from a 32-byte record (p1, t) and the rest
-// (vv, u, v, uv, uu) from the triangle's records, loaded only past the plane
+// (u, v, uv, uu) from the triangle's records, loaded only past the plane
 __device__ __forceinline__ bool test_split(const MeshDev& g, float4 q, float4 pt, float ox, float oy,
                                            float oz, float dx, float dy, float dz, FastHit& h) {
     float num = q.x * (pt.x - ox) + q.y * (pt.y - oy) + q.z * (pt.z - oz);
@@ -240,9 +250,10 @@ __device__ __forceinline__ bool test_split(const MeshDev& g, float4 q, float4 pt
     float r = num / den;
     if (!((0.0f < r) & (r < 1.0f))) return false;
     const uint32_t t = __float_as_uint(pt.w);
-    const float vv = __ldg(&g.plane[t].vv);
-    return test_rec(g, make_float4(q.x, q.y, q.z, pt.x), make_float4(pt.y, pt.z, vv, pt.w), ox, oy, oz,
-                    dx, dy, dz, h);
+    const float4* bb = reinterpret_cast<const float4*>(g.bary + t);
+    const float4 u4 = __ldg(bb), v4 = __ldg(bb + 1);
+    return test_rec_uv(make_float4(q.x, q.y, q.z, pt.x), make_float4(pt.y, pt.z, tri_vv(g, t, u4, v4), pt.w), u4, v4,
+                       ox, oy, oz, dx, dy, dz, h);
 }
 
 // a 16-byte record k (plane in the record, triangle index beside it)

@@ -126,7 +126,7 @@ __device__ __forceinline__ void record_plane(const AccelDev& acc, uint32_t k, bo
 
 // a hit filed by crossing parameter (bits in the x / y slots); the owner
 // recomputes the point and distance in its own registers
-__device__ __forceinline__ void prec_file_hit(FlatWarp& H, uint32_t owner, uint32_t t, uint32_t type, double r) {
+__device__ __forceinline__ void prec_file_hit(HitWarp& H, uint32_t owner, uint32_t t, uint32_t type, double r) {
     const uint32_t slot = atomicAdd(&H.n[owner], 1u);
     if (slot < (uint32_t)kFlatSlots) {
         H.t[slot][owner] = t; H.type[slot][owner] = type;
@@ -137,7 +137,7 @@ __device__ __forceinline__ void prec_file_hit(FlatWarp& H, uint32_t owner, uint3
 
 // FP32 pruning of record k for owner o: returns the triangle to test in
 // FP64, or 0xFFFFFFFF
-__device__ __forceinline__ uint32_t prec_prune(const FlatWarp& H, const AccelDev& acc, uint32_t k, bool full,
+__device__ __forceinline__ uint32_t prec_prune(const HitWarp& H, const AccelDev& acc, uint32_t k, bool full,
                                                uint32_t o, PrecCount& pc) {
     float4 q;
     uint32_t t;
@@ -150,7 +150,7 @@ __device__ __forceinline__ uint32_t prec_prune(const FlatWarp& H, const AccelDev
 }
 
 // FP64 test of triangle t against owner o's sub-segment; files a hit
-__device__ __forceinline__ void prec_test(FlatWarp& H, const PrecWarp& P, const MeshDev& g, uint32_t t, uint32_t o,
+__device__ __forceinline__ void prec_test(HitWarp& H, const PrecWarp& P, const MeshDev& g, uint32_t t, uint32_t o,
                                           PrecCount& pc) {
     pc.exact++;
     double r;
@@ -168,7 +168,7 @@ __device__ __forceinline__ void prec_test(FlatWarp& H, const PrecWarp& P, const 
 // the margin of 0.05.  Other triangles (and a segment parallel to the plane
 // in FP32) always go to the FP64 test.
 static constexpr float kPreST = 0.05f;
-__device__ __forceinline__ bool prec_pretest(const FlatWarp& H, const MeshDev& g, uint32_t t, uint32_t o) {
+__device__ __forceinline__ bool prec_pretest(const HitWarp& H, const MeshDev& g, uint32_t t, uint32_t o) {
     const float4* pp = reinterpret_cast<const float4*>(g.plane + t);
     const float4 a = __ldg(pp), c = __ldg(pp + 1);  // {n, p1.x}, {p1.y, p1.z, vv, info}
     const float4* bb = reinterpret_cast<const float4*>(g.bary + t);
@@ -191,7 +191,7 @@ __device__ __forceinline__ bool prec_pretest(const FlatWarp& H, const MeshDev& g
 
 // appends the lanes' (t, o) to the FP64 queue (fn: warp-uniform length) and
 // tests full groups of 32 in FP64; all lanes call it
-__device__ __forceinline__ void prec_enqueue64(FlatWarp& H, PrecWarp& P, const MeshDev& g, uint32_t lane,
+__device__ __forceinline__ void prec_enqueue64(HitWarp& H, PrecWarp& P, const MeshDev& g, uint32_t lane,
                                                uint32_t t, uint32_t o, uint32_t& fn, PrecCount& pc) {
     const bool live = t != 0xFFFFFFFFu;
     const uint32_t b = __ballot_sync(0xFFFFFFFFu, live);
@@ -213,7 +213,7 @@ __device__ __forceinline__ void prec_enqueue64(FlatWarp& H, PrecWarp& P, const M
 // appends the lanes' surviving (t, o) to the warp's queue (qn: warp-uniform
 // length) and pre-tests full groups of 32 from its top, passing the
 // survivors to the FP64 queue; all lanes call it
-__device__ __forceinline__ void prec_enqueue(FlatWarp& H, PrecWarp& P, const MeshDev& g, uint32_t lane,
+__device__ __forceinline__ void prec_enqueue(HitWarp& H, PrecWarp& P, const MeshDev& g, uint32_t lane,
                                              uint32_t t, uint32_t o, uint32_t& qn, uint32_t& fn, PrecCount& pc) {
     const uint32_t FULL = 0xFFFFFFFFu;
     const bool live = t != 0xFFFFFFFFu;
@@ -278,7 +278,7 @@ static __device__ __noinline__ void ref_scan64(const MeshDev& g, double ox, doub
 }
 
 // a lane whose box is too wide for the warp's list: its own records
-static __device__ __noinline__ void prec_solo(FlatWarp& H, PrecWarp& P, const MeshDev& g, const AccelDev& acc,
+static __device__ __noinline__ void prec_solo(HitWarp& H, PrecWarp& P, const MeshDev& g, const AccelDev& acc,
                                               bool full, uint32_t lane, float fpx, float fpy, float fpz,
                                               PrecCount& pc) {
     const float4 O = H.o[lane];
@@ -299,7 +299,7 @@ static __device__ __noinline__ void prec_solo(FlatWarp& H, PrecWarp& P, const Me
 // it); the counterpart of flat_round_mode.  On return, for open lanes, found
 // and the hit (triangle ht, type htype, point hx, hy, hz) hold the
 // reference's collision result for the sub-segment o -> p.
-__device__ __forceinline__ void prec_round(FlatWarp& H, PrecWarp& P, const MeshDev& g, const AccelDev& acc,
+__device__ __forceinline__ void prec_round(HitWarp& H, PrecWarp& P, const MeshDev& g, const AccelDev& acc,
                                            uint32_t lane, bool open, double ox, double oy, double oz, double px,
                                            double py, double pz, uint32_t excluded, bool& found, uint32_t& ht,
                                            uint32_t& htype, double& hx, double& hy, double& hz, PrecCount& pc) {
