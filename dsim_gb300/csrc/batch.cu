@@ -116,6 +116,10 @@ struct ThinDraws {
 // cell-local jobs run in k_batch_step64 and k_batch_step_local.  THREADS:
 // block size (64, 128 or 256); MINB counts 128-thread blocks per SM, so every
 // block shape of one occupancy has the same register budget per thread.
+// Mesh lanes keep what a round does not read in shared memory (LaneState), and
+// 32-byte records past the plane test are finished 32 at a time (FlatQueue):
+// 52,000 mesh and 52,000 cylinder spins in six jobs 11.5 -> 10.6 ms for 800
+// steps.
 template <int MINB, int LAYOUT, int THREADS = kFlatThreads>
 __global__ void __launch_bounds__(THREADS, MINB * kFlatThreads / THREADS)
 k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
@@ -123,6 +127,8 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
              unsigned long long* jobCounts) {
     constexpr int MESH = LAYOUT == 3 ? 1 : LAYOUT;  // the record path of the mesh instantiations
     __shared__ FlatWarp wh[LAYOUT == 3 ? 1 : THREADS / 32];
+    __shared__ LaneState wc[LAYOUT == 3 ? 1 : THREADS / 32];
+    __shared__ FlatQueue wq[LAYOUT == 1 ? THREADS / 32 : 1];
     // gradient moments and their compensation live in shared memory (touched
     // once per step), which keeps the collision loop's registers free
     __shared__ float mom[6][THREADS];
@@ -167,29 +173,29 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
     float mag = S.f[F_MAG][i];
     const uint32_t meta = S.u[U_META][i];
     uint32_t comp = meta & 0xFFu, fiber = meta >> 8;
-    const uint32_t k0 = J.key0, k1 = J.key1;
-    const float* __restrict__ wave = J.wave;
     uint32_t nrefl = 0, nperm = 0, st = 0;
     const SubDev& sub = subS[wi];
     if (LAYOUT != 3) {
         const MeshDev& g = sub.g;
         const AccelDev& acc = sub.acc;
-        const float perm = J.perm;
-        const uint32_t reflType = J.reflType, maxSub = J.maxSub;
-        uint32_t it = 0;
+        LaneState& C = wc[LAYOUT == 3 ? 0u : wi];
+        float &cmag = C.mag[lane], &umax = C.umax[lane], &umin = C.umin[lane], &u = C.u[lane];
+        uint32_t &ccomp = C.comp[lane], &cfiber = C.fiber[lane], &crefl = C.nrefl[lane], &cperm = C.nperm[lane],
+                 &status = C.status[lane], &it = C.it[lane], &sub_n = C.sub[lane];
+        cmag = mag; ccomp = comp; cfiber = fiber;
+        umax = u = 1.0f; umin = 0.0f;
+        crefl = cperm = status = it = sub_n = 0;
         bool active = valid && nsteps > 0;
         bool fresh = active;
-        Draw d;
-        d.nx = d.ny = d.nz = 0.0f; d.u = 1.0f;
+        // the position is o at the top of a step, the start of its current sub-segment within one
         float ox = x, oy = y, oz = z, px = x, py = y, pz = z;
-        uint32_t excluded = 0xFFFFFFFFu, sub_n = 0;
-        float umax = 1.0f, umin = 0.0f;
+        uint32_t excluded = 0xFFFFFFFFu;
         while (__any_sync(FULL, active)) {
             if (fresh) {
-                d = philox_draw(id, (uint64_t)(ls0 + it), 0u, k0, k1);
-                ox = x; oy = y; oz = z;
-                const float sd = J.sd[comp & 3u];
-                px = x + d.nx * sd; py = y + d.ny * sd; pz = z + d.nz * sd;
+                const Draw d = philox_draw(id, (uint64_t)(ls0 + it), 0u, J.key0, J.key1);
+                u = d.u;
+                const float sd = J.sd[ccomp & 3u];
+                px = ox + d.nx * sd; py = oy + d.ny * sd; pz = oz + d.nz * sd;
                 excluded = 0xFFFFFFFFu;
                 umax = 1.0f; umin = 0.0f;
                 sub_n = 0;
@@ -198,14 +204,15 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
             const bool open = active;
             bool found;
             FastHit best;
-            flat_round_mode<MESH>(H, g, acc, lane, open, ox, oy, oz, px, py, pz, excluded, found, best);
+            flat_round_mode<MESH>(H, g, acc, lane, open, ox, oy, oz, px, py, pz, excluded, found, best,
+                                  LAYOUT == 1 ? &wq[LAYOUT == 1 ? wi : 0u] : nullptr);
             if (open) {
                 bool finish = !found;
                 if (found) {
-                    apply_hit(g, best, d.u, perm, reflType, umax, umin, ox, oy, oz, px, py, pz, comp, fiber,
-                              excluded, nrefl, nperm);
-                    if (++sub_n >= maxSub) {
-                        st |= kStatusSubsegCap;
+                    apply_hit(g, best, u, J.perm, J.reflType, umax, umin, ox, oy, oz, px, py, pz, ccomp, cfiber,
+                              excluded, crefl, cperm);
+                    if (++sub_n >= J.maxSub) {
+                        status |= kStatusSubsegCap;
                         px = ox; py = oy; pz = oz;
                         finish = true;
                     }
@@ -215,22 +222,26 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
                     if (ex > J.clampHi) ex = J.clampHi; else if (ex < J.clampLo) ex = J.clampLo;
                     if (ey > J.clampHi) ey = J.clampHi; else if (ey < J.clampLo) ey = J.clampLo;
                     if (ez > J.clampHi) ez = J.clampHi; else if (ez < J.clampLo) ez = J.clampLo;
-                    x = ex; y = ey; z = ez;
-                    const float T2 = J.T2[comp & 3u];
-                    if (T2 > 0.0f) mag += -mag / T2 * J.dt;
-                    const float w = __ldg(wave + ls0 + it);
-                    kahan_add(mom[0][tx], mom[3][tx], w * x);
-                    kahan_add(mom[1][tx], mom[4][tx], w * y);
-                    kahan_add(mom[2][tx], mom[5][tx], w * z);
+                    ox = ex; oy = ey; oz = ez;
+                    const float T2 = J.T2[ccomp & 3u];
+                    if (T2 > 0.0f) cmag += -cmag / T2 * J.dt;
+                    const float w = __ldg(J.wave + ls0 + it);
+                    kahan_add(mom[0][tx], mom[3][tx], w * ox);
+                    kahan_add(mom[1][tx], mom[4][tx], w * oy);
+                    kahan_add(mom[2][tx], mom[5][tx], w * oz);
                     if (++it >= nsteps) active = false;
                     else fresh = true;
                 }
             }
             __syncwarp();
         }
+        x = ox; y = oy; z = oz;
+        mag = cmag; comp = ccomp; fiber = cfiber; nrefl = crefl; nperm = cperm; st = status;
     } else if (valid) {
         const uint32_t live = __activemask();  // converged: the lanes with a spin
         ThinDraws draws;
+        const uint32_t k0 = J.key0, k1 = J.key1;
+        const float* __restrict__ wave = J.wave;
         const CylDev& g = sub.c;
         const float perm = J.perm;
         uint32_t imo = comp, nearest = fiber;
@@ -282,12 +293,16 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
 // near-degenerate intersections, Kahan moments.  Between chunks the position
 // is kept in the double fields as origin + offset; the float fields get its
 // rounded value (sort keys, float readers).
+// 4 blocks per SM: the round's two queues and FP64 re-test take 128 registers
+// (ms of runs of 200 steps at 4 / 5 / 6: 65,536 mesh spins 6.9 / 6.9 / 7.9,
+// 196,608 20.5 / 20.4 / 23.1).
 template <int LAYOUT>
 __global__ void __launch_bounds__(kFlatThreads, 4)
 k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
                    const uint32_t* __restrict__ stepNow, uint32_t chunk, uint32_t* status,
                    unsigned long long* jobCounts) {
     __shared__ HitWarp wh[kFlatWarps];
+    __shared__ LaneState wc[kFlatWarps];
     __shared__ LocalWarp wl[kFlatWarps];
     __shared__ float mom[6][kFlatThreads];
     __shared__ JobDev jobS[kFlatWarps];
@@ -322,15 +337,23 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
     const uint32_t id = S.u[U_ID][i];
     const bool valid = id != 0xFFFFFFFFu && lane < mine.y;
     // position = lattice origin (multiple of 1/16) + FP32 offset in [0, 1/16)
-    float gx = 0.0f, gy = 0.0f, gz = 0.0f, x = 0.0f, y = 0.0f, z = 0.0f, mag = 0.0f;
-    uint32_t comp = 0, fiber = 0;
+    float &gx = Lw.gx[lane], &gy = Lw.gy[lane], &gz = Lw.gz[lane];  // local_round keeps it there too
+    gx = gy = gz = 0.0f;
+    float ox = 0.0f, oy = 0.0f, oz = 0.0f;
+    LaneState& C = wc[wi];
+    float &mag = C.mag[lane], &umax = C.umax[lane], &umin = C.umin[lane], &u = C.u[lane];
+    uint32_t &comp = C.comp[lane], &fiber = C.fiber[lane], &nrefl = C.nrefl[lane], &nperm = C.nperm[lane],
+             &st = C.status[lane], &it = C.it[lane], &sub_n = C.sub[lane];
+    mag = umin = 0.0f;
+    umax = u = 1.0f;
+    comp = fiber = nrefl = nperm = st = it = sub_n = 0;
     mom[0][tx] = 0.0f; mom[1][tx] = 0.0f; mom[2][tx] = 0.0f;
     mom[3][tx] = 0.0f; mom[4][tx] = 0.0f; mom[5][tx] = 0.0f;
     if (valid) {
         const double X = S.d[D_X][i], Y = S.d[D_Y][i], Z = S.d[D_Z][i];
         const double Gx = floor(X * 16.0) * 0.0625, Gy = floor(Y * 16.0) * 0.0625, Gz = floor(Z * 16.0) * 0.0625;
         gx = (float)Gx; gy = (float)Gy; gz = (float)Gz;
-        x = (float)(X - Gx); y = (float)(Y - Gy); z = (float)(Z - Gz);
+        ox = (float)(X - Gx); oy = (float)(Y - Gy); oz = (float)(Z - Gz);
         mag = S.f[F_MAG][i];
         mom[0][tx] = S.f[F_MX][i]; mom[1][tx] = S.f[F_MY][i]; mom[2][tx] = S.f[F_MZ][i];
         mom[3][tx] = S.f[F_CX][i]; mom[4][tx] = S.f[F_CY][i]; mom[5][tx] = S.f[F_CZ][i];
@@ -339,24 +362,18 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
     }
     const MeshDev& g = subS[wi].g;
     const AccelDev& acc = subS[wi].acc;
-    const float perm = J.perm;
-    const uint32_t reflType = J.reflType, maxSub = J.maxSub;
-    const uint32_t k0 = J.key0, k1 = J.key1;
-    const float* __restrict__ wave = J.wave;
-    uint32_t nrefl = 0, nperm = 0, st = 0, it = 0, excluded = 0xFFFFFFFFu, sub_n = 0;
+    uint32_t excluded = 0xFFFFFFFFu;
     PrecCount pc;
     bool active = valid && nsteps > 0;
     bool fresh = active;
-    Draw d;
-    d.nx = d.ny = d.nz = 0.0f; d.u = 1.0f;
-    float umax = 1.0f, umin = 0.0f;
-    float ox = x, oy = y, oz = z, px = x, py = y, pz = z;
+    // the position is o at the top of a step, the start of its current sub-segment within one
+    float px = ox, py = oy, pz = oz;
     while (__any_sync(FULL, active)) {
         if (fresh) {
-            d = philox_draw(id, (uint64_t)(ls0 + it), 0u, k0, k1);
-            ox = x; oy = y; oz = z;
+            const Draw d = philox_draw(id, (uint64_t)(ls0 + it), 0u, J.key0, J.key1);
+            u = d.u;
             const float sd = J.sd[comp & 3u];
-            px = x + d.nx * sd; py = y + d.ny * sd; pz = z + d.nz * sd;
+            px = ox + d.nx * sd; py = oy + d.ny * sd; pz = oz + d.nz * sd;
             excluded = 0xFFFFFFFFu;
             umax = 1.0f; umin = 0.0f;
             sub_n = 0;
@@ -369,9 +386,9 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
         if (open) {
             bool finish = !found;
             if (found) {
-                apply_hit(g, best, d.u, perm, reflType, umax, umin, ox, oy, oz, px, py, pz, comp, fiber, excluded,
+                apply_hit(g, best, u, J.perm, J.reflType, umax, umin, ox, oy, oz, px, py, pz, comp, fiber, excluded,
                           nrefl, nperm);
-                if (++sub_n >= maxSub) {
+                if (++sub_n >= J.maxSub) {
                     st |= kStatusSubsegCap;
                     px = ox; py = oy; pz = oz;
                     finish = true;
@@ -387,13 +404,13 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
                 const float sx = floor_small(px * 16.0f) * kLatticeH, sy = floor_small(py * 16.0f) * kLatticeH,
                             sz = floor_small(pz * 16.0f) * kLatticeH;
                 gx += sx; gy += sy; gz += sz;
-                x = px - sx; y = py - sy; z = pz - sz;
+                ox = px - sx; oy = py - sy; oz = pz - sz;
                 const float T2 = J.T2[comp & 3u];
                 if (T2 > 0.0f) mag += -mag / T2 * J.dt;
-                const float w = __ldg(wave + ls0 + it);
-                kahan_add(mom[0][tx], mom[3][tx], w * (gx + x));
-                kahan_add(mom[1][tx], mom[4][tx], w * (gy + y));
-                kahan_add(mom[2][tx], mom[5][tx], w * (gz + z));
+                const float w = __ldg(J.wave + ls0 + it);
+                kahan_add(mom[0][tx], mom[3][tx], w * (gx + ox));
+                kahan_add(mom[1][tx], mom[4][tx], w * (gy + oy));
+                kahan_add(mom[2][tx], mom[5][tx], w * (gz + oz));
                 if (++it >= nsteps) active = false;
                 else fresh = true;
             }
@@ -401,7 +418,7 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
         __syncwarp();
     }
     if (valid) {
-        const double X = (double)gx + (double)x, Y = (double)gy + (double)y, Z = (double)gz + (double)z;
+        const double X = (double)gx + (double)ox, Y = (double)gy + (double)oy, Z = (double)gz + (double)oz;
         S.d[D_X][i] = X; S.d[D_Y][i] = Y; S.d[D_Z][i] = Z; S.d[D_MAG][i] = (double)mag;
         S.f[F_X][i] = (float)X; S.f[F_Y][i] = (float)Y; S.f[F_Z][i] = (float)Z;
         S.f[F_MAG][i] = mag;
@@ -849,7 +866,10 @@ struct dsim_batch {
     uint32_t* keys = nullptr;
     uint32_t *hist = nullptr, *hstart = nullptr, *scratch = nullptr;
     uint64_t keyCap = 0, K = 0;
-    uint32_t chunk = 20, occupancy = 4, graphChunks = 8;
+    // 5 blocks per SM: ms of runs of 200 steps at 4 / 5 / 6 / 7 (half of the spins
+    // in meshes, of 100 tubes): 131,072 spins 4.92 / 4.78 / 4.90 / 5.16; 393,216
+    // 15.2 / 14.4 / 14.7 / 14.6; 983,040 31.1 / 29.6 / 29.1 / 30.2
+    uint32_t chunk = 20, occupancy = 5, graphChunks = 8;
     bool chunkSet = false;  // dsim_batch_configure or the autotuner chose the chunk
     uint32_t blockThreads = kFlatThreads;  // block size of the plain step kernels (64, 128, 256)
     // the warps of each kind of step kernel, as uploaded: built from the

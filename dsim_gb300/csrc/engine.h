@@ -82,6 +82,15 @@ inline uint32_t spins_per_warp(uint64_t N, uint32_t warpsPerSm, bool pow2) {
     return p;
 }
 
+// Resident blocks per SM that a step kernel's register budget is taken for, by
+// its blocks: as few (down to `least`) as reach the fewest waves that `most`
+// give.
+inline uint32_t blocks_per_sm(uint32_t blocks, uint32_t least, uint32_t most) {
+    const uint32_t perSm = (blocks + kSmCount - 1) / kSmCount, waves = (perSm + most - 1) / most;
+    const uint32_t k = waves ? (perSm + waves - 1) / waves : 0;
+    return k < least ? least : k;
+}
+
 // ---- accel.cu -------------------------------------------------------------
 // Fine acceleration grid: every triangle is listed in each fine cell it
 // touches (separating-axis test against the cell widened by kAccelEps); cells

@@ -31,16 +31,10 @@
 
 namespace dsim {
 
-// A lane's state that only the ends of steps and the hits read, kept in shared
-// memory: a round's lists and tests hold nearly every register, and what does
-// not fit is spilled around them.  The 14 words take the 7-block form from 204
-// B of spills to 32 and make it the fastest over many waves (us per step at 4 /
-// 5 / 6 / 7 / 8 / 9 blocks per SM: 400,000 spins on 100 tubes 46.6 / 40.8 /
-// 39.0 / 37.0 / 38.7 / 41.7, 1M spins on 400 tubes 119.4 / 103.0 / 98.3 / 97.8
-// / 98.5 / 102.4; in registers, at 5: 41.7 and 105.6).
-struct LaneState {
-    float mag[32], phase[32], umax[32], umin[32], u[32];
-    uint32_t comp[32], fiber[32], id[32], nrefl[32], nperm[32], status[32], it[32], sub[32];
+// and what only this kernel keeps of a lane
+struct WalkLane : LaneState {
+    float phase[32];
+    uint32_t id[32];
 };
 
 // QUEUE (32-byte records): records past the plane test are finished 32 at a
@@ -52,7 +46,7 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
                                                                        MeshStepArgs a, SpinsSorted S,
                                                                        int rng) {
     __shared__ FlatWarp wh[kFlatWarps];
-    __shared__ LaneState wc[kFlatWarps];
+    __shared__ WalkLane wc[kFlatWarps];
     __shared__ FlatQueue wq[QUEUE ? kFlatWarps : 1];
     __shared__ FlatStage ws[STAGE ? kFlatWarps : 1];
     const uint32_t FULL = 0xFFFFFFFFu;
@@ -66,7 +60,7 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
     const bool valid = lane < a.perWarp && i < S.N;
     // the position is o at the top of a step, the start of its current sub-segment within one
     float ox = 0.0f, oy = 0.0f, oz = 0.0f;
-    LaneState& C = wc[threadIdx.x >> 5];
+    WalkLane& C = wc[threadIdx.x >> 5];
     float &mag = C.mag[lane], &phase = C.phase[lane], &umax = C.umax[lane], &umin = C.umin[lane], &u = C.u[lane];
     uint32_t &comp = C.comp[lane], &fiber = C.fiber[lane], &id = C.id[lane], &nrefl = C.nrefl[lane],
              &nperm = C.nperm[lane], &status = C.status[lane], &it = C.it[lane], &sub = C.sub[lane];
@@ -195,9 +189,8 @@ int launch_mesh_step_flat(const MeshDev& g, const AccelDev& acc, const MeshStepA
         // 17.1 / 17.7 / 13.7*; 150,000 19.1* / 18.6 / 19.5 / 20.4; 220,000 26.6 /
         // 25.2 / 22.4* / 23.9; 400,000 46.6 / 40.6 / 38.8 / 37.0*; 600,000 66.2 /
         // 57.7 / 55.5 / 55.4*
-        const uint32_t perSm = (grid.x + kSmCount - 1) / kSmCount, waves = (perSm + 6) / 7;
-        const uint32_t k = (perSm + waves - 1) / waves;
-        if (k <= 4) k_mesh_step_flat<false, 4, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
+        const uint32_t k = blocks_per_sm(grid.x, 4, 7);
+        if (k == 4) k_mesh_step_flat<false, 4, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
         else if (k == 5) k_mesh_step_flat<false, 5, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
         else if (k == 6) k_mesh_step_flat<false, 6, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);
         else k_mesh_step_flat<false, 7, 1, true><<<grid, block, 0, st>>>(g, acc, a, S, rng);

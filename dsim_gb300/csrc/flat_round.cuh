@@ -105,6 +105,19 @@ __device__ __forceinline__ bool filed_walk(const HitWarp& H, uint32_t q, uint32_
     return H.type[q][lane] & kHitWalk;
 }
 
+// A lane's state that only the ends of steps and the hits read, kept in shared
+// memory: a round's lists and tests hold nearly every register, and what does
+// not fit is spilled around them.  In the plain step these words take the form
+// of 7 blocks per SM from 204 B of spills to 32 and make it the fastest over
+// many waves (us per step at 4 / 5 / 6 / 7 / 8 / 9 blocks per SM: 400,000 spins
+// on 100 tubes 46.6 / 40.8 / 39.0 / 37.0 / 38.7 / 41.7, 1M spins on 400 tubes
+// 119.4 / 103.0 / 98.3 / 97.8 / 98.5 / 102.4; in registers, at 5: 41.7 and
+// 105.6).
+struct LaneState {
+    float mag[32], umax[32], umin[32], u[32];
+    uint32_t comp[32], fiber[32], nrefl[32], nperm[32], status[32], it[32], sub[32];
+};
+
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, uint32_t lane) {
 #pragma unroll
     for (uint32_t o = 1; o < 32; o <<= 1) {

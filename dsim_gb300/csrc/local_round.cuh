@@ -373,9 +373,10 @@ __device__ __noinline__ bool local_overflow(HitWarp& H, LocalWarp& Lw, const Mes
 
 // One collision round of the local form for every lane of the warp (all 32
 // lanes call it).  The sub-segment o -> p is in the lane's local frame at
-// origin (gx, gy, gz); on return, for open lanes, found / best hold the
-// collision result with the hit point in the same frame.  LAYOUT 1 or 2
-// compiles only the 32- or 64-byte record path; 0 dispatches on acc.wide.
+// origin (gx, gy, gz), which the caller keeps in the lane's Lw.gx, gy, gz; on
+// return, for open lanes, found / best hold the collision result with the hit
+// point in the same frame.  LAYOUT 1 or 2 compiles only the 32- or 64-byte
+// record path; 0 dispatches on acc.wide.
 template <int LAYOUT = 0>
 __device__ __forceinline__ void local_round(HitWarp& H, LocalWarp& Lw, const MeshDev& g, const AccelDev& acc,
                                             uint32_t lane, bool open, float gx, float gy, float gz, float ox,
@@ -389,7 +390,6 @@ __device__ __forceinline__ void local_round(HitWarp& H, LocalWarp& Lw, const Mes
     const FlatBox box = flat_box(acc, open, aox, aoy, aoz, apx, apy, apz);
     H.o[lane] = make_float4(ox, oy, oz, __uint_as_float(excluded));
     H.d[lane] = make_float4(dx, dy, dz, __uint_as_float(box.lo0 | (box.lo1 << 10) | (box.lo2 << 20)));
-    Lw.gx[lane] = gx; Lw.gy[lane] = gy; Lw.gz[lane] = gz;
     H.n[lane] = 0;
     FlatList l = flat_list(H, box, lane);
     uint32_t qn = 0, fn = 0;  // queue lengths (warp-uniform)

@@ -100,7 +100,7 @@ int dsim_batch_submit(dsim_batch* b, const dsim_job_desc* job, const float* pos3
                       const uint8_t* compartment, const uint32_t* fiber, uint32_t* jobId);
 /* chunk: steps between spin sorts and per launch.  Until it is configured (or
  * autotuned) dsim_batch_advance rounds to whole chunks of 20 steps and launches
- * up to 1000 at a time, to about the end of the next job; occupancy: 4 (default), 5, 6 or 8
+ * up to 1000 at a time, to about the end of the next job; occupancy: 4, 5 (until then), 6 or 8
  * resident blocks per SM for the step kernel; graphChunks: chunks captured in
  * one CUDA graph launch (0 = plain launches, default 8) */
 int dsim_batch_configure(dsim_batch* b, uint32_t chunk, uint32_t occupancy, uint32_t graphChunks);
