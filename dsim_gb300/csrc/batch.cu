@@ -501,6 +501,10 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
     const AccelDev& acc = subS[wi].acc;
     const double perm = (double)J.perm;
     const double hiC = 1.0 - (double)J.spinR, loC = -1.0 + (double)J.spinR;
+    // a point whose float coordinates keep inside this needs no clamp
+    const float inside = (float)hiC - 1e-6f;
+    uint32_t decayOf = 4u;  // the compartment that T2 and rT2 are of
+    double T2 = 0.0, rT2 = 0.0;
     const uint32_t reflType = J.reflType, maxSub = J.maxSub;
     const uint32_t k0 = J.key0, k1 = J.key1;
     const float* __restrict__ wave = J.wave;
@@ -539,12 +543,18 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
                 }
             }
             if (finish) {
-                if (px > hiC) px = hiC; else if (px < loC) px = loC;
-                if (py > hiC) py = hiC; else if (py < loC) py = loC;
-                if (pz > hiC) pz = hiC; else if (pz < loC) pz = loC;
+                if (!(fmaxf(fabsf((float)px), fmaxf(fabsf((float)py), fabsf((float)pz))) < inside)) {
+                    if (px > hiC) px = hiC; else if (px < loC) px = loC;
+                    if (py > hiC) py = hiC; else if (py < loC) py = loC;
+                    if (pz > hiC) pz = hiC; else if (pz < loC) pz = loC;
+                }
                 x = px; y = py; z = pz;
-                const float T2 = J.T2[comp & 3u];
-                if (T2 > 0.0f) mag += -mag / (double)T2 * (double)J.dt;
+                if ((comp & 3u) != decayOf) {
+                    decayOf = comp & 3u;
+                    T2 = (double)J.T2[decayOf];
+                    rT2 = 1.0 / T2;
+                }
+                if (T2 > 0.0) mag += div_by(-mag, T2, rT2) * (double)J.dt;
                 const double w = (double)__ldg(wave + ls0 + it);
                 Mx += w * x; My += w * y; Mz += w * z;
                 if (++it >= nsteps) active = false;
@@ -1081,20 +1091,29 @@ k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
         Cyl64 form = {(double)__ldg(&J.inR)};
         bool clear = false;
         const double hiC = 1.0 - (double)__ldg(&J.spinR), loC = -1.0 + (double)__ldg(&J.spinR);
+        // a point whose float coordinates keep inside this needs no clamp
+        const float inside = (float)hiC - 1e-6f;
         const double dt = (double)__ldg(&J.dt);
         const uint32_t k0 = __ldg(&J.key0), k1 = __ldg(&J.key1);
         const float* __restrict__ wave = J.wave;
+        uint32_t decayOf = 3u;  // the region that T2 and rT2 are of
+        double T2 = 0.0, rT2 = 0.0;
         for (uint32_t it = 0; it < nsteps; it++) {
             const Draw d = draws.step(it, W.per, lane, live, id, ls0, k0, k1);
             const double sd = (double)__ldg(&J.sd[imo == 0 ? 0 : (imo == 1 ? 1 : 2)]);
             const P3<double> o = {x, y, z};
             P3<double> p = {x + (double)d.nx * sd, y + (double)d.ny * sd, z + (double)d.nz * sd};
             cyl_membranes(g, form, o, p, (double)d.u, perm, imo, nearest, nrefl, nperm, st, clear);
-            cyl_clamp(p, loC, hiC, clear);
+            if (!(fmaxf(fabsf((float)p.x), fmaxf(fabsf((float)p.y), fabsf((float)p.z))) < inside))
+                cyl_clamp(p, loC, hiC, clear);
             x = p.x; y = p.y; z = p.z;
             if (imo <= 2) {
-                const float T2 = __ldg(&J.T2[imo]);
-                if (T2 > 0.0f) mag += -mag / (double)T2 * dt;
+                if (imo != decayOf) {
+                    decayOf = imo;
+                    T2 = (double)__ldg(&J.T2[imo]);
+                    rT2 = 1.0 / T2;
+                }
+                if (T2 > 0.0) mag += div_by(-mag, T2, rT2) * dt;
             }
             const double w = (double)__ldg(wave + ls0 + it);
             Mx += w * x; My += w * y; Mz += w * z;

@@ -117,6 +117,17 @@ __device__ __forceinline__ Draw philox_draw(uint32_t spin, uint64_t step, uint32
     d.u = u4;
     return d;
 }
+
+// a / b from r = 1 / b correctly rounded, to the same bits: a q within an ulp,
+// its exact remainder and one correction (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
+// 34, 1990, theorem 2), where nothing over- or underflows; b a positive float's
+// value.  3 FP64 operations for the dozen of a division.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+    if (!(fabs(a) > 1e-200 && fabs(a) < 1e200)) return a / b;
+    const double q = a * r;
+    return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
 #endif  // __CUDACC__
 
 // ---- geometry records held in HBM for the mesh path ---------------------

@@ -173,7 +173,7 @@ __device__ __forceinline__ bool prec_pretest(const HitWarp& H, const MeshDev& g,
     const float4 a = __ldg(pp), c = __ldg(pp + 1);  // {n, p1.x}, {p1.y, p1.z, vv, info}
     const float4* bb = reinterpret_cast<const float4*>(g.bary + t);
     const float4 u4 = __ldg(bb), v4 = __ldg(bb + 1);  // {u, v.x}, {v.y, v.z, uv, uu}
-    const float uv = v4.z, uu = v4.w, vv = fabsf(c.z);
+    const float uv = v4.z, uu = fabsf(v4.w), vv = fabsf(c.z);  // signs: k_tri_regular
     const float mn = fminf(uu, vv), mx = fmaxf(uu, vv);
     if (!((uv * uv <= 0.82f * uu * vv) & (mx <= 100.0f * mn) & (mn >= 1e-6f))) return true;
     const float4 O = H.o[o], D4 = H.d[o];
