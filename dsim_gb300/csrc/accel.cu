@@ -119,11 +119,30 @@ __device__ __forceinline__ void cell_span(uint32_t k, uint32_t nf, double& lo, d
     hi = (k == nf - 1) ? 1.0e6 : -1.0 + (double)(k + 1) * Lf + (double)kAccelEps;
 }
 
+// The corners of a triangle relative to the middle of cell k on one axis, in
+// float (the middle to 1e-15, against 1e-9 that tri_box_overlap32 allows for)
+struct CellAxis {
+    float v[3];
+};
+__device__ __forceinline__ CellAxis cell_axis(uint32_t k, double Lf, float c0, float c1, float c2) {
+    const double ctr = -1.0 + ((double)k + 0.5) * Lf;
+    CellAxis a;
+    a.v[0] = (float)((double)c0 - ctr);
+    a.v[1] = (float)((double)c1 - ctr);
+    a.v[2] = (float)((double)c2 - ctr);
+    return a;
+}
+
+// Pass 1 counts, pass 2 fills.  touched: per triangle of up to kMaskCells cells
+// in its range, the ones pass 1 found it in by their order, so that pass 2 tests
+// none again; a larger triangle's are tested in both.  The FP64 parts of a test
+// are formed once per cell of each axis.  640,000 triangles: count 0.45 -> 0.30
+// ms, fill 0.50 -> 0.09 ms.
 template <bool FILL>
 __global__ void k_accel_cells(uint32_t nT, const TriPlane* __restrict__ plane,
                               const TriBary* __restrict__ bary, uint32_t nf, float invLf,
                               uint32_t* counter, const uint32_t* __restrict__ start, AccelRec* rec,
-                              uint32_t* tri, AccelRecWide* recw, AccelRecFull* recf) {
+                              uint32_t* tri, AccelRecWide* recw, AccelRecFull* recf, uint64_t* touched) {
     uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nT) return;
     TriPlane P = plane[t];
@@ -134,36 +153,45 @@ __global__ void k_accel_cells(uint32_t nT, const TriPlane* __restrict__ plane,
     const float c0[3] = {P.p1x, P.p1y, P.p1z};
     const float c1[3] = {P.p1x + B.vx, P.p1y + B.vy, P.p1z + B.vz};
     const float c2[3] = {P.p1x + B.ux, P.p1y + B.uy, P.p1z + B.uz};
-    const bool many = (hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * (hi[2] - lo[2] + 1) > 1;
-    for (uint32_t x = lo[0]; x <= hi[0]; x++)
-        for (uint32_t y = lo[1]; y <= hi[1]; y++)
-            for (uint32_t z = lo[2]; z <= hi[2]; z++) {
-                if (many) {
-                    double bl[3], bh[3], ctr[3], h[3];
-                    float v32[3][3], h32[3];
-                    cell_span(x, nf, bl[0], bh[0]);
-                    cell_span(y, nf, bl[1], bh[1]);
-                    cell_span(z, nf, bl[2], bh[2]);
-                    for (int k = 0; k < 3; k++) {
-                        ctr[k] = 0.5 * (bl[k] + bh[k]);
-                        h[k] = 0.5 * (bh[k] - bl[k]);
-                        h32[k] = (float)h[k];
-                        v32[0][k] = (float)((double)c0[k] - ctr[k]);
-                        v32[1][k] = (float)((double)c1[k] - ctr[k]);
-                        v32[2][k] = (float)((double)c2[k] - ctr[k]);
-                    }
-                    const int clear = tri_box_overlap32(v32, h32);
+    const uint64_t cells = (uint64_t)(hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * (hi[2] - lo[2] + 1);
+    const bool many = cells > 1, masked = cells <= kMaskCells, test = many && !(FILL && masked);
+    uint64_t mask = FILL && masked ? touched[t] : 0ull, bit = 1ull;
+    // the outermost cells are open: left to the FP64 axes
+    const double Lf = 2.0 / (double)nf;
+    const float hf = (float)(0.5 * Lf + (double)kAccelEps);
+    const float h32[3] = {hf, hf, hf};
+    CellAxis ax = {}, ay = {}, az;
+    for (uint32_t x = lo[0]; x <= hi[0]; x++) {
+        if (test) ax = cell_axis(x, Lf, c0[0], c1[0], c2[0]);
+        for (uint32_t y = lo[1]; y <= hi[1]; y++) {
+            if (test) ay = cell_axis(y, Lf, c0[1], c1[1], c2[1]);
+            for (uint32_t z = lo[2]; z <= hi[2]; z++, bit <<= 1) {
+                if (test) {
+                    az = cell_axis(z, Lf, c0[2], c1[2], c2[2]);
+                    const float v32[3][3] = {{ax.v[0], ay.v[0], az.v[0]},
+                                             {ax.v[1], ay.v[1], az.v[1]},
+                                             {ax.v[2], ay.v[2], az.v[2]}};
+                    const bool open = min(x, min(y, z)) == 0 || max(x, max(y, z)) == nf - 1;
+                    const int clear = open ? 2 : tri_box_overlap32(v32, h32);
                     if (clear == 0) continue;
                     if (clear == 2) {
-                        double v[3][3];
+                        const uint32_t at[3] = {x, y, z};
+                        double v[3][3], h[3];
                         for (int k = 0; k < 3; k++) {
-                            v[0][k] = (double)c0[k] - ctr[k];
-                            v[1][k] = (double)c1[k] - ctr[k];
-                            v[2][k] = (double)c2[k] - ctr[k];
+                            double bl, bh;
+                            cell_span(at[k], nf, bl, bh);
+                            const double ctr = 0.5 * (bl + bh);
+                            h[k] = 0.5 * (bh - bl);
+                            v[0][k] = (double)c0[k] - ctr;
+                            v[1][k] = (double)c1[k] - ctr;
+                            v[2][k] = (double)c2[k] - ctr;
                         }
                         if (!tri_box_overlap(v, h)) continue;
                     }
+                } else if (FILL && masked && !(mask & bit)) {
+                    continue;
                 }
+                if (!FILL) mask |= bit;
                 uint32_t key = morton3(x, y, z);
                 uint32_t slot = atomicAdd(counter + key, 1u);
                 if (FILL) {
@@ -188,17 +216,20 @@ __global__ void k_accel_cells(uint32_t nT, const TriPlane* __restrict__ plane,
                     }
                 }
             }
+        }
+    }
+    if (!FILL && masked) touched[t] = mask;
 }
 
 int launch_accel_cells(bool fill, uint32_t nT, const TriPlane* plane, const TriBary* bary,
                        uint32_t nf, uint32_t* counter, const uint32_t* start, AccelRec* rec,
-                       uint32_t* tri, AccelRecWide* recw, cudaStream_t st, AccelRecFull* recf) {
+                       uint32_t* tri, AccelRecWide* recw, uint64_t* touched, cudaStream_t st, AccelRecFull* recf) {
     if (nT == 0) return kOk;
     float invLf = (float)nf / 2.0f;
     if (fill)
-        k_accel_cells<true><<<(nT + 127) / 128, 128, 0, st>>>(nT, plane, bary, nf, invLf, counter, start, rec, tri, recw, recf);
+        k_accel_cells<true><<<(nT + 127) / 128, 128, 0, st>>>(nT, plane, bary, nf, invLf, counter, start, rec, tri, recw, recf, touched);
     else
-        k_accel_cells<false><<<(nT + 127) / 128, 128, 0, st>>>(nT, plane, bary, nf, invLf, counter, start, rec, tri, recw, recf);
+        k_accel_cells<false><<<(nT + 127) / 128, 128, 0, st>>>(nT, plane, bary, nf, invLf, counter, start, rec, tri, recw, recf, touched);
     DSIM_CUDA_TRY(cudaGetLastError());
     return kOk;
 }

@@ -109,12 +109,14 @@ static int accel_build(dsim_mesh* m, uint32_t nf) {
     uint32_t* counter = nullptr;
     uint32_t* scratch = nullptr;
     cudaStream_t st = 0;
-    if ((rc = dev_alloc(&counter, nkeys))) return rc;
+    const size_t pairs = ((size_t)nkeys + 1) / 2;  // the counters, then the touched cells' bits
+    if ((rc = dev_alloc(&counter, 2 * (pairs + m->nT)))) return rc;
+    uint64_t* touched = reinterpret_cast<uint64_t*>(counter) + pairs;
     if ((rc = dev_alloc(&scratch, scan_scratch_words(nkeys)))) { cudaFree(counter); return rc; }
     do {
         if ((rc = dev_alloc(&m->acc_start, (size_t)nkeys + 1, &m->accBytes))) break;
         if (cudaMemsetAsync(counter, 0, (size_t)nkeys * 4, st) != cudaSuccess) { rc = kErrCuda; break; }
-        if ((rc = launch_accel_cells(false, m->nT, m->plane, m->bary, nf, counter, nullptr, nullptr, nullptr, nullptr, st))) break;
+        if ((rc = launch_accel_cells(false, m->nT, m->plane, m->bary, nf, counter, nullptr, nullptr, nullptr, nullptr, touched, st))) break;
         if ((rc = launch_scan_exclusive(counter, m->acc_start, nkeys, scratch, st))) break;
         uint32_t total = 0;
         if (cudaMemcpyAsync(&total, m->acc_start + nkeys, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -129,7 +131,7 @@ static int accel_build(dsim_mesh* m, uint32_t nf) {
             if ((rc = dev_alloc(&m->acc_tri, total, &m->accBytes))) break;
         }
         if (cudaMemsetAsync(counter, 0, (size_t)nkeys * 4, st) != cudaSuccess) { rc = kErrCuda; break; }
-        if ((rc = launch_accel_cells(true, m->nT, m->plane, m->bary, nf, counter, m->acc_start, m->acc_rec, m->acc_tri, m->acc_recw, st, m->acc_recf))) break;
+        if ((rc = launch_accel_cells(true, m->nT, m->plane, m->bary, nf, counter, m->acc_start, m->acc_rec, m->acc_tri, m->acc_recw, touched, st, m->acc_recf))) break;
         if ((rc = dev_alloc(&m->acc_cell, (size_t)nf * nf * nf, &m->accBytes))) break;
         if ((rc = launch_accel_slabs(nf, m->plane, m->bary, m->acc_start, m->acc_tri, m->acc_recw, m->acc_recf, m->acc_cell, st))) break;
         if (cudaStreamSynchronize(st) != cudaSuccess) { rc = kErrCuda; break; }
@@ -327,7 +329,10 @@ static int mesh_build(dsim_mesh* m, const std::vector<float>& Vn, const std::vec
     rc = kOk;
     do {
         if (cudaMemsetAsync(counter, 0, ncells * 4, st) != cudaSuccess) { rc = kErrCuda; break; }
-        if ((rc = launch_tri_cells(false, m->nT, m->V, m->trgls, m->n, m->L, counter, nullptr, nullptr, st))) break;
+        // its room holds the touched cells' bits until the lists are made
+        if ((rc = dev_alloc(&m->tri_cells, m->nT, &m->bytes))) break;
+        uint64_t* touched = reinterpret_cast<uint64_t*>(m->tri_cells);
+        if ((rc = launch_tri_cells(false, m->nT, m->V, m->trgls, m->n, m->L, counter, nullptr, nullptr, touched, st))) break;
         if ((rc = launch_scan_exclusive(counter, m->cell_start, ncells, scratch, st))) break;
         uint32_t total = 0;
         if (cudaMemcpyAsync(&total, m->cell_start + ncells, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -335,9 +340,8 @@ static int mesh_build(dsim_mesh* m, const std::vector<float>& Vn, const std::vec
         m->entries = total;
         if ((rc = dev_alloc(&m->cell_tri, total, &m->bytes))) break;
         if (cudaMemsetAsync(counter, 0, ncells * 4, st) != cudaSuccess) { rc = kErrCuda; break; }
-        if ((rc = launch_tri_cells(true, m->nT, m->V, m->trgls, m->n, m->L, counter, m->cell_start, m->cell_tri, st))) break;
+        if ((rc = launch_tri_cells(true, m->nT, m->V, m->trgls, m->n, m->L, counter, m->cell_start, m->cell_tri, touched, st))) break;
         if ((rc = launch_sort_cells(ncells, m->cell_start, m->cell_tri, st))) break;
-        if ((rc = dev_alloc(&m->tri_cells, m->nT, &m->bytes))) break;
         if (m->nT > ncells) {  // the scan scratch is sized for ncells; use a count of its own
             uint32_t* tcount = nullptr;
             if ((rc = dev_alloc(&tcount, m->nT))) break;

@@ -181,17 +181,19 @@ int derive(State& s, const uint32_t* tic, const uint32_t* cc) {
     uint32_t nkeys = accel_keys(nf);
     uint32_t* counter = nullptr;
     uint32_t* scr = nullptr;
-    DSIM_CUDA_TRY(cudaMalloc(&counter, (size_t)nkeys * 4));
+    const size_t pairs = ((size_t)nkeys + 1) / 2;  // the counters, then the touched cells' bits
+    DSIM_CUDA_TRY(cudaMalloc(&counter, (pairs + nT) * 8));
+    uint64_t* touched = reinterpret_cast<uint64_t*>(counter) + pairs;
     DSIM_CUDA_TRY(cudaMalloc(&scr, scan_scratch_words(nkeys) * 4));
     DSIM_CUDA_TRY(cudaMalloc(&s.acc_start, ((size_t)nkeys + 1) * 4));
     DSIM_CUDA_TRY(cudaMemset(counter, 0, (size_t)nkeys * 4));
-    rc = launch_accel_cells(false, nT, s.plane, s.bary, nf, counter, nullptr, nullptr, nullptr, nullptr, 0);
+    rc = launch_accel_cells(false, nT, s.plane, s.bary, nf, counter, nullptr, nullptr, nullptr, nullptr, touched, 0);
     if (!rc) rc = launch_scan_exclusive(counter, s.acc_start, nkeys, scr, 0);
     uint32_t accTotal = 0;
     if (!rc && cudaMemcpy(&accTotal, s.acc_start + nkeys, 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = kErrCuda;
     if (!rc && cudaMalloc(&s.acc_recw, (size_t)(accTotal ? accTotal : 1) * sizeof(AccelRecWide)) != cudaSuccess) rc = kErrNoMem;
     if (!rc && cudaMemset(counter, 0, (size_t)nkeys * 4) != cudaSuccess) rc = kErrCuda;
-    if (!rc) rc = launch_accel_cells(true, nT, s.plane, s.bary, nf, counter, s.acc_start, nullptr, nullptr, s.acc_recw, 0);
+    if (!rc) rc = launch_accel_cells(true, nT, s.plane, s.bary, nf, counter, s.acc_start, nullptr, nullptr, s.acc_recw, touched, 0);
     if (!rc && cudaMalloc(&s.acc_cell, (size_t)nf * nf * nf * sizeof(AccelCell)) != cudaSuccess) rc = kErrNoMem;
     if (!rc) rc = launch_accel_slabs(nf, s.plane, s.bary, s.acc_start, nullptr, s.acc_recw, nullptr, s.acc_cell, 0);
     cudaFree(counter);

@@ -141,9 +141,14 @@ __host__ __device__ inline uint32_t accel_keys(uint32_t nf) {
     for (uint32_t b = 0; b < 10; b++) s |= ((v >> b) & 1u) << (3 * b);
     return (s | (s << 1) | (s << 2)) + 1;
 }
+// Both passes of a list build (count, fill) over the triangles' cells; touched:
+// nT words that the count leaves for the fill, one bit per cell of a
+// triangle's range where that has at most kMaskCells
+static constexpr uint32_t kMaskCells = 64;
 int launch_accel_cells(bool fill, uint32_t nT, const TriPlane* plane, const TriBary* bary,
                        uint32_t nf, uint32_t* counter, const uint32_t* start, AccelRec* rec,
-                       uint32_t* tri, AccelRecWide* recw, cudaStream_t st, AccelRecFull* recf = nullptr);
+                       uint32_t* tri, AccelRecWide* recw, uint64_t* touched, cudaStream_t st,
+                       AccelRecFull* recf = nullptr);
 // the cells' slabs from their records (any layout) and the triangles' corners
 int launch_accel_slabs(uint32_t nf, const TriPlane* plane, const TriBary* bary, const uint32_t* start,
                        const uint32_t* tri, const AccelRecWide* recw, const AccelRecFull* recf, AccelCell* cell,
@@ -184,7 +189,7 @@ int launch_records_from_helpers(uint32_t nT, const float* V, const float* H,
                                 const uint32_t* triInfo, TriPlane* plane, TriBary* bary,
                                 cudaStream_t st);
 int launch_tri_cells(bool fill, uint32_t nT, const float* V, const uint32_t* trgls, uint32_t n,
-                     float L, uint32_t* counter, const uint32_t* start, uint32_t* cell_tri,
+                     float L, uint32_t* counter, const uint32_t* start, uint32_t* cell_tri, uint64_t* touched,
                      cudaStream_t st);
 int launch_sort_cells(uint32_t ncells, const uint32_t* start, uint32_t* cell_tri, cudaStream_t st);
 int launch_dense_to_csr(uint32_t ncells, uint32_t maxTPC, uint32_t nT, const uint32_t* counter,

@@ -167,12 +167,15 @@ __device__ bool tri_cube_overlap(f3 p1, f3 p2, f3 p3, f3 cmin, f3 cmax) {
     return false;
 }
 
-// pass 1 (count) and pass 2 (fill) of the grid build, one thread per triangle
+// Pass 1 (count) and pass 2 (fill) of the grid build, one thread per triangle;
+// touched: as k_accel_cells keeps it, so that pass 2 need not repeat the tests
+// (up to 48 segment-triangle tests a cell).  640,000 triangles: fill 0.37 ->
+// 0.03 ms.
 template <bool FILL>
 __global__ void k_tri_cells(uint32_t nT, const float* __restrict__ V,
                             const uint32_t* __restrict__ trgls, uint32_t n, float L,
                             uint32_t* counter, const uint32_t* __restrict__ start,
-                            uint32_t* cell_tri) {
+                            uint32_t* cell_tri, uint64_t* touched) {
     uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nT) return;
     uint32_t i1 = trgls[3 * t], i2 = trgls[3 * t + 1], i3 = trgls[3 * t + 2];
@@ -188,18 +191,25 @@ __global__ void k_tri_cells(uint32_t nT, const float* __restrict__ V,
     if (p2.z > mx.z) mx.z = p2.z; if (p3.z > mx.z) mx.z = p3.z;
     uint32_t x0 = cube_coord(mn.x, L, n), y0 = cube_coord(mn.y, L, n), z0 = cube_coord(mn.z, L, n);
     uint32_t x1 = cube_coord(mx.x, L, n), y1 = cube_coord(mx.y, L, n), z1 = cube_coord(mx.z, L, n);
+    const uint64_t cells = x0 <= x1 && y0 <= y1 && z0 <= z1
+                               ? (uint64_t)(x1 - x0 + 1) * (y1 - y0 + 1) * (z1 - z0 + 1) : 0;
+    const bool masked = cells <= kMaskCells;
+    uint64_t mask = FILL && masked ? touched[t] : 0ull, bit = 1ull;
     for (uint32_t xc = x0; xc <= x1; xc++)
         for (uint32_t yc = y0; yc <= y1; yc++)
-            for (uint32_t zc = z0; zc <= z1; zc++) {
+            for (uint32_t zc = z0; zc <= z1; zc++, bit <<= 1) {
+                if (FILL && masked && !(mask & bit)) continue;
                 uint32_t cube = n * n * zc + n * yc + xc;
                 f3 cmin = mk3(-1.0f + (float)xc * L, -1.0f + (float)yc * L, -1.0f + (float)zc * L);
                 f3 cmax = mk3(-1.0f + (float)(xc + 1) * L, -1.0f + (float)(yc + 1) * L,
                               -1.0f + (float)(zc + 1) * L);
-                if (tri_cube_overlap(p1, p2, p3, cmin, cmax)) {
+                if ((FILL && masked) || tri_cube_overlap(p1, p2, p3, cmin, cmax)) {
+                    if (!FILL) mask |= bit;
                     uint32_t slot = atomicAdd(counter + cube, 1u);
                     if (FILL) cell_tri[start[cube] + slot] = t;
                 }
             }
+    if (!FILL && masked) touched[t] = mask;
 }
 
 // Ascending triangle order inside each cell (the reference's list order): one
@@ -268,14 +278,16 @@ int launch_records_from_mesh(uint32_t nT, const float* V, const uint32_t* trgls,
     return kOk;
 }
 
-// every triangle's reference cells: one thread per cell appends the cell to
-// each of its triangles' records (order within a record is irrelevant)
+// Every triangle's reference cells: a warp per cell appends the cell to each of
+// its triangles' records (order within a record is irrelevant).  A thread per
+// cell left 640,000 triangles' lists to the longest ones: 0.10 -> 0.02 ms.
 __global__ void k_tri_cell_lists(uint32_t n, const uint32_t* __restrict__ cell_start,
                                  const uint32_t* __restrict__ cell_tri, uint32_t* count, uint4* out) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= n * n * n) return;
     const uint32_t packed = (c % n) | (((c / n) % n) << 10) | ((c / (n * n)) << 20);
-    for (uint32_t k = cell_start[c]; k < cell_start[c + 1]; k++) {
+    const uint32_t e = cell_start[c + 1];
+    for (uint32_t k = cell_start[c] + (threadIdx.x & 31u); k < e; k += 32) {
         const uint32_t t = cell_tri[k];
         const uint32_t slot = atomicAdd(count + t, 1u);
         if (slot < 4) reinterpret_cast<uint32_t*>(out + t)[slot] = packed;
@@ -291,7 +303,7 @@ int launch_tri_cell_lists(uint32_t n, uint32_t nT, const uint32_t* cell_start, c
     if (nT == 0) return kOk;
     DSIM_CUDA_TRY(cudaMemsetAsync(count, 0, (size_t)nT * 4, st));
     DSIM_CUDA_TRY(cudaMemsetAsync(out, 0xFF, (size_t)nT * sizeof(uint4), st));
-    k_tri_cell_lists<<<(n * n * n + 255) / 256, 256, 0, st>>>(n, cell_start, cell_tri, count, out);
+    k_tri_cell_lists<<<(n * n * n + 7) / 8, 256, 0, st>>>(n, cell_start, cell_tri, count, out);
     k_tri_cell_many<<<(nT + 255) / 256, 256, 0, st>>>(nT, count, out);
     DSIM_CUDA_TRY(cudaGetLastError());
     return kOk;
@@ -313,13 +325,13 @@ int launch_records_from_helpers(uint32_t nT, const float* V, const float* H, con
 }
 
 int launch_tri_cells(bool fill, uint32_t nT, const float* V, const uint32_t* trgls, uint32_t n,
-                     float L, uint32_t* counter, const uint32_t* start, uint32_t* cell_tri,
+                     float L, uint32_t* counter, const uint32_t* start, uint32_t* cell_tri, uint64_t* touched,
                      cudaStream_t st) {
     if (nT == 0) return kOk;
     if (fill)
-        k_tri_cells<true><<<(nT + 127) / 128, 128, 0, st>>>(nT, V, trgls, n, L, counter, start, cell_tri);
+        k_tri_cells<true><<<(nT + 127) / 128, 128, 0, st>>>(nT, V, trgls, n, L, counter, start, cell_tri, touched);
     else
-        k_tri_cells<false><<<(nT + 127) / 128, 128, 0, st>>>(nT, V, trgls, n, L, counter, start, cell_tri);
+        k_tri_cells<false><<<(nT + 127) / 128, 128, 0, st>>>(nT, V, trgls, n, L, counter, start, cell_tri, touched);
     DSIM_CUDA_TRY(cudaGetLastError());
     return kOk;
 }

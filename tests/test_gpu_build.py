@@ -79,3 +79,24 @@ def test_fine_grid_entries_equal_the_fp64_axes(engine, tmp_path, nf):
     V = np.asarray(mo.vertices, F).reshape(-1, 3)
     T = np.asarray(mo.trgls).reshape(-1, 3)
     assert m.accel_info()["entries"] == _entries64(V, T, nf)
+
+
+@pytest.mark.parametrize("size,nf", [(0.02, 64), (0.055, 64), (0.12, 64), (0.3, 64), (0.7, 9)])
+def test_fine_grid_entries_of_triangles_of_few_and_many_cells(engine, size, nf):
+    """Triangles whose ranges hold from one cell to hundreds (the fill reads the count's bits up to 64 cells and tests
+    the cells of larger ones again): entries as the FP64 axes have them, and both passes agree (the sums are the lists')."""
+    from dsim_gb300.engine import Mesh
+    rng = np.random.default_rng(int(size * 1000))
+    T = 400
+    ctr = rng.uniform(-0.9, 0.9, (T, 1, 3))
+    V = np.clip(ctr + rng.uniform(-size / 2, size / 2, (T, 3, 3)), -0.99, 0.99).astype(F).reshape(-1, 3)
+    tri = np.arange(3 * T, dtype=np.uint32).reshape(-1, 3)
+    m = Mesh.from_arrays(V, tri, np.zeros(T, np.uint32), np.zeros(T, np.uint32), 1.0, numCubes=8)
+    m.set_accel(nf)
+    assert m.accel_info()["entries"] == _entries64(V, tri, nf)
+    lists = m.grid()
+    cc, tic, maxtpc = O.populate_cubes(V.reshape(-1), tri.reshape(-1), 8)
+    assert np.array_equal(np.diff(lists[0].astype(np.int64)), cc.astype(np.int64))
+    dense = tic.reshape(-1, maxtpc)
+    for c in np.nonzero(cc)[0]:
+        assert np.array_equal(lists[1][lists[0][c]:lists[0][c + 1]], dense[c, :cc[c]])
