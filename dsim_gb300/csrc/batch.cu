@@ -54,7 +54,7 @@ struct JobDev {
     uint32_t key0, key1;
     uint32_t flags;               // DSIM_JOB_PRECISE or DSIM_JOB_LOCAL
     float spinR;                  // spin radius (the precision form clamps to +-(1 - spinR) in FP64)
-    uint32_t sortRegion;          // cylinders: spins outside every fiber sort after those inside
+    uint32_t sortRegion;          // cylinders: spins outside every fiber sort after those inside, each kind by id
 };
 
 static_assert(sizeof(JobDev) % 4 == 0 && sizeof(SubDev) % 4 == 0, "records are copied by 32-bit words");
@@ -594,27 +594,36 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
 
 __global__ void k_batch_advance(uint32_t* stepNow, uint32_t chunk) { *stepNow += chunk; }
 
-// sort key: job's base + Morton code of the spin's cell in a 2^bits grid
-// over the box; padding goes to the job's last key
+// sort key: job's base + Morton code of the spin's cell in a 2^bits grid over
+// the box (mesh jobs), or region and scattered id (cylinder jobs); padding goes
+// to the job's last key
 __global__ void k_batch_keys(const JobDev* __restrict__ jobs, BatchSpins S, uint32_t* keys,
                              uint32_t* hist) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= S.N) return;
     const JobDev& J = jobs[S.u[U_JOB][i]];
-    const uint32_t bits = J.sortBits, n = 1u << bits;
+    const uint32_t bits = J.sortBits, n = 1u << bits, id = S.u[U_ID][i];
     uint32_t key;
-    if (S.u[U_ID][i] == 0xFFFFFFFFu) {
+    if (id == 0xFFFFFFFFu) {
         key = J.sortBase + ((J.sortRegion ? 2u : 1u) << (3 * bits)) - 1u;
-    } else {
+    } else if (J.sortRegion) {
         // cylinder jobs: a spin outside every fiber scans its cell's fiber
-        // list (twice), one inside tests its own fiber once, so the two
-        // kinds go to separate warps: region (imo == 2) above the cell code
-        const uint32_t region = J.sortRegion && (S.u[U_META][i] & 0xFFu) >= 2u ? 1u : 0u;
+        // list, one inside tests its own fiber, so the two kinds go to
+        // separate warps; within a kind the spins are spread by their ids.
+        // Neighbours share the crowded cells: in Morton order a few warps held
+        // most of the long steps and set a launch's time (FP64 form, kcycles a
+        // step of a warp: mean 5.9, largest 21.5), while the fiber lists stay in
+        // L1 in any order.  ms of runs in Morton order / spread: two FP64 jobs
+        // 8.9 / 8.3, two of 32,768 spins 8.2 / 7.2, six local jobs of 65,536
+        // 21.5 / 20.7, six plain ones 14.0 / 13.5.
+        const uint32_t region = (S.u[U_META][i] & 0xFFu) >= 2u ? 1u : 0u;
+        key = J.sortBase + (region << (3 * bits)) + ((id * 0x9E3779B1u) >> (32u - 3u * bits));
+    } else {
         const float s = 0.5f * (float)n;
         uint32_t a = (uint32_t)fminf(fmaxf(floorf((S.f[F_X][i] + 1.0f) * s), 0.0f), (float)(n - 1));
         uint32_t b = (uint32_t)fminf(fmaxf(floorf((S.f[F_Y][i] + 1.0f) * s), 0.0f), (float)(n - 1));
         uint32_t c = (uint32_t)fminf(fmaxf(floorf((S.f[F_Z][i] + 1.0f) * s), 0.0f), (float)(n - 1));
-        key = J.sortBase + (region << (3 * bits)) + morton3(a, b, c);
+        key = J.sortBase + morton3(a, b, c);
     }
     keys[i] = key;
     atomicAdd(hist + key, 1u);
