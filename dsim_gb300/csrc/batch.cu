@@ -80,13 +80,22 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
     s = t;
 }
 
-// The warps of one kind of step kernel: first slot and number of slots (of one
-// job) of each, at most `per` (spins_per_warp over the kind's spins).  A launch
-// covers the kind's unfinished jobs only, whatever else the batch holds.
+// The warps of one kind of step kernel: first slot, number of slots (of one
+// job) and the stride between them of each, at most `per` slots (spins_per_warp
+// over the kind's spins).  A launch covers the kind's unfinished jobs only,
+// whatever else the batch holds.  Mesh slots are dealt out (kDealWarps).
 struct StepWarps {
-    const uint2* warp;
+    const uint2* warp;  // first slot; number | stride << 8
     uint32_t count, per;
 };
+struct WarpSlots {
+    uint32_t first, n, stride;
+    __device__ __forceinline__ uint32_t slot(uint32_t at) const { return first + min(at, n - 1u) * stride; }
+};
+__device__ __forceinline__ WarpSlots warp_slots(const StepWarps& W, uint32_t w) {
+    const uint2 q = __ldg(W.warp + w);
+    return {q.x, q.y & 0xFFu, q.y >> 8};
+}
 
 // Draws for a warp whose lanes repeat its `per` spins (a power of two; lane l
 // holds spin l mod per): every 32 / per steps all lanes draw at once, lane l for
@@ -140,10 +149,10 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
     if (w >= W.count) return;  // whole warp
     // mesh: the lanes past the warp's spins help with the records; cylinders:
     // they repeat the spins (ThinDraws)
-    const uint2 mine = __ldg(W.warp + w);
+    const WarpSlots mine = warp_slots(W, w);
     const uint32_t at = LAYOUT == 3 ? lane & (W.per - 1u) : lane;
-    const uint32_t i = mine.x + min(at, mine.y - 1u);
-    const uint32_t jb = S.u[U_JOB][mine.x];
+    const uint32_t i = mine.slot(at);
+    const uint32_t jb = S.u[U_JOB][mine.first];
     // the warp's job and substrate records, copied to shared memory once and
     // read from there (kept out of the collision loop's registers)
     __shared__ JobDev jobS[THREADS / 32];
@@ -166,7 +175,7 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
     const uint32_t ls0 = now - start;
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
-    const bool valid = id != 0xFFFFFFFFu && at < mine.y;
+    const bool valid = id != 0xFFFFFFFFu && at < mine.n;
     float x = S.f[F_X][i], y = S.f[F_Y][i], z = S.f[F_Z][i];
     mom[0][tx] = S.f[F_MX][i]; mom[1][tx] = S.f[F_MY][i]; mom[2][tx] = S.f[F_MZ][i];
     mom[3][tx] = S.f[F_CX][i]; mom[4][tx] = S.f[F_CY][i]; mom[5][tx] = S.f[F_CZ][i];
@@ -315,9 +324,9 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
     LocalWarp& Lw = wl[wi];
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (w >= W.count) return;  // whole warp
-    const uint2 mine = __ldg(W.warp + w);
-    const uint32_t i = mine.x + min(lane, mine.y - 1u);
-    const uint32_t jb = S.u[U_JOB][mine.x];
+    const WarpSlots mine = warp_slots(W, w);
+    const uint32_t i = mine.slot(lane);
+    const uint32_t jb = S.u[U_JOB][mine.first];
     {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(jobs + jb);
         uint32_t* dst = reinterpret_cast<uint32_t*>(jobS + wi);
@@ -335,7 +344,7 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
     const uint32_t ls0 = now - start;
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
-    const bool valid = id != 0xFFFFFFFFu && lane < mine.y;
+    const bool valid = id != 0xFFFFFFFFu && lane < mine.n;
     // position = lattice origin (multiple of 1/16) + FP32 offset in [0, 1/16)
     float &gx = Lw.gx[lane], &gy = Lw.gy[lane], &gz = Lw.gz[lane];  // local_round keeps it there too
     gx = gy = gz = 0.0f;
@@ -466,9 +475,9 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
     PrecWarp& P = wp[wi];
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (w >= W.count) return;  // whole warp
-    const uint2 mine = __ldg(W.warp + w);
-    const uint32_t i = mine.x + min(lane, mine.y - 1u);
-    const uint32_t jb = S.u[U_JOB][mine.x];
+    const WarpSlots mine = warp_slots(W, w);
+    const uint32_t i = mine.slot(lane);
+    const uint32_t jb = S.u[U_JOB][mine.first];
     {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(jobs + jb);
         uint32_t* dst = reinterpret_cast<uint32_t*>(jobS + wi);
@@ -486,7 +495,7 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
     const uint32_t ls0 = now - start;
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
-    const bool valid = id != 0xFFFFFFFFu && lane < mine.y;
+    const bool valid = id != 0xFFFFFFFFu && lane < mine.n;
     double x = 0.0, y = 0.0, z = 0.0, mag = 0.0, Mx = 0.0, My = 0.0, Mz = 0.0;
     uint32_t comp = 0, fiber = 0;
     if (valid) {
@@ -983,17 +992,21 @@ bool job_finished(const dsim_batch* b, const BatchJob& j) {
     return b->stepNow >= j.d.start && b->stepNow - j.d.start >= j.d.steps;
 }
 
-// Warps per SM below which a kind's warps hold fewer than 32 spins.  us per step
-// at 32 / 16 / 8 / 4 / 2 spins a warp: FP32 mesh 16,384 spins 12.2 / 8.4 / 6.5 /
-// 7.9 / 11.2, 32,768 13.7 / 9.2 / 10.2; cell-local mesh 16,384 17.0 / 13.0 / 10.4 /
-// 13.1, 32,768 18.8 / 14.7 / 18.5; FP64 mesh 4096 26.8 / 19.8 / 15.8 / 14.5 / 17.7,
-// 16,384 32.3 / 28.7 / 31.6; FP32 cylinders 16,384 6.3 / 5.7 / 4.0 / 3.4 / 3.9,
-// 49,152 8.5 / 6.7 / 5.8 / 6.3; cell-local cylinders 32,768 11.4 / 8.6 / 7.3 / 7.4;
-// FP64 cylinders 4096 28.9 / 20.2 / 17.9 / 16.2 / 20.6, 32,768 48.5 / 46.7 / 52.3
+// Warps per SM below which a kind's warps hold fewer than 32 spins.  FP32 mesh, ms
+// of runs at 12 / 16 / 20 / 24 (with as many cylinder spins beside them): six jobs
+// of 4957 to 35,814 spins 11.5 / 10.8 / 10.0 / 10.9; one mesh job of 8192 spins 1.54 /
+// 1.62 / 1.68 / 1.70, of 16,384 2.26 / 2.24 / 2.24 / 2.39, of 40,960 3.42 / 3.23 / 3.26 /
+// 3.46, of 65,536 4.25 / 4.16 / 4.05 / 4.44.  The others, us per step at 32 / 16 / 8 /
+// 4 / 2 spins a warp: cell-local mesh 16,384 spins 17.0 / 13.0 / 10.4 / 13.1, 32,768
+// 18.8 / 14.7 / 18.5; FP64 mesh 4096 26.8 / 19.8 / 15.8 / 14.5 / 17.7, 16,384 32.3 /
+// 28.7 / 31.6; FP32 cylinders 16,384 6.3 / 5.7 / 4.0 / 3.4 / 3.9, 49,152 8.5 / 6.7 / 5.8 /
+// 6.3; cell-local cylinders 32,768 11.4 / 8.6 / 7.3 / 7.4; FP64 cylinders 4096 28.9 /
+// 20.2 / 17.9 / 16.2 / 20.6, 32,768 48.5 / 46.7 / 52.3.
 uint32_t warps_per_sm(StepKind k) {
     switch (k) {
         case kStepCyl: case kStepCylLocal: return 41;
         case kStepMesh64: case kStepCyl64: return 8;
+        case kStepMesh: case kStepMeshFull: return 20;
         default: return 16;
     }
 }
@@ -1013,8 +1026,14 @@ int build_warps(dsim_batch* b) {
         const uint32_t per = spins_per_warp_of((StepKind)k, spins[k]);
         for (const auto& j : b->jobs) {
             if (job_finished(b, j) || kind_of(b, j) != (StepKind)k) continue;
-            for (uint32_t q = 0; q < j.pad; q += per)
-                list.push_back(make_uint2((uint32_t)j.slot0 + q, std::min(per, j.pad - q)));
+            const uint32_t warps = (j.pad + per - 1) / per;
+            const bool deal = k != kStepCyl && k != kStepCyl64 && k != kStepCylLocal;
+            for (uint32_t w = 0; w < warps; w++) {
+                // w0: the first of the warps that share slots, `dealt` of them, n slots in all
+                const uint32_t w0 = deal ? w / kDealWarps * kDealWarps : w, dealt = deal ? std::min(kDealWarps, warps - w0) : 1u;
+                const uint32_t n = std::min(j.pad - w0 * per, dealt * per), q = w - w0;
+                list.push_back(make_uint2((uint32_t)j.slot0 + w0 * per + q, (n - q + dealt - 1) / dealt | dealt << 8));
+            }
         }
         b->kinds[k].count = (uint32_t)(list.size() - first[k]);
         b->kinds[k].per = per;
@@ -1072,9 +1091,9 @@ k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (w >= W.count) return;  // whole warp
-    const uint2 mine = __ldg(W.warp + w);
-    const uint32_t at = lane & (W.per - 1u), i = mine.x + min(at, mine.y - 1u);  // the lanes repeat the spins
-    const uint32_t jb = S.u[U_JOB][mine.x];
+    const WarpSlots mine = warp_slots(W, w);
+    const uint32_t at = lane & (W.per - 1u), i = mine.slot(at);  // the lanes repeat the spins
+    const uint32_t jb = S.u[U_JOB][mine.first];
     const JobDev& J = jobs[jb];
     const SubDev& sub = subs[__ldg(&J.sub)];
     const uint32_t now = *stepNow;
@@ -1083,7 +1102,7 @@ k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
     const uint32_t ls0 = now - start;
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
-    const bool valid = id != 0xFFFFFFFFu && at < mine.y;
+    const bool valid = id != 0xFFFFFFFFu && at < mine.n;
     uint32_t nrefl = 0, nperm = 0, st = 0;
     if (valid) {
         const uint32_t live = __activemask();  // converged: the lanes with a spin
@@ -1169,9 +1188,9 @@ k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict
     const uint32_t tx = threadIdx.x;
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (w >= W.count) return;  // whole warp
-    const uint2 mine = __ldg(W.warp + w);
-    const uint32_t at = lane & (W.per - 1u), i = mine.x + min(at, mine.y - 1u);  // the lanes repeat the spins
-    const uint32_t jb = S.u[U_JOB][mine.x];
+    const WarpSlots mine = warp_slots(W, w);
+    const uint32_t at = lane & (W.per - 1u), i = mine.slot(at);  // the lanes repeat the spins
+    const uint32_t jb = S.u[U_JOB][mine.first];
     const JobDev& J = jobs[jb];
     const SubDev& sub = subs[__ldg(&J.sub)];
     const uint32_t now = *stepNow;
@@ -1180,7 +1199,7 @@ k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict
     const uint32_t ls0 = now - start;
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
-    const bool valid = id != 0xFFFFFFFFu && at < mine.y;
+    const bool valid = id != 0xFFFFFFFFu && at < mine.n;
     uint32_t nrefl = 0, nperm = 0, st = 0;
     CylLocal form = {__ldg(&J.inR), {0.0f, 0.0f, 0.0f}, 0u, 0u};
     if (valid) {

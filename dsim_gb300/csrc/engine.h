@@ -82,6 +82,18 @@ inline uint32_t spins_per_warp(uint64_t N, uint32_t warpsPerSm, bool pow2) {
     return p;
 }
 
+// Mesh spins lie in the order of their cells, and neighbours are slow together
+// (crowded cells, tight places with many reflections).  So the spins of up to
+// kDealWarps consecutive warps are dealt out among them in turn: each warp gets
+// some of every kind, and a launch no longer waits for a few warps (kcycles a
+// step of a warp with consecutive spins, mean / largest: 65,536 spins 20.2 / 34.1;
+// 100,001 18.4 / 26.1), while the cells of a block stay close.  us per step by
+// consecutive / 4 / 16 / 64 / 256 warps / all: 65,536 spins on 25 tubes with
+// myelin 16.5 / 14.8 / 13.9 / 13.4 / 14.1 / 14.6; 100,001 on 100 tubes 12.1 /
+// 11.6 / 11.2 / 11.2 / 11.5 / 11.5; 400,000 37.3 / 36.6 / 36.0 / 36.2 / 36.0 /
+// 37.5; 4096 on 25 tubes 4.24 / 4.28 / 4.29 / 4.17 / 4.18 / 4.57.
+static constexpr uint32_t kDealWarps = 64;
+
 // Resident blocks per SM that a step kernel's register budget is taken for, by
 // its blocks: as few (down to `least`) as reach the fewest waves that `most`
 // give.

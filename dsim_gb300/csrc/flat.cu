@@ -56,8 +56,10 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
         if (lane == 0) stage_init(&ws[threadIdx.x >> 5]);
         __syncwarp();
     }
-    const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * a.perWarp + lane;
-    const bool valid = lane < a.perWarp && i < S.N;
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (S.N + a.perWarp - 1) / a.perWarp;
+    const uint32_t w0 = w & ~(kDealWarps - 1u), dealt = min(kDealWarps, warps - w0);  // the warps that share spins
+    const uint32_t i = w0 * a.perWarp + lane * dealt + (w - w0);
+    const bool valid = w < warps && lane < a.perWarp && i < S.N;
     // the position is o at the top of a step, the start of its current sub-segment within one
     float ox = 0.0f, oy = 0.0f, oz = 0.0f;
     WalkLane& C = wc[threadIdx.x >> 5];
@@ -159,12 +161,16 @@ __global__ void __launch_bounds__(kFlatThreads, MINB) k_mesh_step_flat(MeshDev g
     if (status) atomicOr(a.status, status);
 }
 
-// Spins per warp: at most 16 warps per SM below 32 spins a warp.  us per step, 25 tubes
-// with myelin, 32 / 16 / 8 / 4 / 2 / 1 spins a warp: 1000 spins 12.9 / 7.9 /
-// 5.6 / 4.4 / 3.7 / 3.5; 8192 spins 14.0 / 9.3 / 6.8 / 6.1 / 8.2 / 9.8; 24,576
-// spins 15.4 / 10.4 / 9.7 / 11.9; 40,960 spins 16.3 / 11.8 / 14.4; 65,536
-// spins 17.6 / 18.9
-uint32_t mesh_spins_per_warp(uint32_t N) { return spins_per_warp(N, 16, false); }
+// Spins per warp: below 32 of them at most 24 warps per SM, where a warp then
+// still holds 16, else 20.  us per step at 12 / 16 / 20 / 24 / 28 warps per SM: 4096
+// spins on 25 tubes with myelin 4.35 / 4.15 / 4.11 / 4.13 / 5.31; 30,000 spins on
+// 100 tubes 7.01 / 6.28 / 6.18 / 6.63 / 7.33; 45,000 8.51 / 7.96 / 7.51 / 7.57 /
+// 8.27; 60,000 9.85 / 9.16 / 8.76 / 8.72 / 9.29; 80,000 10.5 / 10.4 / 10.1 / 9.8 /
+// 10.6; 65,536 on 25 tubes with myelin 14.9 / 13.6 / 12.9 / 12.4 / 13.0.  32 spins a
+// warp at 1000 spins 12.9, at 8192 14.0.
+uint32_t mesh_spins_per_warp(uint32_t N) {
+    return spins_per_warp(N, N >= 24u * 16u * kSmCount ? 24 : 20, false);
+}
 
 int launch_mesh_step_flat(const MeshDev& g, const AccelDev& acc, const MeshStepArgs& args,
                           const SpinsSorted& S, int rng, cudaStream_t st, int occupancy, bool queue, bool stage) {

@@ -1,8 +1,9 @@
 """Launch shapes: with few spins a warp advances fewer than 32 of them, and the
 mesh step picks its blocks per SM by the count.  The spins' walks do not depend
 on either: the first n of a large set equal, bit for bit, a set of those n
-alone, at counts around the changes of the rules (152 SMs x 16 warps for
-meshes, then 4 to 8 blocks of 128 per SM; x 33 warps for cylinders)."""
+alone, at counts around the changes of the rules (152 SMs x 20 or 24 warps for
+meshes, then 4 to 7 blocks of 128 per SM; x 33 warps for cylinders), and whatever
+warp they are dealt to."""
 import numpy as np
 import pytest
 
@@ -21,7 +22,7 @@ def _mesh(case, m, n):
     return (*s.get(), s.counts())
 
 
-@pytest.mark.parametrize("n", [1, 31, 2433, 4865, 40961, 77825, 97281, 116737, 136193])
+@pytest.mark.parametrize("n", [1, 31, 2433, 3041, 4865, 40961, 58367, 58368, 77825, 97281, 116737, 136193])
 def test_mesh_walks_do_not_depend_on_spins_per_warp(engine, tmp_path, n):
     from dsim_gb300.engine import Mesh
     case = MeshCase(tmp_path, membranes="AM", N=165001)
