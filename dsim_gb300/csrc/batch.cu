@@ -5,8 +5,8 @@
 // [slot0_j, slot0_j + pad_j) with pad_j = nSpins rounded up to 32, so every
 // warp belongs to one job and reads that job's substrate and parameters once.
 // Padding slots carry id 0xFFFFFFFF and do no work.  Every chunk the spins
-// are re-sorted by (job, Morton cell of a per-job sort grid) -- the job
-// ranges are preserved because job j's keys follow job j-1's -- and one step
+// are re-sorted by (job, Morton cell of a per-job sort grid; for cylinder jobs
+// region and scattered id) -- the job ranges are preserved because job j's keys follow job j-1's -- and one step
 // kernel advances every running job by up to `chunk` steps.  The chunk loop
 // (sort, step, step-counter advance) is captured in a CUDA graph.
 //

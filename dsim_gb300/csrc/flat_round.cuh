@@ -17,12 +17,14 @@
 // overflowed).
 //
 // Bound by instruction issue and L2 latency together (400,000 spins on 640,000
-// triangles: issue 51 %, long-scoreboard stalls 3.1 of 8.2 cycles an
-// instruction, DRAM idle).  Warp instructions per step of 32 spins went 3031 ->
-// 2513 (slabs) -> 2164 (this layout: owners by mask and rank instead of
-// five-shuffle searches, no integer division, full windows, one copy of the
-// exact test, no walk over cells for nine hits in ten); 6.6e9 -> 9.1e9
-// spin-steps/s there, 6.8e9 -> 9.4e9 for 1M spins on 2.56M triangles.
+// triangles, 5 blocks per SM: issue 47 %, long-scoreboard stalls 4.0 of 9.0 cycles
+// an instruction, DRAM idle), so by how many warps an SM can hold.  Warp
+// instructions per step of 32 spins went 3031 -> 2513 (slabs) -> 2164 (owners by
+// mask and rank instead of five-shuffle searches, no integer division, full
+// windows, one copy of the exact test, no walk over cells for nine hits in ten):
+// 6.6e9 -> 9.1e9 spin-steps/s there, 6.8e9 -> 9.4e9 for 1M spins on 2.56M
+// triangles; then 11.1e9 and 10.8e9 with a lane's state in shared memory
+// (LaneState), 7 blocks per SM and the spins dealt out (kDealWarps).
 #pragma once
 #include "common.cuh"
 #include "engine.h"

@@ -65,16 +65,16 @@ int dsim_mesh_info(const dsim_mesh* m, uint64_t info[8]);
 /* The step kernels find candidate triangles in a finer acceleration grid
  * (each triangle listed in every fine cell it touches) and
  * apply the reference grid's first-cell-with-hit rule only to the hits, which
- * gives the same results.  Built with 2.5 * numCubes cells per axis by default;
+ * gives the same results.  Built with 2.25 * numCubes cells per axis by default;
  * dsim_mesh_set_accel rebuilds it (0 = scan the reference grid directly).
  * info = {cells per axis, entries, device bytes}. */
 int dsim_mesh_set_accel(dsim_mesh* m, uint32_t cellsPerAxis);
 /* step kernel on the fine grid (all give the same results; default 8; other
  * values are refused): 5, 6, 7 the warp's candidate records flattened into one
  * list, lanes stepping independently (8, 6, 4 resident blocks of 128 threads
- * per SM); 8 as 6 at 5 blocks per SM (96 registers, no spills), with the
- * records that pass the plane test queued and finished 32 at a time; 9 as 6, with each lane's part of every 64-record
- * window copied into shared memory by TMA bulk copies (cp.async.bulk,
+ * per SM); 8 as 6 at 4 to 7 blocks per SM by the number of spins, with the
+ * records that pass the plane test queued and finished 32 at a time; 9 as 6,
+ * with each lane's part of every 64-record window copied into shared memory by TMA bulk copies (cp.async.bulk,
  * mbarrier completion) while the previous window is tested (8 and 9: 32-byte
  * records) */
 int dsim_mesh_set_kernel(dsim_mesh* m, uint32_t variant);
@@ -151,9 +151,10 @@ int dsim_spins_scanned(dsim_spins* s, uint32_t* scannedN, int reset);
 int dsim_spins_status(dsim_spins* s, uint32_t* status, int reset);
 /* Spins are reordered by fine-grid cell every `steps` steps of a mesh run
  * (default 1000, i.e. once at the start of a call of up to 1000 steps; 0 =
- * never) so that neighbouring threads read the same cell records; one step
- * kernel launch covers the steps between reorderings.  Each spin keeps its
- * identity (random stream, counters, getters). */
+ * never) so that a block's threads read the same cell records; one step
+ * kernel launch covers the steps between reorderings.  So few spins that each
+ * has a warp of its own are not reordered.  Each spin keeps its identity
+ * (random stream, counters, getters). */
 int dsim_spins_set_sort_interval(dsim_spins* s, uint32_t steps);
 /* Global index of this object's spin 0 in the Philox counter (default 0).
  * A job split over several GPUs gives each shard the index of its first spin,
