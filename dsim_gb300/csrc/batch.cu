@@ -460,7 +460,11 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
 // draws as the plain form.  Positions and magnitudes persist in the double
 // fields; the float fields receive their rounded values (sort keys, float
 // readers) and the moment pair (m, c) holds M as m - c.
-__global__ void __launch_bounds__(kFlatThreads, 2)
+// 3 blocks per SM (168 registers): two of them, all that a thin mesh job gives an
+// SM, leave room beside them for the blocks of a cylinder job in the same launch.
+// ms of runs at 2 / 3 / 4: two jobs of 15,747 mesh and 13,586 cylinder spins 9.0 /
+// 8.3 / 9.3, two of 32,768 7.2 / 7.0 / 7.5, six of 32,768 21.9 / 22.1 / 22.3.
+__global__ void __launch_bounds__(kFlatThreads, 3)
 k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
                const uint32_t* __restrict__ stepNow, uint32_t chunk, uint32_t* status,
                unsigned long long* jobCounts) {
