@@ -453,6 +453,12 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
     if (st) atomicOr(status, st);
 }
 
+// LaneState of the FP64 form
+struct LaneState64 {
+    double mag[32], m[3][32], umax[32], umin[32], u[32], T2[32], rT2[32];
+    uint32_t comp[32], fiber[32], nrefl[32], nperm[32], status[32], it[32], sub[32], decayOf[32];
+};
+
 // Precision-form mesh jobs (DSIM_JOB_PRECISE): the step of cpuIntegrate
 // (dSim3/src/spinKernelCpu.cpp:430-499) in FP64 -- position, sub-segments,
 // hits and reflections (prec_round.cuh), the clamp to +-(1 - spinRadius), the
@@ -460,16 +466,19 @@ k_batch_step_local(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
 // draws as the plain form.  Positions and magnitudes persist in the double
 // fields; the float fields receive their rounded values (sort keys, float
 // readers) and the moment pair (m, c) holds M as m - c.
-// 3 blocks per SM (168 registers): two of them, all that a thin mesh job gives an
-// SM, leave room beside them for the blocks of a cylinder job in the same launch.
-// ms of runs at 2 / 3 / 4: two jobs of 15,747 mesh and 13,586 cylinder spins 9.0 /
-// 8.3 / 9.3, two of 32,768 7.2 / 7.0 / 7.5, six of 32,768 21.9 / 22.1 / 22.3.
-__global__ void __launch_bounds__(kFlatThreads, 3)
+// Thin jobs at 3 blocks per SM (162 registers): two of them, all that such a job
+// gives an SM, leave room beside them for the blocks of a cylinder job in the same
+// launch; full warps at 4 (128).  ms of runs at 2 / 3 / 4: two jobs of 15,747 mesh
+// and 13,586 cylinder spins 8.2 / 8.2 / 9.0 (9.0 with 198 registers), two of 32,768
+// 7.0 / 7.0 / 7.2, six of 32,768 (full warps) 22.4 / 22.3 / 21.2.
+template <int MINB>
+__global__ void __launch_bounds__(kFlatThreads, MINB)
 k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, BatchSpins S, StepWarps W,
                const uint32_t* __restrict__ stepNow, uint32_t chunk, uint32_t* status,
                unsigned long long* jobCounts) {
     __shared__ HitWarp wh[kFlatWarps];
     __shared__ PrecWarp wp[kFlatWarps];
+    __shared__ LaneState64 wc[kFlatWarps];
     __shared__ JobDev jobS[kFlatWarps];
     __shared__ SubDev subS[kFlatWarps];
     const uint32_t FULL = 0xFFFFFFFFu;
@@ -500,10 +509,18 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
     const bool valid = id != 0xFFFFFFFFu && lane < mine.n;
-    double x = 0.0, y = 0.0, z = 0.0, mag = 0.0, Mx = 0.0, My = 0.0, Mz = 0.0;
-    uint32_t comp = 0, fiber = 0;
+    double ox = 0.0, oy = 0.0, oz = 0.0;
+    LaneState64& C = wc[wi];
+    double &mag = C.mag[lane], &Mx = C.m[0][lane], &My = C.m[1][lane], &Mz = C.m[2][lane], &umax = C.umax[lane],
+           &umin = C.umin[lane], &u = C.u[lane], &T2 = C.T2[lane], &rT2 = C.rT2[lane];
+    uint32_t &comp = C.comp[lane], &fiber = C.fiber[lane], &nrefl = C.nrefl[lane], &nperm = C.nperm[lane],
+             &st = C.status[lane], &it = C.it[lane], &sub_n = C.sub[lane], &decayOf = C.decayOf[lane];
+    mag = Mx = My = Mz = umin = T2 = rT2 = 0.0;
+    u = umax = 1.0;
+    comp = fiber = nrefl = nperm = st = it = sub_n = 0;
+    decayOf = 4u;  // the compartment that T2 and rT2 are of
     if (valid) {
-        x = S.d[D_X][i]; y = S.d[D_Y][i]; z = S.d[D_Z][i]; mag = S.d[D_MAG][i];
+        ox = S.d[D_X][i]; oy = S.d[D_Y][i]; oz = S.d[D_Z][i]; mag = S.d[D_MAG][i];
         Mx = (double)S.f[F_MX][i] - (double)S.f[F_CX][i];
         My = (double)S.f[F_MY][i] - (double)S.f[F_CY][i];
         Mz = (double)S.f[F_MZ][i] - (double)S.f[F_CZ][i];
@@ -516,23 +533,20 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
     const double hiC = 1.0 - (double)J.spinR, loC = -1.0 + (double)J.spinR;
     // a point whose float coordinates keep inside this needs no clamp
     const float inside = (float)hiC - 1e-6f;
-    uint32_t decayOf = 4u;  // the compartment that T2 and rT2 are of
-    double T2 = 0.0, rT2 = 0.0;
     const uint32_t reflType = J.reflType, maxSub = J.maxSub;
     const uint32_t k0 = J.key0, k1 = J.key1;
     const float* __restrict__ wave = J.wave;
-    uint32_t nrefl = 0, nperm = 0, st = 0, it = 0, excluded = 0xFFFFFFFFu, sub_n = 0;
+    uint32_t excluded = 0xFFFFFFFFu;
     PrecCount pc;
     bool active = valid && nsteps > 0;
     bool fresh = active;
-    double u = 1.0, umax = 1.0, umin = 0.0;
-    double ox = x, oy = y, oz = z, px = x, py = y, pz = z;
+    // the position is o at the top of a step, the start of its current sub-segment within one
+    double px = ox, py = oy, pz = oz;
     while (__any_sync(FULL, active)) {
         if (fresh) {
             const Draw d = philox_draw(id, (uint64_t)(ls0 + it), 0u, k0, k1);
-            ox = x; oy = y; oz = z;
             const double sd = (double)J.sd[comp & 3u];
-            px = x + (double)d.nx * sd; py = y + (double)d.ny * sd; pz = z + (double)d.nz * sd;
+            px = ox + (double)d.nx * sd; py = oy + (double)d.ny * sd; pz = oz + (double)d.nz * sd;
             u = (double)d.u;
             excluded = 0xFFFFFFFFu;
             umax = 1.0; umin = 0.0;
@@ -561,7 +575,7 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
                     if (py > hiC) py = hiC; else if (py < loC) py = loC;
                     if (pz > hiC) pz = hiC; else if (pz < loC) pz = loC;
                 }
-                x = px; y = py; z = pz;
+                ox = px; oy = py; oz = pz;
                 if ((comp & 3u) != decayOf) {
                     decayOf = comp & 3u;
                     T2 = (double)J.T2[decayOf];
@@ -569,7 +583,7 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
                 }
                 if (T2 > 0.0) mag += div_by(-mag, T2, rT2) * (double)J.dt;
                 const double w = (double)__ldg(wave + ls0 + it);
-                Mx += w * x; My += w * y; Mz += w * z;
+                Mx += w * ox; My += w * oy; Mz += w * oz;
                 if (++it >= nsteps) active = false;
                 else fresh = true;
             }
@@ -577,8 +591,8 @@ k_batch_step64(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs,
         __syncwarp();
     }
     if (valid) {
-        S.d[D_X][i] = x; S.d[D_Y][i] = y; S.d[D_Z][i] = z; S.d[D_MAG][i] = mag;
-        S.f[F_X][i] = (float)x; S.f[F_Y][i] = (float)y; S.f[F_Z][i] = (float)z;
+        S.d[D_X][i] = ox; S.d[D_Y][i] = oy; S.d[D_Z][i] = oz; S.d[D_MAG][i] = mag;
+        S.f[F_X][i] = (float)ox; S.f[F_Y][i] = (float)oy; S.f[F_Z][i] = (float)oz;
         S.f[F_MAG][i] = (float)mag;
         const float mx = (float)Mx, my = (float)My, mz = (float)Mz;
         S.f[F_MX][i] = mx; S.f[F_MY][i] = my; S.f[F_MZ][i] = mz;
@@ -1347,8 +1361,12 @@ int enqueue_chunk(dsim_batch* b, uint32_t steps) {
                                                                      b->d_status, b->d_counts);
                 break;
             case kStepMesh64:
-                k_batch_step64<<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
-                                                              b->d_status, b->d_counts);
+                if (W.per < 32)
+                    k_batch_step64<3><<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
+                                                                     b->d_status, b->d_counts);
+                else
+                    k_batch_step64<4><<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,
+                                                                     b->d_status, b->d_counts);
                 break;
             case kStepCyl64:
                 k_batch_step_cyl64<<<grid, kFlatThreads, 0, st>>>(b->d_subs, b->d_jobs, D, W, b->d_stepNow, steps,

@@ -59,3 +59,22 @@ def test_jobs_do_not_depend_on_launch_shapes(engine, tmp_path, form, n):
                     assert np.array_equal(a, b_)
             for a, b_ in zip(p0, p1):
                 assert np.array_equal(a, b_)
+
+
+@pytest.mark.parametrize("form", ["plain", "local", "precise"])
+def test_full_warps_walk_as_thin_ones(engine, tmp_path, form):
+    """A mesh job large enough for 32 spins a warp in every form, against its first spins alone (thin warps)."""
+    from dsim_gb300.engine import Batch, Mesh
+    mc, cc = MeshCase(tmp_path, membranes="AM", N=99000), CylCase(tmp_path, N=10)
+    m = Mesh.load(mc.path, mc.spaceScale)
+    out = []
+    for n in (mc.N, 1000):
+        b = Batch(1 << 17, 1)
+        j = b.submit(b.add_mesh(m), **_jobs(mc, cc, n, 30, form)[0])
+        b.run()
+        assert b.status() == 0
+        out.append((*b.get(j, n), *(b.get_precise(j, n) if form != "plain" else ())))
+        b.close()
+    for a, b_ in zip(*out):
+        a, b_ = np.asarray(a), np.asarray(b_)
+        assert np.array_equal(a.reshape(mc.N, -1)[:1000], b_.reshape(1000, -1))
