@@ -157,7 +157,15 @@ int derive(State& s, const uint32_t* tic, const uint32_t* cc) {
     uint32_t total = 0;
     if (!rc && cudaMemcpy(&total, s.cell_start + ncells, 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = kErrCuda;
     if (!rc && cudaMalloc(&s.cell_tri, (size_t)(total ? total : 1) * 4) != cudaSuccess) rc = kErrNoMem;
-    if (!rc) rc = launch_dense_to_csr(ncells, s.maxTPC, nT, cc, tic, s.cell_start, s.cell_tri, s.status, 0);
+    if (!rc) rc = launch_dense_to_csr(ncells, s.maxTPC, nT, total, cc, tic, s.cell_start, s.cell_tri, s.status, 0);
+    // the caller's grid is refused here, before a kernel takes its entries for triangles
+    uint32_t st = 0;
+    if (!rc && cudaMemcpy(&st, s.status, 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = kErrCuda;
+    if (!rc && st) {
+        cudaFree(scratch);
+        set_last_error(kErrFormat, "integrateSystem: trianglesInCubes names a triangle >= %u or a cell above k_maxTrianglesPerCube", nT);
+        return kErrFormat;
+    }
     // each triangle's reference cells (a hit then needs no list search)
     uint32_t* perTri = nullptr;
     if (!rc && (cudaMalloc(&s.tri_cells, (size_t)nT * sizeof(uint4)) != cudaSuccess ||
@@ -165,15 +173,9 @@ int derive(State& s, const uint32_t* tic, const uint32_t* cc) {
         rc = kErrNoMem;
     if (!rc) rc = launch_tri_cell_lists(s.numCubes, nT, s.cell_start, s.cell_tri, perTri, s.tri_cells, 0);
     if (!rc) rc = launch_tri_regular(nT, s.numCubes, s.tri_cells, s.bary, s.plane, 0);
-    uint32_t st = 0;
-    if (!rc && cudaMemcpy(&st, s.status, 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = kErrCuda;
     cudaFree(scratch);
     cudaFree(perTri);
     if (rc) { set_last_error(rc, "integrateSystem: deriving cell lists failed"); return rc; }
-    if (st) {
-        set_last_error(kErrFormat, "integrateSystem: trianglesInCubes names a triangle >= %u or a cell above k_maxTrianglesPerCube", nT);
-        return kErrFormat;
-    }
     // fine acceleration grid from the records (triangle corners p1, p1 + v, p1 + u),
     // 2.25 fine cells per reference cell edge, 32-byte records
     uint32_t nf = s.numCubes * 9 / 4 <= 1024 ? s.numCubes * 9 / 4 : 1024;

@@ -204,7 +204,7 @@ int launch_tri_cells(bool fill, uint32_t nT, const float* V, const uint32_t* trg
                      float L, uint32_t* counter, const uint32_t* start, uint32_t* cell_tri, uint64_t* touched,
                      cudaStream_t st);
 int launch_sort_cells(uint32_t ncells, const uint32_t* start, uint32_t* cell_tri, cudaStream_t st);
-int launch_dense_to_csr(uint32_t ncells, uint32_t maxTPC, uint32_t nT, const uint32_t* counter,
+int launch_dense_to_csr(uint32_t ncells, uint32_t maxTPC, uint32_t nT, uint32_t total, const uint32_t* counter,
                         const uint32_t* dense, const uint32_t* start, uint32_t* cell_tri,
                         uint32_t* status, cudaStream_t st);
 

@@ -247,11 +247,12 @@ __global__ void __launch_bounds__(128) k_sort_cells(uint32_t ncells, const uint3
     }
 }
 
-// dense reference grid [cell][maxTPC] -> CSR lists (order kept).  Entries
-// that name a triangle >= nT, or cells holding more than maxTPC entries, set
-// kStatusBadCell and are replaced by triangle 0's index only as a placeholder
-// (the caller refuses to run on such a grid).
-__global__ void k_dense_to_csr(uint32_t ncells, uint32_t maxTPC, uint32_t nT,
+// dense reference grid [cell][maxTPC] -> CSR lists (order kept) of `total`
+// entries.  An entry that names a triangle >= nT, or a cell that counts more than
+// maxTPC entries, sets kStatusBadCell; the lists then hold placeholders and words
+// that were never written, and the caller reads the status before anything else
+// reads them.
+__global__ void k_dense_to_csr(uint32_t ncells, uint32_t maxTPC, uint32_t nT, uint32_t total,
                                const uint32_t* __restrict__ counter,
                                const uint32_t* __restrict__ dense, const uint32_t* __restrict__ start,
                                uint32_t* cell_tri, uint32_t* status) {
@@ -260,6 +261,8 @@ __global__ void k_dense_to_csr(uint32_t ncells, uint32_t maxTPC, uint32_t nT,
     uint32_t k = counter[c], s = start[c];
     if (k > maxTPC) { atomicOr(status, kStatusBadCell); k = maxTPC; }
     for (uint32_t j = 0; j < k; j++) {
+        // counters whose sum passes 2^32 leave a cell_tri of fewer entries than their starts say
+        if (s >= total || total - s <= j) { atomicOr(status, kStatusBadCell); return; }
         uint32_t t = dense[(size_t)c * maxTPC + j];
         if (t >= nT) { atomicOr(status, kStatusBadCell); t = 0; }
         cell_tri[s + j] = t;
@@ -342,10 +345,10 @@ int launch_sort_cells(uint32_t ncells, const uint32_t* start, uint32_t* cell_tri
     return kOk;
 }
 
-int launch_dense_to_csr(uint32_t ncells, uint32_t maxTPC, uint32_t nT, const uint32_t* counter,
+int launch_dense_to_csr(uint32_t ncells, uint32_t maxTPC, uint32_t nT, uint32_t total, const uint32_t* counter,
                         const uint32_t* dense, const uint32_t* start, uint32_t* cell_tri,
                         uint32_t* status, cudaStream_t st) {
-    k_dense_to_csr<<<(ncells + 255) / 256, 256, 0, st>>>(ncells, maxTPC, nT, counter, dense, start,
+    k_dense_to_csr<<<(ncells + 255) / 256, 256, 0, st>>>(ncells, maxTPC, nT, total, counter, dense, start,
                                                           cell_tri, status);
     DSIM_CUDA_TRY(cudaGetLastError());
     return kOk;
