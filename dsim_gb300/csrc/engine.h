@@ -190,7 +190,7 @@ int launch_records_from_mesh(uint32_t nT, const float* V, const uint32_t* trgls,
 int launch_tri64(uint32_t nT, const float* V, const uint32_t* trgls, Tri64* out, cudaStream_t st);
 // every triangle's reference cells (x | y << 10 | z << 20, n cells per axis)
 // from the cell lists: up to 4 in a uint4 (unused entries kCellNone), kCellMany
-// in every entry when there are more
+// in every entry when there are more, or n is above 1024
 static constexpr uint32_t kCellNone = 0xFFFFFFFFu, kCellMany = 0xFFFFFFFEu;
 int launch_tri_cell_lists(uint32_t n, uint32_t nT, const uint32_t* cell_start, const uint32_t* cell_tri,
                           uint32_t* count, uint4* out, cudaStream_t st);

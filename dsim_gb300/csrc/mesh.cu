@@ -283,10 +283,12 @@ int launch_records_from_mesh(uint32_t nT, const float* V, const uint32_t* trgls,
 
 // Every triangle's reference cells: a warp per cell appends the cell to each of
 // its triangles' records (order within a record is irrelevant).  A thread per
-// cell left 640,000 triangles' lists to the longest ones: 0.10 -> 0.02 ms.
+// cell left 640,000 triangles' lists to the longest ones: 0.10 -> 0.02 ms.  The
+// threads of all cells' warps pass 2^32 from 513 cells per axis on, so the cell is
+// formed from the block and the warp, not from a thread's index.
 __global__ void k_tri_cell_lists(uint32_t n, const uint32_t* __restrict__ cell_start,
                                  const uint32_t* __restrict__ cell_tri, uint32_t* count, uint4* out) {
-    const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (c >= n * n * n) return;
     const uint32_t packed = (c % n) | (((c / n) % n) << 10) | ((c / (n * n)) << 20);
     const uint32_t e = cell_start[c + 1];
@@ -296,9 +298,9 @@ __global__ void k_tri_cell_lists(uint32_t n, const uint32_t* __restrict__ cell_s
         if (slot < 4) reinterpret_cast<uint32_t*>(out + t)[slot] = packed;
     }
 }
-__global__ void k_tri_cell_many(uint32_t nT, const uint32_t* __restrict__ count, uint4* out) {
+__global__ void k_tri_cell_many(uint32_t nT, bool all, const uint32_t* __restrict__ count, uint4* out) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < nT && count[t] > 4) out[t] = make_uint4(kCellMany, kCellMany, kCellMany, kCellMany);
+    if (t < nT && (all || count[t] > 4)) out[t] = make_uint4(kCellMany, kCellMany, kCellMany, kCellMany);
 }
 
 int launch_tri_cell_lists(uint32_t n, uint32_t nT, const uint32_t* cell_start, const uint32_t* cell_tri,
@@ -306,8 +308,10 @@ int launch_tri_cell_lists(uint32_t n, uint32_t nT, const uint32_t* cell_start, c
     if (nT == 0) return kOk;
     DSIM_CUDA_TRY(cudaMemsetAsync(count, 0, (size_t)nT * 4, st));
     DSIM_CUDA_TRY(cudaMemsetAsync(out, 0xFF, (size_t)nT * sizeof(uint4), st));
-    k_tri_cell_lists<<<(n * n * n + 7) / 8, 256, 0, st>>>(n, cell_start, cell_tri, count, out);
-    k_tri_cell_many<<<(nT + 255) / 256, 256, 0, st>>>(nT, count, out);
+    // more cells per axis than a packed cell holds (a plug-in host's own grid): every list is searched
+    const bool all = n > 1024;
+    if (!all) k_tri_cell_lists<<<(n * n * n + 7) / 8, 256, 0, st>>>(n, cell_start, cell_tri, count, out);
+    k_tri_cell_many<<<(nT + 255) / 256, 256, 0, st>>>(nT, all, count, out);
     DSIM_CUDA_TRY(cudaGetLastError());
     return kOk;
 }
