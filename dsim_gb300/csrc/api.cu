@@ -328,7 +328,7 @@ static int mesh_build(dsim_mesh* m, const std::vector<float>& Vn, const std::vec
     if ((rc = dev_alloc(&m->cell_start, (size_t)ncells + 1, &m->bytes))) { cudaFree(counter); cudaFree(scratch); return rc; }
     rc = kOk;
     do {
-        if (cudaMemsetAsync(counter, 0, ncells * 4, st) != cudaSuccess) { rc = kErrCuda; break; }
+        if (cudaMemsetAsync(counter, 0, (size_t)ncells * 4, st) != cudaSuccess) { rc = kErrCuda; break; }
         // its room holds the touched cells' bits until the lists are made
         if ((rc = dev_alloc(&m->tri_cells, m->nT, &m->bytes))) break;
         uint64_t* touched = reinterpret_cast<uint64_t*>(m->tri_cells);
@@ -339,7 +339,7 @@ static int mesh_build(dsim_mesh* m, const std::vector<float>& Vn, const std::vec
             cudaStreamSynchronize(st) != cudaSuccess) { rc = kErrCuda; break; }
         m->entries = total;
         if ((rc = dev_alloc(&m->cell_tri, total, &m->bytes))) break;
-        if (cudaMemsetAsync(counter, 0, ncells * 4, st) != cudaSuccess) { rc = kErrCuda; break; }
+        if (cudaMemsetAsync(counter, 0, (size_t)ncells * 4, st) != cudaSuccess) { rc = kErrCuda; break; }
         if ((rc = launch_tri_cells(true, m->nT, m->V, m->trgls, m->n, m->L, counter, m->cell_start, m->cell_tri, touched, st))) break;
         if ((rc = launch_sort_cells(ncells, m->cell_start, m->cell_tri, st))) break;
         if (m->nT > ncells) {  // the scan scratch is sized for ncells; use a count of its own

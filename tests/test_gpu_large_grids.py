@@ -36,7 +36,7 @@ def _walk(cubes, pos, steps=60):
     return out
 
 
-@pytest.mark.parametrize("cubes", [512, 513, 600])
+@pytest.mark.parametrize("cubes", [512, 513, 600, 1024])
 def test_walks_do_not_depend_on_the_cells(engine, cubes):
     rng = np.random.default_rng(8)
     pos = rng.uniform(-0.95, 0.95, (3000, 3)).astype(F)
