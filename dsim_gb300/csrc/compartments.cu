@@ -47,7 +47,8 @@ __global__ void __launch_bounds__(128) k_compartments(MeshDev g, AccelDev acc, S
                                                       uint32_t maxTries, uint32_t maxMoves, uint32_t* status,
                                                       uint32_t* moved) {
     const uint32_t FULL = 0xFFFFFFFFu, lane = threadIdx.x & 31u;
-    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // warp-uniform, as all but the walk
+    // warp-uniform, as all but the walk; the threads of all spins' warps pass 2^32 from 2^27 spins on
+    const uint32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (i >= S.N) return;
     float sx = S.x[i], sy = S.y[i], sz = S.z[i];
     const uint32_t id = S.id[i];
@@ -186,9 +187,9 @@ int launch_compartments(const MeshDev& g, const AccelDev& acc, const SpinsSorted
                         float startBox, uint64_t seed, uint32_t maxTries, uint32_t maxMoves, uint32_t* status,
                         uint32_t* moved, cudaStream_t st) {
     if (S.N == 0) return kOk;
-    k_compartments<<<(S.N + 3) / 4, 128, 0, st>>>(g, acc, S, maxabs[0], maxabs[1], maxabs[2], startBox,
-                                                      (uint32_t)seed, (uint32_t)(seed >> 32), maxTries, maxMoves,
-                                                      status, moved);
+    const uint32_t grid = (uint32_t)(((uint64_t)S.N + 3) / 4);
+    k_compartments<<<grid, 128, 0, st>>>(g, acc, S, maxabs[0], maxabs[1], maxabs[2], startBox, (uint32_t)seed,
+                                         (uint32_t)(seed >> 32), maxTries, maxMoves, status, moved);
     DSIM_CUDA_TRY(cudaGetLastError());
     return kOk;
 }
