@@ -122,9 +122,10 @@ __device__ __forceinline__ Draw philox_draw(uint32_t spin, uint64_t step, uint32
 // its exact remainder and one correction (P. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
 // 34, 1990, theorem 2), where nothing over- or underflows; b a positive float's
-// value.  3 FP64 operations for the dozen of a division.
+// value.  An infinite b (r = 0) and an a near either end of the range take the
+// division.  3 FP64 operations for the dozen of a division.
 __device__ __forceinline__ double div_by(double a, double b, double r) {
-    if (!(fabs(a) > 1e-200 && fabs(a) < 1e200)) return a / b;
+    if (!(fabs(a) > 1e-200 && fabs(a) < 1e200) || __double2hiint(r) == 0) return a / b;
     const double q = a * r;
     return __fma_rn(__fma_rn(-q, b, a), r, q);
 }
