@@ -100,7 +100,9 @@ __device__ __forceinline__ WarpSlots warp_slots(const StepWarps& W, uint32_t w) 
 // Draws for a warp whose lanes repeat its `per` spins (a power of two; lane l
 // holds spin l mod per): every 32 / per steps all lanes draw at once, lane l for
 // its spin's step number l / per of the coming ones, and a step takes its draw
-// by shuffles.  live: the lanes with a spin.
+// by shuffles.  live: the lanes with a spin, by a ballot of the whole warp (inside
+// the branch of those lanes nothing makes them run together, and __activemask
+// would name whichever did).
 struct ThinDraws {
     Draw drawn;
     __device__ __forceinline__ Draw step(uint32_t it, uint32_t per, uint32_t lane, uint32_t live, uint32_t id,
@@ -184,6 +186,7 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
     uint32_t comp = meta & 0xFFu, fiber = meta >> 8;
     uint32_t nrefl = 0, nperm = 0, st = 0;
     const SubDev& sub = subS[wi];
+    const uint32_t live = LAYOUT == 3 ? __ballot_sync(FULL, valid) : 0u;  // ThinDraws
     if (LAYOUT != 3) {
         const MeshDev& g = sub.g;
         const AccelDev& acc = sub.acc;
@@ -247,7 +250,6 @@ k_batch_step(const SubDev* __restrict__ subs, const JobDev* __restrict__ jobs, B
         x = ox; y = oy; z = oz;
         mag = cmag; comp = ccomp; fiber = cfiber; nrefl = crefl; nperm = cperm; st = status;
     } else if (valid) {
-        const uint32_t live = __activemask();  // converged: the lanes with a spin
         ThinDraws draws;
         const uint32_t k0 = J.key0, k1 = J.key1;
         const float* __restrict__ wave = J.wave;
@@ -1121,9 +1123,9 @@ k_batch_step_cyl64(const SubDev* __restrict__ subs, const JobDev* __restrict__ j
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
     const bool valid = id != 0xFFFFFFFFu && at < mine.n;
+    const uint32_t live = __ballot_sync(FULL, valid);  // ThinDraws
     uint32_t nrefl = 0, nperm = 0, st = 0;
     if (valid) {
-        const uint32_t live = __activemask();  // converged: the lanes with a spin
         ThinDraws draws;
         const CylDev g = sub.c;
         double x = S.d[D_X][i], y = S.d[D_Y][i], z = S.d[D_Z][i], mag = S.d[D_MAG][i];
@@ -1218,10 +1220,10 @@ k_batch_step_cyl_local(const SubDev* __restrict__ subs, const JobDev* __restrict
     const uint32_t nsteps = min(chunk, steps - ls0);
     const uint32_t id = S.u[U_ID][i];
     const bool valid = id != 0xFFFFFFFFu && at < mine.n;
+    const uint32_t live = __ballot_sync(FULL, valid);  // ThinDraws
     uint32_t nrefl = 0, nperm = 0, st = 0;
     CylLocal form = {__ldg(&J.inR), {0.0f, 0.0f, 0.0f}, 0u, 0u};
     if (valid) {
-        const uint32_t live = __activemask();  // converged: the lanes with a spin
         ThinDraws draws;
         const CylDev g = sub.c;
         const double X = S.d[D_X][i], Y = S.d[D_Y][i], Z = S.d[D_Z][i];
