@@ -720,6 +720,7 @@ static int ensure_sort_buffers(dsim_spins* s, uint32_t nb) {
     if (s->sortNb != nb) {
         cudaFree(s->hist); cudaFree(s->hstart); cudaFree(s->hscratch);
         s->hist = s->hstart = s->hscratch = nullptr;
+        s->sortNb = 0;
         uint32_t nkeys = accel_keys(nb);
         if ((rc = dev_alloc(&s->hist, nkeys, &s->bytes)) || (rc = dev_alloc(&s->hstart, (size_t)nkeys + 1, &s->bytes)) ||
             (rc = dev_alloc(&s->hscratch, scan_scratch_words(nkeys), &s->bytes)))

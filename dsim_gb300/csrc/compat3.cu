@@ -91,7 +91,7 @@ struct State {
     uint32_t* wu[4] = {nullptr};    // meta, id (two sets)
     uint32_t* keys = nullptr;
     uint32_t *hist = nullptr, *hstart = nullptr, *hscratch = nullptr;
-    uint32_t histNf = 0;
+    uint32_t histKeys = 0;  // sort keys they hold (they grow to the largest call's, at most the fine grid's)
     uint32_t sortEvery = 1000;  // reorder by fine cell once per call of up to 1000 steps
     void release() {
         cudaFree(plane); cudaFree(bary); cudaFree(cell_start); cudaFree(cell_tri); cudaFree(tri_cells);
@@ -219,15 +219,15 @@ int ensure_work(State& s, uint32_t N) {
         DSIM_CUDA_TRY(cudaMalloc(&s.keys, (size_t)N * 4));
         s.cap = N;
     }
-    const uint32_t nb = sort_grid(N, s.nf);
-    if (s.histNf != nb) {
+    const uint32_t nkeys = accel_keys(sort_grid(N, s.nf));
+    if (s.histKeys < nkeys) {
         cudaFree(s.hist); cudaFree(s.hstart); cudaFree(s.hscratch);
         s.hist = s.hstart = s.hscratch = nullptr;
-        uint32_t nkeys = accel_keys(nb);
+        s.histKeys = 0;
         DSIM_CUDA_TRY(cudaMalloc(&s.hist, (size_t)nkeys * 4));
         DSIM_CUDA_TRY(cudaMalloc(&s.hstart, ((size_t)nkeys + 1) * 4));
         DSIM_CUDA_TRY(cudaMalloc(&s.hscratch, scan_scratch_words(nkeys) * 4));
-        s.histNf = nb;
+        s.histKeys = nkeys;
     }
     return kOk;
 }
@@ -380,7 +380,7 @@ void integrateSystem(float* pos, unsigned int* randSeed, dsim_spinData* spinInfo
     for (uint32_t done = 0; done < iterations; done += chunk) {
         uint32_t n = iterations - done < chunk ? iterations - done : chunk;
         if (s.sortEvery && mesh_spins_per_warp(N) > 1) {
-            rc = launch_sort_spins(s.set(cur, N), s.set(1 - cur, N), s.histNf, s.keys, s.hist, s.hstart,
+            rc = launch_sort_spins(s.set(cur, N), s.set(1 - cur, N), sort_grid(N, s.nf), s.keys, s.hist, s.hstart,
                                    s.hscratch, 0);
             if (rc) { fail(rc); return; }
             cur = 1 - cur;

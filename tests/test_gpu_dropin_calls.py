@@ -1,6 +1,7 @@
 """libdsim3 calls a host can make between two good ones: a grid whose counters or
 entries are out of range is refused before any kernel takes its words for
-triangles, and the next call on a good grid walks as the oracle does."""
+triangles, and the next call on a good grid walks as the oracle does; calls of
+different spin counts keep the plug-in's buffers at the largest one's."""
 import ctypes as C
 
 import numpy as np
@@ -61,10 +62,13 @@ class Host:
 
     def step(self, dev, N, d):
         """One call of integrateSystem replaying d [iterations][N][4]; the status it left."""
+        return self.call(dev, N, self.put(np.ascontiguousarray(d).reshape(-1)), len(d))
+
+    def call(self, dev, N, draws, iterations):
         c = self.case
-        self.L.dsim3_set_replay(self.put(np.ascontiguousarray(d).reshape(-1)), None)
+        self.L.dsim3_set_replay(draws, None)
         self.L.integrateSystem(*dev, float(c.dt), float(c.permeability), N, self.Float3(*[float(x) for x in c.g]),
-                               float(c.pc), len(d), self.dTic, self.dCc)
+                               float(c.pc), iterations, self.dTic, self.dCc)
         return self.L.dsim3_last_status()
 
     def read(self, dev, N):
@@ -132,3 +136,32 @@ def test_grid_out_of_range_is_refused(host, fault):
     host.write(host.dTic, host.tic)
     assert host.step(dev, N, d) == 0, host.L.dsim3_last_error()
     _equal(host.read(dev, N), host.oracle(N, d))
+
+
+def _free_bytes():
+    free, total = C.c_size_t(), C.c_size_t()
+    assert C.CDLL("libcuda.so.1").cuMemGetInfo_v2(C.byref(free), C.byref(total)) == 0
+    return free.value
+
+
+def test_calls_of_different_spin_counts(engine, tmp_path):
+    """Two systems in turn: after the larger one's first call no call changes the free memory, and each walks as alone."""
+    big, small, its = 720_000, 9000, 3
+    h = Host(MeshCase(tmp_path, membranes="AM", N=big))
+    try:
+        d = draws(its, big, seed=33)
+        dB, dS = h.put(d.reshape(-1)), h.put(np.ascontiguousarray(d[:, :small]).reshape(-1))
+        devs = [h.spins(n) for n in (big, small, big, small)]
+        assert h.call(devs[0], big, dB, its) == 0, h.L.dsim3_last_error()
+        h.L.threadSync()
+        free = [_free_bytes()]
+        for dev, n, dd in ((devs[1], small, dS), (devs[2], big, dB), (devs[3], small, dS)):
+            assert h.call(dev, n, dd, its) == 0, h.L.dsim3_last_error()
+            h.L.threadSync()
+            free.append(_free_bytes())
+        assert free == [free[0]] * 4
+        want = h.oracle(small, np.ascontiguousarray(d[:, :small]))
+        for dev in devs:
+            _equal(h.read(dev, small), want)
+    finally:
+        h.close()
