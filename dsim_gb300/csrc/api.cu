@@ -799,11 +799,15 @@ int dsim_spins_set(dsim_spins* s, const float* pos3, const float* mag, const flo
 int dsim_spins_get(dsim_spins* s, float* pos3, float* mag, float* phase, uint8_t* comp,
                    uint16_t* fiber) {
     if (!s) return kErrInvalid;
+    // the slots go back to spin order, so that a signal read after this adds in
+    // that order and not in the last sort's, which its atomics decide
+    int rc = spins_unpermute(s);
+    if (rc) return rc;
     StageArrays A = {};
     HostSection sec[] = {{pos3, 12, (void**)&A.pos}, {mag, 4, (void**)&A.mag}, {phase, 4, (void**)&A.phase},
                          {fiber, 2, (void**)&A.fiber16}, {comp, 1, (void**)&A.comp}};
     const size_t total = stage_layout(s, sec, 5);
-    int rc = launch_stage_store(s->sorted(), A, s->st);
+    rc = launch_stage_store(s->sorted(), A, s->st);
     return rc ? rc : stage_out(s, sec, 5, total);
 }
 
