@@ -255,11 +255,13 @@ __device__ __forceinline__ float slab_margin(const TriBary& B, float vv) {
 // by kRegularEps) that does not list them, that lie in more than four cells,
 // or whose float test may report a point farther off (slab_margin).  Any other
 // triangle is listed by the cell of a hit point that keeps 2 kRegularEps from
-// the cell's faces (flat_only_hit).  The reference's overlap test is decided by
+// the cell's faces (flat_only_hit).  walkAll: every one (a plug-in host whose cell
+// edge is not 2 / n: the walk then visits other cells than those that hold a
+// point).  The reference's overlap test is decided by
 // rounding where a triangle ends on a face, as the rings of a tessellated tube
 // often do, so touching a face alone says nothing.  The sign of uu tells a test
 // to look vv up: it is flagged, or not v . v to the last bit (tri_vv).
-__global__ void k_tri_regular(uint32_t nT, uint32_t n, const uint4* __restrict__ cells,
+__global__ void k_tri_regular(uint32_t nT, uint32_t n, bool walkAll, const uint4* __restrict__ cells,
                               TriBary* bary, TriPlane* plane) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nT) return;
@@ -273,7 +275,7 @@ __global__ void k_tri_regular(uint32_t nT, uint32_t n, const uint4* __restrict__
     const float c2[3] = {P.p1x + B.ux, P.p1y + B.uy, P.p1z + B.uz};
     uint32_t lo[3], hi[3];
     float mn[3], mx[3];
-    bool regular = c.x != kCellMany && slab_margin(B, vv) <= eps;
+    bool regular = !walkAll && c.x != kCellMany && slab_margin(B, vv) <= eps;
     for (int k = 0; k < 3; k++) {
         mn[k] = fminf(c0[k], fminf(c1[k], c2[k]));
         mx[k] = fmaxf(c0[k], fmaxf(c1[k], c2[k]));
@@ -308,10 +310,10 @@ __global__ void k_tri_regular(uint32_t nT, uint32_t n, const uint4* __restrict__
     if (!regular || vv != B.vx * B.vx + B.vy * B.vy + B.vz * B.vz) bary[t].uu = -fabsf(B.uu);
 }
 
-int launch_tri_regular(uint32_t nT, uint32_t n, const uint4* cells, TriBary* bary, TriPlane* plane,
+int launch_tri_regular(uint32_t nT, uint32_t n, bool walkAll, const uint4* cells, TriBary* bary, TriPlane* plane,
                        cudaStream_t st) {
     if (nT == 0) return kOk;
-    k_tri_regular<<<(nT + 127) / 128, 128, 0, st>>>(nT, n, cells, bary, plane);
+    k_tri_regular<<<(nT + 127) / 128, 128, 0, st>>>(nT, n, walkAll, cells, bary, plane);
     DSIM_CUDA_TRY(cudaGetLastError());
     return kOk;
 }

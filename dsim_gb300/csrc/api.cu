@@ -352,7 +352,7 @@ static int mesh_build(dsim_mesh* m, const std::vector<float>& Vn, const std::vec
         } else if ((rc = launch_tri_cell_lists(m->n, m->nT, m->cell_start, m->cell_tri, counter, m->tri_cells, st))) {
             break;
         }
-        if ((rc = launch_tri_regular(m->nT, m->n, m->tri_cells, m->bary, m->plane, st))) break;
+        if ((rc = launch_tri_regular(m->nT, m->n, false, m->tri_cells, m->bary, m->plane, st))) break;
         std::vector<uint32_t> cs(ncells + 1);
         if (cudaMemcpyAsync(cs.data(), m->cell_start, cs.size() * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) { rc = kErrCuda; break; }

@@ -11,6 +11,7 @@
 // compares a device-side content hash of vertices, helpers, triInfo and the
 // grid (one read of each, nothing copied back), so arrays rewritten in place
 // at the same addresses are noticed.
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -66,6 +67,7 @@ struct State {
         const void *V, *H, *TI, *tic, *cc;
         int nH, nTI;
         uint32_t n, maxTPC;
+        float L;
         bool operator==(const Key& o) const { return !memcmp(this, &o, sizeof(Key)); }
     } key;
     bool have = false;
@@ -122,7 +124,7 @@ int derive(State& s, const uint32_t* tic, const uint32_t* cc) {
     State::Key k;
     memset(&k, 0, sizeof(k));
     k.V = s.V; k.H = s.H; k.TI = s.triInfo; k.tic = tic; k.cc = cc; k.nH = s.nH; k.nTI = s.nTI;
-    k.n = s.numCubes; k.maxTPC = s.maxTPC;
+    k.n = s.numCubes; k.maxTPC = s.maxTPC; k.L = s.cubeLength;
     uint64_t h[5] = {0, 0, 0, 0, 0};
     if (s.V && s.H && s.triInfo && tic && cc && s.nV > 0 && s.nH > 0 && s.nTI > 0) {
         if (!s.hashDev) DSIM_CUDA_TRY(cudaMalloc(&s.hashDev, sizeof(unsigned long long) * 5));
@@ -172,7 +174,9 @@ int derive(State& s, const uint32_t* tic, const uint32_t* cc) {
                 cudaMalloc(&perTri, (size_t)nT * 4) != cudaSuccess))
         rc = kErrNoMem;
     if (!rc) rc = launch_tri_cell_lists(s.numCubes, nT, s.cell_start, s.cell_tri, perTri, s.tri_cells, 0);
-    if (!rc) rc = launch_tri_regular(nT, s.numCubes, s.tri_cells, s.bary, s.plane, 0);
+    // the host's cells are the box's, to rounding: only then does a list hold what is inside its cell
+    const bool boxCells = fabs(0.5 * (double)s.cubeLength * (double)s.numCubes - 1.0) <= 1e-6;
+    if (!rc) rc = launch_tri_regular(nT, s.numCubes, !boxCells, s.tri_cells, s.bary, s.plane, 0);
     cudaFree(scratch);
     cudaFree(perTri);
     if (rc) { set_last_error(rc, "integrateSystem: deriving cell lists failed"); return rc; }

@@ -194,8 +194,9 @@ int launch_tri64(uint32_t nT, const float* V, const uint32_t* trgls, Tri64* out,
 static constexpr uint32_t kCellNone = 0xFFFFFFFFu, kCellMany = 0xFFFFFFFEu;
 int launch_tri_cell_lists(uint32_t n, uint32_t nT, const uint32_t* cell_start, const uint32_t* cell_tri,
                           uint32_t* count, uint4* out, cudaStream_t st);
-// accel.cu: flags (sign of vv) the triangles whose hits need the walk over the reference cells
-int launch_tri_regular(uint32_t nT, uint32_t n, const uint4* cells, TriBary* bary, TriPlane* plane,
+// accel.cu: flags (sign of vv) the triangles whose hits need the walk over the
+// reference cells; all of them (walkAll) where the cells are not the box's n per axis
+int launch_tri_regular(uint32_t nT, uint32_t n, bool walkAll, const uint4* cells, TriBary* bary, TriPlane* plane,
                        cudaStream_t st);
 int launch_records_from_helpers(uint32_t nT, const float* V, const float* H,
                                 const uint32_t* triInfo, TriPlane* plane, TriBary* bary,

@@ -1,7 +1,8 @@
 """libdsim3 calls a host can make between two good ones: a grid whose counters or
 entries are out of range is refused before any kernel takes its words for
 triangles, and the next call on a good grid walks as the oracle does; calls of
-different spin counts keep the plug-in's buffers at the largest one's."""
+different spin counts keep the plug-in's buffers at the largest one's; a cell edge
+of the host's own is taken as it is."""
 import ctypes as C
 
 import numpy as np
@@ -36,11 +37,14 @@ class Host:
                               ("k_maxTrianglesPerCube", self.W, np.uint32), ("k_cubeLength", F(2.0) / F(CUBES), F),
                               ("k_reflectionType", 1, np.uint32), ("k_permeability", case.permeability, F),
                               ("k_deltaTime", case.dt, F)):
-            a = np.array([val], ty)
-            L.copyConstantToDevice(name.encode(), a.ctypes.data, 0, 4)
+            self.constant(name, val, ty)
         for name, tab in (("k_T2Values", case.T2), ("k_stdDevs", case.stdDevs)):
             a = np.ascontiguousarray(tab, F)
             L.copyConstantToDevice(name.encode(), a.ctypes.data, 0, 16)
+
+    def constant(self, name, val, ty):
+        a = np.array([val], ty)
+        self.L.copyConstantToDevice(name.encode(), a.ctypes.data, 0, 4)
 
     def put(self, arr):
         arr = np.ascontiguousarray(arr)
@@ -77,9 +81,10 @@ class Host:
         self.L.copyArrayFromDevice(s.ctypes.data, dev[2], 0, s.nbytes)
         return pos, s
 
-    def oracle(self, N, d):
+    def oracle(self, N, d, edge=F(2.0) / F(CUBES)):
         c, mo = self.case, self.mo
         p = O.params3(c.stdDevs, c.T2, c.permeability, c.dt, CUBES, self.W)
+        p.cubeLength = edge
         pos, mag, ph = c.pos[:3 * N].copy(), c.mag[:N].copy(), c.phase[:N].copy()
         comp, fib = c.comp[:N].copy(), c.fiber[:N].copy()
         capped, _ = O.integrate3(p, pos, np.zeros(2 * N, np.uint32), mag, ph, comp, fib, mo.vertices, mo.helpers,
@@ -165,3 +170,18 @@ def test_calls_of_different_spin_counts(engine, tmp_path):
             _equal(h.read(dev, small), want)
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("scale", [1.0 + 1e-7, 1.0 + 1e-5, 1.001, 0.99, 1.3])
+def test_cell_edge_of_the_hosts_own(host, scale):
+    """k_cubeLength other than the box's 2 / k_numCubes: the reference's walk then visits cells that need not list the
+    triangles inside them, and a hit of such a triangle does not count.  Between two calls with the box's own edge."""
+    N, own = host.case.N, F(2.0) / F(CUBES)
+    d = draws(40, N, seed=35)
+    want = {}
+    for edge in (own, F(float(own) * scale), own):
+        host.constant("k_cubeLength", edge, F)
+        dev = host.spins(N)
+        assert host.step(dev, N, d) == 0, host.L.dsim3_last_error()
+        want[edge] = want[edge] if edge in want else host.oracle(N, d, edge)
+        _equal(host.read(dev, N), want[edge])
