@@ -1095,8 +1095,8 @@ int dsim_mesh_compartments(dsim_mesh* m, dsim_spins* s, uint64_t seed, float sta
         return kErrInvalid;
     }
     DSIM_CUDA_TRY(cudaMemsetAsync(s->moved, 0, 4, s->st));
-    int rc = launch_compartments(m->dev(), m->acc(), s->sorted(), m->maxabs, startBoxSize, seed, 20, 8, s->status,
-                                 s->moved, s->st);
+    int rc = launch_compartments(m->dev(), m->acc(), m->accEntries, s->sorted(), m->maxabs, startBoxSize, seed, 20, 8,
+                                 s->status, s->moved, s->st);
     if (rc) return rc;
     uint32_t h = 0;
     DSIM_CUDA_TRY(cudaMemcpyAsync(&h, s->moved, 4, cudaMemcpyDeviceToHost, s->st));

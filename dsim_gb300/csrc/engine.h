@@ -217,9 +217,10 @@ int build_cyl_grid_gpu(const float4* fibers, uint32_t nF, uint32_t n, uint32_t m
                        uint32_t* counter, uint32_t* cubes, float4* cubeF, uint32_t* maxCount, cudaStream_t st);
 
 // ---- compartments.cu ------------------------------------------------------
-int launch_compartments(const MeshDev& g, const AccelDev& acc, const SpinsSorted& S, const float maxabs[3],
-                        float startBox, uint64_t seed, uint32_t maxTries, uint32_t maxMoves, uint32_t* status,
-                        uint32_t* moved, cudaStream_t st);
+// entries: of the fine grid's lists
+int launch_compartments(const MeshDev& g, const AccelDev& acc, uint64_t entries, const SpinsSorted& S,
+                        const float maxabs[3], float startBox, uint64_t seed, uint32_t maxTries, uint32_t maxMoves,
+                        uint32_t* status, uint32_t* moved, cudaStream_t st);
 
 // ---- scan.cu --------------------------------------------------------------
 // content hashes of n device arrays of 32-bit words (nwords[k] words at

@@ -2,7 +2,9 @@
 (numpy): lines along each axis, through grids of one to many cells, from spins in
 and outside the box, and lines that cross as many membranes as the search keeps,
 and one more (status bit 4).  Spins whose line comes within 1e-4 of an edge or of
-its own ends are left out: there the search may tilt the line at random."""
+its own ends are left out: there the search may tilt the line at random.  Many
+spins are searched a thread each, few a warp each: the same spins find the same
+either way, tilts included."""
 import numpy as np
 import pytest
 
@@ -116,3 +118,42 @@ def test_lines_across_as_many_membranes_as_are_kept(engine, count, nf):
     assert np.array_equal(comp[ok], want[few][ok]) and np.array_equal(fiber[ok], wfib[few][ok])
     if not few.all():
         assert _search(V, T, mem, fib, pos[~few], nf)[3] & 4
+
+
+def _all(V, T, mem, fib, pos, nf):
+    from dsim_gb300.engine import Mesh, Spins
+    m = Mesh.from_arrays(V, T, mem, fib, 1.0)
+    m.set_accel(nf)
+    s = Spins(len(pos))
+    s.set(pos.reshape(-1), None, None, np.full(len(pos), 9, np.uint8), np.full(len(pos), 9, np.uint16))
+    m.compartments(s, seed=4)
+    p, _, _, comp, fiber = s.get()
+    return p.reshape(-1, 3), comp, fiber, s.status()
+
+
+@pytest.mark.parametrize("membranes,nf,scale", [("AM", 112, 10.0), ("G", 20, 6.0), ("AM", 3, 12.0)])
+def test_many_spins_find_what_few_do(engine, tmp_path, membranes, nf, scale):
+    case = MeshCase(tmp_path, membranes=membranes, n_axons=4)
+    t = case.tube
+    V = (t["vertices"] / F(scale)).astype(F)
+    rng = np.random.default_rng(nf)
+    pos = rng.uniform(-1.2, 1.2, (300_000, 3)).astype(F)            # a thread each: 100,000 and a quarter of the entries
+    pos[:500, :2] = np.asarray(t["centres"])[rng.integers(0, 4, 500)] / scale     # on an axis: lines along edges
+    pos[:500, 2] = rng.integers(-8, 9, 500) / scale
+    few = 1500                                                      # a warp each, at 3 layers of cells too
+    many, some = _all(V, t["trgls"], t["membrane"], t["fiber"], pos, nf), _all(V, t["trgls"], t["membrane"], t["fiber"],
+                                                                               pos[:few], nf)
+    assert many[3] == some[3] == 0
+    for a, b in zip(many[:3], some[:3]):
+        assert np.array_equal(a[:few].view(np.uint8), b.view(np.uint8))
+    assert len(np.unique(some[1])) == (3 if membranes == "AM" else 2)
+
+
+@pytest.mark.parametrize("count", [32, 33])
+def test_many_spins_across_as_many_membranes_as_are_kept(engine, count):
+    V, T, mem, fib = _shells(count)
+    pos = np.full((150_000, 3), 0.01, F) * np.array([1, -2, 0.5], F)
+    comp, fiber, moved, status = _search(V, T, mem, fib, pos, 112)
+    assert moved == 0 and status == (4 if count > 32 else 0)
+    if count == 32:
+        assert np.all(comp == 3) and np.all(fiber == 0)
