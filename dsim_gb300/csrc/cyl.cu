@@ -352,8 +352,18 @@ int launch_cyl_step(const CylDev& g, const CylStepArgs& args, const CylSpinsDev&
     // 10,000 spins 3.7 / 3.1 / 2.7 / 2.3 / 2.3 / 2.5; 40,000 spins 3.9 / 3.4 /
     // 3.2 / 3.7; 80,000 spins 4.1 / 3.9 / 4.6; 120,000 spins 4.7 / 4.8
     a.perWarp = spins_per_warp(S.N, 33, true);
+    // Free walks (no membrane stops a spin) are draws and little else, which copies of
+    // a spin only repeat: thin warps only where each spin has its own.  us of runs of
+    // 128 steps thin / full: 3000 spins 62 / 79, 10,000 101 / 79, 60,000 139 / 120.
+    const bool walls = a.perm < 1.0f;
+    if (!walls && a.perWarp > 1) a.perWarp = 32;
+    // The order takes a launch, a clear and a gather of every spin's record: worth it
+    // from a dozen steps on (us of runs of 4 / 16 / 128 steps without and with, 64
+    // cylinders: 30,000 spins 42 and 49 / 82 and 80 / 405 and 373; 1M 151 and 161 / 469
+    // and 420 / 3312 and 3034), not for a spin alone in its warp (1000: 26 and 32 / 48
+    // and 53 / 198 and 200) and never without membranes.
     const uint32_t* order = nullptr;
-    if (scratch.order) {
+    if (scratch.order && walls && a.perWarp > 1 && a.iterations >= 12) {
         DSIM_CUDA_TRY(cudaMemsetAsync(scratch.count, 0, 8, st));
         k_cyl_order<<<(S.N + 255) / 256, 256, 0, st>>>(S.N, g.nF, reinterpret_cast<const uint4*>(S.seed4),
                                                        scratch.order, scratch.count);
