@@ -220,19 +220,15 @@ void cyl_hold(const dsim_cyl* c, int delta) {
 int mesh_rebuild_accel(dsim_mesh* m, uint32_t nf) { return accel_build(m, nf); }
 }  // namespace dsim
 
-// staging bytes per spin: position, magnitude, phase and two words (cylinders)
-static constexpr size_t kStageBytes = 28;
-
 struct dsim_spins {
     uint32_t N = 0;
     cudaStream_t st = nullptr;
-    float *x = nullptr, *y = nullptr, *z = nullptr, *mag = nullptr, *phase = nullptr;
-    uint32_t* meta = nullptr;
-    // reordering by cell (fast mesh path): stable ids, second buffer set
-    uint32_t* id = nullptr;
-    float *x2 = nullptr, *y2 = nullptr, *z2 = nullptr, *mag2 = nullptr, *phase2 = nullptr;
-    uint32_t *meta2 = nullptr, *id2 = nullptr, *keys = nullptr, *hist = nullptr, *hstart = nullptr,
-             *hscratch = nullptr;
+    // x, y, z, magnitude, phase, meta and stable id of every slot, `pitch` words each
+    uint32_t* block = nullptr;
+    // the same again (lazy): a reordering's target, and between calls the room where
+    // the host's arrays land on their way to and from the slots (28 bytes a spin at most)
+    uint32_t* block2 = nullptr;
+    uint32_t *keys = nullptr, *hist = nullptr, *hstart = nullptr, *hscratch = nullptr;
     uint32_t sortNb = 0;        // key grid of the allocated sort buffers
     uint32_t sortEvery = 1000;  // steps between reorderings (0 = never): once per call of up to 1000 steps
     uint64_t launches = 0;      // kernels launched by dsim_mesh_run / dsim_cyl_run on this object
@@ -248,34 +244,33 @@ struct dsim_spins {
     size_t drawsCap = 0;
     float4* grad = nullptr;     // per-step gradient table (lazy, grows)
     size_t gradCap = 0;
-    unsigned char* stage = nullptr;  // the host's arrays on the device (kStageBytes per spin)
     uint32_t* moved = nullptr;  // spins the compartment search moved
     double* partials = nullptr; // signal scratch
-    double* sig = nullptr;      // 15 doubles
+    double* sig = nullptr;      // 15 doubles, then the words of status and moved
     void* flush = nullptr;
     size_t flushCap = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     uint64_t bytes = 0;
+    size_t pitch() const { return ((size_t)N + 63) & ~(size_t)63; }
     SpinsDev dev() const {
+        const SpinsSorted t = sorted();
         SpinsDev S;
-        S.x = x; S.y = y; S.z = z; S.mag = mag; S.phase = phase; S.meta = meta; S.seed = nullptr;
+        S.x = t.x; S.y = t.y; S.z = t.z; S.mag = t.mag; S.phase = t.phase; S.meta = t.meta; S.seed = nullptr;
         S.N = N;
         return S;
     }
-    SpinsSorted sorted() const {
+    SpinsSorted slots(uint32_t* b) const {
+        const size_t p = pitch();
+        float* f = reinterpret_cast<float*>(b);
         SpinsSorted S;
-        S.x = x; S.y = y; S.z = z; S.mag = mag; S.phase = phase; S.meta = meta; S.id = id; S.N = N;
+        S.x = f; S.y = f + p; S.z = f + 2 * p; S.mag = f + 3 * p; S.phase = f + 4 * p;
+        S.meta = b + 5 * p; S.id = b + 6 * p; S.N = N;
         return S;
     }
-    SpinsSorted sorted2() const {
-        SpinsSorted S;
-        S.x = x2; S.y = y2; S.z = z2; S.mag = mag2; S.phase = phase2; S.meta = meta2; S.id = id2; S.N = N;
-        return S;
-    }
-    void swap_buffers() {
-        std::swap(x, x2); std::swap(y, y2); std::swap(z, z2); std::swap(mag, mag2);
-        std::swap(phase, phase2); std::swap(meta, meta2); std::swap(id, id2);
-    }
+    SpinsSorted sorted() const { return slots(block); }
+    SpinsSorted sorted2() const { return slots(block2); }
+    void swap_buffers() { std::swap(block, block2); }
+    unsigned char* stage() const { return reinterpret_cast<unsigned char*>(block2); }
 };
 
 // ---------------------------------------------------------------------------
@@ -652,13 +647,10 @@ void dsim_cyl_free(dsim_cyl* c) { cyl_release(c); }
 static void spins_release(dsim_spins* s) {
     if (!s) return;
     if (s->st) cudaStreamSynchronize(s->st);
-    cudaFree(s->x); cudaFree(s->y); cudaFree(s->z); cudaFree(s->mag); cudaFree(s->phase);
-    cudaFree(s->meta); cudaFree(s->cpos); cudaFree(s->cseed); cudaFree(s->corder); cudaFree(s->counts);
-    cudaFree(s->status); cudaFree(s->tested); cudaFree(s->draws); cudaFree(s->grad); cudaFree(s->partials);
-    cudaFree(s->sig); cudaFree(s->flush); cudaFree(s->stage); cudaFree(s->moved);
-    cudaFree(s->id); cudaFree(s->x2); cudaFree(s->y2); cudaFree(s->z2); cudaFree(s->mag2);
-    cudaFree(s->phase2); cudaFree(s->meta2); cudaFree(s->id2); cudaFree(s->keys); cudaFree(s->hist);
-    cudaFree(s->hstart); cudaFree(s->hscratch);
+    cudaFree(s->block); cudaFree(s->block2); cudaFree(s->cpos); cudaFree(s->cseed); cudaFree(s->corder);
+    cudaFree(s->counts); cudaFree(s->tested); cudaFree(s->draws); cudaFree(s->grad); cudaFree(s->partials);
+    cudaFree(s->sig); cudaFree(s->flush); cudaFree(s->keys); cudaFree(s->hist); cudaFree(s->hstart);
+    cudaFree(s->hscratch);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     if (s->st) cudaStreamDestroy(s->st);
@@ -674,15 +666,13 @@ int dsim_spins_create(uint32_t N, dsim_spins** out) {
     do {
         if (cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess) { rc = kErrCuda; break; }
         if (cudaEventCreate(&s->ev0) != cudaSuccess || cudaEventCreate(&s->ev1) != cudaSuccess) { rc = kErrCuda; break; }
-        if ((rc = dev_alloc(&s->x, N, &s->bytes)) || (rc = dev_alloc(&s->y, N, &s->bytes)) ||
-            (rc = dev_alloc(&s->z, N, &s->bytes)) || (rc = dev_alloc(&s->mag, N, &s->bytes)) ||
-            (rc = dev_alloc(&s->phase, N, &s->bytes)) || (rc = dev_alloc(&s->meta, N, &s->bytes)) ||
-            (rc = dev_alloc(&s->counts, (size_t)2 * N, &s->bytes)) || (rc = dev_alloc(&s->status, 1, &s->bytes)) ||
+        if ((rc = dev_alloc(&s->block, 7 * s->pitch(), &s->bytes)) ||
+            (rc = dev_alloc(&s->counts, (size_t)2 * N, &s->bytes)) ||
             (rc = dev_alloc(&s->partials, reduce_scratch_doubles(N), &s->bytes)) ||
-            (rc = dev_alloc(&s->sig, 15, &s->bytes)) || (rc = dev_alloc(&s->id, N, &s->bytes)) ||
-            (rc = dev_alloc(&s->moved, 1, &s->bytes)) ||
-            (rc = dev_alloc(&s->stage, (size_t)N * kStageBytes, &s->bytes)))
+            (rc = dev_alloc(&s->sig, 16, &s->bytes)))
             break;
+        s->status = reinterpret_cast<uint32_t*>(s->sig + 15);
+        s->moved = s->status + 1;
         if (cudaMemsetAsync(s->counts, 0, (size_t)8 * N, s->st) != cudaSuccess ||
             cudaMemsetAsync(s->status, 0, 4, s->st) != cudaSuccess) { rc = kErrCuda; break; }
         if ((rc = launch_stage_load(StageArrays(), s->sorted(), s->st))) break;  // ids 0, 1, ...
@@ -708,15 +698,14 @@ static int spins_unpermute(dsim_spins* s) {
     return kOk;
 }
 
+static int ensure_block2(dsim_spins* s) {
+    return s->block2 ? kOk : dev_alloc(&s->block2, 7 * s->pitch(), &s->bytes);
+}
+
 static int ensure_sort_buffers(dsim_spins* s, uint32_t nb) {
-    int rc;
-    if (!s->x2) {
-        if ((rc = dev_alloc(&s->x2, s->N, &s->bytes)) || (rc = dev_alloc(&s->y2, s->N, &s->bytes)) ||
-            (rc = dev_alloc(&s->z2, s->N, &s->bytes)) || (rc = dev_alloc(&s->mag2, s->N, &s->bytes)) ||
-            (rc = dev_alloc(&s->phase2, s->N, &s->bytes)) || (rc = dev_alloc(&s->meta2, s->N, &s->bytes)) ||
-            (rc = dev_alloc(&s->id2, s->N, &s->bytes)) || (rc = dev_alloc(&s->keys, s->N, &s->bytes)))
-            return rc;
-    }
+    int rc = ensure_block2(s);
+    if (rc) return rc;
+    if (!s->keys && (rc = dev_alloc(&s->keys, s->N, &s->bytes))) return rc;
     if (s->sortNb != nb) {
         cudaFree(s->hist); cudaFree(s->hstart); cudaFree(s->hscratch);
         s->hist = s->hstart = s->hscratch = nullptr;
@@ -731,33 +720,35 @@ static int ensure_sort_buffers(dsim_spins* s, uint32_t nb) {
 }
 
 // ---- the host's arrays --------------------------------------------------------
-// One host array and its section of the staging buffer.
+// One host array and its section of the room it passes through.
 struct HostSection {
     void* host;
     size_t elem;  // bytes per spin
     void** dev;
 };
-// Where all the given arrays together are at most this they travel as one copy
-// through a host buffer: a pageable copy takes about 12 us however short, a
-// host memcpy of this size as much.
+// Where several arrays together are at most this they travel as one copy through
+// a host buffer: a pageable copy takes about 12 us however short, a host memcpy of
+// this size as much.
 static constexpr size_t kOneCopyBytes = 256 << 10;
 
 static size_t stage_layout(dsim_spins* s, HostSection* sec, int n) {
     size_t at = 0;  // widest elements first: every section is aligned
     for (int k = 0; k < n; k++) {
-        *sec[k].dev = sec[k].host ? s->stage + at : nullptr;
+        *sec[k].dev = sec[k].host ? s->stage() + at : nullptr;
         if (sec[k].host) at += sec[k].elem * s->N;
     }
     return at;
 }
-static int stage_in(dsim_spins* s, HostSection* sec, int n) {
+// buf: the caller's, kept until it has waited for the stream
+static int stage_in(dsim_spins* s, HostSection* sec, int n, std::vector<unsigned char>& buf) {
     const size_t total = stage_layout(s, sec, n);
-    if (total <= kOneCopyBytes) {
-        std::vector<unsigned char> buf(total);
+    int given = 0;
+    for (int k = 0; k < n; k++) given += sec[k].host != nullptr;
+    if (given > 1 && total <= kOneCopyBytes) {
+        buf.resize(total);
         for (int k = 0; k < n; k++)
-            if (sec[k].host) memcpy(buf.data() + ((unsigned char*)*sec[k].dev - s->stage), sec[k].host, sec[k].elem * s->N);
-        if (total) DSIM_CUDA_TRY(cudaMemcpyAsync(s->stage, buf.data(), total, cudaMemcpyHostToDevice, s->st));
-        DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
+            if (sec[k].host) memcpy(buf.data() + ((unsigned char*)*sec[k].dev - s->stage()), sec[k].host, sec[k].elem * s->N);
+        if (total) DSIM_CUDA_TRY(cudaMemcpyAsync(s->stage(), buf.data(), total, cudaMemcpyHostToDevice, s->st));
         return kOk;
     }
     for (int k = 0; k < n; k++)
@@ -768,10 +759,10 @@ static int stage_in(dsim_spins* s, HostSection* sec, int n) {
 static int stage_out(dsim_spins* s, const HostSection* sec, int n, size_t total) {
     if (total <= kOneCopyBytes) {
         std::vector<unsigned char> buf(total);
-        if (total) DSIM_CUDA_TRY(cudaMemcpyAsync(buf.data(), s->stage, total, cudaMemcpyDeviceToHost, s->st));
+        if (total) DSIM_CUDA_TRY(cudaMemcpyAsync(buf.data(), s->stage(), total, cudaMemcpyDeviceToHost, s->st));
         DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
         for (int k = 0; k < n; k++)
-            if (sec[k].host) memcpy(sec[k].host, buf.data() + ((unsigned char*)*sec[k].dev - s->stage), sec[k].elem * s->N);
+            if (sec[k].host) memcpy(sec[k].host, buf.data() + ((unsigned char*)*sec[k].dev - s->stage()), sec[k].elem * s->N);
         return kOk;
     }
     for (int k = 0; k < n; k++)
@@ -785,15 +776,16 @@ int dsim_spins_set(dsim_spins* s, const float* pos3, const float* mag, const flo
                    const uint8_t* comp, const uint16_t* fiber) {
     if (!s) return kErrInvalid;
     int rc = spins_unpermute(s);  // what is not given stays with its spin
-    if (rc) return rc;
+    if (rc || (rc = ensure_block2(s))) return rc;
     StageArrays A = {};
     HostSection sec[] = {{const_cast<float*>(pos3), 12, (void**)&A.pos}, {const_cast<float*>(mag), 4, (void**)&A.mag},
                          {const_cast<float*>(phase), 4, (void**)&A.phase},
                          {const_cast<uint16_t*>(fiber), 2, (void**)&A.fiber16},
                          {const_cast<uint8_t*>(comp), 1, (void**)&A.comp}};
-    if ((rc = stage_in(s, sec, 5)) || (rc = launch_stage_load(A, s->sorted(), s->st))) return rc;
+    std::vector<unsigned char> buf;
+    if (!(rc = stage_in(s, sec, 5, buf))) rc = launch_stage_load(A, s->sorted(), s->st);
     DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
-    return kOk;
+    return rc;
 }
 
 int dsim_spins_get(dsim_spins* s, float* pos3, float* mag, float* phase, uint8_t* comp,
@@ -802,7 +794,7 @@ int dsim_spins_get(dsim_spins* s, float* pos3, float* mag, float* phase, uint8_t
     // the slots go back to spin order, so that a signal read after this adds in
     // that order and not in the last sort's, which its atomics decide
     int rc = spins_unpermute(s);
-    if (rc) return rc;
+    if (rc || (rc = ensure_block2(s))) return rc;
     StageArrays A = {};
     HostSection sec[] = {{pos3, 12, (void**)&A.pos}, {mag, 4, (void**)&A.mag}, {phase, 4, (void**)&A.phase},
                          {fiber, 2, (void**)&A.fiber16}, {comp, 1, (void**)&A.comp}};
@@ -823,27 +815,30 @@ int dsim_spins_set_cyl(dsim_spins* s, const float* pos3, const float* mag, const
                        const uint32_t* imo, const uint32_t* nearest) {
     if (!s || !pos3) return kErrInvalid;
     int rc = ensure_cyl(s);
-    if (rc) return rc;
+    if (rc || (rc = ensure_block2(s))) return rc;
     StageArrays A = {};
     HostSection sec[] = {{const_cast<float*>(pos3), 12, (void**)&A.pos}, {const_cast<float*>(mag), 4, (void**)&A.mag},
                          {const_cast<float*>(phase), 4, (void**)&A.phase},
                          {const_cast<uint32_t*>(imo), 4, (void**)&A.imo},
                          {const_cast<uint32_t*>(nearest), 4, (void**)&A.nearest}};
-    const CylSpinsDev D = {s->cpos, s->cseed, s->mag, s->N};
-    if ((rc = stage_in(s, sec, 5)) || (rc = launch_stage_load_cyl(A, D, s->st))) return rc;
+    const CylSpinsDev D = {s->cpos, s->cseed, s->sorted().mag, s->N};
+    std::vector<unsigned char> buf;
+    if (!(rc = stage_in(s, sec, 5, buf))) rc = launch_stage_load_cyl(A, D, s->st);
     DSIM_CUDA_TRY(cudaStreamSynchronize(s->st));
-    return kOk;
+    return rc;
 }
 
 int dsim_spins_get_cyl(dsim_spins* s, float* pos3, float* mag, float* phase, uint32_t* imo,
                        uint32_t* nearest) {
     if (!s || !s->cpos) return kErrInvalid;
+    int rc = ensure_block2(s);
+    if (rc) return rc;
     StageArrays A = {};
     HostSection sec[] = {{pos3, 12, (void**)&A.pos}, {mag, 4, (void**)&A.mag}, {phase, 4, (void**)&A.phase},
                          {imo, 4, (void**)&A.imo}, {nearest, 4, (void**)&A.nearest}};
     const size_t total = stage_layout(s, sec, 5);
-    const CylSpinsDev S = {s->cpos, s->cseed, s->mag, s->N};
-    int rc = launch_stage_store_cyl(S, A, s->st);
+    const CylSpinsDev S = {s->cpos, s->cseed, s->sorted().mag, s->N};
+    rc = launch_stage_store_cyl(S, A, s->st);
     return rc ? rc : stage_out(s, sec, 5, total);
 }
 
@@ -1041,7 +1036,7 @@ int dsim_cyl_run(dsim_cyl* c, dsim_spins* s, const dsim_cyl_params* p, const flo
     int rc = upload_grad_draws(s, gradPerStep, replayDraws, iterations, &a.grad, &a.draws);
     if (rc) return rc;
     CylSpinsDev S;
-    S.pos = s->cpos; S.seed4 = s->cseed; S.mag = s->mag; S.N = s->N;
+    S.pos = s->cpos; S.seed4 = s->cseed; S.mag = s->sorted().mag; S.N = s->N;
     uint32_t launches = 0;
     rc = launch_cyl_step(c->dev(), a, S, {s->corder, s->corder + s->N}, replayDraws ? kRngReplay : kRngPhilox, s->st,
                          &launches);
