@@ -12,6 +12,9 @@
 #include <unordered_map>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #pragma GCC visibility push(default)
 #include "../../include/dsim.h"
 #pragma GCC visibility pop
@@ -756,6 +759,16 @@ static int stage_in(dsim_spins* s, HostSection* sec, int n, std::vector<unsigned
             DSIM_CUDA_TRY(cudaMemcpyAsync(*sec[k].dev, sec[k].host, sec[k].elem * s->N, cudaMemcpyHostToDevice, s->st));
     return kOk;
 }
+// Makes the pages of a caller's array present, their contents as they are.  A
+// device copy into pages that were never written (a fresh calloc) lets the device
+// fault on each: 28 MB took 20.6 ms, and take 0.9 with the pages made here first.
+// (Reading and writing back a byte of each maps the zero page first: 9 ms.)
+static void make_pages(void* p, size_t bytes) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const size_t lo = (size_t)p & ~(page - 1), hi = ((size_t)p + bytes + page - 1) & ~(page - 1);
+    constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE, Linux 5.14; without it the copy does what it did
+    if (bytes) madvise(reinterpret_cast<void*>(lo), hi - lo, kPopulateWrite);
+}
 static int stage_out(dsim_spins* s, const HostSection* sec, int n, size_t total) {
     if (total <= kOneCopyBytes) {
         std::vector<unsigned char> buf(total);
@@ -765,6 +778,8 @@ static int stage_out(dsim_spins* s, const HostSection* sec, int n, size_t total)
             if (sec[k].host) memcpy(sec[k].host, buf.data() + ((unsigned char*)*sec[k].dev - s->stage()), sec[k].elem * s->N);
         return kOk;
     }
+    for (int k = 0; k < n; k++)
+        if (sec[k].host) make_pages(sec[k].host, sec[k].elem * s->N);
     for (int k = 0; k < n; k++)
         if (sec[k].host)
             DSIM_CUDA_TRY(cudaMemcpyAsync(sec[k].host, *sec[k].dev, sec[k].elem * s->N, cudaMemcpyDeviceToHost, s->st));
