@@ -1012,6 +1012,14 @@ bool job_finished(const dsim_batch* b, const BatchJob& j) {
     return b->stepNow >= j.d.start && b->stepNow - j.d.start >= j.d.steps;
 }
 
+// A launch of few steps, by a configured chunk: the warps' reading of their job and
+// substrate and their strided slots are then most of it, so they are fewer and (but
+// for FP64 steps) take neighbouring slots.  us of 48 steps of 300,000 mesh spins at
+// chunks of 1 / 2 / 4 / 8 as long launches and so: 5132 / 3686 / 2897 / 2292 and 4034 /
+// 3079 / 2561 / 2099; of 60 cell-local jobs of 400, mesh and cylinders: 3137 / 2046 /
+// 1558 / 1059 and 2372 / 1644 / 1333 / 937.
+bool short_launches(const dsim_batch* b) { return b->chunkSet && b->chunk <= 8; }
+
 // Warps per SM below which a kind's warps hold fewer than 32 spins.  FP32 mesh, ms
 // of runs at 12 / 16 / 20 / 24 (with as many cylinder spins beside them): six jobs
 // of 4957 to 35,814 spins 11.5 / 10.8 / 10.0 / 10.9; one mesh job of 8192 spins 1.54 /
@@ -1022,16 +1030,19 @@ bool job_finished(const dsim_batch* b, const BatchJob& j) {
 // 28.7 / 31.6; FP32 cylinders 16,384 6.3 / 5.7 / 4.0 / 3.4 / 3.9, 49,152 8.5 / 6.7 / 5.8 /
 // 6.3; cell-local cylinders 32,768 11.4 / 8.6 / 7.3 / 7.4; FP64 cylinders 4096 28.9 /
 // 20.2 / 17.9 / 16.2 / 20.6, 32,768 48.5 / 46.7 / 52.3.
-uint32_t warps_per_sm(StepKind k) {
+// No more than the configured blocks per SM hold at once: 60,000 FP32 mesh spins at 4
+// blocks, launches of 48 steps, 626 us at 20 warps and 469 at 16.
+uint32_t warps_per_sm(const dsim_batch* b, StepKind k) {
+    if (short_launches(b)) return 8;
     switch (k) {
         case kStepCyl: case kStepCylLocal: return 41;
         case kStepMesh64: case kStepCyl64: return 8;
-        case kStepMesh: case kStepMeshFull: return 20;
+        case kStepMesh: case kStepMeshFull: return std::min(20u, 4u * b->occupancy);
         default: return 16;
     }
 }
-uint32_t spins_per_warp_of(StepKind k, uint64_t spins) {
-    return spins_per_warp(spins, warps_per_sm(k), k == kStepCyl || k == kStepCylLocal || k == kStepCyl64);
+uint32_t spins_per_warp_of(const dsim_batch* b, StepKind k, uint64_t spins) {
+    return spins_per_warp(spins, warps_per_sm(b, k), k == kStepCyl || k == kStepCylLocal || k == kStepCyl64);
 }
 
 // lists the warps of the unfinished jobs by kind
@@ -1043,11 +1054,11 @@ int build_warps(dsim_batch* b) {
         if (!job_finished(b, j)) spins[kind_of(b, j)] += j.nSpins;
     for (int k = 0; k < kStepKinds; k++) {
         first[k] = list.size();
-        const uint32_t per = spins_per_warp_of((StepKind)k, spins[k]);
+        const uint32_t per = spins_per_warp_of(b, (StepKind)k, spins[k]);
         for (const auto& j : b->jobs) {
             if (job_finished(b, j) || kind_of(b, j) != (StepKind)k) continue;
             const uint32_t warps = (j.pad + per - 1) / per;
-            const bool deal = k != kStepCyl && k != kStepCyl64 && k != kStepCylLocal;
+            const bool deal = k == kStepMesh64 || (k != kStepCyl && k != kStepCyl64 && k != kStepCylLocal && !short_launches(b));
             for (uint32_t w = 0; w < warps; w++) {
                 // w0: the first of the warps that share slots, `dealt` of them, n slots in all
                 const uint32_t w0 = deal ? w / kDealWarps * kDealWarps : w, dealt = deal ? std::min(kDealWarps, warps - w0) : 1u;
@@ -1086,7 +1097,7 @@ int ensure_warps(dsim_batch* b) {
             if (!job_finished(b, j)) left[kind_of(b, j)] += j.nSpins;
         for (int k = 0; k < kStepKinds; k++)
             stale = stale || (b->kinds[k].count > 0 &&
-                              (left[k] == 0 || 4 * spins_per_warp_of((StepKind)k, left[k]) <= 3 * b->kinds[k].per));
+                              (left[k] == 0 || 4 * spins_per_warp_of(b, (StepKind)k, left[k]) <= 3 * b->kinds[k].per));
     }
     return stale ? build_warps(b) : kOk;
 }
@@ -1695,6 +1706,7 @@ int dsim_batch_configure(dsim_batch* b, uint32_t chunk, uint32_t occupancy, uint
     b->chunkSet = true;
     b->occupancy = occupancy;
     b->graphChunks = graphChunks;
+    b->warpsValid = false;  // the warps go by them
     invalidate_graph(b);
     return kOk;
 }
@@ -2063,6 +2075,7 @@ int dsim_batch_autotune(dsim_batch* b, uint32_t trialSteps, uint32_t best[3], fl
     float bestT = 3.4e38f;
     uint32_t bg = 0, bo = b->occupancy, bc = b->chunk;
     const uint32_t graph0 = b->graphChunks;
+    const bool set0 = b->chunkSet;
     b->chunkSet = true;  // the candidates' chunks, and then the best one
     cudaError_t e = save();
     auto set_grid = [&](uint32_t halves) -> int {
@@ -2123,7 +2136,9 @@ int dsim_batch_autotune(dsim_batch* b, uint32_t trialSteps, uint32_t best[3], fl
     cudaEventDestroy(e1);
     cudaFree(snap);
     b->occupancy = bo; b->chunk = bc; b->graphChunks = graph0;
+    b->warpsValid = false;
     invalidate_graph(b);
+    if (rc || e != cudaSuccess) b->chunkSet = set0;
     if (rc) return rc;
     if (e != cudaSuccess) { set_last_cuda_error(e, "dsim_batch_autotune", __FILE__, __LINE__); return kErrCuda; }
     best[0] = bo; best[1] = bc; best[2] = bg;
