@@ -214,11 +214,19 @@ __global__ void k_tri_cells(uint32_t nT, const float* __restrict__ V,
 
 // Ascending triangle order inside each cell (the reference's list order): one
 // warp per cell; an entry's place is the number of smaller entries (a triangle
-// is listed once per cell), counted from a copy in shared memory.  Cells of
-// more than kSortCell entries are insertion-sorted in place by one lane.  An
-// insertion sort per thread, whose every shift is a dependent global load and
-// store, took 0.55 ms for the 640,000-triangle mesh; this takes 0.03 ms.
+// is listed once per cell), counted from a copy in shared memory.  An insertion
+// sort per thread, whose every shift is a dependent global load and store, took
+// 0.55 ms for the 640,000-triangle mesh; this takes 0.03 ms.  Cells of more than
+// kSortCell entries are sorted in place by a bitonic network whose comparators all
+// ascend (each merge begins with the mirror image of its second half; K. E.
+// Batcher, "Sorting networks and their applications", AFIPS 32, 1968), so that
+// entries past the end, larger than all, never move and are left out.
 static constexpr uint32_t kSortCell = 512;
+__device__ __forceinline__ void sort_pair(uint32_t* v, uint32_t i, uint32_t j, uint32_t k) {
+    if (j >= k) return;
+    const uint32_t a = v[i], b = v[j];
+    if (a > b) { v[i] = b; v[j] = a; }
+}
 __global__ void __launch_bounds__(128) k_sort_cells(uint32_t ncells, const uint32_t* __restrict__ start,
                                                     uint32_t* cell_tri) {
     __shared__ uint32_t sh[4][kSortCell];
@@ -228,13 +236,22 @@ __global__ void __launch_bounds__(128) k_sort_cells(uint32_t ncells, const uint3
     const uint32_t b = start[c], k = start[c + 1] - b;
     if (k < 2) return;
     if (k > kSortCell) {
-        if (lane == 0)
-            for (uint32_t i = b + 1; i < b + k; i++) {
-                const uint32_t v = cell_tri[i];
-                uint32_t j = i;
-                while (j > b && cell_tri[j - 1] > v) { cell_tri[j] = cell_tri[j - 1]; j--; }
-                cell_tri[j] = v;
+        uint32_t* v = cell_tri + b;
+        for (uint32_t half = 1; half < k; half *= 2) {
+            const uint32_t pairs = (k + 2 * half - 1) / (2 * half) * half;
+            for (uint32_t p = lane; p < pairs; p += 32) {
+                const uint32_t from = p / half * 2 * half, at = p & (half - 1u);
+                sort_pair(v, from + at, from + 2 * half - 1u - at, k);
             }
+            __syncwarp();
+            for (uint32_t d = half / 2; d > 0; d /= 2) {
+                for (uint32_t p = lane; p < pairs; p += 32) {
+                    const uint32_t i = p / d * 2 * d + (p & (d - 1u));
+                    sort_pair(v, i, i + d, k);
+                }
+                __syncwarp();
+            }
+        }
         return;
     }
     for (uint32_t i = lane; i < k; i += 32) sh[w][i] = cell_tri[b + i];
