@@ -86,7 +86,9 @@ __device__ __forceinline__ int tri_box_overlap32(const float v[3][3], const floa
     for (int c = 0; c < 3; c++)
 #pragma unroll
         for (int k = 0; k < 3; k++) W = fmaxf(W, fabsf(v[c][k]));
-    if (!(W < 4.0f)) return 2;  // also a NaN, or the half-open outermost cells
+    // also infinite; a NaN is passed over by the maximum, and a triangle with one
+    // reports no hit (its normal has one), whatever cells list it
+    if (!(W < 4.0f)) return 2;
     const float err2 = 64.0f * 5.9604645e-08f * W * W, err3 = 512.0f * 5.9604645e-08f * W * W * W;
     bool sure = true;
 #pragma unroll

@@ -172,9 +172,10 @@ int launch_sort_spins(const SpinsSorted& S, const SpinsSorted& D, uint32_t nb, u
 // sort: 1000 spins 35 us)
 uint32_t sort_grid(uint32_t N, uint32_t nf);
 int launch_unpermute(const SpinsSorted& S, const SpinsSorted& D, cudaStream_t st);
-// flat.cu: the mesh step (warp-flattened candidate lists); occupancy 4, 6 or
-// 8 blocks per SM; queue: plane-test survivors finished 32 at a time; stage:
-// each cell's records staged in shared memory by bulk (TMA) copies
+// flat.cu: the mesh step (warp-flattened candidate lists); queue: plane-test
+// survivors finished 32 at a time, at 4 to 7 blocks per SM by the number of spins
+// (32-byte records); stage: each cell's records staged in shared memory by bulk
+// (TMA) copies; occupancy: 4, 6 or 8 blocks per SM of the other forms
 uint32_t mesh_spins_per_warp(uint32_t N);
 int launch_mesh_step_flat(const MeshDev& g, const AccelDev& acc, const MeshStepArgs& a,
                           const SpinsSorted& S, int rng, cudaStream_t st, int occupancy = 8,

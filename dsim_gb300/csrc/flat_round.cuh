@@ -24,7 +24,10 @@
 // windows, one copy of the exact test, no walk over cells for nine hits in ten):
 // 6.6e9 -> 9.1e9 spin-steps/s there, 6.8e9 -> 9.4e9 for 1M spins on 2.56M
 // triangles; then 11.1e9 and 10.8e9 with a lane's state in shared memory
-// (LaneState), 7 blocks per SM and the spins dealt out (kDealWarps).
+// (LaneState), 7 blocks per SM and the spins dealt out (kDealWarps).  All on tubes
+// that do not overlap.  Where they do, single spins caught between surfaces make
+// long chains of rounds that a launch waits for: the 10,000-step walk of 1M spins
+// on 2.56M triangles of overlapping tubes went 2.93e9 -> 3.56e9.
 #pragma once
 #include "common.cuh"
 #include "engine.h"

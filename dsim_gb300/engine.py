@@ -383,6 +383,8 @@ class Batch:
         return jid.value
 
     def configure(self, chunk=20, occupancy=4, graph_chunks=8, block=None):
+        """All of them at once: a batch that is not configured chooses launches of up to 1000 steps and 5 blocks per SM,
+        and there is no way back to that."""
         check(native().dsim_batch_configure(self.h, int(chunk), int(occupancy), int(graph_chunks)))
         if block is not None:
             check(native().dsim_batch_set_block(self.h, int(block)))

@@ -65,8 +65,10 @@ int dsim_mesh_info(const dsim_mesh* m, uint64_t info[8]);
 /* The step kernels find candidate triangles in a finer acceleration grid
  * (each triangle listed in every fine cell it touches) and
  * apply the reference grid's first-cell-with-hit rule only to the hits, which
- * gives the same results.  Built with 2.25 * numCubes cells per axis by default;
- * dsim_mesh_set_accel rebuilds it (0 = scan the reference grid directly).
+ * gives the same results.  Built with 2.25 * numCubes cells per axis by default,
+ * at most 1024; dsim_mesh_set_accel rebuilds it (1 to 1024; 0 is refused).  It
+ * holds 16 bytes a cell (17 GB at 1024 per axis), 4 bytes a Morton key (as many
+ * keys as cells, up to the next power of 8) and 16 to 64 bytes an entry.
  * info = {cells per axis, entries, device bytes}. */
 int dsim_mesh_set_accel(dsim_mesh* m, uint32_t cellsPerAxis);
 /* step kernel on the fine grid (all give the same results; default 8; other
@@ -131,6 +133,9 @@ int dsim_cyl_fine_lists(const float* fiberPos4, uint32_t nFibers, uint32_t numCu
 void dsim_cyl_free(dsim_cyl* c);
 
 /* ---- spin state (device resident, one CUDA stream per object) ---------- */
+/* 36 bytes of device memory a spin when made; 28 more from the first set, get or
+ * reordering on (a second set of slots, through which arrays come and go too), 4
+ * for a sort's keys, and for cylinder runs 36.  dsim_spins_bytes tells. */
 int dsim_spins_create(uint32_t N, dsim_spins** out);
 uint32_t dsim_spins_count(const dsim_spins* s);
 /* mesh state: pos3 (x,y,z per spin), mag, phase, compartment, fiber */

@@ -100,7 +100,9 @@ int dsim_batch_submit(dsim_batch* b, const dsim_job_desc* job, const float* pos3
                       const uint8_t* compartment, const uint32_t* fiber, uint32_t* jobId);
 /* chunk: steps between spin sorts and per launch.  Until it is configured (or
  * autotuned) dsim_batch_advance rounds to whole chunks of 20 steps and launches
- * up to 1000 at a time, to about the end of the next job; occupancy: 4, 5 (until then), 6 or 8
+ * up to 1000 at a time, to about the end of the next job; configuring anything
+ * here fixes the chunk for the batch's life.  Chunks of up to 8 steps list their
+ * warps for short launches.  occupancy: 4, 5 (until then), 6 or 8
  * resident blocks per SM for the step kernel; graphChunks: chunks captured in
  * one CUDA graph launch (0 = plain launches, default 8) */
 int dsim_batch_configure(dsim_batch* b, uint32_t chunk, uint32_t occupancy, uint32_t graphChunks);
@@ -132,8 +134,8 @@ int dsim_batch_get(dsim_batch* b, uint32_t jobId, float* pos3, float* mag, float
                    uint8_t* compartment, uint32_t* fiber);
 /* per-job {reflections or rejections, permeations} and status bits */
 int dsim_batch_counts(dsim_batch* b, uint32_t jobId, uint64_t counts[2]);
-/* precision and cell-local forms: {fine-grid records examined, FP64 triangle
- * tests}; cell-local cylinder jobs: {distance tests, FP64 decisions} */
+/* precision and cell-local forms: {fine-grid records examined (of cells that the
+ * sub-segment may meet), FP64 triangle tests}; cell-local cylinder jobs: {distance tests, FP64 decisions} */
 int dsim_batch_precision_counts(dsim_batch* b, uint32_t jobId, uint64_t out[2]);
 /* precision and cell-local forms: FP64 positions (3 per spin) and magnitudes
  * in spin order; DSIM_EINVAL for a plain job.  Synchronous. */
